@@ -248,7 +248,12 @@ __device__ __forceinline__ void round_bf16_pair(float& a, float& b) {
   b = bf16_hi(packed);
 }
 
-// Element traits so that one kernel body serves f32 and bf16 tensors.
+template <typename T>
+struct IsHalf { static constexpr bool value = false; };
+template <>
+struct IsHalf<__half> { static constexpr bool value = true; };
+
+// Element traits so that one kernel body serves f32, bf16 and fp16 tensors.
 template <typename T>
 struct Elem;
 template <>
@@ -266,9 +271,13 @@ struct Elem<__nv_bfloat16> {
   __device__ static void store(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
   __device__ static float round(float v) { return round_bf16(v); }
   __device__ static void round_pair(float& a, float& b) { round_bf16_pair(a, b); }  // one conversion
+  // two elements in a 32-bit word
+  __device__ static float lo(uint32_t pair) { return bf16_lo(pair); }
+  __device__ static float hi(uint32_t pair) { return bf16_hi(pair); }
+  __device__ static uint32_t pack(float a, float b) { return pack_bf16x2(a, b); }
 };
 template <>
-struct Elem<__half> {  // fp16 tensors run on the generic (non-tensor-core) kernels only
+struct Elem<__half> {
   static constexpr int kPerVec = 8;
   __device__ static float load(const __half* p) { return __half2float(*p); }
   __device__ static void store(__half* p, float v) { *p = __float2half_rn(v); }
@@ -277,6 +286,12 @@ struct Elem<__half> {  // fp16 tensors run on the generic (non-tensor-core) kern
     const float2 r = __half22float2(__floats2half2_rn(a, b));
     a = r.x;
     b = r.y;
+  }
+  __device__ static float lo(uint32_t pair) { return __low2float(*reinterpret_cast<const __half2*>(&pair)); }
+  __device__ static float hi(uint32_t pair) { return __high2float(*reinterpret_cast<const __half2*>(&pair)); }
+  __device__ static uint32_t pack(float a, float b) {
+    const __half2 pair = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&pair);
   }
 };
 
@@ -398,6 +413,20 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
       "{%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// The same with fp16 A and B.
+__device__ __forceinline__ void mma_f16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+      "{%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <typename T>
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (IsHalf<T>::value) mma_f16_16816(d, a, b0, b1);
+  else mma_bf16_16816(d, a, b0, b1);
 }
 
 // ---- TMA (tensor-map bulk copies) and mbarriers ----------------------------------

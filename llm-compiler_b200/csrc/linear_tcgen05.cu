@@ -1,7 +1,7 @@
 // serve.linear on the 5th-generation tensor cores: tcgen05.mma with the accumulator in tensor
 // memory (TMEM), operands staged in shared memory by TMA.
 //
-// y[M,N] = x[M,K] W[N,K]^T, both operands K-major bf16. One CTA computes a 128 x bn tile over
+// y[M,N] = x[M,K] W[N,K]^T, both operands K-major and both bf16 or both fp16. One CTA computes a 128 x bn tile over
 // one K slice (bn: a runtime multiple of 16 up to the template's BN accumulator columns of
 // TMEM, fp32). Roles inside the CTA of 4 warps:
 //   warp 0, one elected lane  TMA producer: per k-block one A_ROWS x 64 box of x and one bn x 64
@@ -46,10 +46,13 @@ constexpr int kEpiloguePartial = 100;  // internal: fp32 split-K partials, no ro
 // write r(r(x W^T) + residual) themselves: no partials in global memory, no reduce kernel
 constexpr int kEpilogueClusterResidual = 101;
 
-struct Tcgen05Params {
-  const __nv_bfloat16* bias;
-  const __nv_bfloat16* residual;
-  __nv_bfloat16* out;
+// T: the element type of x, W, bias, residual and y, __nv_bfloat16 or __half. (The decode chain's forms
+// exist for bf16 only; fp16 projections take the plain form and the persistent kernel.)
+template <typename T>
+struct Tcgen05ParamsOf {
+  const T* bias;
+  const T* residual;
+  T* out;
   float* partials;  // [splits, m, n] fp32 when epilogue == kEpiloguePartial
   int32_t* status;
   int m, k, n, epilogue, splits;
@@ -68,7 +71,7 @@ struct Tcgen05Params {
   // RMSNorm folded into the projection (norm_input != nullptr): the A operand is the
   // un-normalised x, the norm weight is already multiplied into W's columns, and the epilogue
   // scales row r of the accumulator by rsqrt(mean(x_r^2) + eps) before bias / SwiGLU.
-  const __nv_bfloat16* norm_input = nullptr;
+  const T* norm_input = nullptr;
   int64_t norm_row_stride = 0;
   float norm_eps = 0.0f;
   // Partial-sum producer only: the CTAs of the first N tile also leave sum(x_r^2) over their K
@@ -83,6 +86,7 @@ struct Tcgen05Params {
   const float* norm_squares = nullptr;
   int norm_slices = 0;
 };
+using Tcgen05Params = Tcgen05ParamsOf<__nv_bfloat16>;
 
 // silu for the fused SwiGLU epilogue: x / (1 + 2^(-x log2 e)) on the special-function unit
 // (ex2.approx, rcp.approx: a few ulp of fp32, far below the bf16 rounding that follows). An
@@ -93,47 +97,49 @@ __device__ __forceinline__ float silu_f32(float x) {
 }
 
 // Bias onto 32 accumulator columns (16-byte loads where all 32 columns exist and are aligned).
-__device__ __forceinline__ void add_bias(const Tcgen05Params& p, int col0, int n_end, float (&v)[32]) {
+template <typename T>
+__device__ __forceinline__ void add_bias(const Tcgen05ParamsOf<T>& p, int col0, int n_end, float (&v)[32]) {
   const bool whole = col0 + 32 <= n_end;
   if (p.bias != nullptr) {
     if (whole && (reinterpret_cast<uintptr_t>(p.bias + col0) & 15u) == 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const uint4 b = __ldg(reinterpret_cast<const uint4*>(p.bias + col0) + i);
-        v[8 * i] += bf16_lo(b.x); v[8 * i + 1] += bf16_hi(b.x);
-        v[8 * i + 2] += bf16_lo(b.y); v[8 * i + 3] += bf16_hi(b.y);
-        v[8 * i + 4] += bf16_lo(b.z); v[8 * i + 5] += bf16_hi(b.z);
-        v[8 * i + 6] += bf16_lo(b.w); v[8 * i + 7] += bf16_hi(b.w);
+        v[8 * i] += Elem<T>::lo(b.x); v[8 * i + 1] += Elem<T>::hi(b.x);
+        v[8 * i + 2] += Elem<T>::lo(b.y); v[8 * i + 3] += Elem<T>::hi(b.y);
+        v[8 * i + 4] += Elem<T>::lo(b.z); v[8 * i + 5] += Elem<T>::hi(b.z);
+        v[8 * i + 6] += Elem<T>::lo(b.w); v[8 * i + 7] += Elem<T>::hi(b.w);
       }
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (col0 + i < n_end) v[i] += __bfloat162float(p.bias[col0 + i]);
+        if (col0 + i < n_end) v[i] += Elem<T>::load(p.bias + col0 + i);
     }
   }
 }
 
 // r(r(x W^T + b) + residual) for 32 columns of one output row.
-__device__ __forceinline__ void add_residual(const Tcgen05Params& p, int epilogue, int row, int col0,
-                                             int n_end, float (&v)[32]) {
+template <typename T>
+__device__ __forceinline__ void add_residual(const Tcgen05ParamsOf<T>& p, int epilogue, int row, int col0, int n_end,
+                                             float (&v)[32]) {
   const bool whole = col0 + 32 <= n_end;
   const int64_t o = static_cast<int64_t>(row) * p.n + col0;
   if (epilogue == B200_EPILOGUE_RESIDUAL) {  // r(r(x W^T + b) + residual)
 #pragma unroll
-    for (int i = 0; i < 32; i += 2) round_bf16_pair(v[i], v[i + 1]);
+    for (int i = 0; i < 32; i += 2) Elem<T>::round_pair(v[i], v[i + 1]);
     if (whole && (reinterpret_cast<uintptr_t>(p.residual + o) & 15u) == 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const uint4 r = *(reinterpret_cast<const uint4*>(p.residual + o) + i);
-        v[8 * i] = __fadd_rn(v[8 * i], bf16_lo(r.x)); v[8 * i + 1] = __fadd_rn(v[8 * i + 1], bf16_hi(r.x));
-        v[8 * i + 2] = __fadd_rn(v[8 * i + 2], bf16_lo(r.y)); v[8 * i + 3] = __fadd_rn(v[8 * i + 3], bf16_hi(r.y));
-        v[8 * i + 4] = __fadd_rn(v[8 * i + 4], bf16_lo(r.z)); v[8 * i + 5] = __fadd_rn(v[8 * i + 5], bf16_hi(r.z));
-        v[8 * i + 6] = __fadd_rn(v[8 * i + 6], bf16_lo(r.w)); v[8 * i + 7] = __fadd_rn(v[8 * i + 7], bf16_hi(r.w));
+        v[8 * i] = __fadd_rn(v[8 * i], Elem<T>::lo(r.x)); v[8 * i + 1] = __fadd_rn(v[8 * i + 1], Elem<T>::hi(r.x));
+        v[8 * i + 2] = __fadd_rn(v[8 * i + 2], Elem<T>::lo(r.y)); v[8 * i + 3] = __fadd_rn(v[8 * i + 3], Elem<T>::hi(r.y));
+        v[8 * i + 4] = __fadd_rn(v[8 * i + 4], Elem<T>::lo(r.z)); v[8 * i + 5] = __fadd_rn(v[8 * i + 5], Elem<T>::hi(r.z));
+        v[8 * i + 6] = __fadd_rn(v[8 * i + 6], Elem<T>::lo(r.w)); v[8 * i + 7] = __fadd_rn(v[8 * i + 7], Elem<T>::hi(r.w));
       }
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (col0 + i < n_end) v[i] = __fadd_rn(v[i], __bfloat162float(p.residual[o + i]));
+        if (col0 + i < n_end) v[i] = __fadd_rn(v[i], Elem<T>::load(p.residual + o + i));
     }
   }  // (without a residual the store below is the one rounding)
 }
@@ -141,24 +147,25 @@ __device__ __forceinline__ void add_residual(const Tcgen05Params& p, int epilogu
 // y_j = r(silu(r(gate_j))) * r(up_j) for the 16 (gate, up) column pairs of a 32-column chunk;
 // the caller's store rounds the product. The roundings go through the conversion unit, which
 // the exponentials and reciprocals of silu also queue for, so they are taken in pairs.
+template <typename T>
 __device__ __forceinline__ void swiglu_of_chunk(float (&v)[32], float (&y)[16]) {
 #pragma unroll
   for (int j = 0; j < 16; j += 2) {
-    round_bf16_pair(v[2 * j], v[2 * j + 1]);
-    round_bf16_pair(v[2 * j + 2], v[2 * j + 3]);
+    Elem<T>::round_pair(v[2 * j], v[2 * j + 1]);
+    Elem<T>::round_pair(v[2 * j + 2], v[2 * j + 3]);
     float g0 = silu_f32(v[2 * j]), g1 = silu_f32(v[2 * j + 2]);
-    round_bf16_pair(g0, g1);
+    Elem<T>::round_pair(g0, g1);
     y[j] = g0 * v[2 * j + 1];
     y[j + 1] = g1 * v[2 * j + 3];
   }
 }
 
-// The bf16 epilogue of 32 accumulator columns of one output row: bias, then SwiGLU (columns
-// 2j / 2j+1 are gate_j / up_j) or the residual, with the reference's bf16 rounding points.
+// The epilogue of 32 accumulator columns of one output row: bias, then SwiGLU (columns
+// 2j / 2j+1 are gate_j / up_j) or the residual, with the reference's rounding points.
 // EPI >= 0: the epilogue is known at compile time (the decode chain's instantiations carry
 // only their own); -1: taken from the parameters.
-template <int EPI = -1>
-__device__ __forceinline__ void store_chunk(const Tcgen05Params& p, int row, int col0, int n_end,
+template <int EPI = -1, typename T>
+__device__ __forceinline__ void store_chunk(const Tcgen05ParamsOf<T>& p, int row, int col0, int n_end,
                                             float (&v)[32]) {
   const int epilogue = EPI >= 0 ? EPI : p.epilogue;
   const int out_cols = epilogue == B200_EPILOGUE_SWIGLU ? p.n / 2 : p.n;
@@ -166,35 +173,35 @@ __device__ __forceinline__ void store_chunk(const Tcgen05Params& p, int row, int
   add_bias(p, col0, n_end, v);
   if (epilogue == B200_EPILOGUE_SWIGLU) {
     // columns 2j / 2j+1 are gate_j / up_j
-    __nv_bfloat16* dst = p.out + static_cast<int64_t>(row) * out_cols + col0 / 2;
+    T* dst = p.out + static_cast<int64_t>(row) * out_cols + col0 / 2;
     float y[16];
-    swiglu_of_chunk(v, y);
+    swiglu_of_chunk<T>(v, y);
     if (col0 + 32 <= n_end && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
         reinterpret_cast<uint4*>(dst)[i] =
-            make_uint4(pack_bf16x2(y[8 * i], y[8 * i + 1]), pack_bf16x2(y[8 * i + 2], y[8 * i + 3]),
-                       pack_bf16x2(y[8 * i + 4], y[8 * i + 5]), pack_bf16x2(y[8 * i + 6], y[8 * i + 7]));
+            make_uint4(Elem<T>::pack(y[8 * i], y[8 * i + 1]), Elem<T>::pack(y[8 * i + 2], y[8 * i + 3]),
+                       Elem<T>::pack(y[8 * i + 4], y[8 * i + 5]), Elem<T>::pack(y[8 * i + 6], y[8 * i + 7]));
     } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j)
-        if (col0 + 2 * j + 1 < n_end) dst[j] = __float2bfloat16_rn(y[j]);
+        if (col0 + 2 * j + 1 < n_end) Elem<T>::store(dst + j, y[j]);
     }
     return;
   }
   const int64_t o = static_cast<int64_t>(row) * p.n + col0;
   add_residual(p, epilogue, row, col0, n_end, v);
-  __nv_bfloat16* dst = p.out + o;
+  T* dst = p.out + o;
   if (whole && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       reinterpret_cast<uint4*>(dst)[i] =
-          make_uint4(pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
-                     pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
+          make_uint4(Elem<T>::pack(v[8 * i], v[8 * i + 1]), Elem<T>::pack(v[8 * i + 2], v[8 * i + 3]),
+                     Elem<T>::pack(v[8 * i + 4], v[8 * i + 5]), Elem<T>::pack(v[8 * i + 6], v[8 * i + 7]));
   } else {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if (col0 + i < n_end) dst[i] = __float2bfloat16_rn(v[i]);
+      if (col0 + i < n_end) Elem<T>::store(dst + i, v[i]);
   }
 }
 
@@ -210,12 +217,13 @@ constexpr int kFormCluster = 2;  // split-K over a thread-block cluster, residua
 constexpr int kFormNorm = 3;     // folded RMSNorm, bias, no other epilogue (an LM head)
 constexpr int kFormNormSwiglu = 4;  // folded RMSNorm + SwiGLU (a gate|up projection)
 
-template <int BN, int STAGES, int A_ROWS, int FORM>
+template <int BN, int STAGES, int A_ROWS, int FORM, typename T = __nv_bfloat16>
 __global__ void __launch_bounds__(kThreads)
-linear_tcgen05_kernel(const Tcgen05Params p, const __grid_constant__ CUtensorMap a_map,
+linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtensorMap a_map,
                       const __grid_constant__ CUtensorMap b_map) {
   constexpr bool kCluster = FORM == kFormCluster, kPartial = FORM == kFormPartial;
   constexpr bool kNorm = FORM == kFormNorm || FORM == kFormNormSwiglu;
+  static_assert(FORM == kFormPlain || !IsHalf<T>::value, "the decode chain's forms are bf16");
   constexpr int kEpilogue = FORM == kFormNormSwiglu ? B200_EPILOGUE_SWIGLU : FORM == kFormNorm ? B200_EPILOGUE_NONE : -1;
   constexpr int kABytes = A_ROWS * 128;
   // TMEM is allocated in powers of two of at least 32 columns
@@ -223,7 +231,7 @@ linear_tcgen05_kernel(const Tcgen05Params p, const __grid_constant__ CUtensorMap
   constexpr int kBBytes = BN * 128;
   constexpr int kStageBytes = kABytes + kBBytes;
   const int bn = p.bn;
-  const uint32_t idesc = instruction_descriptor(kBM, bn);
+  const uint32_t idesc = instruction_descriptor(kBM, bn, false, false, IsHalf<T>::value);
   const uint32_t stage_tx_bytes = static_cast<uint32_t>(kABytes + bn * 128);
 
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -610,14 +618,15 @@ constexpr int kPersistentStages = 4;
 constexpr int kPersistentThreads = 192;
 constexpr int kPersistentBN = 256;
 
+template <typename T>
 __global__ void __launch_bounds__(kPersistentThreads, 1)
-linear_tcgen05_persistent_kernel(const Tcgen05Params p, const __grid_constant__ CUtensorMap a_map,
+linear_tcgen05_persistent_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtensorMap a_map,
                                  const __grid_constant__ CUtensorMap b_map) {
   constexpr int STAGES = kPersistentStages;
   constexpr int kABytes = kBM * 128;
   constexpr int kStageBytes = kABytes + kPersistentBN * 128;
   const int bn = p.bn;
-  const uint32_t idesc = instruction_descriptor(kBM, bn);
+  const uint32_t idesc = instruction_descriptor(kBM, bn, false, false, IsHalf<T>::value);
   const uint32_t stage_tx_bytes = static_cast<uint32_t>(kABytes + bn * 128);
 
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -747,12 +756,12 @@ linear_tcgen05_persistent_kernel(const Tcgen05Params p, const __grid_constant__ 
               float v[32], y[16];
               tmem_load_32x32(t_addr + c0 + quarter * 32, v);
               if (row < p.m) add_bias(p, col0 + quarter * 32, n_end, v);
-              swiglu_of_chunk(v, y);
+              swiglu_of_chunk<T>(v, y);
 #pragma unroll
               for (int i = 0; i < 2; ++i)
                 packed[quarter * 2 + i] =
-                    make_uint4(pack_bf16x2(y[8 * i], y[8 * i + 1]), pack_bf16x2(y[8 * i + 2], y[8 * i + 3]),
-                               pack_bf16x2(y[8 * i + 4], y[8 * i + 5]), pack_bf16x2(y[8 * i + 6], y[8 * i + 7]));
+                    make_uint4(Elem<T>::pack(y[8 * i], y[8 * i + 1]), Elem<T>::pack(y[8 * i + 2], y[8 * i + 3]),
+                               Elem<T>::pack(y[8 * i + 4], y[8 * i + 5]), Elem<T>::pack(y[8 * i + 6], y[8 * i + 7]));
             }
           } else {
 #pragma unroll
@@ -766,8 +775,8 @@ linear_tcgen05_persistent_kernel(const Tcgen05Params p, const __grid_constant__ 
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 packed[half * 4 + i] =
-                    make_uint4(pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
-                               pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
+                    make_uint4(Elem<T>::pack(v[8 * i], v[8 * i + 1]), Elem<T>::pack(v[8 * i + 2], v[8 * i + 3]),
+                               Elem<T>::pack(v[8 * i + 4], v[8 * i + 5]), Elem<T>::pack(v[8 * i + 6], v[8 * i + 7]));
             }
           }
           __syncwarp();  // the previous round's reads of the staging tile are done
@@ -814,12 +823,13 @@ linear_tcgen05_persistent_kernel(const Tcgen05Params p, const __grid_constant__ 
   trace.mark(1);
 }
 
-int launch_persistent(const Tcgen05Params& p, const CUtensorMap& a_map, const CUtensorMap& b_map,
+template <typename T>
+int launch_persistent(const Tcgen05ParamsOf<T>& p, const CUtensorMap& a_map, const CUtensorMap& b_map,
                       cudaStream_t stream) {
   // the stage ring, 4 KB of store staging per epilogue warp, alignment slack
   constexpr int smem = kPersistentStages * (kBM + kPersistentBN) * 128 + 4 * 4096 + 1024;
   static_assert(smem <= 227 * 1024, "stage ring exceeds shared memory");
-  auto kernel = linear_tcgen05_persistent_kernel;
+  auto kernel = linear_tcgen05_persistent_kernel<T>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return B200_ERR_LAUNCH;
   if (p.bn <= 0 || p.bn > kPersistentBN || p.bn % 16 != 0) return B200_ERR_BAD_ARGUMENT;
@@ -845,8 +855,8 @@ bool small_rings() {
   return value;
 }
 
-template <int BN, int STAGES, int A_ROWS, int FORM>
-int launch(const Tcgen05Params& p, const CUtensorMap& a_map, const CUtensorMap& b_map,
+template <int BN, int STAGES, int A_ROWS, int FORM, typename T>
+int launch(const Tcgen05ParamsOf<T>& p, const CUtensorMap& a_map, const CUtensorMap& b_map,
            cudaStream_t stream) {
   // the instantiation must be the one the parameters describe
   if ((FORM == kFormCluster) != (p.epilogue == kEpilogueClusterResidual) ||
@@ -867,11 +877,11 @@ int launch(const Tcgen05Params& p, const CUtensorMap& a_map, const CUtensorMap& 
     smem += 2 * p.splits * owned * 16;  // a send and a receive region
     if (smem > 227 * 1024) return B200_ERR_UNSUPPORTED;
   }
-  auto kernel = linear_tcgen05_kernel<BN, STAGES, A_ROWS, FORM>;
+  auto kernel = linear_tcgen05_kernel<BN, STAGES, A_ROWS, FORM, T>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return B200_ERR_LAUNCH;
   const int64_t tiles_n = ceil_div(p.n, p.bn), tiles_m = ceil_div(p.m, kBM);
-  Tcgen05Params q = p;
+  Tcgen05ParamsOf<T> q = p;
   static const bool n_fastest_always = [] {  // B200_TILE_ORDER=n: the comparison run
     const char* text = getenv("B200_TILE_ORDER");
     return text != nullptr && strcmp(text, "n") == 0;
@@ -896,11 +906,12 @@ int launch(const Tcgen05Params& p, const CUtensorMap& a_map, const CUtensorMap& 
 }
 
 // serve.linear proper: with or without the folded RMSNorm
-template <int BN, int STAGES, int A_ROWS>
-int launch_linear(const Tcgen05Params& p, const CUtensorMap& a_map, const CUtensorMap& b_map,
+template <int BN, int STAGES, int A_ROWS, typename T>
+int launch_linear(const Tcgen05ParamsOf<T>& p, const CUtensorMap& a_map, const CUtensorMap& b_map,
                   cudaStream_t stream) {
   if (p.norm_input == nullptr) return launch<BN, STAGES, A_ROWS, kFormPlain>(p, a_map, b_map, stream);
-  return p.epilogue == B200_EPILOGUE_SWIGLU ? launch<BN, STAGES, A_ROWS, kFormNormSwiglu>(p, a_map, b_map, stream)
+  if constexpr (IsHalf<T>::value) return B200_ERR_UNSUPPORTED;
+  else return p.epilogue == B200_EPILOGUE_SWIGLU ? launch<BN, STAGES, A_ROWS, kFormNormSwiglu>(p, a_map, b_map, stream)
                                             : launch<BN, STAGES, A_ROWS, kFormNorm>(p, a_map, b_map, stream);
 }
 
@@ -1051,10 +1062,11 @@ PartialPlan plan_partial(int64_t m, int64_t k, int64_t n) {
 // Called by b200_linear. Returns B200_ERR_UNSUPPORTED when this path does not apply (a
 // tensor map cannot describe the operands, or a decode-size M with too few N tiles to fill
 // the GPU without split-K), in which case the caller uses the warp-level kernel.
-int linear_tcgen05(const void* input, const void* weight, const void* bias, const void* residual,
-                   void* output, int64_t m, int64_t k, int64_t n, int64_t input_row_stride,
-                   int epilogue, int32_t* status, cudaStream_t stream, bool fold_norm,
-                   double norm_eps, const float* norm_squares, int norm_slices) {
+template <typename T>
+int linear_tcgen05_of(const void* input, const void* weight, const void* bias, const void* residual,
+                      void* output, int64_t m, int64_t k, int64_t n, int64_t input_row_stride,
+                      int epilogue, int32_t* status, cudaStream_t stream, bool fold_norm,
+                      double norm_eps, const float* norm_squares, int norm_slices) {
   if (ceil_div(m, kBM) > 65535) return B200_ERR_UNSUPPORTED;
   if (fold_norm && m > 128) return B200_ERR_UNSUPPORTED;  // the idle-warp scheme: one or two rows a thread
   int bn;
@@ -1138,10 +1150,10 @@ int linear_tcgen05(const void* input, const void* weight, const void* bias, cons
   if (!make_bf16_matrix_map(&a_map, input, m, k, input_row_stride, m <= 64 ? 64 : kBM) ||
       !make_bf16_matrix_map(&b_map, weight, n, k, k, bn))
     return B200_ERR_UNSUPPORTED;
-  Tcgen05Params p;
-  p.bias = static_cast<const __nv_bfloat16*>(bias);
-  p.residual = static_cast<const __nv_bfloat16*>(residual);
-  p.out = static_cast<__nv_bfloat16*>(output);
+  Tcgen05ParamsOf<T> p;
+  p.bias = static_cast<const T*>(bias);
+  p.residual = static_cast<const T*>(residual);
+  p.out = static_cast<T*>(output);
   p.partials = nullptr;
   p.status = status;
   p.m = static_cast<int>(m);
@@ -1154,7 +1166,7 @@ int linear_tcgen05(const void* input, const void* weight, const void* bias, cons
   p.wait_limit = wait_limit();
   p.drop_loads = drop_loads();
   if (fold_norm) {
-    p.norm_input = static_cast<const __nv_bfloat16*>(input);
+    p.norm_input = static_cast<const T*>(input);
     p.norm_row_stride = input_row_stride;
     p.norm_eps = static_cast<float>(norm_eps);
     p.norm_squares = norm_slices > 0 ? norm_squares : nullptr;
@@ -1176,6 +1188,15 @@ int linear_tcgen05(const void* input, const void* weight, const void* bias, cons
   if (bn == 256) return launch_linear<256, 4, 128>(p, a_map, b_map, stream);
   if (bn == 128) return launch_linear<128, 3, 128>(p, a_map, b_map, stream);
   return launch_linear<64, 4, 128>(p, a_map, b_map, stream);
+}
+
+int linear_tcgen05(const void* input, const void* weight, const void* bias, const void* residual,
+                   void* output, int64_t m, int64_t k, int64_t n, int64_t input_row_stride, int dtype,
+                   int epilogue, int32_t* status, cudaStream_t stream, bool fold_norm,
+                   double norm_eps, const float* norm_squares, int norm_slices) {
+  auto* run = dtype == B200_F16 ? linear_tcgen05_of<__half> : linear_tcgen05_of<__nv_bfloat16>;
+  return run(input, weight, bias, residual, output, m, k, n, input_row_stride, epilogue, status, stream,
+             fold_norm, norm_eps, norm_squares, norm_slices);
 }
 
 int linear_partial_splits(int64_t m, int64_t k, int64_t n) { return plan_partial(m, k, n).splits; }
@@ -1231,7 +1252,7 @@ int linear_splitk_residual_tcgen05(const void* input, const void* weight, const 
   const int a_rows = m <= 64 ? 64 : 128;
   // enough N x M tiles to fill the GPU without cutting K: the plain kernel with the residual epilogue
   if (plan.splits <= 1)
-    return linear_tcgen05(input, weight, nullptr, residual, output, m, k, n, input_row_stride,
+    return linear_tcgen05(input, weight, nullptr, residual, output, m, k, n, input_row_stride, B200_BF16,
                           B200_EPILOGUE_RESIDUAL, status, stream, false, 0.0, nullptr, 0);
   CUtensorMap a_map, b_map;
   if (!make_bf16_matrix_map(&a_map, input, m, k, input_row_stride, a_rows) ||
@@ -1311,7 +1332,7 @@ extern "C" int b200_linear_rms_input(const void* input, const void* folded_weigh
   if (m > 128) return B200_ERR_TOO_LARGE;
   if (k % 8 != 0 || input_row_stride % 8 != 0) return B200_ERR_UNSUPPORTED;
   if (!aligned16(input) || !aligned16(folded_weight)) return B200_ERR_ALIGNMENT;
-  return linear_tcgen05(input, folded_weight, bias, nullptr, output, m, k, n, input_row_stride,
+  return linear_tcgen05(input, folded_weight, bias, nullptr, output, m, k, n, input_row_stride, B200_BF16,
                         epilogue, status, static_cast<cudaStream_t>(stream), true, epsilon,
                         static_cast<const float*>(row_squares), static_cast<int>(row_square_slices));
 }

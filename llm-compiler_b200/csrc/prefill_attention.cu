@@ -2,12 +2,18 @@
 // B x 1 x T x T mask, or with proven causality (fully masked key tiles are skipped and
 // the mask is not read).
 //
-// bf16 kernel (warp-level tensor cores): a CTA of 4 warps owns 64 query rows of one
+// bf16 / fp16 kernel (warp-level tensor cores): a CTA of 4 warps owns 64 query rows of one
 // (sequence, q head); each warp keeps 16 rows of Q as A fragments and streams 64-key
 // K/V tiles through a cp.async ring of XOR-swizzled rows; S = Q K^T and O += P V are
 // m16n8k16 tiles with an fp32 online softmax in the log2 domain. The output is written
 // token-major (B x T x Hq x D) so that the transpose + reshape that follows in the
 // graph is a view.
+//
+// fp16 takes this kernel for every mask and mode. Its scores stay in the natural domain (an additive mask may hold
+// the type's lowest value, whose multiple by log2 e would overflow to -inf and turn a uniform row into NaN), and
+// its probabilities, which the CUDA-core kernel holds in fp32, enter P V as the sum of two fp16 numbers: high part
+// and remainder, 22 bits. 2 x 515 tokens, 14 heads of 64: 1851 us on the CUDA-core kernel (one CTA per query row,
+// keys and values re-read by every row) -> 26 us.
 //
 // fp32 kernel: CUDA cores with IEEE fp32 dots for small full-precision graphs.
 #include <math.h>
@@ -23,12 +29,13 @@ constexpr int kBM = 64;  // query rows per CTA
 constexpr int kBN = 64;  // keys per tile
 constexpr float kLog2e = 1.4426950408889634f;
 
+template <typename T>
 struct PrefillParams {
-  const __nv_bfloat16* q;
-  const __nv_bfloat16* k;
-  const __nv_bfloat16* v;
+  const T* q;
+  const T* k;
+  const T* v;
   const void* mask;
-  __nv_bfloat16* out;
+  T* out;
   int64_t qs[3], ks[3], vs[3];  // batch, head, token strides (elements)
   int64_t ms[4];                // mask strides: batch, head, query, key
   int batch, q_heads, kv_heads, groups, tokens;
@@ -53,8 +60,38 @@ __device__ __forceinline__ uint32_t tile_offset(int row, int chunk) {
   return static_cast<uint32_t>(row * (D * 2) + (((chunk & ~7) | ((chunk ^ row) & 7)) << 4));
 }
 
-template <int D, int STAGES>
-__global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const PrefillParams p) {
+// One output row by a whole warp, key by key, touching only the keys that the row sees: what an fp16 row is put right
+// with when its tile product met an infinite or NaN value row of a key that it does not see (0 * inf; fp16
+// activations do overflow). A row that is NaN by itself stays so.
+template <typename T, int D>
+__device__ __noinline__ void attend_row(const PrefillParams<T>& p, int b, int hq, int qrow) {
+  const int lane = threadIdx.x & 31, kvh = hq / p.groups;
+  const T* q = p.q + b * p.qs[0] + hq * p.qs[1] + static_cast<int64_t>(qrow) * p.qs[2];
+  float m = -INFINITY, l = 0.0f, acc[D / 32] = {};
+  const int key_end = p.causal ? qrow + 1 : p.tokens;
+  for (int key = 0; key < key_end; ++key) {
+    const T* k = p.k + b * p.ks[0] + kvh * p.ks[1] + static_cast<int64_t>(key) * p.ks[2];
+    const T* v = p.v + b * p.vs[0] + kvh * p.vs[1] + static_cast<int64_t>(key) * p.vs[2];
+    float s = 0.0f;
+    for (int d = lane; d < D; d += 32) s = fmaf(Elem<T>::load(q + d), Elem<T>::load(k + d), s);
+    s = warp_sum(s);
+    s = p.compat ? Elem<T>::round(Elem<T>::round(s) * p.scale) : s * p.scale;
+    if (p.mask != nullptr)
+      s += load_mask(p.mask, p.mask_dtype,
+                     b * p.ms[0] + static_cast<int64_t>(qrow) * p.ms[2] + static_cast<int64_t>(key) * p.ms[3]);
+    const float m_new = fmaxf(m, s), m_safe = m_new == -INFINITY ? 0.0f : m_new;
+    const float alpha = expf(m - m_safe), pr = expf(s - m_safe);
+    l = l * alpha + pr;
+    for (int i = 0; i < D / 32; ++i) acc[i] = acc[i] * alpha + pr * Elem<T>::load(v + lane + 32 * i);
+    m = m_new;
+  }
+  T* out = p.out + ((static_cast<int64_t>(b) * p.tokens + qrow) * p.q_heads + hq) * D;
+  for (int i = 0; i < D / 32; ++i) Elem<T>::store(out + lane + 32 * i, acc[i] / l);
+}
+
+template <typename T, int D, int STAGES>
+__global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const PrefillParams<T> p) {
+  constexpr bool kHalf = IsHalf<T>::value;
   constexpr int kChunksPerRow = D / 8;
   constexpr int kTileBytes = kBN * D * 2;
   constexpr int kQBytes = kBM * D * 2;
@@ -72,13 +109,13 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
   const int b = blockIdx.z;
   const int kvh = hq / p.groups;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int T = p.tokens;
+  const int tokens = p.tokens;
 
-  const __nv_bfloat16* qg = p.q + b * p.qs[0] + hq * p.qs[1];
-  const __nv_bfloat16* kg = p.k + b * p.ks[0] + kvh * p.ks[1];
-  const __nv_bfloat16* vg = p.v + b * p.vs[0] + kvh * p.vs[1];
+  const T* qg = p.q + b * p.qs[0] + hq * p.qs[1];
+  const T* kg = p.k + b * p.ks[0] + kvh * p.ks[1];
+  const T* vg = p.v + b * p.vs[0] + kvh * p.vs[1];
 
-  const int key_end = p.causal ? min(T, q0 + kBM) : T;
+  const int key_end = p.causal ? min(tokens, q0 + kBM) : tokens;
   const int n_tiles = (key_end + kBN - 1) / kBN;
 
   auto issue_kv = [&](int tile) {
@@ -90,7 +127,7 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
       const int id = i * kThreads + threadIdx.x;
       const int r = id / kChunksPerRow, c = id % kChunksPerRow;
       const int token = t0 + r;
-      const bool valid = token < T;
+      const bool valid = token < tokens;
       const uint32_t soff = tile_offset<D>(r, c);
       cp_async16_zfill(kdst + soff, valid ? kg + token * p.ks[2] + c * 8 : kg, valid ? 16 : 0);
       cp_async16_zfill(vdst + soff, valid ? vg + token * p.vs[2] + c * 8 : vg, valid ? 16 : 0);
@@ -103,7 +140,7 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
     const int id = i * kThreads + threadIdx.x;
     const int r = id / kChunksPerRow, c = id % kChunksPerRow;
     const int token = q0 + r;
-    const bool valid = token < T;
+    const bool valid = token < tokens;
     cp_async16_zfill(q_sm + tile_offset<D>(r, c), valid ? qg + token * p.qs[2] + c * 8 : qg,
                      valid ? 16 : 0);
   }
@@ -120,7 +157,10 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
 #pragma unroll
   for (int i = 0; i < kNTiles; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.0f;
 
-  const float scale_log2 = p.scale * kLog2e;
+  // scores in the log2 domain (bf16) or the natural one (fp16: see the top of this file)
+  constexpr float kUnit = kHalf ? 1.0f : kLog2e;
+  const float scale = p.scale * kUnit;
+  auto probability = [](float x) { return fast_exp2(kHalf ? x * kLog2e : x); };
   const int mat = lane >> 3;
   const int row_lo = q0 + warp * 16 + (lane >> 2);  // this thread's query rows: row_lo, row_lo + 8
 
@@ -155,8 +195,8 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
         uint32_t kb[4];
         const int r = np * 16 + ((mat >> 1) << 3) + (lane & 7);
         ldmatrix_x4(kb, ksm + tile_offset<D>(r, ks * 2 + (mat & 1)));
-        mma_bf16_16816(sacc[np * 2], qa[ks], kb[0], kb[1]);
-        mma_bf16_16816(sacc[np * 2 + 1], qa[ks], kb[2], kb[3]);
+        mma_16816<T>(sacc[np * 2], qa[ks], kb[0], kb[1]);
+        mma_16816<T>(sacc[np * 2 + 1], qa[ks], kb[2], kb[3]);
       }
     }
 
@@ -169,16 +209,16 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
         const int key = k0 + nt * 8 + (lane & 3) * 2 + (e & 1);
         float s;
         if (p.compat)
-          s = round_bf16(round_bf16(sacc[nt][e]) * p.scale) * kLog2e;
+          s = Elem<T>::round(Elem<T>::round(sacc[nt][e]) * p.scale) * kUnit;
         else
-          s = sacc[nt][e] * scale_log2;
-        const bool visible = key < T && qrow < T && (!p.causal || key <= qrow);
+          s = sacc[nt][e] * scale;
+        const bool visible = key < tokens && qrow < tokens && (!p.causal || key <= qrow);
         if (visible) {
           if (p.mask != nullptr)
             s += load_mask(p.mask, p.mask_dtype,
                            b * p.ms[0] + static_cast<int64_t>(qrow) * p.ms[2] +
                                static_cast<int64_t>(key) * p.ms[3]) *
-                 kLog2e;
+                 kUnit;
         } else {
           s = -INFINITY;
         }
@@ -194,7 +234,7 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
       const float m_new = fmaxf(m_run[r], mx);
       m_safe[r] = m_new == -INFINITY ? 0.0f : m_new;
-      alpha[r] = fast_exp2(m_run[r] - m_safe[r]);
+      alpha[r] = probability(m_run[r] - m_safe[r]);
       m_run[r] = m_new;
       l_run[r] *= alpha[r];
     }
@@ -207,26 +247,34 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
     }
 #pragma unroll
     for (int kk = 0; kk < kBN / 16; ++kk) {
-      uint32_t pa[4];
+      uint32_t pa[4], pa_low[kHalf ? 4 : 1];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int nt = kk * 2 + half;
-        const float p0 = fast_exp2(sacc[nt][0] - m_safe[0]);
-        const float p1 = fast_exp2(sacc[nt][1] - m_safe[0]);
-        const float p2 = fast_exp2(sacc[nt][2] - m_safe[1]);
-        const float p3 = fast_exp2(sacc[nt][3] - m_safe[1]);
+        const float p0 = probability(sacc[nt][0] - m_safe[0]);
+        const float p1 = probability(sacc[nt][1] - m_safe[0]);
+        const float p2 = probability(sacc[nt][2] - m_safe[1]);
+        const float p3 = probability(sacc[nt][3] - m_safe[1]);
         l_run[0] += p0 + p1;
         l_run[1] += p2 + p3;
-        pa[half * 2] = pack_bf16x2(p0, p1);
-        pa[half * 2 + 1] = pack_bf16x2(p2, p3);
+        pa[half * 2] = Elem<T>::pack(p0, p1);
+        pa[half * 2 + 1] = Elem<T>::pack(p2, p3);
+        if constexpr (kHalf) {
+          pa_low[half * 2] = Elem<T>::pack(p0 - Elem<T>::lo(pa[half * 2]), p1 - Elem<T>::hi(pa[half * 2]));
+          pa_low[half * 2 + 1] = Elem<T>::pack(p2 - Elem<T>::lo(pa[half * 2 + 1]), p3 - Elem<T>::hi(pa[half * 2 + 1]));
+        }
       }
 #pragma unroll
       for (int np = 0; np < kNTiles / 2; ++np) {
         uint32_t vb[4];
         const int r = kk * 16 + ((mat & 1) << 3) + (lane & 7);
         ldmatrix_x4_trans(vb, vsm + tile_offset<D>(r, np * 2 + (mat >> 1)));
-        mma_bf16_16816(oacc[np * 2], pa, vb[0], vb[1]);
-        mma_bf16_16816(oacc[np * 2 + 1], pa, vb[2], vb[3]);
+        mma_16816<T>(oacc[np * 2], pa, vb[0], vb[1]);
+        mma_16816<T>(oacc[np * 2 + 1], pa, vb[2], vb[3]);
+        if constexpr (kHalf) {
+          mma_16816<T>(oacc[np * 2], pa_low, vb[0], vb[1]);
+          mma_16816<T>(oacc[np * 2 + 1], pa_low, vb[2], vb[3]);
+        }
       }
     }
   }
@@ -237,22 +285,30 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
   }
+  bool nan_row[2] = {false, false};
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int qrow = row_lo + r * 8;
-    if (qrow >= T) continue;
+    if (qrow >= tokens) continue;
     const float inv = 1.0f / l_run[r];  // all-masked row: 0 * inf = NaN, as the oracle
-    __nv_bfloat16* orow = p.out + ((static_cast<int64_t>(b) * T + qrow) * p.q_heads + hq) * D;
+    T* orow = p.out + ((static_cast<int64_t>(b) * tokens + qrow) * p.q_heads + hq) * D;
 #pragma unroll
     for (int nt = 0; nt < kNTiles; ++nt) {
       const int col = nt * 8 + (lane & 3) * 2;
       *reinterpret_cast<uint32_t*>(orow + col) =
-          pack_bf16x2(oacc[nt][r * 2] * inv, oacc[nt][r * 2 + 1] * inv);
+          Elem<T>::pack(oacc[nt][r * 2] * inv, oacc[nt][r * 2 + 1] * inv);
+      nan_row[r] = nan_row[r] || isnan(oacc[nt][r * 2] * inv) || isnan(oacc[nt][r * 2 + 1] * inv);
     }
+  }
+  if constexpr (kHalf) {
+    __syncwarp();  // the rows stored above come before those that are stored again
+    for (int i = 0; i < 16; ++i)
+      if (__any_sync(0xffffffffu, (lane >> 2) == (i & 7) && nan_row[i >> 3]))
+        attend_row<T, D>(p, b, hq, q0 + warp * 16 + i);
   }
 }
 
-// ---- generic path (fp32, fp16, head sizes 16 / 32 / 256): one CTA per (query token, q head,
+// ---- generic path (fp32, head sizes 16 / 32 / 256, fp16 without 16-byte rows): one CTA per (query token, q head,
 // sequence), fp32 arithmetic on the CUDA cores, one rounding on the way out (and, in the
 // compatible mode of a 16-bit type, the reference's two roundings of the scores) ----------
 template <int D, typename T>
@@ -313,10 +369,10 @@ __global__ void prefill_attention_generic_kernel(const T* __restrict__ q, const 
   }
 }
 
-template <int D, int STAGES>
-int launch_bf16(const PrefillParams& p, cudaStream_t stream) {
+template <int D, int STAGES, typename T>
+int launch_warp_level(const PrefillParams<T>& p, cudaStream_t stream) {
   constexpr int smem = kBM * D * 2 + STAGES * 2 * kBN * D * 2;
-  auto kernel = prefill_attention_kernel<D, STAGES>;
+  auto kernel = prefill_attention_kernel<T, D, STAGES>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return B200_ERR_LAUNCH;
   dim3 grid((p.tokens + kBM - 1) / kBM, p.q_heads, p.batch);
@@ -372,7 +428,14 @@ extern "C" int b200_prefill_attention(const void* query, const void* key, const 
   const int64_t* ms = mask != nullptr ? mask_strides : zero4;
 
   if (!known_dtype(dtype)) return B200_ERR_UNSUPPORTED;
-  if (dtype != B200_BF16 || (head_dim != 64 && head_dim != 128)) {
+  // 16-byte loads of every row: what the tensor-core kernels need (bf16 is refused without them, fp16 keeps the
+  // CUDA-core kernel)
+  bool rows16 = aligned16(query) && aligned16(key) && aligned16(value) &&
+                (reinterpret_cast<uintptr_t>(output) & 3u) == 0;
+  for (int i = 0; i < 3; ++i)
+    rows16 = rows16 && query_strides[i] % 8 == 0 && key_strides[i] % 8 == 0 && value_strides[i] % 8 == 0;
+  const bool tensor_core = (head_dim == 64 || head_dim == 128) && (dtype == B200_BF16 || (dtype == B200_F16 && rows16));
+  if (!tensor_core) {
     if (head_dim != 16 && head_dim != 32 && head_dim != 64 && head_dim != 128 && head_dim != 256)
       return B200_ERR_UNSUPPORTED;
     if (tokens > 65535 * 64) return B200_ERR_TOO_LARGE;
@@ -398,15 +461,11 @@ extern "C" int b200_prefill_attention(const void* query, const void* key, const 
     });
     return launch_status();
   }
-  if (!aligned16(query) || !aligned16(key) || !aligned16(value) ||
-      (reinterpret_cast<uintptr_t>(output) & 3u) != 0)
-    return B200_ERR_ALIGNMENT;
-  for (int i = 0; i < 3; ++i)
-    if (query_strides[i] % 8 != 0 || key_strides[i] % 8 != 0 || value_strides[i] % 8 != 0)
-      return B200_ERR_ALIGNMENT;
+  if (!rows16) return B200_ERR_ALIGNMENT;
 
-  if (mode == B200_MODE_FAST && ((mask == nullptr && causal) ||
-                                 (mask != nullptr && !causal && mask_dtype == B200_F32 && workspace != nullptr))) {
+  if (dtype == B200_BF16 && mode == B200_MODE_FAST &&
+      ((mask == nullptr && causal) ||
+       (mask != nullptr && !causal && mask_dtype == B200_F32 && workspace != nullptr))) {
     // the tensor-core kernel: causal-proved, or the additive-mask contract with its tile pre-pass
     const int code = prefill_attention_tcgen05(query, key, value, output, batch, q_heads, kv_heads,
                                                tokens, head_dim, query_strides, key_strides,
@@ -415,26 +474,30 @@ extern "C" int b200_prefill_attention(const void* query, const void* key, const 
     if (code != B200_ERR_UNSUPPORTED) return code;
   }
 
-  PrefillParams p;
-  p.q = static_cast<const __nv_bfloat16*>(query);
-  p.k = static_cast<const __nv_bfloat16*>(key);
-  p.v = static_cast<const __nv_bfloat16*>(value);
-  p.mask = mask;
-  p.out = static_cast<__nv_bfloat16*>(output);
-  for (int i = 0; i < 3; ++i) {
-    p.qs[i] = query_strides[i];
-    p.ks[i] = key_strides[i];
-    p.vs[i] = value_strides[i];
-  }
-  for (int i = 0; i < 4; ++i) p.ms[i] = ms[i];
-  p.batch = static_cast<int>(batch);
-  p.q_heads = static_cast<int>(q_heads);
-  p.kv_heads = static_cast<int>(kv_heads);
-  p.groups = groups;
-  p.tokens = static_cast<int>(tokens);
-  p.mask_dtype = mask_dtype;
-  p.causal = causal ? 1 : 0;
-  p.compat = mode == B200_MODE_PYTORCH_COMPATIBLE ? 1 : 0;
-  p.scale = static_cast<float>(scale);
-  return head_dim == 64 ? launch_bf16<64, 3>(p, s) : launch_bf16<128, 2>(p, s);
+  auto warp_level = [&](auto tag) {
+    using T = typename decltype(tag)::type;
+    PrefillParams<T> p;
+    p.q = static_cast<const T*>(query);
+    p.k = static_cast<const T*>(key);
+    p.v = static_cast<const T*>(value);
+    p.mask = mask;
+    p.out = static_cast<T*>(output);
+    for (int i = 0; i < 3; ++i) {
+      p.qs[i] = query_strides[i];
+      p.ks[i] = key_strides[i];
+      p.vs[i] = value_strides[i];
+    }
+    for (int i = 0; i < 4; ++i) p.ms[i] = ms[i];
+    p.batch = static_cast<int>(batch);
+    p.q_heads = static_cast<int>(q_heads);
+    p.kv_heads = static_cast<int>(kv_heads);
+    p.groups = groups;
+    p.tokens = static_cast<int>(tokens);
+    p.mask_dtype = mask_dtype;
+    p.causal = causal ? 1 : 0;
+    p.compat = mode == B200_MODE_PYTORCH_COMPATIBLE ? 1 : 0;
+    p.scale = static_cast<float>(scale);
+    return head_dim == 64 ? launch_warp_level<64, 3>(p, s) : launch_warp_level<128, 2>(p, s);
+  };
+  return dtype == B200_F16 ? warp_level(TypeTag<__half>{}) : warp_level(TypeTag<__nv_bfloat16>{});
 }

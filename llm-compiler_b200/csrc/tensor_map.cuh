@@ -29,7 +29,7 @@ inline EncodeTiledFn tensor_map_encoder() {
   return encode;
 }
 
-// bf16 row-major matrix [rows, cols] with a row pitch of `row_stride` elements, tiled in boxes
+// 16-bit (bf16; fp16 alike, a copy only moves bits) row-major matrix [rows, cols] with a row pitch of `row_stride` elements, tiled in boxes
 // of box_rows x 64 columns (128-byte rows) with the 128B swizzle; out-of-range reads give zeros.
 inline bool make_bf16_matrix_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols,
                                  int64_t row_stride, int box_rows) {

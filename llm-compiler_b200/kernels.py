@@ -18,8 +18,8 @@ import torch
 
 from . import _lib
 
-# (fp16 runs on the generic CUDA-core kernels: the reference's kernels accept it,
-# backends/triton_linear.py:100-105, and no benchmark configuration uses it)
+# (fp16: projections and prompt attention on the tensor cores where rows allow 16-byte loads, the rest on generic
+# CUDA-core kernels; the reference's kernels accept it, backends/triton_linear.py:100-105)
 _DTYPE_CODES = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
 _MODES = {"fast": _lib.MODE_FAST, "pytorch_compatible": _lib.MODE_PYTORCH_COMPATIBLE}
 _EPILOGUES = {"none": _lib.EPILOGUE_NONE, "residual": _lib.EPILOGUE_RESIDUAL,

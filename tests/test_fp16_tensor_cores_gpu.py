@@ -1,0 +1,92 @@
+"""fp16 projections and prompt attention on the tensor cores, against the CUDA-core kernels that the same calls take
+when a base address is not a multiple of 16 bytes, and against the oracle.
+
+Tolerance: either kernel sums exact fp16 products in fp32 (order: K x 2^-24 of the summands, below a thousandth of what
+follows) and rounds a result to 11 bits; a SwiGLU rounds three factors, attention one quotient. 4 x 2^-11 of the
+largest result covers the worst of them."""
+
+import pytest
+import torch
+
+from oracle import serve_ops
+import llm_compiler_b200 as b200
+from llm_compiler_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+
+BOUND = 4 * 2.0 ** -11
+
+
+def unaligned(tensor):
+    """The same values one element behind a 16-byte boundary."""
+    storage = torch.empty(tensor.numel() + 8, dtype=tensor.dtype, device=tensor.device)
+    view = storage[1:1 + tensor.numel()].view(tensor.shape)
+    view.copy_(tensor)
+    assert view.data_ptr() % 16
+    return view
+
+
+def close(actual, expected):
+    actual, expected = actual.float().cpu(), expected.float().cpu()
+    assert torch.equal(torch.isnan(actual), torch.isnan(expected))
+    assert torch.equal(actual.isinf(), expected.isinf())
+    actual, expected = (t[expected.isfinite()] for t in (actual, expected))
+    if expected.numel():
+        assert (actual - expected).abs().max().item() <= BOUND * expected.abs().max().item()
+
+
+# around the row tiles (16 / 32 / 64 warp-level, 64, 128), the persistent kernel's first size, few and many columns,
+# remainders of the 64-wide K blocks
+@pytest.mark.parametrize("epilogue", ["none", "bias", "residual", "swiglu"])
+@pytest.mark.parametrize("m,k,n", [(1, 8, 16), (1, 896, 896), (16, 72, 130), (17, 896, 9728), (64, 136, 2400),
+                                   (65, 896, 1152), (128, 4864, 896), (129, 72, 264), (1023, 200, 896),
+                                   (1024, 896, 1152), (1100, 72, 904)])
+def test_linear(m, k, n, epilogue):
+    g = torch.Generator().manual_seed(m + k + n)
+    x, w = torch.randn(m, k, generator=g).half().cuda(), (0.1 * torch.randn(n, k, generator=g)).half().cuda()
+    bias = torch.randn(n, generator=g).half().cuda() if epilogue in ("bias", "swiglu") else None
+    residual = torch.randn(m, n, generator=g).half().cuda() if epilogue == "residual" else None
+    options = dict(residual=residual, epilogue="none" if epilogue == "bias" else epilogue)
+    close(b200.b200_linear(x, w, bias, **options), b200.b200_linear(unaligned(x), w, bias, **options))
+    kernels.runtime().check_status()
+
+
+def test_linear_overflow_stays_in_its_row_and_column():
+    x, w = torch.full((70, 64), 100.0).half().cuda(), torch.full((136, 64), 1.0).half().cuda()
+    x[3] = 60000.0  # the sum overflows fp16
+    x[5, 7] = float("inf")
+    w[9, 0] = float("nan")
+    close(b200.b200_linear(x, w), b200.b200_linear(unaligned(x), w))
+
+
+@pytest.mark.parametrize("mode", ["fast", "pytorch_compatible"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("t", [1, 15, 64, 65, 130])
+def test_prefill_attention(t, d, mode):
+    g = torch.Generator().manual_seed(t + d)
+    batch, heads, kv_heads = 2, 6, 2
+    q = torch.randn(batch, t, heads, d, generator=g).half().cuda().transpose(1, 2)
+    k, v = (torch.randn(batch, kv_heads, t, d, generator=g).half().cuda() for _ in range(2))
+    lowest = torch.zeros(batch, 1, t, t)
+    lowest[:, :, :, t // 2:] = torch.finfo(torch.float32).min  # soft mask of the lowest value: some rows see only it
+    lowest[1, :, t // 3] = torch.finfo(torch.float32).min
+    hidden = torch.zeros(1, 1, t, t).expand(batch, 1, t, t).clone()
+    hidden[:, :, t // 2] = -torch.inf  # a row that sees nothing is NaN
+    options = dict(scale=d ** -0.5, numerical_mode=mode)
+    for mask in (None, lowest.cuda(), hidden.cuda(), serve_ops.causal_mask(batch, t).half().cuda()):
+        kept = unaligned(q.transpose(1, 2)).transpose(1, 2)
+        close(b200.b200_prefill_attention(q, k, v, mask, causal=mask is None, **options),
+              b200.b200_prefill_attention(kept, k, v, mask, causal=mask is None, **options))
+    expected = serve_ops.prefill_attention(q.cpu(), k.cpu(), v.cpu(), serve_ops.causal_mask(batch, t),
+                                           groups=heads // kv_heads, scale=d ** -0.5)
+    close(b200.b200_prefill_attention(q, k, v, None, causal=True, **options), expected)
+
+
+def test_prefill_attention_does_not_read_values_that_a_row_does_not_see():
+    g = torch.Generator().manual_seed(4)
+    q, k, v = (torch.randn(1, 2, 100, 64, generator=g).half().cuda() for _ in range(3))
+    v[0, 1, 70] = float("inf")
+    k[0, 0, 90] = float("nan")
+    out = b200.b200_prefill_attention(q, k, v, None, scale=0.125, causal=True)
+    assert out[0, 1, :70].isfinite().all() and not out[0, 1, 70:].isfinite().any()
+    assert out[0, 0, :90].isfinite().all() and out[0, 0, 90:].isnan().all()
