@@ -133,6 +133,24 @@ inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 blo
   return launch_chained_cluster(kernel, grid, block, smem, stream, 1u, static_cast<Args&&>(args)...);
 }
 
+// Launches `kernel` in clusters of `splits` CTAs along grid z, stream-ordered behind everything before it.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_cluster_z(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream,
+                                    unsigned splits, Args&&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(threads);
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = 1;
+  attribute.val.clusterDim.y = 1;
+  attribute.val.clusterDim.z = splits;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 // ---- Timeline trace (only in builds with -DB200_TRACE) -----------------------------------
 // Thread 0 of every block of a traced kernel records {kernel id, block, SM, globaltimer and
 // SM clock at the top, after the dependency wait, at the end} into a caller-provided device

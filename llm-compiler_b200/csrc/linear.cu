@@ -207,10 +207,10 @@ __global__ void __launch_bounds__(WM* WN * 32) linear_warp_kernel(const LinearPa
   }
 }
 
-// ------------------------------------------------------- generic: fp32, fp16 ----
-// fp32 arithmetic on the CUDA cores for the element types the tensor-core kernels do not
-// take; a 16-bit type is rounded where the reference's kernels round theirs (the result,
-// the sum in front of a residual add, gate / up / silu(gate) of a SwiGLU).
+// ------------------------------------------------------- CUDA cores: fp32, fp16 ----
+// fp32 arithmetic for fp32 tensors and for the fp16 calls that the tensor-core kernels do not take; a 16-bit type is
+// rounded where the reference's kernels round theirs (the result, the sum in front of a residual add, gate / up /
+// silu(gate) of a SwiGLU). Two kernels: a few rows stream W (linear_rows_kernel), more rows are a tiled product.
 template <typename T>
 struct LinearParamsGeneric {
   const T* x;
@@ -222,68 +222,190 @@ struct LinearParamsGeneric {
   int m, k, n, epilogue;
 };
 
+// One output, or with SwiGLU the output of the column pair (n, n + 1): v0 is column n's sum, v1 column n + 1's.
 template <typename T>
-__global__ void __launch_bounds__(256) linear_generic_kernel(const LinearParamsGeneric<T> p) {
-  constexpr int BM = 64, BN = 64, BKF = 16;
-  __shared__ float As[BKF][BM + 1];
-  __shared__ float Bs[BKF][BN + 1];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int m_base = blockIdx.y * BM, n_base = blockIdx.x * BN;
-  float acc[4][4] = {};  // a sum of the blocks' sums: rounding errors grow with K / 16 + 16, not with K
-  for (int k0 = 0; k0 < p.k; k0 += BKF) {
-    for (int id = threadIdx.x; id < BM * BKF; id += 256) {
-      const int r = id / BKF, c = id % BKF;
-      const int m = m_base + r, kk = k0 + c;
-      As[c][r] = (m < p.m && kk < p.k) ? Elem<T>::load(p.x + static_cast<int64_t>(m) * p.x_row_stride + kk) : 0.0f;
-      const int n = n_base + r;
-      Bs[c][r] = (n < p.n && kk < p.k) ? Elem<T>::load(p.w + static_cast<int64_t>(n) * p.k + kk) : 0.0f;
+__device__ __forceinline__ void epilogue_generic(const LinearParamsGeneric<T>& p, int m, int n, float v0, float v1) {
+  if (m >= p.m || n >= p.n) return;
+  if (p.bias != nullptr) v0 += Elem<T>::load(p.bias + n);
+  if (p.epilogue == B200_EPILOGUE_SWIGLU) {
+    if (n & 1) return;
+    if (p.bias != nullptr) v1 += Elem<T>::load(p.bias + n + 1);
+    const float gate = Elem<T>::round(silu_f32(Elem<T>::round(v0)));
+    Elem<T>::store(p.out + static_cast<int64_t>(m) * (p.n / 2) + n / 2, gate * Elem<T>::round(v1));
+    return;
+  }
+  const int64_t o = static_cast<int64_t>(m) * p.n + n;
+  if (p.epilogue == B200_EPILOGUE_RESIDUAL) v0 = __fadd_rn(Elem<T>::round(v0), Elem<T>::load(p.residual + o));
+  Elem<T>::store(p.out + o, v0);
+}
+
+// fp32, up to 8 rows of x per CTA: bound by reading W once. A warp holds 4 rows of W against all rows of x, its lanes
+// side by side along K in 16-byte loads; KSPLIT warps of the CTA share the K range of the same 4 rows and add their
+// sums in warp order, so that a projection of few columns still puts enough loads in flight. x comes out of L1. The
+// sums are short chains joined by a tree (K / (32 KSPLIT) terms a lane), below the error of the tiled kernel's order.
+// Qwen2-0.5B decode step, 4 rows: 318 us a projection in 64 x 64 tiles (60 idle rows, one serial K loop per CTA)
+// -> 10.0 us on average.
+constexpr int kRowsThreads = 256, kRowsColumns = 4, kRowsOfX = 8;
+
+template <int KSPLIT>
+__global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearParamsGeneric<float> p) {
+  constexpr int kGroups = kRowsThreads / 32 / KSPLIT;  // groups of 4 columns in a CTA
+  __shared__ float sums[kRowsThreads / 32][kRowsOfX * kRowsColumns];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = (blockIdx.x * kGroups + warp / KSPLIT) * kRowsColumns, slice = warp % KSPLIT;
+  const int m0 = blockIdx.y * kRowsOfX, rows = min(kRowsOfX, p.m - m0);
+  float acc[kRowsOfX][kRowsColumns] = {};
+  const float* w[kRowsColumns];
+#pragma unroll
+  for (int j = 0; j < kRowsColumns; ++j) w[j] = p.w + static_cast<int64_t>(min(n0 + j, p.n - 1)) * p.k;
+  const float* x = p.x + m0 * p.x_row_stride;
+#pragma unroll 4
+  for (int k = (slice * 32 + lane) * 4; k < p.k; k += KSPLIT * 128) {
+    float4 wv[kRowsColumns];
+#pragma unroll
+    for (int j = 0; j < kRowsColumns; ++j) wv[j] = __ldg(reinterpret_cast<const float4*>(w[j] + k));
+#pragma unroll
+    for (int i = 0; i < kRowsOfX; ++i) {
+      if (i >= rows) break;
+      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + i * p.x_row_stride + k));
+#pragma unroll
+      for (int j = 0; j < kRowsColumns; ++j)
+        acc[i][j] = fmaf(xv.w, wv[j].w, fmaf(xv.z, wv[j].z, fmaf(xv.y, wv[j].y, fmaf(xv.x, wv[j].x, acc[i][j]))));
     }
-    __syncthreads();
-    float block[4][4] = {};
+  }
 #pragma unroll
-    for (int kk = 0; kk < BKF; ++kk) {
-      float a[4], b[4];
+  for (int i = 0; i < kRowsOfX; ++i) {
+    if (i >= rows) break;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+    for (int j = 0; j < kRowsColumns; ++j) {
+      const float sum = warp_sum(acc[i][j]);
+      if (lane == 0) sums[warp][i * kRowsColumns + j] = sum;
+    }
+  }
+  __syncthreads();
+  // one thread per output of the CTA's groups: 32 of them each, so at most all threads
+  const int group = threadIdx.x >> 5, item = threadIdx.x & 31, i = item / kRowsColumns, j = item % kRowsColumns;
+  if (group >= kGroups || i >= rows) return;
+  float v0 = 0.0f, v1 = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
+  for (int s = 0; s < KSPLIT; ++s) {
+    v0 += sums[group * KSPLIT + s][item];
+    v1 += sums[group * KSPLIT + s][item ^ 1];
+  }
+  epilogue_generic(p, m0 + i, (blockIdx.x * kGroups + group) * kRowsColumns + j, v0, v1);
+}
+
+// Tiled product: 64 x 64 outputs a CTA, 4 x 8 a thread, K in blocks of 16 whose sums are added to the accumulators
+// (rounding errors grow with K / 16 + 16, not with K). The next block travels in registers while this one is
+// multiplied. Where the tiles are fewer than the SMs, the K range is cut over the CTAs of a cluster (up to 8 along
+// grid z), which add their tiles in rank order through distributed shared memory: no workspace, one launch.
+// VEC: rows of x and W allow 16-byte loads. fp32, 9728 x 896 on 600 rows: 397 us (26 TFLOP/s); with the attention of
+// prefill_attention.cu, Qwen2-0.5B in fp32 on 2 x 300 tokens takes 20.9 ms (54.6 with 4 x 4 outputs a thread, unbuffered).
+constexpr int kTiledThreads = 128, kTile = 64, kTileK = 16;
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(kTiledThreads) linear_tiled_kernel(const LinearParamsGeneric<T> p) {
+  constexpr int kPitch = kTile + 4;
+  __shared__ __align__(16) float tiles[2][2][kTileK][kPitch];  // [buffer][x, W][k][row]: also the tile handed over
+  static_assert(sizeof(tiles) >= sizeof(float) * kTile * kTile, "the tile's sums must fit the operand buffers");
+  const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;  // 8 columns of 8, 16 rows of 4
+  const int m_base = blockIdx.y * kTile, n_base = blockIdx.x * kTile;
+  const int splits = gridDim.z, blocks = (p.k + kTileK - 1) / kTileK, per = (blocks + splits - 1) / splits;
+  const int first = blockIdx.z * per, last = min(first + per, blocks);
+
+  float staged[2][8];
+  auto fetch = [&](int block) {
+    if constexpr (VEC) {  // two 16-byte loads of 4 k each (fp32)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = threadIdx.x / 4 + 32 * h, k = block * kTileK + threadIdx.x % 4 * 4;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+        if (m_base + r < p.m && k < p.k)
+          a = __ldg(reinterpret_cast<const float4*>(p.x + (m_base + r) * p.x_row_stride + k));
+        if (n_base + r < p.n && k < p.k)
+          b = __ldg(reinterpret_cast<const float4*>(p.w + static_cast<int64_t>(n_base + r) * p.k + k));
+        staged[0][h * 4] = a.x; staged[0][h * 4 + 1] = a.y; staged[0][h * 4 + 2] = a.z; staged[0][h * 4 + 3] = a.w;
+        staged[1][h * 4] = b.x; staged[1][h * 4 + 1] = b.y; staged[1][h * 4 + 2] = b.z; staged[1][h * 4 + 3] = b.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int id = i * kTiledThreads + threadIdx.x, r = id / kTileK, k = block * kTileK + id % kTileK;
+        staged[0][i] = m_base + r < p.m && k < p.k ? Elem<T>::load(p.x + (m_base + r) * p.x_row_stride + k) : 0.0f;
+        staged[1][i] = n_base + r < p.n && k < p.k ? Elem<T>::load(p.w + static_cast<int64_t>(n_base + r) * p.k + k) : 0.0f;
+      }
+    }
+  };
+  auto place = [&](int buffer) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int id = i * kTiledThreads + threadIdx.x;
+      const int r = VEC ? threadIdx.x / 4 + 32 * (i / 4) : id / kTileK;
+      const int k = VEC ? threadIdx.x % 4 * 4 + i % 4 : id % kTileK;
+      tiles[buffer][0][k][r] = staged[0][i];
+      tiles[buffer][1][k][r] = staged[1][i];
+    }
+  };
+
+  float acc[4][8] = {};
+  if (first < last) {
+    fetch(first);
+    place(0);
+  }
+  __syncthreads();
+  for (int block = first; block < last; ++block) {
+    const int buffer = (block - first) & 1;
+    if (block + 1 < last) fetch(block + 1);
+    float sum[4][8] = {};
+#pragma unroll
+    for (int k = 0; k < kTileK; ++k) {
+      const float4 a = *reinterpret_cast<const float4*>(&tiles[buffer][0][k][ty * 4]);
+      const float4 b0 = *reinterpret_cast<const float4*>(&tiles[buffer][1][k][tx * 4]);
+      const float4 b1 = *reinterpret_cast<const float4*>(&tiles[buffer][1][k][32 + tx * 4]);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) block[i][j] = fmaf(a[i], b[j], block[i][j]);
+        for (int j = 0; j < 8; ++j) sum[i][j] = fmaf(av[i], bv[j], sum[i][j]);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += block[i][j];
+      for (int j = 0; j < 8; ++j) acc[i][j] += sum[i][j];
+    if (block + 1 < last) place(buffer ^ 1);
     __syncthreads();
   }
+  auto column = [&](int j) { return (j >> 2) * 32 + tx * 4 + (j & 3); };
+  if (splits == 1) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m_base + ty * 4 + i;
-    if (m >= p.m) continue;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n_base + tx * 4 + j;
-      if (n >= p.n) continue;
-      float v = acc[i][j];
-      if (p.bias != nullptr) v += Elem<T>::load(p.bias + n);
-      if (p.epilogue == B200_EPILOGUE_SWIGLU) {
-        // gate in even columns, up in odd columns: pair them inside the thread
-        if ((j & 1) == 0) {
-          float u = acc[i][j + 1];
-          if (p.bias != nullptr) u += Elem<T>::load(p.bias + n + 1);
-          const float gate = Elem<T>::round(silu_f32(Elem<T>::round(v)));
-          Elem<T>::store(p.out + static_cast<int64_t>(m) * (p.n / 2) + n / 2, gate * Elem<T>::round(u));
-        }
-        continue;
-      }
-      const int64_t o = static_cast<int64_t>(m) * p.n + n;
-      if (p.epilogue == B200_EPILOGUE_RESIDUAL)
-        v = __fadd_rn(Elem<T>::round(v), Elem<T>::load(p.residual + o));
-      Elem<T>::store(p.out + o, v);
-    }
+      for (int j = 0; j < 8; ++j)
+        epilogue_generic(p, m_base + ty * 4 + i, n_base + column(j), acc[i][j], j < 7 ? acc[i][j + 1] : 0.0f);
+    return;
   }
+  float* mine = &tiles[0][0][0][0];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; j += 4)
+      *reinterpret_cast<float4*>(mine + (ty * 4 + i) * kTile + column(j)) =
+          make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+  cluster_sync();
+  const int rank = cluster_cta_rank();
+  for (int unit = rank * kTiledThreads + threadIdx.x; unit < kTile * kTile / 4; unit += splits * kTiledThreads) {
+    float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int s = 0; s < splits; ++s) {
+      const float4 t = load_cluster_f32x4(smem_u32(mine + unit * 4), s);
+      total.x += t.x; total.y += t.y; total.z += t.z; total.w += t.w;
+    }
+    const int m = m_base + unit / (kTile / 4), n = n_base + unit % (kTile / 4) * 4;
+    epilogue_generic(p, m, n, total.x, total.y);
+    epilogue_generic(p, m, n + 1, total.y, 0.0f);
+    epilogue_generic(p, m, n + 2, total.z, total.w);
+    epilogue_generic(p, m, n + 3, total.w, 0.0f);
+  }
+  cluster_sync();  // no CTA leaves while another reads its tile
 }
 
 struct TilePlan {
@@ -374,27 +496,61 @@ extern "C" int64_t b200_linear_workspace_bytes(int64_t m, int64_t k, int64_t n, 
                                  t.partial_floats_per_tile_split * 4;
 }
 
+// Rows up to which W is streamed (linear_rows_kernel, its time grows with every 8 rows) instead of multiplied in tiles
+// (the same time for 1 to 64 rows). 9728 x 896: 18.0, 31.9 us for 8, 16 rows, 51 us in tiles; 896 x 4864: 10.3, 19.1
+// against 32 us.
+constexpr int64_t kRowsLimit = 16;
+
+template <int KSPLIT>
+static void launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
+  constexpr int kColumns = kRowsThreads / 32 / KSPLIT * kRowsColumns;
+  dim3 grid(static_cast<unsigned>(ceil_div(p.n, kColumns)), static_cast<unsigned>(ceil_div(p.m, kRowsOfX)));
+  linear_rows_kernel<KSPLIT><<<grid, kRowsThreads, 0, s>>>(p);
+}
+
+template <typename T>
 static int linear_generic(const void* input, const void* weight, const void* bias, const void* residual, void* output,
-                          int64_t m, int64_t k, int64_t n, int64_t input_row_stride, int dtype, int epilogue,
-                          cudaStream_t s) {
-  dim3 grid(static_cast<unsigned>(ceil_div(n, 64)), static_cast<unsigned>(ceil_div(m, 64)));
-  if (grid.y > 65535) return B200_ERR_TOO_LARGE;
-  with_element_type(dtype, [&](auto tag) {
-    using T = typename decltype(tag)::type;
-    LinearParamsGeneric<T> p;
-    p.x = static_cast<const T*>(input);
-    p.w = static_cast<const T*>(weight);
-    p.bias = static_cast<const T*>(bias);
-    p.residual = static_cast<const T*>(residual);
-    p.out = static_cast<T*>(output);
-    p.x_row_stride = input_row_stride;
-    p.m = static_cast<int>(m);
-    p.k = static_cast<int>(k);
-    p.n = static_cast<int>(n);
-    p.epilogue = epilogue;
-    linear_generic_kernel<T><<<grid, 256, 0, s>>>(p);
-  });
-  return launch_status();
+                          int64_t m, int64_t k, int64_t n, int64_t input_row_stride, int epilogue, cudaStream_t s) {
+  LinearParamsGeneric<T> p;
+  p.x = static_cast<const T*>(input);
+  p.w = static_cast<const T*>(weight);
+  p.bias = static_cast<const T*>(bias);
+  p.residual = static_cast<const T*>(residual);
+  p.out = static_cast<T*>(output);
+  p.x_row_stride = input_row_stride;
+  p.m = static_cast<int>(m);
+  p.k = static_cast<int>(k);
+  p.n = static_cast<int>(n);
+  p.epilogue = epilogue;
+  bool vec = false;
+  if constexpr (sizeof(T) == 4) {
+    vec = k % 4 == 0 && input_row_stride % 4 == 0 && aligned16(input) && aligned16(weight);
+    if (vec && m <= kRowsLimit) {
+      // K over as many warps as still leave each some 4 loads per lane, fewer where the columns alone fill the GPU
+      const int64_t warps = ceil_div(n, kRowsColumns) * ceil_div(m, kRowsOfX);
+      if (warps >= 32 * kNumSMs || k <= 256) launch_rows<1>(p, s);
+      else if (warps >= 16 * kNumSMs || k <= 512) launch_rows<2>(p, s);
+      else if (warps >= 8 * kNumSMs || k <= 1024) launch_rows<4>(p, s);
+      else launch_rows<8>(p, s);
+      return launch_status();
+    }
+  }
+  const int64_t tiles_m = ceil_div(m, kTile), tiles_n = ceil_div(n, kTile);
+  if (tiles_m > 65535) return B200_ERR_TOO_LARGE;
+  // CTAs of a tile: as many K slices (of at least 8 blocks) as bring some 4 CTAs to every SM
+  int64_t splits = 1;
+  while (splits < 8 && tiles_m * tiles_n * splits * 2 <= 4 * kNumSMs && ceil_div(k, kTileK) >= 16 * splits) splits *= 2;
+  dim3 grid(static_cast<unsigned>(tiles_n), static_cast<unsigned>(tiles_m), static_cast<unsigned>(splits));
+  auto launch_with = [&](auto kernel) {
+    if (splits == 1) kernel<<<grid, kTiledThreads, 0, s>>>(p);
+    else if (launch_cluster_z(kernel, grid, kTiledThreads, s, static_cast<unsigned>(splits), p) != cudaSuccess)
+      return B200_ERR_LAUNCH;
+    return launch_status();
+  };
+  if constexpr (sizeof(T) == 4) {
+    if (vec) return launch_with(linear_tiled_kernel<T, true>);
+  }
+  return launch_with(linear_tiled_kernel<T, false>);
 }
 
 // The tensor-core kernels, bf16 or fp16 (T): tcgen05, or the warp-level kernel where that declines.
@@ -452,7 +608,7 @@ extern "C" int b200_linear(const void* input, const void* weight, const void* bi
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   if (dtype == B200_F32)
-    return linear_generic(input, weight, bias, residual, output, m, k, n, input_row_stride, dtype, epilogue, s);
+    return linear_generic<float>(input, weight, bias, residual, output, m, k, n, input_row_stride, epilogue, s);
   if (dtype == B200_F16) {
     // fp16 on the tensor cores where 16-byte copies reach every row (the four projections of a Qwen2-0.5B layer on
     // 1030 rows: 478 us each on average on the CUDA cores, 21.6 us here); what they do not reach (and a caller
@@ -460,7 +616,7 @@ extern "C" int b200_linear(const void* input, const void* weight, const void* bi
     const int64_t need = b200_linear_workspace_bytes(m, k, n, dtype, epilogue);
     if (k % 8 != 0 || input_row_stride % 8 != 0 || !aligned16(input) || !aligned16(weight) ||
         (need > 0 && (!workspace || workspace_bytes < need)))
-      return linear_generic(input, weight, bias, residual, output, m, k, n, input_row_stride, dtype, epilogue, s);
+      return linear_generic<__half>(input, weight, bias, residual, output, m, k, n, input_row_stride, epilogue, s);
     return linear_tensor_core<__half>(input, weight, bias, residual, output, m, k, n, input_row_stride, dtype,
                                       epilogue, workspace, workspace_bytes, status, s);
   }
