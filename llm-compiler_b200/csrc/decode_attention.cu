@@ -1016,76 +1016,200 @@ __global__ void decode_merge_kernel(const float* __restrict__ ws_o, const float*
   out[static_cast<int64_t>(bh) * head_dim + threadIdx.x] = __float2bfloat16_rn(o_all / l_all);
 }
 
-// ---- fp32 path (CUDA cores, IEEE fp32 dots): small graphs in full precision ----------
-// One CTA per (sequence, q head); thread t walks tokens t, t+blockDim, ... with its own
-// online-softmax state, then the CTA merges. Matches the oracle to fp32 round-off.
-// The generic kernel: fp32, fp16, and the head sizes the tensor-core kernels do not take
-// (16, 32, 256). One CTA of 64 threads per (sequence, query head), thread t owning tokens
-// t, t + 64, ...; all arithmetic in fp32 on the CUDA cores, one rounding on the way out (and,
-// in the compatible mode of a 16-bit type, the reference's two roundings of the scores).
+// ---- CUDA cores: fp32, fp16, and the head sizes the tensor-core kernels do not take (16, 32, 256) ----
+// All arithmetic in fp32, one rounding on the way out (and, in the compatible mode of a 16-bit type, the reference's two
+// roundings of the scores). A CTA serves up to 8 query heads of one KV head from one read of its keys and values, in
+// tiles through shared memory (the next tile travels in registers meanwhile); the context of a (sequence, KV head) is
+// cut over the CTAs of a cluster, which merge through distributed shared memory: no workspace. Each CTA takes whole
+// tiles. Bound by latency at small contexts, else by the shared-memory reads of P and V (7 query heads x 600 tokens of
+// 64 in fp32, 4 sequences: 64.8 us with one CTA and thread-serial rows per query head -> 9.0 us).
+constexpr int kSplitHeads = 8, kSplitThreads = 256;
+template <int D>
+constexpr int kSplitTile = D <= 64 ? 64 : 4096 / D;  // tokens of a tile
+
+template <typename T>
+struct SplitParams {
+  const T* q;
+  const T* kbuf;
+  const T* vbuf;
+  const int64_t* lengths;
+  const void* mask;
+  T* out;
+  int32_t* status;
+  int64_t q_batch_stride, q_head_stride, mask_batch_stride;
+  int q_heads, kv_heads, groups, capacity, mask_len, mask_dtype, splits;
+  float scale;
+  bool compat, vec;  // vec: buffers that start on 16 bytes
+};
+
 template <int D, typename T>
-__global__ void decode_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ kbuf,
-                                                const T* __restrict__ vbuf,
-                                                const int64_t* __restrict__ lengths,
-                                                const void* __restrict__ mask, T* __restrict__ out,
-                                                int q_heads, int kv_heads, int groups, int capacity,
-                                                int mask_len, int64_t q_batch_stride,
-                                                int64_t q_head_stride, int64_t mask_batch_stride,
-                                                int mask_dtype, float scale, bool compat,
-                                                int32_t* status) {
-  constexpr int kT = D > 128 ? 32 : 64;  // (the merge buffer of 64 threads x 256 columns would not fit)
-  const int hq = blockIdx.x;
-  const int b = blockIdx.y;
-  const int kvh = hq / groups;
-  int64_t len = lengths[b];
-  if (len > mask_len) {
-    if (threadIdx.x == 0 && hq == 0 && status != nullptr)
-      atomicOr(status, B200_STATUS_LENGTH_OVER_MASK);
-    len = mask_len;
+__global__ void __launch_bounds__(kSplitThreads) decode_attention_split_kernel(const SplitParams<T> p) {
+  constexpr int kTile = kSplitTile<D>, kPitch = D + 4, kVec = Elem<T>::kPerVec;
+  constexpr int kItems = (kTile * D + kSplitThreads * kVec - 1) / (kSplitThreads * kVec);  // 16-byte loads a thread
+  constexpr int kGroups = D >= kSplitThreads ? 1 : kSplitThreads / D < kSplitHeads ? kSplitThreads / D : kSplitHeads;
+  constexpr int kEach = kSplitHeads / kGroups;  // heads a thread accumulates
+  __shared__ __align__(16) float sq[kSplitHeads][D], sk[kTile][kPitch], sv[kTile][D], sp[kSplitHeads][kTile];
+  __shared__ float sm[kSplitHeads], sl[kSplitHeads], sa[kSplitHeads];
+  float(*so)[D] = reinterpret_cast<float(*)[D]>(&sk[0][0]);  // this CTA's part of the outputs, behind its last tile
+  static_assert(kTile * kPitch >= kSplitHeads * D, "the outputs must fit the keys' tile");
+  const int blocks = (p.groups + kSplitHeads - 1) / kSplitHeads;
+  const int unit = blockIdx.x / p.splits, rank = blockIdx.x % p.splits, b = blockIdx.y;
+  const int kvh = unit / blocks, head0 = unit % blocks * kSplitHeads;
+  const int heads = min(kSplitHeads, p.groups - head0), hq = kvh * p.groups + head0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int64_t len = p.lengths[b];
+  if (len > p.mask_len) {
+    if (threadIdx.x == 0 && blockIdx.x == 0 && p.status != nullptr) atomicOr(p.status, B200_STATUS_LENGTH_OVER_MASK);
+    len = p.mask_len;
   }
   if (len < 0) len = 0;
-  __shared__ float sq[D];
-  __shared__ float sm[kT], sl[kT];
-  __shared__ float so[kT][D + 1];
-  for (int d = threadIdx.x; d < D; d += kT)
-    sq[d] = Elem<T>::load(q + b * q_batch_stride + hq * q_head_stride + d);
-  __syncthreads();
-  float m = -INFINITY, l = 0.0f, acc[D];
+  const int tiles = static_cast<int>((len + kTile - 1) / kTile), per = (tiles + p.splits - 1) / p.splits;
+  const int first = rank * per, last = min(first + per, tiles);
+
+  Vec16<T> keys[kItems], values[kItems];
+  auto fetch = [&](int tile) {
 #pragma unroll
-  for (int d = 0; d < D; ++d) acc[d] = 0.0f;
-  for (int t = threadIdx.x; t < len; t += kT) {
-    const T* krow = kbuf + ((static_cast<int64_t>(b) * capacity + t) * kv_heads + kvh) * D;
-    const T* vrow = vbuf + ((static_cast<int64_t>(b) * capacity + t) * kv_heads + kvh) * D;
-    float s = 0.0f;
+    for (int i = 0; i < kItems; ++i) {
+      const int at = (i * kSplitThreads + threadIdx.x) * kVec, row = at / D;
+      const int64_t token = static_cast<int64_t>(tile) * kTile + row;
+      const int64_t o = ((b * static_cast<int64_t>(p.capacity) + token) * p.kv_heads + kvh) * D + at % D;
+      const bool valid = row < kTile && token < len;  // rows past the length may hold anything: zeros instead
+      if (valid && p.vec) {
+        keys[i].load(p.kbuf + o);
+        values[i].load(p.vbuf + o);
+      } else {
 #pragma unroll
-    for (int d = 0; d < D; ++d) s = fmaf(sq[d], Elem<T>::load(krow + d), s);
-    s = compat ? Elem<T>::round(Elem<T>::round(s) * scale) : s * scale;
-    if (mask != nullptr) s += load_mask(mask, mask_dtype, b * mask_batch_stride + t);
-    const float m_new = fmaxf(m, s);
-    const float m_safe = m_new == -INFINITY ? 0.0f : m_new;
-    const float alpha = expf(m - m_safe);
-    const float pr = expf(s - m_safe);
-    l = l * alpha + pr;
-#pragma unroll
-    for (int d = 0; d < D; ++d) acc[d] = acc[d] * alpha + pr * Elem<T>::load(vrow + d);
-    m = m_new;
-  }
-  sm[threadIdx.x] = m;
-  sl[threadIdx.x] = l;
-#pragma unroll
-  for (int d = 0; d < D; ++d) so[threadIdx.x][d] = acc[d];
-  __syncthreads();
-  for (int d = threadIdx.x; d < D; d += kT) {
-    float m_all = -INFINITY;
-    for (int t = 0; t < kT; ++t) m_all = fmaxf(m_all, sm[t]);
-    float l_all = 0.0f, o_all = 0.0f;
-    for (int t = 0; t < kT; ++t) {
-      const float wgt = sm[t] == -INFINITY ? 0.0f : expf(sm[t] - m_all);
-      l_all += sl[t] * wgt;
-      o_all += so[t][d] * wgt;
+        for (int e = 0; e < kVec; ++e) {
+          keys[i].v[e] = valid ? Elem<T>::load(p.kbuf + o + e) : 0.0f;
+          values[i].v[e] = valid ? Elem<T>::load(p.vbuf + o + e) : 0.0f;
+        }
+      }
     }
-    Elem<T>::store(out + (static_cast<int64_t>(b) * q_heads + hq) * D + d, o_all / l_all);
+  };
+  if (first < last) fetch(first);
+  for (int i = threadIdx.x; i < kSplitHeads * D; i += kSplitThreads)
+    sq[i / D][i % D] = i / D < heads
+        ? Elem<T>::load(p.q + b * p.q_batch_stride + (hq + i / D) * p.q_head_stride + i % D) : 0.0f;
+  if (threadIdx.x < kSplitHeads) {
+    sm[threadIdx.x] = -INFINITY;
+    sl[threadIdx.x] = 0.0f;
   }
+  const int column = threadIdx.x % D, group = threadIdx.x / D;  // (threads beyond kGroups groups only load and score)
+  float acc[kEach] = {};
+  for (int tile = first; tile < last; ++tile) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const int at = (i * kSplitThreads + threadIdx.x) * kVec, row = at / D;
+      if (kItems * kSplitThreads * kVec > kTile * D && row >= kTile) break;
+#pragma unroll
+      for (int e = 0; e < kVec; e += 4) {
+        *reinterpret_cast<float4*>(&sk[row][at % D + e]) =
+            make_float4(keys[i].v[e], keys[i].v[e + 1], keys[i].v[e + 2], keys[i].v[e + 3]);
+        *reinterpret_cast<float4*>(&sv[row][at % D + e]) =
+            make_float4(values[i].v[e], values[i].v[e + 1], values[i].v[e + 2], values[i].v[e + 3]);
+      }
+    }
+    __syncthreads();
+    if (tile + 1 < last) fetch(tile + 1);
+    for (int item = threadIdx.x; item < kSplitHeads * kTile; item += kSplitThreads) {
+      const int h = item / kTile, t = item % kTile;
+      const int64_t token = static_cast<int64_t>(tile) * kTile + t;
+      float s = 0.0f;
+#pragma unroll 8
+      for (int d = 0; d < D; d += 4) {
+        const float4 k4 = *reinterpret_cast<const float4*>(&sk[t][d]), q4 = *reinterpret_cast<const float4*>(&sq[h][d]);
+        s = fmaf(q4.x, k4.x, s); s = fmaf(q4.y, k4.y, s); s = fmaf(q4.z, k4.z, s); s = fmaf(q4.w, k4.w, s);
+      }
+      s = p.compat ? Elem<T>::round(Elem<T>::round(s) * p.scale) : s * p.scale;
+      if (token >= len) s = -INFINITY;
+      else if (p.mask != nullptr) s += load_mask(p.mask, p.mask_dtype, b * p.mask_batch_stride + token);
+      sp[h][t] = s;
+    }
+    __syncthreads();
+    {  // warp h: running maximum and sum of head h
+      float s[(kTile + 31) / 32], top = -INFINITY, sum = 0.0f;
+#pragma unroll
+      for (int i = 0; i < (kTile + 31) / 32; ++i) {
+        s[i] = lane + 32 * i < kTile ? sp[warp][lane + 32 * i] : -INFINITY;
+        top = fmaxf(top, s[i]);
+      }
+      const float m = sm[warp], m_new = fmaxf(m, warp_max(top)), m_safe = m_new == -INFINITY ? 0.0f : m_new;
+#pragma unroll
+      for (int i = 0; i < (kTile + 31) / 32; ++i) {
+        s[i] = expf(s[i] - m_safe);
+        sum += s[i];
+        if (lane + 32 * i < kTile) sp[warp][lane + 32 * i] = s[i];
+      }
+      sum = warp_sum(sum);
+      __syncwarp();
+      if (lane == 0) {
+        const float alpha = expf(m - m_safe);
+        sa[warp] = alpha;
+        sm[warp] = m_new;
+        sl[warp] = sl[warp] * alpha + sum;
+      }
+    }
+    __syncthreads();
+    if (group < kGroups) {
+      float part[kEach] = {};
+#pragma unroll 4
+      for (int t = 0; t < kTile; t += 4) {
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = sv[t + j][column];
+#pragma unroll
+        for (int i = 0; i < kEach; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(&sp[group + i * kGroups][t]);
+          part[i] = fmaf(w.w, v[3], fmaf(w.z, v[2], fmaf(w.y, v[1], fmaf(w.x, v[0], part[i]))));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kEach; ++i) acc[i] = acc[i] * sa[group + i * kGroups] + part[i];
+    }
+  }
+  if (group < kGroups)
+#pragma unroll
+    for (int i = 0; i < kEach; ++i) so[group + i * kGroups][column] = acc[i];
+  cluster_sync();
+  for (int h = rank; h < heads; h += p.splits) {
+    for (int d = threadIdx.x; d < D; d += kSplitThreads) {
+      float m_all = -INFINITY, l_all = 0.0f, o_all = 0.0f;
+      for (int r = 0; r < p.splits; ++r) m_all = fmaxf(m_all, load_cluster_f32(smem_u32(&sm[h]), r));
+      for (int r = 0; r < p.splits; ++r) {
+        const float m = load_cluster_f32(smem_u32(&sm[h]), r);
+        const float weight = m == -INFINITY ? 0.0f : expf(m - m_all);
+        l_all += load_cluster_f32(smem_u32(&sl[h]), r) * weight;
+        o_all += load_cluster_f32(smem_u32(&so[h][d]), r) * weight;
+      }
+      Elem<T>::store(p.out + (static_cast<int64_t>(b) * p.q_heads + hq + h) * D + d, o_all / l_all);
+    }
+  }
+  cluster_sync();  // no CTA leaves while another reads its part
+}
+
+template <int D, typename T>
+int launch_split(SplitParams<T> p, int64_t batch, int64_t max_length, cudaStream_t stream) {
+  // CTAs of a (sequence, KV head, 8 query heads): up to 8 while some 4 fit on every SM and a CTA gets a tile of the
+  // longest context
+  const int64_t units = batch * p.kv_heads * ceil_div(p.groups, kSplitHeads);
+  int splits = 1;
+  while (splits < 8 && units * splits * 2 <= 4 * kNumSMs && max_length >= 2 * splits * kSplitTile<D>) splits *= 2;
+  p.splits = splits;
+  const int64_t head_units = p.kv_heads * ceil_div(p.groups, kSplitHeads);
+  if (head_units * splits > INT32_MAX) return B200_ERR_TOO_LARGE;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(head_units * splits), static_cast<unsigned>(batch));
+  config.blockDim = dim3(kSplitThreads);
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = static_cast<unsigned>(splits);
+  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  if (cudaLaunchKernelEx(&config, decode_attention_split_kernel<D, T>, p) != cudaSuccess) return B200_ERR_LAUNCH;
+  return launch_status();
 }
 
 template <int D>
@@ -1410,25 +1534,37 @@ static int decode_attention_impl(const void* query, const void* key_buffer,
     if (sequence_order != nullptr) return B200_ERR_UNSUPPORTED;  // (a service order is the tensor-core kernel's)
     if (head_dim != 16 && head_dim != 32 && head_dim != 64 && head_dim != 128 && head_dim != 256)
       return B200_ERR_UNSUPPORTED;
-    dim3 grid(static_cast<unsigned>(q_heads), static_cast<unsigned>(batch));
-    const bool compat = mode == B200_MODE_PYTORCH_COMPATIBLE && dtype != B200_F32;
+    int code = B200_ERR_UNSUPPORTED;
     with_element_type(dtype, [&](auto tag) {
       using T = typename decltype(tag)::type;
-      auto run = [&](auto kernel) {
-        kernel<<<grid, head_dim > 128 ? 32 : 64, 0, s>>>(
-            static_cast<const T*>(query), static_cast<const T*>(key_buffer),
-            static_cast<const T*>(value_buffer), lengths, mask, static_cast<T*>(output),
-            static_cast<int>(q_heads), static_cast<int>(kv_heads), groups, static_cast<int>(capacity),
-            static_cast<int>(mask_len), q_batch_stride, q_head_stride, mask_batch_stride, mask_dtype,
-            static_cast<float>(scale), compat, status);
-      };
-      if (head_dim == 16) run(decode_attention_generic_kernel<16, T>);
-      else if (head_dim == 32) run(decode_attention_generic_kernel<32, T>);
-      else if (head_dim == 64) run(decode_attention_generic_kernel<64, T>);
-      else if (head_dim == 128) run(decode_attention_generic_kernel<128, T>);
-      else run(decode_attention_generic_kernel<256, T>);
+      SplitParams<T> p;
+      p.q = static_cast<const T*>(query);
+      p.kbuf = static_cast<const T*>(key_buffer);
+      p.vbuf = static_cast<const T*>(value_buffer);
+      p.lengths = lengths;
+      p.mask = mask;
+      p.out = static_cast<T*>(output);
+      p.status = status;
+      p.q_batch_stride = q_batch_stride;
+      p.q_head_stride = q_head_stride;
+      p.mask_batch_stride = mask_batch_stride;
+      p.q_heads = static_cast<int>(q_heads);
+      p.kv_heads = static_cast<int>(kv_heads);
+      p.groups = groups;
+      p.capacity = static_cast<int>(capacity);
+      p.mask_len = static_cast<int>(mask_len);
+      p.mask_dtype = mask_dtype;
+      p.scale = static_cast<float>(scale);
+      p.compat = mode == B200_MODE_PYTORCH_COMPATIBLE && dtype != B200_F32;
+      p.vec = aligned16(key_buffer) && aligned16(value_buffer);
+      const int64_t longest = max_length_hint > 0 && max_length_hint < mask_len ? max_length_hint : mask_len;
+      if (head_dim == 16) code = launch_split<16>(p, batch, longest, s);
+      else if (head_dim == 32) code = launch_split<32>(p, batch, longest, s);
+      else if (head_dim == 64) code = launch_split<64>(p, batch, longest, s);
+      else if (head_dim == 128) code = launch_split<128>(p, batch, longest, s);
+      else code = launch_split<256>(p, batch, longest, s);
     });
-    return launch_status();
+    return code;
   }
   if (!aligned16(key_buffer) || !aligned16(value_buffer) ||
       (reinterpret_cast<uintptr_t>(query) & 3u) != 0 || q_head_stride % 2 != 0 ||

@@ -55,6 +55,9 @@ __device__ __forceinline__ float load_mask(const void* mask, int dtype, int64_t 
   return __bfloat162float(static_cast<const __nv_bfloat16*>(mask)[index]);
 }
 
+template <bool B>
+struct Flag { static constexpr bool value = B; };
+
 template <int D>
 __device__ __forceinline__ uint32_t tile_offset(int row, int chunk) {
   return static_cast<uint32_t>(row * (D * 2) + (((chunk & ~7) | ((chunk ^ row) & 7)) << 4));
@@ -308,65 +311,159 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
   }
 }
 
-// ---- generic path (fp32, head sizes 16 / 32 / 256, fp16 without 16-byte rows): one CTA per (query token, q head,
-// sequence), fp32 arithmetic on the CUDA cores, one rounding on the way out (and, in the
-// compatible mode of a 16-bit type, the reference's two roundings of the scores) ----------
-template <int D, typename T>
-__global__ void prefill_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k,
-                                                 const T* __restrict__ v,
-                                                 const void* __restrict__ mask, T* __restrict__ out,
-                                                 int q_heads, int groups, int tokens, int64_t qs0,
-                                                 int64_t qs1, int64_t qs2, int64_t ks0, int64_t ks1,
-                                                 int64_t ks2, int64_t vs0, int64_t vs1, int64_t vs2,
-                                                 int64_t ms0, int64_t ms2, int64_t ms3,
-                                                 int mask_dtype, int causal, float scale,
-                                                 bool compat) {
-  constexpr int kT = D > 128 ? 32 : 64;  // (the merge buffer of 64 threads x 256 columns would not fit)
-  const int qt = blockIdx.x, hq = blockIdx.y, b = blockIdx.z;
-  const int kvh = hq / groups;
-  __shared__ float sq[D];
-  __shared__ float sm[kT], sl[kT];
-  __shared__ float so[kT][D + 1];
-  for (int d = threadIdx.x; d < D; d += kT) sq[d] = Elem<T>::load(q + b * qs0 + hq * qs1 + qt * qs2 + d);
-  __syncthreads();
-  float m = -INFINITY, l = 0.0f, acc[D];
+// ---- CUDA cores: fp32, head sizes 16 / 32 / 256, fp16 without 16-byte rows ----
+// fp32 arithmetic, one rounding on the way out (and, in the compatible mode of a 16-bit type, the reference's two
+// roundings of the scores). A CTA of 16 x 16 threads owns 64 query rows of one (sequence, query head) and walks 64-key
+// tiles: scores 4 x 4 a thread from transposed Q and K tiles, then 4 rows x D / 16 columns of P V, whose 64-key sums
+// are added to the running output one tile at a time (short chains: rounding errors grow with the tiles, not the keys).
+// A key that a row does not see has probability -1 and is skipped: its value may be infinite or NaN. Bound by the FMA
+// rate (4 FMA a shared-memory word) and by the few CTAs of a short prompt.
+// Qwen2-0.5B in fp32, 1 x 1000 tokens: 126.8 -> 34.4 ms a pass with the tiled GEMM of linear.cu (before: one CTA per
+// query row, every row reading all keys and values again).
+template <int D>
+constexpr int kTiledSmem = (2 * D * 68 + 64 * D + 64 * 68) * 4;
+
+template <int D, typename T, bool VEC>
+__global__ void __launch_bounds__(256) prefill_attention_tiled_kernel(const PrefillParams<T> p) {
+  constexpr int kPitch = 68, kColumns = D / 16;
+  extern __shared__ __align__(16) float tiled_smem[];
+  float* q_sm = tiled_smem;              // [D][68]: Q transposed
+  float* k_sm = q_sm + D * kPitch;       // [D][68]: K transposed
+  float* v_sm = k_sm + D * kPitch;       // [64][D]
+  float* p_sm = v_sm + 64 * D;           // [64 keys][68 rows]
+  const int q0 = blockIdx.x * 64, hq = blockIdx.y, b = blockIdx.z, kvh = hq / p.groups;
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  const T* q = p.q + b * p.qs[0] + hq * p.qs[1];
+  const T* k = p.k + b * p.ks[0] + kvh * p.ks[1];
+  const T* v = p.v + b * p.vs[0] + kvh * p.vs[1];
+
+  // 64 rows from `first` on, zeros behind the last token
+  auto load_rows = [&](const T* base, int64_t stride, int first, float* to, bool transposed) {
+    constexpr int kVec = VEC ? Elem<T>::kPerVec : 1;
+    for (int at = threadIdx.x * kVec; at < 64 * D; at += 256 * kVec) {
+      const int row = at / D, d = at % D;
+      float value[kVec];
+      if (first + row >= p.tokens) {
 #pragma unroll
-  for (int d = 0; d < D; ++d) acc[d] = 0.0f;
-  const int key_end = causal ? qt + 1 : tokens;
-  for (int t = threadIdx.x; t < key_end; t += kT) {
-    const T* krow = k + b * ks0 + kvh * ks1 + t * ks2;
-    const T* vrow = v + b * vs0 + kvh * vs1 + t * vs2;
-    float s = 0.0f;
+        for (int e = 0; e < kVec; ++e) value[e] = 0.0f;
+      } else if constexpr (VEC) {
+        Vec16<T> raw;
+        raw.load(base + (first + row) * stride + d);
 #pragma unroll
-    for (int d = 0; d < D; ++d) s = fmaf(sq[d], Elem<T>::load(krow + d), s);
-    s = compat ? Elem<T>::round(Elem<T>::round(s) * scale) : s * scale;
-    if (mask != nullptr)
-      s += load_mask(mask, mask_dtype, b * ms0 + static_cast<int64_t>(qt) * ms2 + t * ms3);
-    const float m_new = fmaxf(m, s);
-    const float m_safe = m_new == -INFINITY ? 0.0f : m_new;
-    const float alpha = expf(m - m_safe);
-    const float pr = expf(s - m_safe);
-    l = l * alpha + pr;
+        for (int e = 0; e < kVec; ++e) value[e] = raw.v[e];
+      } else {
+        value[0] = Elem<T>::load(base + (first + row) * stride + d);
+      }
 #pragma unroll
-    for (int d = 0; d < D; ++d) acc[d] = acc[d] * alpha + pr * Elem<T>::load(vrow + d);
-    m = m_new;
-  }
-  sm[threadIdx.x] = m;
-  sl[threadIdx.x] = l;
-#pragma unroll
-  for (int d = 0; d < D; ++d) so[threadIdx.x][d] = acc[d];
-  __syncthreads();
-  for (int d = threadIdx.x; d < D; d += kT) {
-    float m_all = -INFINITY;
-    for (int t = 0; t < kT; ++t) m_all = fmaxf(m_all, sm[t]);
-    float l_all = 0.0f, o_all = 0.0f;
-    for (int t = 0; t < kT; ++t) {
-      const float wgt = sm[t] == -INFINITY ? 0.0f : expf(sm[t] - m_all);
-      l_all += sl[t] * wgt;
-      o_all += so[t][d] * wgt;
+      for (int e = 0; e < kVec; ++e) to[transposed ? (d + e) * kPitch + row : row * D + d + e] = value[e];
     }
-    Elem<T>::store(out + ((static_cast<int64_t>(b) * tokens + qt) * q_heads + hq) * D + d, o_all / l_all);
+  };
+
+  load_rows(q, p.qs[2], q0, q_sm, true);
+  float m[4], l[4], out[4][kColumns];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kColumns; ++c) out[i][c] = 0.0f;
   }
+  const int key_end = p.causal ? min(p.tokens, q0 + 64) : p.tokens;
+  for (int k0 = 0; k0 < key_end; k0 += 64) {
+    __syncthreads();  // the last tile's products have read K, V and P
+    load_rows(k, p.ks[2], k0, k_sm, true);
+    load_rows(v, p.vs[2], k0, v_sm, false);
+    __syncthreads();
+    float s[4][4] = {};
+#pragma unroll 4
+    for (int d = 0; d < D; ++d) {
+      const float4 a = *reinterpret_cast<const float4*>(q_sm + d * kPitch + ty * 4);
+      const float4 c = *reinterpret_cast<const float4*>(k_sm + d * kPitch + tx * 4);
+      const float av[4] = {a.x, a.y, a.z, a.w}, cv[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = fmaf(av[i], cv[j], s[i][j]);
+    }
+    const bool whole = k0 + 64 <= p.tokens && (!p.causal || k0 + 63 <= q0);  // every row sees every key
+    float alpha[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = q0 + ty * 4 + i;
+      bool seen[4];
+      float top = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = k0 + tx * 4 + j;
+        seen[j] = whole || (key < p.tokens && (!p.causal || key <= row));
+        s[i][j] = p.compat ? Elem<T>::round(Elem<T>::round(s[i][j]) * p.scale) : s[i][j] * p.scale;
+        if (p.mask != nullptr && seen[j] && row < p.tokens)
+          s[i][j] += load_mask(p.mask, p.mask_dtype,
+                               b * p.ms[0] + static_cast<int64_t>(row) * p.ms[2] + static_cast<int64_t>(key) * p.ms[3]);
+        if (seen[j]) top = fmaxf(top, s[i][j]);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      const float m_new = fmaxf(m[i], top), m_safe = m_new == -INFINITY ? 0.0f : m_new;
+      alpha[i] = expf(m[i] - m_safe);
+      m[i] = m_new;
+      float sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = seen[j] ? expf(s[i][j] - m_safe) : -1.0f;
+        sum += seen[j] ? s[i][j] : 0.0f;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l[i] = l[i] * alpha[i] + sum;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<float4*>(p_sm + (tx * 4 + j) * kPitch + ty * 4) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
+    __syncthreads();
+    float part[4][kColumns] = {};
+    auto add_keys = [&](auto masked) {
+#pragma unroll 4
+      for (int key = 0; key < 64; ++key) {
+        const float4 w = *reinterpret_cast<const float4*>(p_sm + key * kPitch + ty * 4);
+        const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int c = 0; c < kColumns; ++c) {
+          const float value = v_sm[key * D + tx + 16 * c];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float next = fmaf(wv[i], value, part[i][c]);
+            part[i][c] = decltype(masked)::value && wv[i] < 0.0f ? part[i][c] : next;
+          }
+        }
+      }
+    };
+    if (whole) add_keys(Flag<false>{});
+    else add_keys(Flag<true>{});
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < kColumns; ++c) out[i][c] = out[i][c] * alpha[i] + part[i][c];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = q0 + ty * 4 + i;
+    if (row >= p.tokens) continue;
+    T* to = p.out + ((static_cast<int64_t>(b) * p.tokens + row) * p.q_heads + hq) * D;
+#pragma unroll
+    for (int c = 0; c < kColumns; ++c) Elem<T>::store(to + tx + 16 * c, out[i][c] / l[i]);
+  }
+}
+
+template <int D, typename T>
+int launch_tiled(const PrefillParams<T>& p, bool vec, cudaStream_t stream) {
+  auto launch = [&](auto kernel) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTiledSmem<D>) != cudaSuccess)
+      return B200_ERR_LAUNCH;
+    kernel<<<dim3((p.tokens + 63) / 64, p.q_heads, p.batch), 256, kTiledSmem<D>, stream>>>(p);
+    return launch_status();
+  };
+  return vec ? launch(prefill_attention_tiled_kernel<D, T, true>) : launch(prefill_attention_tiled_kernel<D, T, false>);
 }
 
 template <int D, int STAGES, typename T>
@@ -428,53 +525,35 @@ extern "C" int b200_prefill_attention(const void* query, const void* key, const 
   const int64_t* ms = mask != nullptr ? mask_strides : zero4;
 
   if (!known_dtype(dtype)) return B200_ERR_UNSUPPORTED;
-  // 16-byte loads of every row: what the tensor-core kernels need (bf16 is refused without them, fp16 keeps the
+  // 16-byte loads of every row: what the tensor-core kernels need (bf16 is refused without them, fp16 then takes the
   // CUDA-core kernel)
-  bool rows16 = aligned16(query) && aligned16(key) && aligned16(value) &&
-                (reinterpret_cast<uintptr_t>(output) & 3u) == 0;
+  const int per_vec = dtype == B200_F32 ? 4 : 8;
+  bool rows16 = aligned16(query) && aligned16(key) && aligned16(value);
   for (int i = 0; i < 3; ++i)
-    rows16 = rows16 && query_strides[i] % 8 == 0 && key_strides[i] % 8 == 0 && value_strides[i] % 8 == 0;
-  const bool tensor_core = (head_dim == 64 || head_dim == 128) && (dtype == B200_BF16 || (dtype == B200_F16 && rows16));
+    rows16 = rows16 && query_strides[i] % per_vec == 0 && key_strides[i] % per_vec == 0 && value_strides[i] % per_vec == 0;
+  const bool pairs = (reinterpret_cast<uintptr_t>(output) & 3u) == 0;
+  const bool tensor_core = (head_dim == 64 || head_dim == 128) &&
+                           (dtype == B200_BF16 || (dtype == B200_F16 && rows16 && pairs));
   if (!tensor_core) {
     if (head_dim != 16 && head_dim != 32 && head_dim != 64 && head_dim != 128 && head_dim != 256)
       return B200_ERR_UNSUPPORTED;
     if (tokens > 65535 * 64) return B200_ERR_TOO_LARGE;
-    dim3 grid(static_cast<unsigned>(tokens), static_cast<unsigned>(q_heads),
-              static_cast<unsigned>(batch));
-    const bool compat = mode == B200_MODE_PYTORCH_COMPATIBLE && dtype != B200_F32;
-    with_element_type(dtype, [&](auto tag) {
-      using T = typename decltype(tag)::type;
-      auto run = [&](auto kernel) {
-        kernel<<<grid, head_dim > 128 ? 32 : 64, 0, s>>>(
-            static_cast<const T*>(query), static_cast<const T*>(key), static_cast<const T*>(value),
-            mask, static_cast<T*>(output), static_cast<int>(q_heads), groups,
-            static_cast<int>(tokens), query_strides[0], query_strides[1], query_strides[2],
-            key_strides[0], key_strides[1], key_strides[2], value_strides[0], value_strides[1],
-            value_strides[2], ms[0], ms[2], ms[3], mask_dtype, causal, static_cast<float>(scale),
-            compat);
-      };
-      if (head_dim == 16) run(prefill_attention_generic_kernel<16, T>);
-      else if (head_dim == 32) run(prefill_attention_generic_kernel<32, T>);
-      else if (head_dim == 64) run(prefill_attention_generic_kernel<64, T>);
-      else if (head_dim == 128) run(prefill_attention_generic_kernel<128, T>);
-      else run(prefill_attention_generic_kernel<256, T>);
-    });
-    return launch_status();
-  }
-  if (!rows16) return B200_ERR_ALIGNMENT;
-
-  if (dtype == B200_BF16 && mode == B200_MODE_FAST &&
-      ((mask == nullptr && causal) ||
-       (mask != nullptr && !causal && mask_dtype == B200_F32 && workspace != nullptr))) {
-    // the tensor-core kernel: causal-proved, or the additive-mask contract with its tile pre-pass
-    const int code = prefill_attention_tcgen05(query, key, value, output, batch, q_heads, kv_heads,
-                                               tokens, head_dim, query_strides, key_strides,
-                                               value_strides, scale, status, s, mask, mask_strides,
-                                               workspace, workspace_bytes, 0, nullptr, 0);
-    if (code != B200_ERR_UNSUPPORTED) return code;
+  } else {
+    if (!rows16 || !pairs) return B200_ERR_ALIGNMENT;
+    if (dtype == B200_BF16 && mode == B200_MODE_FAST &&
+        ((mask == nullptr && causal) ||
+         (mask != nullptr && !causal && mask_dtype == B200_F32 && workspace != nullptr))) {
+      // the tensor-core kernel: causal-proved, or the additive-mask contract with its tile pre-pass
+      const int code = prefill_attention_tcgen05(query, key, value, output, batch, q_heads, kv_heads,
+                                                 tokens, head_dim, query_strides, key_strides,
+                                                 value_strides, scale, status, s, mask, mask_strides,
+                                                 workspace, workspace_bytes, 0, nullptr, 0);
+      if (code != B200_ERR_UNSUPPORTED) return code;
+    }
   }
 
-  auto warp_level = [&](auto tag) {
+  int code = B200_ERR_UNSUPPORTED;
+  with_element_type(dtype, [&](auto tag) {
     using T = typename decltype(tag)::type;
     PrefillParams<T> p;
     p.q = static_cast<const T*>(query);
@@ -495,9 +574,19 @@ extern "C" int b200_prefill_attention(const void* query, const void* key, const 
     p.tokens = static_cast<int>(tokens);
     p.mask_dtype = mask_dtype;
     p.causal = causal ? 1 : 0;
-    p.compat = mode == B200_MODE_PYTORCH_COMPATIBLE ? 1 : 0;
+    p.compat = mode == B200_MODE_PYTORCH_COMPATIBLE && dtype != B200_F32 ? 1 : 0;
     p.scale = static_cast<float>(scale);
-    return head_dim == 64 ? launch_warp_level<64, 3>(p, s) : launch_warp_level<128, 2>(p, s);
-  };
-  return dtype == B200_F16 ? warp_level(TypeTag<__half>{}) : warp_level(TypeTag<__nv_bfloat16>{});
+    if constexpr (sizeof(T) == 2) {
+      if (tensor_core) {
+        code = head_dim == 64 ? launch_warp_level<64, 3>(p, s) : launch_warp_level<128, 2>(p, s);
+        return;
+      }
+    }
+    if (head_dim == 16) code = launch_tiled<16>(p, rows16, s);
+    else if (head_dim == 32) code = launch_tiled<32>(p, rows16, s);
+    else if (head_dim == 64) code = launch_tiled<64>(p, rows16, s);
+    else if (head_dim == 128) code = launch_tiled<128>(p, rows16, s);
+    else code = launch_tiled<256>(p, rows16, s);
+  });
+  return code;
 }
