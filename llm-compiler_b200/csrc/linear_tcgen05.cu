@@ -30,6 +30,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "linear_rows.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
 
@@ -1199,13 +1200,20 @@ int linear_tcgen05(const void* input, const void* weight, const void* bias, cons
              fold_norm, norm_eps, norm_squares, norm_slices);
 }
 
-int linear_partial_splits(int64_t m, int64_t k, int64_t n) { return plan_partial(m, k, n).splits; }
+int linear_partial_splits(int64_t m, int64_t k, int64_t n) {
+  return takes_few_rows(m) ? 1 : plan_partial(m, k, n).splits;
+}
 
 int linear_partial_tcgen05(const void* input, const void* weight, float* partials,
                            float* row_squares, int64_t m, int64_t k, int64_t n,
                            int64_t input_row_stride, int splits, int32_t* status,
                            cudaStream_t stream) {
   if (row_squares != nullptr && m > 128) return B200_ERR_UNSUPPORTED;
+  if (splits == 1 && takes_few_rows(m)) {
+    FewRowsCall c{input, weight, nullptr, nullptr, nullptr, partials, row_squares, m, k, n, input_row_stride,
+                  B200_EPILOGUE_NONE};
+    return linear_few_rows(c, B200_BF16, stream);
+  }
   const PartialPlan plan = plan_partial(m, k, n);
   const int a_rows = m <= 64 ? 64 : 128;
   CUtensorMap a_map, b_map;
@@ -1248,6 +1256,11 @@ int linear_splitk_residual_tcgen05(const void* input, const void* weight, const 
                                    void* output, int64_t m, int64_t k, int64_t n,
                                    int64_t input_row_stride, int32_t* status, cudaStream_t stream,
                                    float* squares_out) {
+  if (squares_out == nullptr && takes_few_rows(m)) {
+    FewRowsCall c{input, weight, nullptr, residual, output, nullptr, nullptr, m, k, n, input_row_stride,
+                  B200_EPILOGUE_RESIDUAL};
+    return linear_few_rows(c, B200_BF16, stream);
+  }
   const PartialPlan plan = plan_cluster(m, k, n);
   const int a_rows = m <= 64 ? 64 : 128;
   // enough N x M tiles to fill the GPU without cutting K: the plain kernel with the residual epilogue
@@ -1289,7 +1302,9 @@ int linear_splitk_residual_tcgen05(const void* input, const void* weight, const 
 
 // Slices of row sums of squares that the cluster split-K projection leaves (N tiles x K slices);
 // 0 when the shape runs without a cluster (then nothing is written).
+// (a projection of a few rows leaves none: the one behind it squares its rows on the way)
 int64_t linear_splitk_slices(int64_t m, int64_t k, int64_t n) {
+  if (takes_few_rows(m)) return 0;
   const PartialPlan plan = plan_cluster(m, k, n);
   return plan.splits <= 1 ? 0 : ceil_div(n, static_cast<int64_t>(plan.bn)) * plan.splits;
 }
@@ -1332,6 +1347,11 @@ extern "C" int b200_linear_rms_input(const void* input, const void* folded_weigh
   if (m > 128) return B200_ERR_TOO_LARGE;
   if (k % 8 != 0 || input_row_stride % 8 != 0) return B200_ERR_UNSUPPORTED;
   if (!aligned16(input) || !aligned16(folded_weight)) return B200_ERR_ALIGNMENT;
+  if (takes_few_rows(m)) {
+    FewRowsCall c{input, folded_weight, bias, nullptr, output, nullptr, nullptr, m, k, n, input_row_stride, epilogue,
+                  true, epsilon};
+    return linear_few_rows(c, B200_BF16, static_cast<cudaStream_t>(stream));
+  }
   return linear_tcgen05(input, folded_weight, bias, nullptr, output, m, k, n, input_row_stride, B200_BF16,
                         epilogue, status, static_cast<cudaStream_t>(stream), true, epsilon,
                         static_cast<const float*>(row_squares), static_cast<int>(row_square_slices));
