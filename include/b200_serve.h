@@ -325,6 +325,38 @@ int b200_linear(const void* input, const void* weight, const void* bias, const v
                 int dtype, int epilogue, void* workspace, int64_t workspace_bytes,
                 int32_t* status, void* stream);
 
+/* ---- Prompt layers -------------------------------------------------------------
+ * The layers of a Qwen2 prompt (qwen2.py:236-304) from empty caches: per layer b200_rms_norm, b200_linear (q|k|v with
+ * bias), RoPE and KV store from position 0 on, causal b200_prefill_attention, b200_linear + residual, b200_rms_norm,
+ * b200_linear + SwiGLU (gate_j / up_j rows alternating), b200_linear + residual. x [batch * tokens, hidden] is updated
+ * in place; the other buffers are scratch of the sizes beside them. With a block table the caches are block pools
+ * (b200_paged_kv_store) and `capacity` is the longest sequence. The workspace serves every b200_linear of the layer
+ * (b200_linear_workspace_bytes). Launches what those calls launch; returns the first error. */
+typedef struct {
+  const void *input_norm, *qkv_weight, *qkv_bias, *o_weight, *post_norm, *gate_up_weight, *down_weight;
+  void *keys, *values;
+} b200_prompt_layer;
+typedef struct {
+  void* x;                     /* [rows, hidden] */
+  void* x_middle;              /* [rows, hidden] */
+  void* h;                     /* [rows, hidden] */
+  void* qkv;                   /* [rows, (q_heads + 2 kv_heads) head_dim] */
+  void* q;                     /* [rows, q_heads head_dim] */
+  void* k;                     /* [rows, kv_heads head_dim] */
+  void* attention;             /* [rows, q_heads head_dim] */
+  void* gated;                 /* [rows, intermediate] */
+  const void *cosine, *sine;   /* [rows, head_dim] */
+  const int64_t* positions;    /* [batch], zeros */
+  const int32_t* block_table;  /* NULL: contiguous caches */
+  void* workspace;
+  int64_t workspace_bytes, batch, tokens, q_heads, kv_heads, head_dim, hidden, intermediate, capacity;
+  int64_t num_blocks, block_size, max_blocks;
+  double epsilon, scale;
+  int dtype, mode;
+} b200_prompt_call;
+int b200_qwen2_prompt_layers(const b200_prompt_layer* layers, int64_t num_layers, const b200_prompt_call* call,
+                             int32_t* status, void* stream);
+
 /* ---- Decode-step chain: split-K partial sums reduced by the operator that follows ----------
  * At decode sizes (M <= 128 rows) the projections are weight streaming: the GEMM is cut into
  * N tiles x K slices so that every SM pulls weights, each CTA writes its fp32 partial tile,

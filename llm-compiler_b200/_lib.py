@@ -95,6 +95,26 @@ class StepOutput(ctypes.Structure):
                [("epsilon", c_double)]
 
 
+class PromptLayer(ctypes.Structure):
+    """b200_prompt_layer of include/b200_serve.h."""
+
+    _fields_ = [(name, c_void_p) for name in
+                ("input_norm", "qkv_weight", "qkv_bias", "o_weight", "post_norm", "gate_up_weight", "down_weight",
+                 "keys", "values")]
+
+
+class PromptCall(ctypes.Structure):
+    """b200_prompt_call of include/b200_serve.h."""
+
+    _fields_ = [(name, c_void_p) for name in
+                ("x", "x_middle", "h", "qkv", "q", "k", "attention", "gated", "cosine", "sine", "positions",
+                 "block_table", "workspace")] + \
+               [(name, c_int64) for name in
+                ("workspace_bytes", "batch", "tokens", "q_heads", "kv_heads", "head_dim", "hidden", "intermediate",
+                 "capacity", "num_blocks", "block_size", "max_blocks")] + \
+               [("epsilon", c_double), ("scale", c_double), ("dtype", c_int), ("mode", c_int)]
+
+
 _DELTA, _RETENTION, _STEP = POINTER(DeltaInputs), POINTER(RetentionInputs), POINTER(StepOutput)
 
 # What b200_abi_version() of a matching library returns (bumped with every signature change).
@@ -143,6 +163,7 @@ SIGNATURES = {
     "b200_linear_workspace_bytes": (c_int64, [c_int64, c_int64, c_int64, c_int, c_int]),
     "b200_linear": (c_int, [c_void_p] * 5 + [c_int64] * 4 + [c_int, c_int, c_void_p, c_int64,
                                                               c_void_p, c_void_p]),
+    "b200_qwen2_prompt_layers": (c_int, [POINTER(PromptLayer), c_int64, POINTER(PromptCall), c_void_p, c_void_p]),
     "b200_linear_partial_splits": (c_int64, [c_int64, c_int64, c_int64]),
     "b200_linear_partial": (c_int, [c_void_p] * 4 + [c_int64] * 5 + [c_void_p, c_void_p]),
     "b200_reduce_residual_rms_norm": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p,

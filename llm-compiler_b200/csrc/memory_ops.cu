@@ -3,6 +3,7 @@
 // advance and greedy argmax. All of them move each byte once with 16-byte accesses;
 // none needs scratch memory.
 #include "common.cuh"
+#include "prompt_layers.cuh"
 
 namespace b200 {
 namespace {
@@ -228,6 +229,52 @@ int rope_typed(const void* q, const void* k, const void* cosine, const void* sin
     else launch(rope_kernel<T, false, int64_t>);
   }
   return launch_status();
+}
+
+// A prompt's RoPE and KV store in one pass over the projection's rows (what rope_kernel and kv_store_kernel do in two,
+// with k read back in between): a thread takes 16 bytes of a head's lower half and the 16 bytes of its upper half, heads
+// of q, k, v side by side, so that a warp reads neighbouring pieces of one row. Bound by memory latency at small
+// prompts, by its reads and writes at large ones: 4 x 4096 tokens of Qwen2-0.5B, 75 MB: 22.2 us in two kernels.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+rope_into_cache_kernel(const T* qkv, const T* cosine, const T* sine, T* q_out, T* keys, T* values, uint32_t total,
+                       uint32_t tokens, uint32_t q_heads, uint32_t kv_heads, uint32_t dim, int64_t capacity) {
+  constexpr uint32_t per = Elem<T>::kPerVec;
+  // What follows may start once the kernel in front has finished: it may take tensor memory that one still needs.
+  // (No __restrict__: nothing may be read ahead of the wait.)
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const uint32_t half = dim / 2, pieces = half / per, heads = q_heads + 2 * kv_heads;
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < total; i += gridDim.x * kThreads) {
+    const uint32_t d0 = i % pieces * per, h = i / pieces % heads, row = i / (pieces * heads);
+    const uint32_t b = row / tokens, t = row % tokens;
+    const T* src = qkv + (static_cast<int64_t>(row) * heads + h) * dim + d0;
+    const int64_t angle = static_cast<int64_t>(row) * dim + d0;
+    Vec16<T> lo, hi;
+    lo.load(src);
+    hi.load(src + half);
+    T* dst;
+    if (h < q_heads)
+      dst = q_out + ((static_cast<int64_t>(b) * q_heads + h) * tokens + t) * dim;
+    else if (h < q_heads + kv_heads)
+      dst = keys + ((b * capacity + t) * kv_heads + h - q_heads) * dim;
+    else
+      dst = values + ((b * capacity + t) * kv_heads + h - q_heads - kv_heads) * dim;
+    if (h < q_heads + kv_heads) {
+      Vec16<T> clo, chi, slo, shi;
+      clo.load(cosine + angle);
+      chi.load(cosine + angle + half);
+      slo.load(sine + angle);
+      shi.load(sine + angle + half);
+#pragma unroll
+      for (int e = 0; e < static_cast<int>(per); ++e) {
+        const float x = lo.v[e], y = hi.v[e];
+        rope_pair<T>(x, y, clo.v[e], chi.v[e], slo.v[e], shi.v[e], lo.v[e], hi.v[e]);
+      }
+    }
+    lo.store(dst + d0);
+    hi.store(dst + half + d0);
+  }
 }
 
 // Decode fusion: one launch rotates q, rotates k into the K buffer and copies v into
@@ -565,6 +612,32 @@ __global__ void argmax_kernel(const T* __restrict__ logits, int64_t* __restrict_
 }
 
 }  // namespace
+}  // namespace b200
+
+namespace b200 {
+int rope_into_cache(const void* qkv, const void* cosine, const void* sine, void* q_out, void* keys, void* values,
+                    int64_t batch, int64_t tokens, int64_t q_heads, int64_t kv_heads, int64_t head_dim, int64_t capacity,
+                    int dtype, cudaStream_t stream) {
+  int code = B200_ERR_UNSUPPORTED;
+  for (const void* p : {qkv, cosine, sine, static_cast<const void*>(q_out), static_cast<const void*>(keys),
+                        static_cast<const void*>(values)})
+    if (!aligned16(p)) return code;
+  with_element_type(dtype, [&](auto tag) {
+    using T = typename decltype(tag)::type;
+    constexpr int per = Elem<T>::kPerVec;
+    if (head_dim % (2 * per) != 0) return;
+    const int64_t total = batch * tokens * (q_heads + 2 * kv_heads) * (head_dim / 2 / per);
+    const int grid = grid_for(total);
+    if (total + static_cast<int64_t>(grid) * kThreads >= (int64_t(1) << 32)) return;  // (32-bit indices)
+    code = launch_chained(rope_into_cache_kernel<T>, dim3(grid), dim3(kThreads), 0, stream, static_cast<const T*>(qkv),
+                          static_cast<const T*>(cosine), static_cast<const T*>(sine), static_cast<T*>(q_out),
+                          static_cast<T*>(keys), static_cast<T*>(values), static_cast<uint32_t>(total),
+                          static_cast<uint32_t>(tokens), static_cast<uint32_t>(q_heads), static_cast<uint32_t>(kv_heads),
+                          static_cast<uint32_t>(head_dim), capacity) == cudaSuccess
+               ? launch_status() : B200_ERR_LAUNCH;
+  });
+  return code;
+}
 }  // namespace b200
 
 using namespace b200;

@@ -40,15 +40,19 @@ __device__ __forceinline__ void finish_pair(float x0, float x1, float inv_rms, f
 constexpr int kMaxCached = 4;  // 16-byte chunks a thread keeps in registers
 
 template <typename T, bool kVector>
-__global__ void rms_norm_fast_kernel(const T* __restrict__ input, const T* __restrict__ weight,
-                                     T* __restrict__ output, int64_t hidden, int64_t row_stride,
+__global__ void rms_norm_fast_kernel(const T* input, const T* weight, T* output, int64_t hidden, int64_t row_stride,
                                      float epsilon, bool round_before_weight) {
   constexpr int per = kVector ? Elem<T>::kPerVec : 1;
+  // What follows may start once the kernel in front has finished: it may take tensor memory that one still needs.
+  // (No __restrict__: nothing may be read ahead of the wait. The weight is read with the row, one latency for both.)
+  grid_dependency_wait();
+  grid_launch_dependents();
   const T* row = input + blockIdx.x * row_stride;
   T* out = output + blockIdx.x * hidden;
   const int64_t chunks = hidden / per;
 
   float cache[kMaxCached][per];
+  Vec16<T> w[kMaxCached];
   float sum = 0.0f;
 #pragma unroll
   for (int i = 0; i < kMaxCached; ++i) {
@@ -57,6 +61,7 @@ __global__ void rms_norm_fast_kernel(const T* __restrict__ input, const T* __res
       if (kVector) {
         Vec16<T> v;
         v.load(row + c * per);
+        w[i].load(weight + c * per);
 #pragma unroll
         for (int j = 0; j < per; ++j) {
           cache[i][j] = v.v[j];
@@ -97,11 +102,10 @@ __global__ void rms_norm_fast_kernel(const T* __restrict__ input, const T* __res
     const int64_t c = threadIdx.x + static_cast<int64_t>(i) * blockDim.x;
     if (c < chunks) {
       if (kVector) {
-        Vec16<T> w, y;
-        w.load(weight + c * per);
+        Vec16<T> y;
 #pragma unroll
         for (int j = 0; j < per; j += 2)
-          finish_pair<T>(cache[i][j], cache[i][j + 1], inv_rms, w.v[j], w.v[j + 1], round_before_weight,
+          finish_pair<T>(cache[i][j], cache[i][j + 1], inv_rms, w[i].v[j], w[i].v[j + 1], round_before_weight,
                          y.v[j], y.v[j + 1]);
         y.store(out + c * per);
       } else {
@@ -131,10 +135,12 @@ constexpr int kRowsPerBlock = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(kRowsPerBlock * 32)
-rms_norm_rows_kernel(const T* __restrict__ input, const T* __restrict__ weight, T* __restrict__ output,
+rms_norm_rows_kernel(const T* input, const T* weight, T* output,
                      int64_t rows, int64_t hidden, int64_t row_stride, float epsilon,
                      bool round_before_weight) {
   constexpr int per = Elem<T>::kPerVec;
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int64_t r = static_cast<int64_t>(blockIdx.x) * kRowsPerBlock + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -143,6 +149,7 @@ rms_norm_rows_kernel(const T* __restrict__ input, const T* __restrict__ weight, 
   const int chunks = static_cast<int>(hidden / per);  // at most 32 * kMaxCached
 
   float cache[kMaxCached][per];
+  Vec16<T> w[kMaxCached];
   float sum = 0.0f;
 #pragma unroll
   for (int i = 0; i < kMaxCached; ++i) {
@@ -150,6 +157,7 @@ rms_norm_rows_kernel(const T* __restrict__ input, const T* __restrict__ weight, 
     if (c < chunks) {
       Vec16<T> v;
       v.load(row + c * per);
+      w[i].load(weight + c * per);
 #pragma unroll
       for (int j = 0; j < per; ++j) {
         cache[i][j] = v.v[j];
@@ -163,11 +171,10 @@ rms_norm_rows_kernel(const T* __restrict__ input, const T* __restrict__ weight, 
   for (int i = 0; i < kMaxCached; ++i) {
     const int c = lane + i * 32;
     if (c < chunks) {
-      Vec16<T> w, y;
-      w.load(weight + c * per);
+      Vec16<T> y;
 #pragma unroll
       for (int j = 0; j < per; j += 2)
-        finish_pair<T>(cache[i][j], cache[i][j + 1], inv_rms, w.v[j], w.v[j + 1], round_before_weight,
+        finish_pair<T>(cache[i][j], cache[i][j + 1], inv_rms, w[i].v[j], w[i].v[j + 1], round_before_weight,
                        y.v[j], y.v[j + 1]);
       y.store(out + c * per);
     }
@@ -278,17 +285,12 @@ int rms_norm_typed(const void* input, const void* weight, void* output, int64_t 
   if (threads < 32) threads = 32;
   if (vec && chunks <= 32 * kMaxCached && rows >= 4 * kNumSMs * kRowsPerBlock) {
     const int grid = static_cast<int>(ceil_div(rows, kRowsPerBlock));
-    rms_norm_rows_kernel<T><<<grid, kRowsPerBlock * 32, 0, stream>>>(x, w, y, rows, hidden, row_stride,
-                                                                   epsilon, rbw);
-    return launch_status();
+    return launch_chained(rms_norm_rows_kernel<T>, dim3(grid), dim3(kRowsPerBlock * 32), 0, stream, x, w, y, rows, hidden,
+                          row_stride, epsilon, rbw) == cudaSuccess ? launch_status() : B200_ERR_LAUNCH;
   }
-  if (vec)
-    rms_norm_fast_kernel<T, true><<<static_cast<int>(rows), threads, 0, stream>>>(
-        x, w, y, hidden, row_stride, epsilon, rbw);
-  else
-    rms_norm_fast_kernel<T, false><<<static_cast<int>(rows), threads, 0, stream>>>(
-        x, w, y, hidden, row_stride, epsilon, rbw);
-  return launch_status();
+  auto kernel = vec ? rms_norm_fast_kernel<T, true> : rms_norm_fast_kernel<T, false>;
+  return launch_chained(kernel, dim3(static_cast<unsigned>(rows)), dim3(static_cast<unsigned>(threads)), 0, stream, x, w, y,
+                        hidden, row_stride, epsilon, rbw) == cudaSuccess ? launch_status() : B200_ERR_LAUNCH;
 }
 
 }  // namespace

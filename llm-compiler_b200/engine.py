@@ -279,31 +279,12 @@ class Qwen2Engine(ServingEngine):
         position_ids = torch.arange(tokens, dtype=torch.int64, device=self.device).repeat(batch, 1)
         x = kernels.b200_embedding(self.embed, ids)
         cosine, sine = kernels.b200_rope_table(position_ids, self.inv_freq, self.dtype)
-        zeros = self.positions  # all zero right now
-        q_size, kv_size = cfg.q_size, cfg.kv_size
-        for index, layer in enumerate(self.layers):
-            h = kernels.b200_rms_norm(x, layer["input_norm"], epsilon=cfg.rms_norm_eps,
-                                      round_before_weight=True, numerical_mode=self.mode)
-            qkv = kernels.b200_linear(h, layer["qkv_w"], layer["qkv_b"])
-            q = qkv[..., :q_size].view(batch, tokens, cfg.num_heads, cfg.head_dim).transpose(1, 2)
-            k = qkv[..., q_size:q_size + kv_size].view(batch, tokens, cfg.num_kv_heads,
-                                                       cfg.head_dim).transpose(1, 2)
-            v = qkv[..., q_size + kv_size:].view(batch, tokens, cfg.num_kv_heads,
-                                                 cfg.head_dim).transpose(1, 2)
-            q, k = kernels.b200_rope(q, k, cosine, sine)
-            if self.paged:
-                kernels.b200_paged_kv_store(self.state.keys[index], self.state.values[index],
-                                            self.state.block_table, k, v, zeros)
-            else:
-                kernels.b200_kv_store(self.state.keys[index], self.state.values[index], k, v, zeros)
-            attn = kernels.b200_prefill_attention(q, k, v, None, scale=self.scale, causal=True,
-                                                  numerical_mode=self.mode)
-            attn = attn.transpose(1, 2).reshape(batch, tokens, q_size)  # a view: memory is B,T,H,D
-            x = kernels.b200_linear(attn, layer["o_w"], residual=x, epilogue="residual")
-            h = kernels.b200_rms_norm(x, layer["post_norm"], epsilon=cfg.rms_norm_eps,
-                                      round_before_weight=True, numerical_mode=self.mode)
-            a = kernels.b200_linear(h, layer["gate_up_w"], epilogue="swiglu")
-            x = kernels.b200_linear(a, layer["down_w"], residual=x, epilogue="residual")
+        # (the launches above are fully serialised, so that the layers' weights may be read ahead)
+        with kernels.launch_mode(programmatic=self.programmatic_launch, constant_weights=self.programmatic_launch):
+            x = kernels.b200_qwen2_prompt_layers(
+                x, self.layers, self.state.keys, self.state.values, cosine, sine, self.positions,  # all zero right now
+                q_heads=cfg.num_heads, scale=self.scale, epsilon=cfg.rms_norm_eps, numerical_mode=self.mode,
+                block_table=self.state.block_table if self.paged else None)
         if all_logits:
             h = kernels.b200_rms_norm(x, self.final_norm, epsilon=cfg.rms_norm_eps,
                                       round_before_weight=True, numerical_mode=self.mode)

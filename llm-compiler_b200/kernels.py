@@ -11,6 +11,7 @@ libb200serve.so, and a missing library or a CPU tensor is an error, never a fall
 from __future__ import annotations
 
 import contextlib
+import ctypes
 import math
 from typing import Optional, Tuple
 
@@ -197,7 +198,8 @@ def _mode(numerical_mode: str) -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # (the raw handle: building a torch.cuda.Stream around it costs 3 us a launch)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _check(code: int, what: str) -> None:
@@ -907,6 +909,65 @@ def b200_linear(tensor: torch.Tensor, weight: torch.Tensor,
     _check(code, "b200_linear")
     _count(rt)
     return output
+
+
+def b200_qwen2_prompt_layers(x: torch.Tensor, layers, keys, values, cosine: torch.Tensor, sine: torch.Tensor,
+                             positions: torch.Tensor, *, q_heads: int, scale: float, epsilon: float,
+                             numerical_mode: str = "fast", block_table: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """All layers of a Qwen2 prompt from empty caches, issued by one native call (the operators' own entry points in
+    the order of qwen2.py:236-304). x: B x T x hidden, dense, updated in place and returned; layers: the packed weights
+    of Qwen2Engine; keys / values: each layer's buffers [B, capacity, kv_heads, head_dim], or with `block_table` its
+    block pools; positions: B zeros."""
+
+    device = _require_cuda(x, cosine, sine, positions, block_table, *keys, *values)
+    batch, tokens, hidden = x.shape
+    _, capacity, kv_heads, dim = keys[0].shape
+    rows, q_size, width = batch * tokens, q_heads * dim, (q_heads + 2 * kv_heads) * dim
+    intermediate = layers[0]["down_w"].shape[1]
+    pool = [0, 0, 0]
+    if block_table is not None:
+        pool = [keys[0].shape[0], capacity, block_table.shape[1]]
+        capacity = pool[1] * pool[2]
+    names = ("input_norm", "qkv_w", "qkv_b", "o_w", "post_norm", "gate_up_w", "down_w")
+    shapes = dict(input_norm=(hidden,), qkv_w=(width, hidden), qkv_b=(width,), o_w=(hidden, q_size), post_norm=(hidden,),
+                  gate_up_w=(2 * intermediate, hidden), down_w=(hidden, intermediate))
+    table = (_lib.PromptLayer * len(layers))()
+    kept = []  # (dense copies of weights that a caller handed over as views)
+    for entry, layer, layer_keys, layer_values in zip(table, layers, keys, values):
+        operands = [layer[name] for name in names]
+        for name, operand in zip(names, operands):
+            if operand.shape != shapes[name] or operand.dtype != x.dtype:
+                raise ValueError(f"{name} must have shape {shapes[name]} and the input's dtype")
+        operands = [_dense(operand) for operand in operands]
+        kept.append(operands)
+        for buffer in (layer_keys, layer_values):
+            if buffer.shape != keys[0].shape or buffer.dtype != x.dtype or not buffer.is_contiguous():
+                raise ValueError("KV buffers must be contiguous tensors of one shape in the input's dtype")
+        (entry.input_norm, entry.qkv_weight, entry.qkv_bias, entry.o_weight, entry.post_norm, entry.gate_up_weight,
+         entry.down_weight) = (operand.data_ptr() for operand in operands)
+        entry.keys, entry.values = layer_keys.data_ptr(), layer_values.data_ptr()
+    if not x.is_contiguous() or tokens > capacity or positions.shape != (batch,) or positions.dtype != torch.int64 or \
+            (block_table is None and keys[0].shape[0] != batch):
+        raise ValueError("prompt rows must be dense and fit the KV buffers")
+    if cosine.shape != (batch, tokens, dim) or sine.shape != (batch, tokens, dim) or \
+            not (cosine.is_contiguous() and sine.is_contiguous() and cosine.dtype == sine.dtype == x.dtype):
+        raise ValueError("cosine/sine must be contiguous B x T x D tensors in the input's dtype")
+    rt, library, code_dtype = runtime(device), _lib.load(), _code(x.dtype)
+    need = max(int(library.b200_linear_workspace_bytes(rows, k, n, code_dtype, epilogue)) for k, n, epilogue in
+               ((hidden, width, _lib.EPILOGUE_NONE), (q_size, hidden, _lib.EPILOGUE_RESIDUAL),
+                (hidden, 2 * intermediate, _lib.EPILOGUE_SWIGLU), (intermediate, hidden, _lib.EPILOGUE_RESIDUAL)))
+    scratch = [torch.empty((rows, columns), dtype=x.dtype, device=device)
+               for columns in (hidden, hidden, width, q_size, kv_heads * dim, q_size, intermediate)]
+    call = _lib.PromptCall(
+        x.data_ptr(), *(buffer.data_ptr() for buffer in scratch), cosine.data_ptr(), sine.data_ptr(),
+        positions.data_ptr(), _ptr(block_table), _ptr(rt.workspace("linear", need)), need, batch, tokens, q_heads, kv_heads,
+        dim, hidden, intermediate, capacity, *pool, float(epsilon), float(scale), code_dtype, _mode(numerical_mode))
+    code = library.b200_qwen2_prompt_layers(table, len(layers), ctypes.byref(call), rt.status.data_ptr(), _stream())
+    _check(code, "b200_qwen2_prompt_layers")
+    # norms, projections, attention, RoPE with the KV store (apart where rows have no 16-byte pieces or blocks)
+    fused = block_table is None and dim % (32 // x.element_size()) == 0
+    _count(rt, (8 if fused else 9) * len(layers))
+    return x
 
 
 def linear_partial_splits(m: int, k: int, n: int) -> int:

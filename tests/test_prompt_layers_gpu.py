@@ -1,0 +1,54 @@
+"""The native prompt loop (csrc/prompt_layers.cu) against its operators called one by one: the same launches but for RoPE
+and KV store in one kernel, whose roundings are the same, so every result is equal bit for bit."""
+
+import pytest
+import torch
+
+from llm_compiler_b200 import kernels, qwen2
+from llm_compiler_b200.engine import Qwen2Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _operator_by_operator(engine, ids):
+    cfg = engine.config
+    batch, tokens = ids.shape
+    x = kernels.b200_embedding(engine.embed, ids.cuda())
+    positions = torch.arange(tokens, device="cuda").repeat(batch, 1)
+    cosine, sine = kernels.b200_rope_table(positions, engine.inv_freq, engine.dtype)
+    norm = dict(epsilon=cfg.rms_norm_eps, round_before_weight=True, numerical_mode=engine.mode)
+    cached = []
+    for layer in engine.layers:
+        qkv = kernels.b200_linear(kernels.b200_rms_norm(x, layer["input_norm"], **norm), layer["qkv_w"], layer["qkv_b"])
+        q, k, v = (part.view(batch, tokens, -1, cfg.head_dim).transpose(1, 2)
+                   for part in qkv.split([cfg.q_size, cfg.kv_size, cfg.kv_size], dim=-1))
+        q, k = kernels.b200_rope(q, k, cosine, sine)
+        cached.append((k.transpose(1, 2), v.transpose(1, 2)))
+        mixed = kernels.b200_prefill_attention(q, k, v, None, scale=engine.scale, causal=True, numerical_mode=engine.mode)
+        x = kernels.b200_linear(mixed.transpose(1, 2).reshape(batch, tokens, -1), layer["o_w"], residual=x, epilogue="residual")
+        gated = kernels.b200_linear(kernels.b200_rms_norm(x, layer["post_norm"], **norm), layer["gate_up_w"], epilogue="swiglu")
+        x = kernels.b200_linear(gated, layer["down_w"], residual=x, epilogue="residual")
+    return kernels.b200_linear(kernels.b200_rms_norm(x[:, -1], engine.final_norm, **norm), engine.lm_head), cached
+
+
+@pytest.mark.parametrize("dtype,heads,kv_heads,dim,layout,mode", [
+    (torch.bfloat16, 14, 2, 64, "contiguous", "fast"), (torch.bfloat16, 6, 3, 128, "contiguous", "fast"),
+    (torch.bfloat16, 14, 2, 64, "paged", "fast"), (torch.bfloat16, 4, 2, 64, "contiguous", "pytorch_compatible"),
+    (torch.float16, 14, 2, 64, "contiguous", "fast"), (torch.float32, 4, 4, 32, "contiguous", "fast"),
+    (torch.bfloat16, 4, 2, 16, "contiguous", "fast"), (torch.float32, 2, 1, 256, "contiguous", "fast")])
+@pytest.mark.parametrize("batch,tokens", [(1, 1), (3, 9), (1, 130), (2, 600)])
+def test_equals_the_operators_one_by_one(dtype, heads, kv_heads, dim, layout, mode, batch, tokens):
+    config = qwen2.Qwen2Config(hidden_size=heads * dim, intermediate_size=3 * heads * dim, num_layers=3, num_heads=heads,
+                               num_kv_heads=kv_heads, vocab_size=1000)
+    weights = qwen2.make_weights(config, seed=tokens, dtype=dtype, device="cuda", reproducible=False)
+    engine = Qwen2Engine(config, weights, batch=batch, capacity=640, kv_layout=layout, numerical_mode=mode)
+    ids = torch.randint(0, 1000, (batch, tokens), generator=torch.Generator().manual_seed(batch))
+    expected, cached = _operator_by_operator(engine, ids)
+    for _ in range(2):  # (the second prompt runs on used caches)
+        assert torch.equal(engine.prefill(ids), expected)
+        for layer, (keys, values) in enumerate(cached):
+            for buffer, rows in ((engine.state.keys[layer], keys), (engine.state.values[layer], values)):
+                for b in range(batch):
+                    stored = buffer[b] if layout == "contiguous" else buffer[engine.state.block_table[b].long()].flatten(0, 1)
+                    assert torch.equal(stored[:tokens], rows[b])
+    kernels.runtime().check_status()
