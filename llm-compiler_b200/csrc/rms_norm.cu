@@ -149,7 +149,6 @@ rms_norm_rows_kernel(const T* input, const T* weight, T* output,
   const int chunks = static_cast<int>(hidden / per);  // at most 32 * kMaxCached
 
   float cache[kMaxCached][per];
-  Vec16<T> w[kMaxCached];
   float sum = 0.0f;
 #pragma unroll
   for (int i = 0; i < kMaxCached; ++i) {
@@ -157,7 +156,6 @@ rms_norm_rows_kernel(const T* input, const T* weight, T* output,
     if (c < chunks) {
       Vec16<T> v;
       v.load(row + c * per);
-      w[i].load(weight + c * per);
 #pragma unroll
       for (int j = 0; j < per; ++j) {
         cache[i][j] = v.v[j];
@@ -171,10 +169,11 @@ rms_norm_rows_kernel(const T* input, const T* weight, T* output,
   for (int i = 0; i < kMaxCached; ++i) {
     const int c = lane + i * 32;
     if (c < chunks) {
-      Vec16<T> y;
+      Vec16<T> w, y;
+      w.load(weight + c * per);
 #pragma unroll
       for (int j = 0; j < per; j += 2)
-        finish_pair<T>(cache[i][j], cache[i][j + 1], inv_rms, w[i].v[j], w[i].v[j + 1], round_before_weight,
+        finish_pair<T>(cache[i][j], cache[i][j + 1], inv_rms, w.v[j], w.v[j + 1], round_before_weight,
                        y.v[j], y.v[j + 1]);
       y.store(out + c * per);
     }

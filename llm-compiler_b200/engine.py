@@ -279,8 +279,10 @@ class Qwen2Engine(ServingEngine):
         position_ids = torch.arange(tokens, dtype=torch.int64, device=self.device).repeat(batch, 1)
         x = kernels.b200_embedding(self.embed, ids)
         cosine, sine = kernels.b200_rope_table(position_ids, self.inv_freq, self.dtype)
-        # (the launches above are fully serialised, so that the layers' weights may be read ahead)
-        with kernels.launch_mode(programmatic=self.programmatic_launch, constant_weights=self.programmatic_launch):
+        # (The launches above are fully serialised, so that the layers' weights may be read ahead. Long prompts have
+        # nothing to hide between launches of 100 us, and waiting CTAs of the next one cost them 1 %: 4 x 4096 tokens.)
+        chained = self.programmatic_launch and batch * tokens <= 4096
+        with kernels.launch_mode(programmatic=chained, constant_weights=chained):
             x = kernels.b200_qwen2_prompt_layers(
                 x, self.layers, self.state.keys, self.state.values, cosine, sine, self.positions,  # all zero right now
                 q_heads=cfg.num_heads, scale=self.scale, epsilon=cfg.rms_norm_eps, numerical_mode=self.mode,
