@@ -1057,6 +1057,8 @@ __global__ void __launch_bounds__(kSplitThreads) decode_attention_split_kernel(c
   const int kvh = unit / blocks, head0 = unit % blocks * kSplitHeads;
   const int heads = min(kSplitHeads, p.groups - head0), hq = kvh * p.groups + head0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  grid_launch_dependents();
   int64_t len = p.lengths[b];
   if (len > p.mask_len) {
     if (threadIdx.x == 0 && blockIdx.x == 0 && p.status != nullptr) atomicOr(p.status, B200_STATUS_LENGTH_OVER_MASK);
@@ -1198,17 +1200,10 @@ int launch_split(SplitParams<T> p, int64_t batch, int64_t max_length, cudaStream
   p.splits = splits;
   const int64_t head_units = p.kv_heads * ceil_div(p.groups, kSplitHeads);
   if (head_units * splits > INT32_MAX) return B200_ERR_TOO_LARGE;
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(static_cast<unsigned>(head_units * splits), static_cast<unsigned>(batch));
-  config.blockDim = dim3(kSplitThreads);
-  config.stream = stream;
-  cudaLaunchAttribute attribute;
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = static_cast<unsigned>(splits);
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  if (cudaLaunchKernelEx(&config, decode_attention_split_kernel<D, T>, p) != cudaSuccess) return B200_ERR_LAUNCH;
+  if (launch_chained_cluster(decode_attention_split_kernel<D, T>,
+                             dim3(static_cast<unsigned>(head_units * splits), static_cast<unsigned>(batch)),
+                             dim3(kSplitThreads), 0, stream, static_cast<unsigned>(splits), p) != cudaSuccess)
+    return B200_ERR_LAUNCH;
   return launch_status();
 }
 

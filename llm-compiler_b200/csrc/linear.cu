@@ -240,60 +240,128 @@ __device__ __forceinline__ void epilogue_generic(const LinearParamsGeneric<T>& p
   Elem<T>::store(p.out + o, v0);
 }
 
-// fp32, up to 8 rows of x per CTA: bound by reading W once. A warp holds 4 rows of W against all rows of x, its lanes
-// side by side along K in 16-byte loads; KSPLIT warps of the CTA share the K range of the same 4 rows and add their
-// sums in warp order, so that a projection of few columns still puts enough loads in flight. x comes out of L1. The
-// sums are short chains joined by a tree (K / (32 KSPLIT) terms a lane), below the error of the tiled kernel's order.
-// Qwen2-0.5B decode step, 4 rows: 318 us a projection in 64 x 64 tiles (60 idle rows, one serial K loop per CTA)
-// -> 10.0 us on average.
-constexpr int kRowsThreads = 256, kRowsColumns = 4, kRowsOfX = 8;
+// fp32, up to 8 rows of x per CTA: bound by reading W once, and in a chain of launches by the time until W flows. As in
+// linear_rows.cu W travels as early as it can (before the dependency wait, where the caller promises constant weights):
+// every lane copies the pieces that it will multiply (cp.async) into a ring of its own, 8 columns x 4 k of a chunk of
+// 128 k, so that many CTAs with few registers keep their loads in flight and the main loop has no barrier. The warps of
+// a CTA (and, with few columns, of a cluster) share the K range; x comes out of L1. The sums are short chains
+// (4 K / 128 / warps terms a lane) joined by a tree of exchanges in which every lane ends up with one output.
+// Qwen2-0.5B decode step, 4 rows: 9728 x 896 16.1 us with W in registers behind the launch, 896 x 4864 9.2, LM head 128.
+constexpr int kRowsWarps = 4, kRowsThreads = kRowsWarps * 32, kRowsColumns = 8, kRowsOfX = 8, kRowsRing = 4;
+constexpr int kRowsChunk = 128, kRowsChunkBytes = kRowsColumns * 512;  // k, and bytes of a warp's piece of W
 
-template <int KSPLIT>
-__global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearParamsGeneric<float> p) {
-  constexpr int kGroups = kRowsThreads / 32 / KSPLIT;  // groups of 4 columns in a CTA
-  __shared__ float sums[kRowsThreads / 32][kRowsOfX * kRowsColumns];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * kGroups + warp / KSPLIT) * kRowsColumns, slice = warp % KSPLIT;
-  const int m0 = blockIdx.y * kRowsOfX, rows = min(kRowsOfX, p.m - m0);
-  float acc[kRowsOfX][kRowsColumns] = {};
-  const float* w[kRowsColumns];
+// Lane i's return value: the sum over the lanes of their v[i].
+__device__ __forceinline__ float sum_transposed(float (&v)[32], int lane) {
 #pragma unroll
-  for (int j = 0; j < kRowsColumns; ++j) w[j] = p.w + static_cast<int64_t>(min(n0 + j, p.n - 1)) * p.k;
-  const float* x = p.x + m0 * p.x_row_stride;
-#pragma unroll 4
-  for (int k = (slice * 32 + lane) * 4; k < p.k; k += KSPLIT * 128) {
-    float4 wv[kRowsColumns];
+  for (int s = 16; s >= 1; s >>= 1) {
+    const bool upper = (lane & s) != 0;
 #pragma unroll
-    for (int j = 0; j < kRowsColumns; ++j) wv[j] = __ldg(reinterpret_cast<const float4*>(w[j] + k));
-#pragma unroll
-    for (int i = 0; i < kRowsOfX; ++i) {
-      if (i >= rows) break;
-      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + i * p.x_row_stride + k));
-#pragma unroll
-      for (int j = 0; j < kRowsColumns; ++j)
-        acc[i][j] = fmaf(xv.w, wv[j].w, fmaf(xv.z, wv[j].z, fmaf(xv.y, wv[j].y, fmaf(xv.x, wv[j].x, acc[i][j]))));
+    for (int i = 0; i < s; ++i) {
+      const float given = upper ? v[i] : v[i + s], kept = upper ? v[i + s] : v[i];
+      v[i] = kept + __shfl_xor_sync(0xffffffffu, given, s);
     }
   }
+  return v[0];
+}
+
+// ROWS: rows of x a CTA takes (4 or 8)
+template <int ROWS>
+__global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearParamsGeneric<float> p, int slots, int early) {
+  extern __shared__ __align__(16) unsigned char rows_ring[];  // [warp][chunk][column][lane]
+  constexpr int kOutputs = ROWS * kRowsColumns;
+  __shared__ float part[kRowsWarps][kOutputs];
+  __shared__ float total[kOutputs];
+  grid_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * kRowsColumns, m0 = blockIdx.y * ROWS, rows = min(ROWS, p.m - m0);
+  const int splits = gridDim.z, rank = blockIdx.z;
+  const int chunks = (p.k + kRowsChunk - 1) / kRowsChunk, parts = splits * kRowsWarps, mine = rank * kRowsWarps + warp;
+  const int first = static_cast<int>(static_cast<int64_t>(chunks) * mine / parts);
+  const int count = static_cast<int>(static_cast<int64_t>(chunks) * (mine + 1) / parts) - first;
+  const uint32_t base = smem_u32(rows_ring) + warp * slots * kRowsChunkBytes + lane * 16;
+  // (pieces beyond K become zeros; columns beyond N repeat the last one and are not stored)
+  auto copy = [&](int c) {
+    if (c >= count) return;
+    const int k = (first + c) * kRowsChunk + lane * 4;
+    const bool there = k < p.k;  // (K is a multiple of 4)
+    const uint32_t at = base + c % kRowsRing * kRowsChunkBytes;
 #pragma unroll
-  for (int i = 0; i < kRowsOfX; ++i) {
-    if (i >= rows) break;
+    for (int j = 0; j < kRowsColumns; ++j)
+      cp_async16_zfill(at + j * 512, p.w + static_cast<int64_t>(min(n0 + j, p.n - 1)) * p.k + (there ? k : 0), there ? 16 : 0);
+  };
+  if (!early) grid_dependency_wait();
+#pragma unroll
+  for (int c = 0; c < kRowsRing; ++c) {
+    copy(c);
+    cp_async_commit();
+  }
+  if (early) grid_dependency_wait();
+
+  float acc[ROWS][kRowsColumns] = {};
+  const float* x = p.x + m0 * p.x_row_stride;
+  for (int c = 0; c < count; ++c) {
+    const int k = (first + c) * kRowsChunk + lane * 4;
+    float4 xv[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      xv[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (i < rows && k < p.k)
+        asm volatile("ld.global.ca.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(xv[i].x), "=f"(xv[i].y), "=f"(xv[i].z), "=f"(xv[i].w)
+                     : "l"(x + i * p.x_row_stride + k) : "memory");
+    }
+    cp_async_wait<kRowsRing - 1>();
+    const uint32_t at = base + c % kRowsRing * kRowsChunkBytes;
 #pragma unroll
     for (int j = 0; j < kRowsColumns; ++j) {
-      const float sum = warp_sum(acc[i][j]);
-      if (lane == 0) sums[warp][i * kRowsColumns + j] = sum;
+      float4 w;
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(w.x), "=f"(w.y), "=f"(w.z), "=f"(w.w)
+                   : "r"(at + j * 512) : "memory");
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+        acc[i][j] = fmaf(xv[i].w, w.w, fmaf(xv[i].z, w.z, fmaf(xv[i].y, w.y, fmaf(xv[i].x, w.x, acc[i][j]))));
     }
+    copy(c + kRowsRing);  // (every lane refills the pieces that it has read itself)
+    cp_async_commit();
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int h = 0; h < kOutputs / 32; ++h) {
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = acc[(h * 32 + i) / kRowsColumns][i % kRowsColumns];
+    part[warp][h * 32 + lane] = sum_transposed(v, lane);
   }
   __syncthreads();
-  // one thread per output of the CTA's groups: 32 of them each, so at most all threads
-  const int group = threadIdx.x >> 5, item = threadIdx.x & 31, i = item / kRowsColumns, j = item % kRowsColumns;
-  if (group >= kGroups || i >= rows) return;
-  float v0 = 0.0f, v1 = 0.0f;
+  if (splits > 1) {
+    if (threadIdx.x < kOutputs) {
+      float sum = 0.0f;
 #pragma unroll
-  for (int s = 0; s < KSPLIT; ++s) {
-    v0 += sums[group * KSPLIT + s][item];
-    v1 += sums[group * KSPLIT + s][item ^ 1];
+      for (int s = 0; s < kRowsWarps; ++s) sum += part[s][threadIdx.x];
+      total[threadIdx.x] = sum;
+    }
+    cluster_sync();
   }
-  epilogue_generic(p, m0 + i, (blockIdx.x * kGroups + group) * kRowsColumns + j, v0, v1);
+  // pairs of neighbouring columns, dealt to the CTAs of the cluster; sums in warp and rank order
+  for (int u = rank + splits * threadIdx.x; u < kOutputs / 2; u += splits * kRowsThreads) {
+    const int i = u / (kRowsColumns / 2), c = u % (kRowsColumns / 2) * 2, at = i * kRowsColumns + c;
+    if (i >= rows) continue;
+    float v0 = 0.0f, v1 = 0.0f;
+    if (splits > 1) {
+      for (int s = 0; s < splits; ++s) {
+        v0 += load_cluster_f32(smem_u32(&total[at]), s);
+        v1 += load_cluster_f32(smem_u32(&total[at + 1]), s);
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < kRowsWarps; ++s) {
+        v0 += part[s][at];
+        v1 += part[s][at + 1];
+      }
+    }
+    epilogue_generic(p, m0 + i, n0 + c, v0, v1);
+    epilogue_generic(p, m0 + i, n0 + c + 1, v1, 0.0f);
+  }
+  if (splits > 1) cluster_sync();  // no CTA leaves while another reads its sums
 }
 
 // Tiled product: 64 x 64 outputs a CTA, 4 x 8 a thread, K in blocks of 16 whose sums are added to the accumulators
@@ -502,11 +570,24 @@ extern "C" int64_t b200_linear_workspace_bytes(int64_t m, int64_t k, int64_t n, 
 // against 32 us.
 constexpr int64_t kRowsLimit = 16;
 
-template <int KSPLIT>
-static void launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
-  constexpr int kColumns = kRowsThreads / 32 / KSPLIT * kRowsColumns;
-  dim3 grid(static_cast<unsigned>(ceil_div(p.n, kColumns)), static_cast<unsigned>(ceil_div(p.m, kRowsOfX)));
-  linear_rows_kernel<KSPLIT><<<grid, kRowsThreads, 0, s>>>(p);
+template <int ROWS>
+static int launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
+  // with few columns as many CTAs of a cluster along K as it takes to hold W in one ring each, up to some eight an SM
+  const int64_t groups = ceil_div(p.n, kRowsColumns), tall = ceil_div(p.m, ROWS), chunks = ceil_div(p.k, kRowsChunk);
+  int64_t splits = ceil_div(chunks, kRowsWarps * kRowsRing);
+  if (splits > 8 * kNumSMs / (groups * tall)) splits = 8 * kNumSMs / (groups * tall);
+  if (splits > 8) splits = 8;
+  if (splits < 1) splits = 1;
+  const int64_t most = ceil_div(chunks, kRowsWarps * splits);
+  const int slots = static_cast<int>(most < kRowsRing ? most : kRowsRing), smem = kRowsWarps * slots * kRowsChunkBytes;
+  if (cudaFuncSetAttribute(linear_rows_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kRowsWarps * kRowsRing * kRowsChunkBytes) != cudaSuccess)
+    return B200_ERR_LAUNCH;
+  const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(tall), static_cast<unsigned>(splits));
+  const int early = (launch_mode() & B200_LAUNCH_CONSTANT_WEIGHTS) != 0 ? 1 : 0;
+  return launch_chained_cluster_xz(linear_rows_kernel<ROWS>, grid, dim3(kRowsThreads), static_cast<size_t>(smem), s, 1u,
+                                   static_cast<unsigned>(splits), p, slots, early) == cudaSuccess
+             ? launch_status() : B200_ERR_LAUNCH;
 }
 
 template <typename T>
@@ -526,15 +607,7 @@ static int linear_generic(const void* input, const void* weight, const void* bia
   bool vec = false;
   if constexpr (sizeof(T) == 4) {
     vec = k % 4 == 0 && input_row_stride % 4 == 0 && aligned16(input) && aligned16(weight);
-    if (vec && m <= kRowsLimit) {
-      // K over as many warps as still leave each some 4 loads per lane, fewer where the columns alone fill the GPU
-      const int64_t warps = ceil_div(n, kRowsColumns) * ceil_div(m, kRowsOfX);
-      if (warps >= 32 * kNumSMs || k <= 256) launch_rows<1>(p, s);
-      else if (warps >= 16 * kNumSMs || k <= 512) launch_rows<2>(p, s);
-      else if (warps >= 8 * kNumSMs || k <= 1024) launch_rows<4>(p, s);
-      else launch_rows<8>(p, s);
-      return launch_status();
-    }
+    if (vec && m <= kRowsLimit) return m <= 4 ? launch_rows<4>(p, s) : launch_rows<8>(p, s);
   }
   const int64_t tiles_m = ceil_div(m, kTile), tiles_n = ceil_div(n, kTile);
   if (tiles_m > 65535) return B200_ERR_TOO_LARGE;

@@ -280,15 +280,14 @@ rope_into_cache_kernel(const T* qkv, const T* cosine, const T* sine, T* q_out, T
 // Decode fusion: one launch rotates q, rotates k into the K buffer and copies v into
 // the V buffer at positions[b]. Vector path only (D/2 a multiple of the vector width).
 template <typename T>
-__global__ void rope_kv_store_kernel(const T* __restrict__ q, const T* __restrict__ k,
-                                     const T* __restrict__ v, const T* __restrict__ cosine,
-                                     const T* __restrict__ sine, T* __restrict__ q_out,
-                                     T* __restrict__ kbuf, T* __restrict__ vbuf,
-                                     const int64_t* __restrict__ positions, int64_t batch,
+__global__ void rope_kv_store_kernel(const T* q, const T* k, const T* v, const T* cosine, const T* sine, T* q_out,
+                                     T* kbuf, T* vbuf, const int64_t* positions, int64_t batch,
                                      int64_t q_heads, int64_t kv_heads, int64_t dim,
                                      int64_t capacity, int64_t qb, int64_t qh, int64_t kb,
                                      int64_t kh, int64_t vb, int64_t vh, int64_t cb,
                                      int32_t* status) {
+  grid_dependency_wait();  // (as in rope_into_cache_kernel)
+  grid_launch_dependents();
   constexpr int per = Elem<T>::kPerVec;
   const int64_t half = dim / 2;
   const int64_t chunks = half / per;
@@ -708,15 +707,18 @@ int b200_rope_kv_store(const void* query, const void* key, const void* value, co
   if (total == 0) return B200_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int grid = grid_for(total);
+  int code = B200_OK;
   with_element_type(dtype, [&](auto tag) {
     using T = typename decltype(tag)::type;
-    rope_kv_store_kernel<T><<<grid, kThreads, 0, s>>>(
-        static_cast<const T*>(query), static_cast<const T*>(key), static_cast<const T*>(value),
-        static_cast<const T*>(cosine), static_cast<const T*>(sine), static_cast<T*>(query_out),
-        static_cast<T*>(key_buffer), static_cast<T*>(value_buffer), positions, batch, q_heads,
-        kv_heads, head_dim, capacity, q_batch_stride, q_head_stride, k_batch_stride,
-        k_head_stride, v_batch_stride, v_head_stride, cos_batch_stride, status);
+    if (launch_chained(rope_kv_store_kernel<T>, dim3(grid), dim3(kThreads), 0, s, static_cast<const T*>(query),
+                       static_cast<const T*>(key), static_cast<const T*>(value), static_cast<const T*>(cosine),
+                       static_cast<const T*>(sine), static_cast<T*>(query_out), static_cast<T*>(key_buffer),
+                       static_cast<T*>(value_buffer), positions, batch, q_heads, kv_heads, head_dim, capacity,
+                       q_batch_stride, q_head_stride, k_batch_stride, k_head_stride, v_batch_stride, v_head_stride,
+                       cos_batch_stride, status) != cudaSuccess)
+      code = B200_ERR_LAUNCH;
   });
+  if (code != B200_OK) return code;
   return launch_status();
 }
 

@@ -373,8 +373,11 @@ class Qwen2Engine(ServingEngine):
     def _decode_step(self) -> None:
         if self.chained:
             self._decode_step_chain()
-        else:
+        elif self.dtype == torch.bfloat16:
             self._decode_step_separate()
+        else:  # (fp32, fp16: the norms, RoPE, attention and projections of few rows wait on the device)
+            with kernels.launch_mode(programmatic=self.programmatic_launch, constant_weights=self.programmatic_launch):
+                self._decode_step_separate()
 
     def _decode_step_chain(self) -> None:
         """Fast bf16 decode step: every small projection is a split-K partial-sum producer on
