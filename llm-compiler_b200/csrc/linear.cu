@@ -14,7 +14,6 @@
 #include <string.h>
 
 #include "common.cuh"
-#include "linear_rows.cuh"
 
 namespace b200 {
 namespace {
@@ -634,10 +633,6 @@ static int linear_tensor_core(const void* input, const void* weight, const void*
                               int epilogue, void* workspace, int64_t workspace_bytes, int32_t* status,
                               cudaStream_t s) {
   if (use_tcgen05(m)) {
-    if (takes_few_rows(m)) {
-      FewRowsCall c{input, weight, bias, residual, output, nullptr, nullptr, m, k, n, input_row_stride, epilogue};
-      return linear_few_rows(c, dtype, s);
-    }
     const int code = linear_tcgen05(input, weight, bias, residual, output, m, k, n, input_row_stride, dtype,
                                     epilogue, status, s);
     if (code != B200_ERR_UNSUPPORTED) return code;

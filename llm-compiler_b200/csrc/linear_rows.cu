@@ -2,20 +2,19 @@
 // 8, in every form that a decode step has: plain with bias / residual / SwiGLU, fp32 sums for the operator behind it,
 // folded RMSNorm.
 //
-// Bound by reading W once and, in a 0.5B model (2 - 17 MB a launch), by the chain launch -> x -> product -> sum ->
-// store. So W travels as early as it can, before the dependency wait, and what is behind the wait is short: one read
-// of x, a handful of warp-level products, one exchange between the warps and the store. Every warp has a K range of
-// its own and every lane a ring of 16-byte pieces that it alone fills (cp.async) and reads: shared memory as more
-// registers, so that the next launch's W finds room while this one is at work, and no barrier in the main loop. The
-// rows of W are the M side of m16n8k16 and the rows of x its N side. The order of k inside a product is free as long
-// as both operands share it: a lane takes 8 neighbouring k of its W rows and of its x row, the first half as one
-// product's fragment, the second half as the next one's.
+// Bound by the chain launch -> x -> product -> sum -> store: the matrices of a 0.5B model are 2 - 17 MB. The tcgen05
+// kernels' prologue, ring of tiles, tensor memory and cluster exchange cost 3.7 us there however small the matrix.
+// Here W travels as early as it can, before the dependency wait, and what is behind the wait is short: one read of x, a
+// chain of warp-level products, one exchange and the store. A warp takes 16 columns of y (the M side of m16n8k16; the
+// rows of x are its N side) and one K slice, and copies both operands into rings of its own: small CTAs with little
+// shared memory, so that the next launch's W finds room while this one is at work.
 //
-// Qwen2-0.5B on 1 row, launches in a chain, against the tcgen05 kernels (whose prologue, ring of tiles, tensor memory and
-// cluster exchange cost 3.7 us however small the matrix): q|k|v 3.7 -> 2.3 us, o 4.9 -> 2.5, gate|up 10.1 -> 4.7
-// (17.4 MB, 3.7 TB/s), down 7.2 -> 4.5, LM head 56 -> 55; 8 rows within 15 % of that. Decode step 935 -> 648 us (8
-// rows: 913 -> 688), four layers of the 7B 692 -> 628 (693 -> 667), Bazirax 1.5b 546 -> 431 (563 -> 454), Lozanex 1.5b
-// 511 -> 465 (745 -> 712).
+// Qwen2-0.5B on 1 row, launches in a chain: q|k|v 3.7 -> 2.7 us, o 4.9 -> 3.6, gate|up 10.1 -> 6.9, down 7.2 -> 5.4 (8
+// rows: 2.8, 3.8, 6.7, 5.5); the layer with its attention 34.3 -> 30.8 us.
+//
+// The sums are those of linear_tcgen05.cu bit for bit: the same K slices, each one chain of 16-deep products in K
+// order, slices and squares added in the same order. (The two kinds of tensor-core instruction round alike.) So a row's
+// result does not depend on how many rows stand beside it, and a token does not change with the kernel.
 #include <stdlib.h>
 
 #include "common.cuh"
@@ -24,12 +23,15 @@
 namespace b200 {
 namespace {
 
-constexpr int kChunk = 32;   // k of two products: 4 lanes x 8
-constexpr int kHalf = 4;     // chunks of half a ring: a copy group
-constexpr int kRows = 8;     // rows of x, the N side of a product
-constexpr int kColumns = 16; // columns of y of a CTA, the M side
-constexpr int kPieces = 2;   // 16-byte pieces of W of a lane and chunk
-constexpr int kWarps = 4, kThreads = kWarps * 32;
+constexpr int kRows = 8, kColumns = 16;
+constexpr int kBlock = 64;                             // k of a ring slot: 128-byte rows
+constexpr int kWBytes = kColumns * 128;
+constexpr int kPitch = kColumns + 4;                   // floats between rows of x in the exchange: conflict-free stores
+constexpr int kPartBytes = kRows * kPitch * 4;
+constexpr int kMaxSlices = 8;                          // warps of a CTA, CTAs of a cluster
+constexpr int kNormFloats = 2048;                      // norm slices x rows that a CTA takes in
+constexpr int kLongRing = 16, kShortRing = 4;          // slots of W of a warp
+__host__ __device__ constexpr int x_ring(int ring) { return ring < 8 ? ring : 8; }  // slots of x
 
 template <typename T>
 struct RowsParams {
@@ -38,213 +40,263 @@ struct RowsParams {
   const T* bias;
   const T* residual;
   T* out;
-  float* sums;         // fp32 sums instead of `out`
-  float* row_squares;  // and sum(x_r^2), written by the first CTA
+  float* sums;
+  float* row_squares;
+  float* squares_out;
+  const float* norm_squares;
   int64_t x_row_stride;
   int m, k, n, epilogue;
-  int fold_norm;
+  int splits, blocks_per_slice, warps;  // K slices, 64-k blocks of each, slices of a CTA
+  int tile_groups;                      // with squares_out: 16-column groups of a tile (the cluster along x)
+  int norm_slices, early;
+  int slots, x_slots;  // what the rings have room for: all of a slice if it is short
   float norm_eps;
-  int slots;  // chunks that a warp's ring has room for: 2 kHalf, or all that it has to multiply if fewer
-  int early;  // W may be read before the kernels in front have finished
 };
 
-// x by way of L1: all CTAs of an SM read the same few kilobytes, whose L2 slices would otherwise answer each of them
-// (gate|up on 8 rows: 6.5 us past L1, 5.3 us through it)
-__device__ __forceinline__ uint4 load_rows_of_x(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.ca.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
-}
-
-// as in the tcgen05 projections: a few ulp of fp32, far below the rounding that follows
+// as in linear_tcgen05.cu
 __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + exp2f(-1.4426950408889634f * x)); }
 
+// x by way of L1: all CTAs of an SM read the same few kilobytes, whose L2 slices would otherwise answer each of them
+__device__ __forceinline__ void copy_through_l1(uint32_t smem_addr, const void* p, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr), "l"(p), "r"(bytes));
+}
+__device__ __forceinline__ uint4 load_shared16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 template <typename T>
 __device__ __forceinline__ float square_pair(uint32_t pair, float sum) {
   const float a = Elem<T>::lo(pair), b = Elem<T>::hi(pair);
   return fmaf(b, b, fmaf(a, a, sum));
 }
 
-template <typename T, bool SQUARES>
-__global__ void __launch_bounds__(kThreads) linear_rows16_kernel(const RowsParams<T> p) {
-  constexpr int kPitch = kColumns + 4;  // conflict-free fragment stores
-  extern __shared__ __align__(16) unsigned char ring[];  // [warp][chunk][piece][lane]
-  __shared__ __align__(16) float part[kWarps][kRows][kPitch];
-  __shared__ float total[kRows][kColumns];
-  __shared__ float squares[kWarps][kRows];
-  __shared__ float total_squares[kRows];
+constexpr int kPlain = 0, kSquares = 1, kNorm = 2;  // HELPER: what the warp behind the multiplying ones does
+
+// RING: slots of a warp for blocks of W (and x_ring(RING) for blocks of x, which are near).
+template <typename T, int HELPER, int RING>
+__global__ void __launch_bounds__(kMaxSlices * 32) linear_rows16_kernel(const RowsParams<T> p) {
+  constexpr int kXRing = x_ring(RING);
+  extern __shared__ __align__(128) unsigned char ring[];  // per warp W, then per warp x, part, norm slices
+  __shared__ float unit_squares[kRows][kColumns / 4];
+  __shared__ float row_scale[kRows];
   grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * kColumns, splits = gridDim.z, rank = blockIdx.z;
-  const int chunks = (p.k + kChunk - 1) / kChunk, parts = splits * kWarps, mine = rank * kWarps + warp;
-  const int first = static_cast<int>(static_cast<int64_t>(chunks) * mine / parts);
-  const int count = static_cast<int>(static_cast<int64_t>(chunks) * (mine + 1) / parts) - first;
-  const uint32_t base = smem_u32(ring) + warp * (p.slots * kPieces * 512) + lane * 16;
+  const int n0 = blockIdx.x * kColumns;
+  const int slice = blockIdx.z * p.warps + warp;
+  const int all_blocks = (p.k + kBlock - 1) / kBlock, first = slice * p.blocks_per_slice;
+  const int count = warp < p.warps ? max(0, min(first + p.blocks_per_slice, all_blocks) - first) : 0;
+  const int x_bytes = p.m * 128;
+  const uint32_t w_base = smem_u32(ring) + warp * p.slots * kWBytes;
+  const uint32_t x_base = smem_u32(ring) + p.warps * p.slots * kWBytes + warp * p.x_slots * x_bytes;
+  float* parts = reinterpret_cast<float*>(ring + p.warps * (p.slots * kWBytes + p.x_slots * x_bytes));
+  auto part = [&](int s, int row, int c) { return parts + (s * kRows + row) * kPitch + c; };
+  float* norm_parts = parts + p.warps * kRows * kPitch;
+  const bool squares = HELPER == kSquares && blockIdx.x == 0;
 
-  // Chunk c of this warp goes to slot c % (2 kHalf). (Pieces beyond K become zeros; columns beyond N are not copied:
-  // what they multiply is not stored.)
+  // Rows of a slot are stored with their 16-byte pieces XOR-ed by the row, as a 128-byte TMA swizzle does. Pieces
+  // beyond K become zeros; columns beyond N and rows beyond M are not copied: what they multiply is not stored.
   auto copy_weights = [&](int c) {
     if (c >= count) return;
-    const int k = (first + c) * kChunk + t * 8;
-    const bool there = k < p.k;  // (K is a multiple of 8: all 8 or none)
-    const uint32_t at = base + c % (2 * kHalf) * (kPieces * 512);
+    const int k = (first + c) * kBlock + (lane & 7) * 8, bytes = k < p.k ? 16 : 0;
+    const uint32_t at = w_base + c % RING * kWBytes;
 #pragma unroll
-    for (int r = 0; r < kPieces; ++r) {
-      const int n = n0 + r * 8 + g;
-      if (n < p.n) cp_async16_zfill(at + r * 512, p.w + static_cast<int64_t>(n) * p.k + (there ? k : 0), there ? 16 : 0);
+    for (int i = 0; i < kColumns / 4; ++i) {
+      const int r = (lane >> 3) + 4 * i, n = n0 + r;
+      if (n < p.n)
+        cp_async16_zfill(at + r * 128 + (swizzle128(r, lane & 7) << 4), p.w + static_cast<int64_t>(n) * p.k + (bytes ? k : 0), bytes);
     }
   };
-  // x is read into registers, all of it that the ring covers at once
-  uint4 xv[2 * kHalf];
-  const T* x_row = p.x + (g < p.m ? g : 0) * p.x_row_stride + t * 8;
-  auto load_row = [&](int slot, int c) {
-    const int k = (first + c) * kChunk;
-    xv[slot] = make_uint4(0u, 0u, 0u, 0u);
-    if (g < p.m && c < count && k + t * 8 < p.k) xv[slot] = load_rows_of_x(x_row + k);
+  auto copy_rows = [&](int c) {
+    if (c >= count) return;
+    const int k = (first + c) * kBlock + (lane & 7) * 8, bytes = k < p.k ? 16 : 0;
+    const uint32_t at = x_base + c % kXRing * x_bytes;
+#pragma unroll
+    for (int i = 0; i < kRows / 4; ++i) {
+      const int r = (lane >> 3) + 4 * i;
+      if (r < p.m) copy_through_l1(at + r * 128 + (swizzle128(r, lane & 7) << 4), p.x + r * p.x_row_stride + (bytes ? k : 0), bytes);
+    }
   };
+  // A copy group per block of W, then one per block of x, then (in the main loop) one per turn, with the block of W
+  // RING and the block of x kXRing further on. Block i is complete once group RING + i is.
   if (!p.early) grid_dependency_wait();
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {  // two copy groups in flight
-#pragma unroll
-    for (int j = 0; j < kHalf; ++j) copy_weights(h * kHalf + j);
+  for (int c = 0; c < RING; ++c) {
+    copy_weights(c);
     cp_async_commit();
   }
   if (p.early) grid_dependency_wait();
 #pragma unroll
-  for (int c = 0; c < 2 * kHalf; ++c) load_row(c, c);
+  for (int c = 0; c < kXRing; ++c) {
+    copy_rows(c);
+    cp_async_commit();
+  }
+  if (squares) {  // (the whole slice stays in the ring: the helper reads x there)
+    cp_async_wait<0>();
+    __syncthreads();
+  }
 
-  float acc[2][4] = {};  // (two chains of products, added at the end)
-  float ss = 0.0f;
-  for (int turn = 0; turn < count; turn += 2 * kHalf) {
+  if (warp < p.warps) {
+    // fragments are read a block ahead of their products: a chain of dependent instructions has no slack for it
+    struct Fragments {
+      uint32_t a[4][4], b[2][4];
+    } now, next;
+    const int row = ((lane >> 3 & 1) << 3) + (lane & 7), x_row = min(lane & 7, p.m - 1);  // (rows beyond M: any row)
+    auto read = [&](Fragments& f, int c) {
+      const uint32_t w_at = w_base + c % RING * kWBytes, x_at = x_base + c % kXRing * x_bytes;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int c0 = turn + h * kHalf;
-      if (c0 >= count) break;
-      cp_async_wait<1>();
-      uint4 v[kHalf][kPieces];
+      for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(f.a[ks], w_at + row * 128 + (swizzle128(row, ks * 2 + (lane >> 4)) << 4));
 #pragma unroll
-      for (int j = 0; j < kHalf; ++j)
-#pragma unroll
-        for (int r = 0; r < kPieces; ++r)
-          if (c0 + j < count)
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(v[j][r].x), "=r"(v[j][r].y), "=r"(v[j][r].z), "=r"(v[j][r].w)
-                         : "r"(base + (h * kHalf + j) * (kPieces * 512) + r * 512) : "memory");
-#pragma unroll
-      for (int j = 0; j < kHalf; ++j) {
-        if (c0 + j >= count) break;
-        const uint4 b = xv[h * kHalf + j], u = v[j][0], d = v[j][1];
-        const uint32_t low[4] = {u.x, d.x, u.y, d.y}, high[4] = {u.z, d.z, u.w, d.w};
-        mma_16816<T>(acc[0], low, b.x, b.y);
-        mma_16816<T>(acc[1], high, b.z, b.w);
-        if (SQUARES) ss = square_pair<T>(b.w, square_pair<T>(b.z, square_pair<T>(b.y, square_pair<T>(b.x, ss))));
+      for (int h = 0; h < 2; ++h) ldmatrix_x4(f.b[h], x_at + x_row * 128 + (swizzle128(x_row, h * 4 + (lane >> 3)) << 4));
+    };
+    float acc[4] = {};
+    if (count > 0) {
+      cp_async_wait<kXRing - 1>();
+      __syncwarp();
+      read(now, 0);
+    }
+    for (int c = 0; c < count; ++c) {
+      if (c + 1 < count) {
+        cp_async_wait<kXRing - 2>();
+        __syncwarp();
+        read(next, c + 1);
       }
 #pragma unroll
-      for (int j = 0; j < kHalf; ++j) {  // (every lane refills the pieces that it has read itself)
-        copy_weights(c0 + 2 * kHalf + j);
-        load_row(h * kHalf + j, c0 + 2 * kHalf + j);
+      for (int ks = 0; ks < 4; ++ks) mma_16816<T>(acc, now.a[ks], now.b[ks / 2][ks % 2 * 2], now.b[ks / 2][ks % 2 * 2 + 1]);
+      // (every lane has read this block's slots: it did so before the barrier above)
+      if (c + kXRing < count) {
+        copy_weights(c + RING);
+        copy_rows(c + kXRing);
       }
       cp_async_commit();
+      now = next;
     }
-  }
-  cp_async_wait<0>();
-
-  // the warps' sums, in warp order (behind them, with several CTAs, in rank order: the same result every time)
-  float* at = &part[warp][2 * t][g];
-  at[0] = acc[0][0] + acc[1][0];
-  at[kPitch] = acc[0][1] + acc[1][1];
-  at[8] = acc[0][2] + acc[1][2];
-  at[kPitch + 8] = acc[0][3] + acc[1][3];
-  if (SQUARES) {
-    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-    ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-    if (t == 0) squares[warp][g] = ss;
+    cp_async_wait<0>();
+    float* at = part(warp, 2 * t, g);
+    at[0] = acc[0];
+    at[kPitch] = acc[1];
+    at[8] = acc[2];
+    at[kPitch + 8] = acc[3];
+  } else if (HELPER == kSquares) {
+    if (squares && lane < p.m) {
+      const int blocks = max(0, min(static_cast<int>(blockIdx.z + 1) * p.blocks_per_slice, all_blocks) -
+                                    static_cast<int>(blockIdx.z) * p.blocks_per_slice);
+      const uint32_t x_row = smem_u32(ring) + p.slots * kWBytes + lane * 128;
+      float ss = 0.0f;
+      for (int c = 0; c < blocks; ++c) {
+        uint4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = load_shared16(x_row + c * x_bytes + (((j + lane) & 7) << 4));
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          ss = square_pair<T>(v[j].w, square_pair<T>(v[j].z, square_pair<T>(v[j].y, square_pair<T>(v[j].x, ss))));
+      }
+      p.row_squares[static_cast<int64_t>(blockIdx.z) * p.m + lane] = ss;
+    }
+  } else if (HELPER == kNorm) {
+#pragma unroll 8
+    for (int i = lane; i < p.norm_slices * p.m; i += 32) norm_parts[i] = __ldcg(p.norm_squares + i);
+    __syncwarp();
+    if (lane < p.m) {
+      float ss = 0.0f;
+#pragma unroll 16
+      for (int i = 0; i < p.norm_slices; ++i) ss += norm_parts[i * p.m + lane];
+      row_scale[lane] = rsqrtf(ss / static_cast<float>(p.k) + p.norm_eps);
+    }
   }
   __syncthreads();
-  if (splits > 1) {
-    for (int u = threadIdx.x; u < kRows * kColumns; u += kThreads) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int s = 0; s < kWarps; ++s) sum += part[s][u / kColumns][u % kColumns];
-      total[u / kColumns][u % kColumns] = sum;
-    }
-    if (SQUARES && threadIdx.x < kRows) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int s = 0; s < kWarps; ++s) sum += squares[s][threadIdx.x];
-      total_squares[threadIdx.x] = sum;
-    }
-    cluster_sync();
-  }
-  // pairs of neighbouring columns, dealt to the CTAs of the cluster
-  for (int u = rank + splits * threadIdx.x; u < kRows * kColumns / 2; u += splits * kThreads) {
-    const int row = u / (kColumns / 2), c = u % (kColumns / 2) * 2, n = n0 + c;
-    if (row >= p.m || n >= p.n) continue;
-    const bool has1 = n + 1 < p.n;
-    float v0 = 0.0f, v1 = 0.0f, sq = 0.0f;
-    if (splits > 1) {
-      for (int s = 0; s < splits; ++s) {
-        v0 += load_cluster_f32(smem_u32(&total[row][c]), s);
-        v1 += load_cluster_f32(smem_u32(&total[row][c + 1]), s);
-        if (SQUARES) sq += load_cluster_f32(smem_u32(&total_squares[row]), s);
-      }
-    } else {
-#pragma unroll
-      for (int s = 0; s < kWarps; ++s) {
-        const float2 v = *reinterpret_cast<const float2*>(&part[s][row][c]);
-        v0 += v.x;
-        v1 += v.y;
-        if (SQUARES) sq += squares[s][row];
-      }
-    }
-    const int64_t o = static_cast<int64_t>(row) * p.n + n;
+  const bool across = gridDim.z > 1 && p.sums == nullptr;  // the slices are the CTAs of a cluster along z
+  if (across) cluster_sync();
+
+  // units of 4 columns, dealt to the CTAs that hold the slices
+  const int owners = across ? p.splits : 1, owner = across ? blockIdx.z : 0;
+  for (int u = owner + owners * threadIdx.x; u < kRows * kColumns / 4; u += owners * blockDim.x) {
+    const int row = u / (kColumns / 4), c = u % (kColumns / 4) * 4, n = n0 + c, have = min(4, p.n - n);
+    if (p.squares_out != nullptr) unit_squares[row][c / 4] = 0.0f;
+    if (row >= p.m || have <= 0) continue;
+    float v[4] = {};
     if (p.sums != nullptr) {
-      p.sums[o] = v0;
-      if (has1) p.sums[o + 1] = v1;
-      if (SQUARES && n == 0 && p.row_squares != nullptr) p.row_squares[row] = sq;
+      float* dst = p.sums + (static_cast<int64_t>(blockIdx.z) * p.m + row) * p.n + n;
+      for (int e = 0; e < have; ++e) dst[e] = *part(0, row, c + e);
       continue;
     }
-    if (SQUARES && p.fold_norm) {
-      const float scale = rsqrtf(sq / static_cast<float>(p.k) + p.norm_eps);
-      v0 *= scale;
-      v1 *= scale;
+    for (int s = 0; s < p.splits; ++s) {
+      const uint32_t at = smem_u32(part(across ? 0 : s, row, c));
+      const float4 q = across ? load_cluster_f32x4(at, s) : *reinterpret_cast<const float4*>(part(s, row, c));
+      v[0] += q.x; v[1] += q.y; v[2] += q.z; v[3] += q.w;
+    }
+    if (HELPER == kNorm) {
+      const float scale = row_scale[row];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] *= scale;
     }
     if (p.bias != nullptr) {
-      v0 += Elem<T>::load(p.bias + n);
-      if (has1) v1 += Elem<T>::load(p.bias + n + 1);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < have) v[e] += Elem<T>::load(p.bias + n + e);
     }
-    Elem<T>::round_pair(v0, v1);
-    if (p.epilogue == B200_EPILOGUE_SWIGLU) {  // column 2j is gate_j, column 2j + 1 is up_j
-      Elem<T>::store(p.out + static_cast<int64_t>(row) * (p.n / 2) + n / 2, Elem<T>::round(silu_fast(v0)) * v1);
+    if (p.epilogue == B200_EPILOGUE_SWIGLU) {  // column 2j is gate_j, column 2j + 1 is up_j (N is even)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        if (e >= have) break;
+        Elem<T>::round_pair(v[e], v[e + 1]);
+        Elem<T>::store(p.out + static_cast<int64_t>(row) * (p.n / 2) + (n + e) / 2, Elem<T>::round(silu_fast(v[e])) * v[e + 1]);
+      }
       continue;
     }
+    const int64_t o = static_cast<int64_t>(row) * p.n + n;
     if (p.epilogue == B200_EPILOGUE_RESIDUAL) {
-      v0 = __fadd_rn(v0, Elem<T>::load(p.residual + o));
-      if (has1) v1 = __fadd_rn(v1, Elem<T>::load(p.residual + o + 1));
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < have) v[e] = __fadd_rn(Elem<T>::round(v[e]), Elem<T>::load(p.residual + o + e));
     }
-    if (has1 && (reinterpret_cast<uintptr_t>(p.out + o) & 3u) == 0) {
-      *reinterpret_cast<uint32_t*>(p.out + o) = Elem<T>::pack(v0, v1);
+    if (have == 4 && (reinterpret_cast<uintptr_t>(p.out + o) & 7u) == 0) {
+      *reinterpret_cast<uint2*>(p.out + o) = make_uint2(Elem<T>::pack(v[0], v[1]), Elem<T>::pack(v[2], v[3]));
     } else {
-      Elem<T>::store(p.out + o, v0);
-      if (has1) Elem<T>::store(p.out + o + 1, v1);
+      for (int e = 0; e < have; ++e) Elem<T>::store(p.out + o + e, v[e]);
+    }
+    if (p.squares_out != nullptr) {  // of what was stored (here N is a multiple of 4)
+      Elem<T>::round_pair(v[0], v[1]);
+      Elem<T>::round_pair(v[2], v[3]);
+      unit_squares[row][c / 4] = fmaf(v[0], v[0], fmaf(v[1], v[1], fmaf(v[2], v[2], v[3] * v[3])));
     }
   }
-  if (splits > 1) cluster_sync();  // no CTA leaves while another reads its sums
+  if (p.squares_out != nullptr) {
+    // unit i of a tile's rows (counted through the rows) belongs to slice i % splits, which adds its own in order
+    cluster_sync();
+    const int tile = blockIdx.x / p.tile_groups, member = blockIdx.x % p.tile_groups;
+    for (int item = threadIdx.x * p.tile_groups + member; item < p.splits * p.m; item += blockDim.x * p.tile_groups) {
+      const int s = item / p.m, row = item % p.m, units = p.tile_groups * (kColumns / 4), begin = row * units;
+      float ss = 0.0f;
+      for (int i = begin + (s - begin % p.splits + p.splits) % p.splits; i < begin + units; i += p.splits)
+        ss += load_cluster_f32(smem_u32(&unit_squares[row][(i - begin) % 4]), (i - begin) / 4);
+      p.squares_out[static_cast<int64_t>(tile * p.splits + s) * p.m + row] = ss;
+    }
+  }
+  if (across || p.squares_out != nullptr) cluster_sync();  // no CTA leaves while another reads its part
 }
+
+template <typename T, int HELPER, int RING>
+int launch_rows16(const RowsParams<T>& p, dim3 grid, int threads, unsigned cluster_x, unsigned cluster_z, cudaStream_t s) {
+  auto kernel = linear_rows16_kernel<T, HELPER, RING>;
+  constexpr int kMost = (RING == kShortRing ? kMaxSlices : 1) * (RING * kWBytes + x_ring(RING) * kRows * 128 + kPartBytes) +
+                        (HELPER == kNorm ? kNormFloats * 4 : 0);
+  const int smem = p.warps * (p.slots * kWBytes + p.x_slots * p.m * 128 + kPartBytes) +
+                   (HELPER == kNorm ? p.norm_slices * p.m * 4 : 0);
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess ||
+      launch_chained_cluster_xz(kernel, grid, dim3(threads), static_cast<size_t>(smem), s, cluster_x, cluster_z, p) !=
+          cudaSuccess)
+    return B200_ERR_LAUNCH;
+  return launch_status();
+}
+
+int64_t blocks_per_slice(const FewRowsCall& c) { return ceil_div(ceil_div(c.k, kBlock), static_cast<int64_t>(c.splits)); }
 
 template <typename T>
 int linear_few_rows_of(const FewRowsCall& c, cudaStream_t stream) {
-  constexpr int kSlotBytes = kWarps * kPieces * 512;
-  // With few columns as many CTAs of a cluster along K as it takes to hold W in one ring each, up to some four CTAs
-  // an SM (896 x 4864 on 1 row: 4.5 us with 5 CTAs a column tile; 7.2 us on the tcgen05 kernel in clusters).
-  const int64_t groups = ceil_div(c.n, kColumns), chunks = ceil_div(c.k, kChunk);
-  int64_t splits = ceil_div(chunks, kWarps * 2 * kHalf);
-  if (splits > 4 * kNumSMs / groups) splits = 4 * kNumSMs / groups;
-  if (splits > 8) splits = 8;
-  if (splits < 1) splits = 1;
-  const int64_t most = ceil_div(chunks, kWarps * splits);
-
+  const int64_t per = blocks_per_slice(c);
+  const bool tiles = c.squares_out != nullptr;  // all slices in a CTA, the CTAs of a tile in a cluster
+  const int ring = tiles ? kShortRing : kLongRing;
   RowsParams<T> p;
   p.x = static_cast<const T*>(c.input);
   p.w = static_cast<const T*>(c.weight);
@@ -253,35 +305,50 @@ int linear_few_rows_of(const FewRowsCall& c, cudaStream_t stream) {
   p.out = static_cast<T*>(c.output);
   p.sums = c.sums;
   p.row_squares = c.row_squares;
+  p.squares_out = c.squares_out;
+  p.norm_squares = c.norm_squares;
   p.x_row_stride = c.input_row_stride;
   p.m = static_cast<int>(c.m);
   p.k = static_cast<int>(c.k);
   p.n = static_cast<int>(c.n);
   p.epilogue = c.epilogue;
-  p.fold_norm = c.fold_norm ? 1 : 0;
-  p.norm_eps = static_cast<float>(c.norm_eps);
-  p.slots = static_cast<int>(most < 2 * kHalf ? most : 2 * kHalf);
+  p.splits = c.splits;
+  p.blocks_per_slice = static_cast<int>(per);
+  p.warps = tiles ? c.splits : 1;
+  p.tile_groups = tiles ? c.tile_columns / kColumns : 1;
+  p.norm_slices = c.norm_slices;
+  p.slots = static_cast<int>(per < ring ? per : ring);
+  p.x_slots = p.slots < x_ring(ring) ? p.slots : x_ring(ring);
   p.early = (launch_mode() & B200_LAUNCH_CONSTANT_WEIGHTS) != 0 ? 1 : 0;
-  const bool squares = c.fold_norm || c.row_squares != nullptr;
-  const dim3 grid(static_cast<unsigned>(groups), 1, static_cast<unsigned>(splits));
-  auto kernel = squares ? linear_rows16_kernel<T, true> : linear_rows16_kernel<T, false>;
-  if (launch_chained_cluster_xz(kernel, grid, dim3(kThreads), static_cast<size_t>(p.slots * kSlotBytes), stream, 1u,
-                                static_cast<unsigned>(splits), p) != cudaSuccess)
-    return B200_ERR_LAUNCH;
-  return launch_status();
+  p.norm_eps = static_cast<float>(c.norm_eps);
+  int64_t groups = ceil_div(c.n, kColumns);
+  if (tiles) {
+    groups = ceil_div(c.n, static_cast<int64_t>(c.tile_columns)) * p.tile_groups;
+    return launch_rows16<T, kPlain, kShortRing>(p, dim3(static_cast<unsigned>(groups)), 32 * c.splits,
+                                                static_cast<unsigned>(p.tile_groups), 1u, stream);
+  }
+  const dim3 grid(static_cast<unsigned>(groups), 1, static_cast<unsigned>(c.splits));
+  if (c.row_squares != nullptr) return launch_rows16<T, kSquares, kLongRing>(p, grid, 64, 1u, 1u, stream);
+  if (c.norm_squares != nullptr) return launch_rows16<T, kNorm, kLongRing>(p, grid, 64, 1u, 1u, stream);
+  return launch_rows16<T, kPlain, kLongRing>(p, grid, 32, 1u, c.sums != nullptr ? 1u : static_cast<unsigned>(c.splits), stream);
 }
 
 }  // namespace
 
-// One column tile of the products: up to 8 rows it is the faster kernel at every size measured. A second one (16 rows)
-// doubles what the CTAs read of x, and wins little where it wins: Qwen2-0.5B 906 -> 876 us a step, four layers of the
-// 7B 696 -> 817, Lozanex 1.5b 854 -> 901.
-bool takes_few_rows(int64_t m) {
+bool takes_few_rows(const FewRowsCall& c) {
   static const int64_t limit = [] {  // B200_FEW_ROWS=0: the comparison run
     const char* text = getenv("B200_FEW_ROWS");
     return text != nullptr ? static_cast<int64_t>(atoi(text)) : kRows;
   }();
-  return m <= limit && m <= kRows;
+  if (c.m > limit || c.m > kRows || c.splits < 1) return false;
+  // A launch that is a chain of latencies. A larger matrix is a stream, which the tcgen05 kernels' TMA rings keep fuller
+  // than one warp a slice can: 151936 x 896 56 against 82 us on 1 row, four layers of Qwen2-7B 688 against 955.
+  if (c.n * c.k > (10 << 20)) return false;
+  if (c.sums == nullptr && c.splits > kMaxSlices) return false;
+  if (c.row_squares != nullptr && blocks_per_slice(c) > x_ring(kLongRing)) return false;  // the helper reads the whole slice
+  if (c.squares_out != nullptr && c.tile_columns > kColumns * kMaxSlices) return false;
+  if (c.norm_squares != nullptr && (c.splits != 1 || c.norm_slices * c.m > kNormFloats)) return false;
+  return true;
 }
 
 int linear_few_rows(const FewRowsCall& call, int dtype, cudaStream_t stream) {

@@ -1215,6 +1215,14 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
     // 60.2 us against 71.2 - 78.3 us for one 208 ... 256-column CTA per SM at N = 151936.
     if (ceil_div(n, 192) >= 4 * kNumSMs) bn = 192;
   }
+  if (m <= 64 && (!fold_norm || norm_slices > 0)) {
+    FewRowsCall c{input, weight, bias, epilogue == B200_EPILOGUE_RESIDUAL ? residual : nullptr, output, m, k, n,
+                  input_row_stride, epilogue};
+    c.norm_squares = fold_norm ? norm_squares : nullptr;
+    c.norm_slices = norm_slices;
+    c.norm_eps = norm_eps;
+    if (takes_few_rows(c)) return linear_few_rows(c, IsHalf<T>::value ? B200_F16 : B200_BF16, stream);
+  }
   CUtensorMap a_map, b_map;
   if (!make_bf16_matrix_map(&a_map, input, m, k, input_row_stride, m <= 64 ? 64 : kBM) ||
       !make_bf16_matrix_map(&b_map, weight, n, k, k, bn))
@@ -1269,7 +1277,7 @@ int linear_tcgen05(const void* input, const void* weight, const void* bias, cons
 }
 
 int linear_partial_splits(int64_t m, int64_t k, int64_t n) {
-  return takes_few_rows(m) ? 1 : plan_partial(m, k, n).splits;
+  return plan_partial(m, k, n).splits;
 }
 
 int linear_partial_tcgen05(const void* input, const void* weight, float* partials,
@@ -1277,10 +1285,11 @@ int linear_partial_tcgen05(const void* input, const void* weight, float* partial
                            int64_t input_row_stride, int splits, int32_t* status,
                            cudaStream_t stream) {
   if (row_squares != nullptr && m > 128) return B200_ERR_UNSUPPORTED;
-  if (splits == 1 && takes_few_rows(m)) {
-    FewRowsCall c{input, weight, nullptr, nullptr, nullptr, partials, row_squares, m, k, n, input_row_stride,
-                  B200_EPILOGUE_NONE};
-    return linear_few_rows(c, B200_BF16, stream);
+  {
+    FewRowsCall c{input, weight, nullptr, nullptr, nullptr, m, k, n, input_row_stride, B200_EPILOGUE_NONE, splits};
+    c.sums = partials;
+    c.row_squares = row_squares;
+    if (takes_few_rows(c)) return linear_few_rows(c, B200_BF16, stream);
   }
   const PartialPlan plan = plan_partial(m, k, n);
   const int a_rows = m <= 64 ? 64 : 128;
@@ -1324,25 +1333,22 @@ int linear_splitk_residual_tcgen05(const void* input, const void* weight, const 
                                    void* output, int64_t m, int64_t k, int64_t n,
                                    int64_t input_row_stride, int32_t* status, cudaStream_t stream,
                                    float* squares_out) {
-  if (squares_out == nullptr && takes_few_rows(m)) {
-    FewRowsCall c{input, weight, nullptr, residual, output, nullptr, nullptr, m, k, n, input_row_stride,
-                  B200_EPILOGUE_RESIDUAL};
-    return linear_few_rows(c, B200_BF16, stream);
-  }
   const PartialPlan plan = plan_cluster(m, k, n);
   // enough N x M tiles to fill the GPU without cutting K: the plain kernel with the residual epilogue
   if (plan.splits <= 1)
     return linear_tcgen05(input, weight, nullptr, residual, output, m, k, n, input_row_stride, B200_BF16,
                           B200_EPILOGUE_RESIDUAL, status, stream, false, 0.0, nullptr, 0);
+  FewRowsCall c{input, weight, nullptr, residual, output, m, k, n, input_row_stride, B200_EPILOGUE_RESIDUAL, plan.splits};
+  c.squares_out = squares_out;
+  c.tile_columns = plan.bn;
+  if (takes_few_rows(c)) return linear_few_rows(c, B200_BF16, stream);
   return launch_cluster_splitk(plan, input, weight, nullptr, residual, output, m, k, n, input_row_stride, status, stream,
                                squares_out);
 }
 
 // Slices of row sums of squares that the cluster split-K projection leaves (N tiles x K slices);
 // 0 when the shape runs without a cluster (then nothing is written).
-// (a projection of a few rows leaves none: the one behind it squares its rows on the way)
 int64_t linear_splitk_slices(int64_t m, int64_t k, int64_t n) {
-  if (takes_few_rows(m)) return 0;
   const PartialPlan plan = plan_cluster(m, k, n);
   return plan.splits <= 1 ? 0 : ceil_div(n, static_cast<int64_t>(plan.bn)) * plan.splits;
 }
@@ -1385,11 +1391,6 @@ extern "C" int b200_linear_rms_input(const void* input, const void* folded_weigh
   if (m > 128) return B200_ERR_TOO_LARGE;
   if (k % 8 != 0 || input_row_stride % 8 != 0) return B200_ERR_UNSUPPORTED;
   if (!aligned16(input) || !aligned16(folded_weight)) return B200_ERR_ALIGNMENT;
-  if (takes_few_rows(m)) {
-    FewRowsCall c{input, folded_weight, bias, nullptr, output, nullptr, nullptr, m, k, n, input_row_stride, epilogue,
-                  true, epsilon};
-    return linear_few_rows(c, B200_BF16, static_cast<cudaStream_t>(stream));
-  }
   return linear_tcgen05(input, folded_weight, bias, nullptr, output, m, k, n, input_row_stride, B200_BF16,
                         epilogue, status, static_cast<cudaStream_t>(stream), true, epsilon,
                         static_cast<const float*>(row_squares), static_cast<int>(row_square_slices));

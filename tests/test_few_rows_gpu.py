@@ -72,17 +72,53 @@ def test_forms_of_the_decode_chain(m, k, n):
     x, w, residual, _ = _operands(m, k, n, torch.bfloat16)
     half, (exact, sums) = 1.01 * _half_ulp(torch.bfloat16), _product(x, w)
     partials, squares = kernels.b200_linear_partial(x, w, row_squares=True)
-    assert partials.shape == (1, m, n) and squares.shape == (1, m)
-    _check(partials[0], exact, sums)
+    assert squares.shape == partials.shape[:2]
+    _check(partials.sum(0), exact, sums)
     exact_squares = x.double().square().sum(-1)
-    _check(squares[0], exact_squares, k * 2.0 ** -23 * exact_squares)
+    _check(squares.sum(0), exact_squares, k * 2.0 ** -23 * exact_squares)
     total = exact + residual.double()
-    out, none = kernels.b200_linear_splitk_residual(x, w, residual, row_squares=True)
-    assert none is None
+    out = kernels.b200_linear_splitk_residual(x, w, residual)
     _check(out, total, sums + half * (exact.abs() + total.abs() + 2 * sums))
-    assert torch.equal(out, kernels.b200_linear_splitk_residual(x, w, residual))
     scale = torch.rsqrt(exact_squares / k + 1e-6)[:, None]
     normed = exact * scale
-    _check(kernels.b200_linear_rms_input(x, w, epsilon=1e-6), normed,
-           1.01 * sums * scale + (half + k * 2.0 ** -23) * normed.abs())
+    for given in (None, squares):
+        _check(kernels.b200_linear_rms_input(x, w, epsilon=1e-6, row_squares=given), normed,
+               1.01 * sums * scale + (half + k * 2.0 ** -23) * normed.abs())
+    kernels.runtime().check_status()
+
+
+# the sizes above whose rows take few blocks, the projections of a Qwen2-0.5B layer, longer K, more
+# column tiles than the GPU holds at once, and one matrix over the limit
+CHAIN = [(1, 896, 1152), (8, 896, 896), (3, 4864, 896), (5, 904, 1092), (2, 3584, 2308), (7, 3584, 2800), (4, 18944, 512),
+         (6, 896, 9728), (2, 264, 30000), (8, 72, 2500), (1, 896, 12000)]
+
+
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("m,k,n", CHAIN)
+def test_a_row_is_the_same_bit_for_bit_in_a_larger_batch(m, k, n, early):
+    """16 rows run on the tcgen05 kernels; the same rows in a batch of up to 8 give the same bits in every form."""
+    x, w, residual, bias = _operands(16, k, n, torch.bfloat16)
+    few = slice(0, m)
+    with kernels.launch_mode(programmatic=early, constant_weights=early):
+        many = kernels.b200_linear_partial(x, w, row_squares=True)
+        mine = kernels.b200_linear_partial(x[few], w, row_squares=True)
+        assert torch.equal(mine[0], many[0][:, few]) and torch.equal(mine[1], many[1][:, few])
+        assert torch.equal(kernels.b200_linear_partial(x[few], w), many[0][:, few])
+        assert torch.equal(kernels.b200_linear_splitk_residual(x[few], w, residual[few]),
+                           kernels.b200_linear_splitk_residual(x, w, residual)[few])
+        out, squares = kernels.b200_linear_splitk_residual(x, w, residual, row_squares=True)
+        out_few, squares_few = kernels.b200_linear_splitk_residual(x[few], w, residual[few], row_squares=True)
+        assert torch.equal(out_few, out[few])
+        assert (squares is None) == (squares_few is None)
+        if squares is not None:
+            assert torch.equal(squares_few, squares[:, few])
+        given = torch.rand((112, 16), device="cuda") + 0.1
+        for epilogue in ("none", "swiglu"):
+            assert torch.equal(kernels.b200_linear(x[few], w, epilogue=epilogue), kernels.b200_linear(x, w, epilogue=epilogue)[few])
+            for parts in (None, given):
+                assert torch.equal(
+                    kernels.b200_linear_rms_input(x[few], w, epsilon=1e-6, epilogue=epilogue,
+                                                  row_squares=None if parts is None else parts[:, few].contiguous()),
+                    kernels.b200_linear_rms_input(x, w, epsilon=1e-6, epilogue=epilogue, row_squares=parts)[few])
+        assert torch.equal(kernels.b200_linear(x[few], w, bias), kernels.b200_linear(x, w, bias)[few])
     kernels.runtime().check_status()
