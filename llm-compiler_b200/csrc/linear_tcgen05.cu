@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "linear_rows.cuh"
+#include "prompt_layers.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
 
@@ -1130,21 +1131,6 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
         if (ceil_div(n, candidate) * tiles_m >= kNumSMs * 3 / 4) return candidate;
       return 64;
     };
-    // A short prompt against a narrow matrix leaves most SMs idle even in 64-column tiles (whose products take the time
-    // of wider ones): K is cut over the CTAs of a cluster as in decoding, from 129 rows on only a long K, where that
-    // pays for adding up the tiles. 896 columns, K 4864: 77 rows 27.1 -> 9.6 us, 300 rows 27.9 -> 16.3, 640 rows 28.1 ->
-    // 20.9; K 896: 77 rows 7.6 -> 6.5, but 512 rows 8.6 -> 10.3 if it did.
-    if constexpr (!IsHalf<T>::value) {
-      const bool pairs = n % 4 == 0 && ((reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(residual) |
-                                         reinterpret_cast<uintptr_t>(bias)) & 7u) == 0;
-      if (!fold_norm && epilogue != B200_EPILOGUE_SWIGLU && pairs && ceil_div(n, 64) * tiles_m < kNumSMs / 2 &&
-          (m <= kBM || ceil_div(k, kBK) >= 32)) {
-        const PartialPlan plan = plan_cluster(m, k, n);
-        if (plan.splits > 1)
-          return launch_cluster_splitk(plan, input, weight, bias, epilogue == B200_EPILOGUE_RESIDUAL ? residual : nullptr,
-                                       output, m, k, n, input_row_stride, status, stream, nullptr);
-      }
-    }
     // A few M tiles (65 .. 1023 rows: large decode batches, short prefills) stream W rather than
     // reuse it: the widest tile that still gives about three quarters of the SMs a CTA, else the
     // narrowest (a 3584-column projection at 256 rows: 112 CTAs of 64 columns instead of 28 of 256).
@@ -1344,6 +1330,26 @@ int linear_splitk_residual_tcgen05(const void* input, const void* weight, const 
   if (takes_few_rows(c)) return linear_few_rows(c, B200_BF16, stream);
   return launch_cluster_splitk(plan, input, weight, nullptr, residual, output, m, k, n, input_row_stride, status, stream,
                                squares_out);
+}
+
+// A short prompt against a narrow matrix leaves most SMs idle even in 64-column tiles (whose products take the time of
+// wider ones): K is cut over the CTAs of a cluster as in decoding, from 129 rows on only a long K, where that pays for
+// adding up the tiles. 896 columns, K 4864: 77 rows 27.1 -> 9.6 us, 300 rows 27.9 -> 16.3, 640 rows 28.1 -> 20.9; K
+// 896: 77 rows 7.6 -> 6.5, but 512 rows 8.6 -> 10.3 if it did. For callers that may choose the order of the sums
+// (b200_linear keeps its own: routers behind it choose experts by the last bits). bf16, y = r(r(x W^T + bias) +
+// residual); B200_ERR_UNSUPPORTED: not such a size, use b200_linear.
+int linear_narrow_prompt(const void* input, const void* weight, const void* bias, const void* residual, void* output,
+                         int64_t m, int64_t k, int64_t n, int32_t* status, cudaStream_t stream) {
+  const uintptr_t ends = reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(residual) |
+                         reinterpret_cast<uintptr_t>(bias);
+  if ((launch_mode() & B200_LAUNCH_LINEAR_WARP_LEVEL) != 0 || m <= 64 || m > 65535 || k % 8 != 0 || n % 4 != 0 ||
+      (ends & 7u) != 0 || !aligned16(input) || !aligned16(weight) ||
+      ceil_div(n, static_cast<int64_t>(64)) * ceil_div(m, static_cast<int64_t>(kBM)) >= kNumSMs / 2 ||
+      (m > kBM && ceil_div(k, static_cast<int64_t>(kBK)) < 32))
+    return B200_ERR_UNSUPPORTED;
+  const PartialPlan plan = plan_cluster(m, k, n);
+  if (plan.splits <= 1) return B200_ERR_UNSUPPORTED;
+  return launch_cluster_splitk(plan, input, weight, bias, residual, output, m, k, n, k, status, stream, nullptr);
 }
 
 // Slices of row sums of squares that the cluster split-K projection leaves (N tiles x K slices);

@@ -1,5 +1,5 @@
-"""Projections of short prompts against the 64-bit product at the lines of the dispatch: few 64-column tiles (K cut over
-a cluster), too few tiles for the persistent kernel, and the row counts around both.
+"""Projections of short prompts against the 64-bit product at the lines of the dispatch: too few tiles for the persistent
+kernel, and the row counts around it. (K cut over a cluster is tested with the prompt's layers and the split-K form.)
 
 Bound of an element: K 2^-23 sum |x w| for fp32 sums in any order, and half an ulp (at most 2^-8 of a bf16 value, 2^-11
 of an fp16 value) for every rounding: one, or two in front of a residual."""
@@ -33,7 +33,7 @@ def test_linear(m, k, n, dtype):
         out = b200.b200_linear(x, w, b, residual=r, epilogue="none" if r is None else "residual")
         assert ((out.double() - total).abs() <= bound).all()
         assert torch.equal(out, b200.b200_linear(x, w, b, residual=r, epilogue="none" if r is None else "residual"))
-    # rows of a wider matrix, and outputs that 8-byte stores cannot reach keep the other kernel
+    # rows of a wider matrix
     wide = torch.randn(m, k + 8, generator=g).to(dtype).cuda()
     strided = b200.b200_linear(wide[:, 8:], w)
     exact = wide[:, 8:].double() @ w.double().T
