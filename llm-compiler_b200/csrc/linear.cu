@@ -245,7 +245,8 @@ __device__ __forceinline__ void epilogue_generic(const LinearParamsGeneric<T>& p
 // 128 k, so that many CTAs with few registers keep their loads in flight and the main loop has no barrier. The warps of
 // a CTA (and, with few columns, of a cluster) share the K range; x comes out of L1. The sums are short chains
 // (4 K / 128 / warps terms a lane) joined by a tree of exchanges in which every lane ends up with one output.
-// Qwen2-0.5B decode step, 4 rows: 9728 x 896 16.1 us with W in registers behind the launch, 896 x 4864 9.2, LM head 128.
+// In a chain of launches, 4 rows, against W in registers behind the launch: 9728 x 896 16.1 -> 8.4 us (4.2 TB/s), 896 x
+// 4864 9.2 -> 6.3, 896 x 896 4.9 -> 2.4, LM head 151936 x 896 128 -> 83 (6.6 TB/s). 8 rows: 11.7, 7.7, 3.0, 121 (FMAs).
 constexpr int kRowsWarps = 4, kRowsThreads = kRowsWarps * 32, kRowsColumns = 8, kRowsOfX = 8, kRowsRing = 4;
 constexpr int kRowsChunk = 128, kRowsChunkBytes = kRowsColumns * 512;  // k, and bytes of a warp's piece of W
 
@@ -564,10 +565,10 @@ extern "C" int64_t b200_linear_workspace_bytes(int64_t m, int64_t k, int64_t n, 
                                  t.partial_floats_per_tile_split * 4;
 }
 
-// Rows up to which W is streamed (linear_rows_kernel, its time grows with every 8 rows) instead of multiplied in tiles
-// (the same time for 1 to 64 rows). 9728 x 896: 18.0, 31.9 us for 8, 16 rows, 51 us in tiles; 896 x 4864: 10.3, 19.1
-// against 32 us.
-constexpr int64_t kRowsLimit = 16;
+// Rows up to which W is streamed (linear_rows_kernel, whose time grows with every 8 rows) instead of multiplied in tiles
+// (the same time for 1 to 64 rows). 9728 x 896: 11.7, 18.0, 33.1, 40.7 us for 8, 16, 32,
+// 40 rows, 58 us in tiles; 896 x 4864: 7.7, 14.5, 24.4, 25.5 against 45 us.
+constexpr int64_t kRowsLimit = 40;
 
 template <int ROWS>
 static int launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
