@@ -280,8 +280,9 @@ class Qwen2Engine(ServingEngine):
         x = kernels.b200_embedding(self.embed, ids)
         cosine, sine = kernels.b200_rope_table(position_ids, self.inv_freq, self.dtype)
         # (The launches above are fully serialised, so that the layers' weights may be read ahead. Long prompts have
-        # nothing to hide between launches of 100 us, and waiting CTAs of the next one cost them 1 %: 4 x 4096 tokens.)
-        chained = self.programmatic_launch and batch * tokens <= 4096
+        # nothing to hide between launches of 100 us, and waiting CTAs of the next one cost them 1 %: 4 x 4096 tokens of
+        # the 0.5B model, some 3000 of the 7B.)
+        chained = self.programmatic_launch and batch * tokens * cfg.hidden_size <= 4 << 20
         with kernels.launch_mode(programmatic=chained, constant_weights=chained):
             x = kernels.b200_qwen2_prompt_layers(
                 x, self.layers, self.state.keys, self.state.values, cosine, sine, self.positions,  # all zero right now
