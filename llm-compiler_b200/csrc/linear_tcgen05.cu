@@ -31,7 +31,6 @@
 
 #include "common.cuh"
 #include "linear_rows.cuh"
-#include "prompt_layers.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
 
@@ -42,12 +41,10 @@ constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kThreads = 128;
 
-constexpr int kMostUnits = 8;  // 16-byte units of a tile that a thread of a cluster adds up, at most
-
 constexpr int kEpiloguePartial = 100;  // internal: fp32 split-K partials, no rounding
 // internal: the K slices of a tile are the CTAs of one thread-block cluster (cluster extent =
 // splits along grid z); they add their fp32 accumulators through distributed shared memory and
-// write r(r(x W^T + bias) + residual) themselves: no partials in global memory, no reduce kernel
+// write r(r(x W^T) + residual) themselves: no partials in global memory, no reduce kernel
 constexpr int kEpilogueClusterResidual = 101;
 
 // T: the element type of x, W, bias, residual and y, __nv_bfloat16 or __half. (The decode chain's forms
@@ -504,8 +501,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
     const int first_row = first_item >> unit_shift, first_col = tile_n * bn + (first_item & ((bn / 4) - 1)) * 4;
     const bool first_valid = threadIdx.x < owned && first_row < rows && first_col < n_end;
     const int64_t first_offset = static_cast<int64_t>(tile_m * kBM + first_row) * p.n + first_col;
-    const bool adds = p.residual != nullptr;
-    uint2 res = first_valid && adds ? *reinterpret_cast<const uint2*>(p.residual + first_offset) : make_uint2(0u, 0u);
+    uint2 res = first_valid ? *reinterpret_cast<const uint2*>(p.residual + first_offset) : make_uint2(0u, 0u);
     const bool landed = mbarrier_wait_bounded(smem_u32(&reduce_bar), 0, p.wait_limit);
     trace.stamp(4);
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -519,7 +515,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
         continue;
       }
       const int64_t o = static_cast<int64_t>(tile_m * kBM + r) * p.n + col;  // n % 4 == 0
-      if (local != threadIdx.x && adds) res = *reinterpret_cast<const uint2*>(p.residual + o);
+      if (local != threadIdx.x) res = *reinterpret_cast<const uint2*>(p.residual + o);
       float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       float4 t[8];
 #pragma unroll
@@ -531,16 +527,10 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
 #pragma unroll
       for (int s0 = 0; s0 < 8; ++s0)
         if (s0 < p.splits) { acc.x += t[s0].x; acc.y += t[s0].y; acc.z += t[s0].z; acc.w += t[s0].w; }
-      if (p.bias != nullptr) {
-        const uint2 b = *reinterpret_cast<const uint2*>(p.bias + col);
-        acc.x += bf16_lo(b.x); acc.y += bf16_hi(b.x); acc.z += bf16_lo(b.y); acc.w += bf16_hi(b.y);
-      }
-      if (adds) {
-        round_bf16_pair(acc.x, acc.y);
-        round_bf16_pair(acc.z, acc.w);
-        acc.x = __fadd_rn(acc.x, bf16_lo(res.x)); acc.y = __fadd_rn(acc.y, bf16_hi(res.x));
-        acc.z = __fadd_rn(acc.z, bf16_lo(res.y)); acc.w = __fadd_rn(acc.w, bf16_hi(res.y));
-      }
+      round_bf16_pair(acc.x, acc.y);
+      round_bf16_pair(acc.z, acc.w);
+      acc.x = __fadd_rn(acc.x, bf16_lo(res.x)); acc.y = __fadd_rn(acc.y, bf16_hi(res.x));
+      acc.z = __fadd_rn(acc.z, bf16_lo(res.y)); acc.w = __fadd_rn(acc.w, bf16_hi(res.y));
       *reinterpret_cast<uint2*>(p.out + o) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
       if (p.squares_out != nullptr) {
         // the squares of what was stored; slice 0's copy of this unit, read by this thread alone, is free
@@ -884,7 +874,7 @@ int launch(const Tcgen05ParamsOf<T>& p, const CUtensorMap& a_map, const CUtensor
   int smem = ring;
   if (p.epilogue == kEpilogueClusterResidual) {
     const int owned = (A_ROWS * p.bn / 4 + p.splits - 1) / p.splits;
-    if (owned > kMostUnits * kThreads) return B200_ERR_UNSUPPORTED;
+    if (owned > 4 * kThreads) return B200_ERR_UNSUPPORTED;
     smem += 2 * p.splits * owned * 16;  // a send and a receive region
     if (smem > 227 * 1024) return B200_ERR_UNSUPPORTED;
   }
@@ -933,7 +923,7 @@ template <int BN, int STAGES, int A_ROWS>
 int resident_clusters(int bn, int splits) {
   const int owned = (A_ROWS * bn / 4 + splits - 1) / splits;
   const int smem = STAGES * (A_ROWS + BN) * 128 + 9216 + 2 * splits * owned * 16;
-  if (owned > kMostUnits * kThreads || smem > 227 * 1024) return 0;
+  if (owned > 4 * kThreads || smem > 227 * 1024) return 0;
   auto kernel = linear_tcgen05_kernel<BN, STAGES, A_ROWS, kFormCluster>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -1013,7 +1003,7 @@ PartialPlan plan_cluster(int64_t m, int64_t k, int64_t n) {
       // (the last slices may come out empty, e.g. 14 k-blocks over 8 slices of 2: such a CTA
       // ships zeros; 8 slices of at most 2 k-blocks measured faster than 4 slices of 4)
       const int64_t per = ceil_div(kb, splits);
-      if (ceil_div(rows * bn / 4, splits) > kMostUnits * kThreads) continue;  // units one CTA can own
+      if (ceil_div(rows * bn / 4, splits) > 4 * kThreads) continue;  // units one CTA can own
       // every cluster resident at once: a second wave would double the time
       if (splits > 1 && resident_clusters_of(cluster_config(static_cast<int>(rows), bn, per), bn,
                                              static_cast<int>(splits)) < tiles)
@@ -1066,45 +1056,6 @@ PartialPlan plan_partial(int64_t m, int64_t k, int64_t n) {
     }
   }
   return best;
-}
-
-// y = r(r(x W^T + bias) + residual) (bias and residual may be absent), K cut over the CTAs of a cluster. bf16, N a
-// multiple of 4, bias / residual / output on 8-byte boundaries.
-int launch_cluster_splitk(const PartialPlan& plan, const void* input, const void* weight, const void* bias,
-                          const void* residual, void* output, int64_t m, int64_t k, int64_t n, int64_t input_row_stride,
-                          int32_t* status, cudaStream_t stream, float* squares_out) {
-  const int a_rows = m <= 64 ? 64 : 128;
-  CUtensorMap a_map, b_map;
-  if (!make_bf16_matrix_map(&a_map, input, m, k, input_row_stride, a_rows) ||
-      !make_bf16_matrix_map(&b_map, weight, n, k, k, plan.bn))
-    return B200_ERR_UNSUPPORTED;
-  Tcgen05Params p;
-  p.bias = static_cast<const __nv_bfloat16*>(bias);
-  p.residual = static_cast<const __nv_bfloat16*>(residual);
-  p.out = static_cast<__nv_bfloat16*>(output);
-  p.partials = nullptr;
-  p.status = status;
-  p.m = static_cast<int>(m);
-  p.k = static_cast<int>(k);
-  p.n = static_cast<int>(n);
-  p.epilogue = kEpilogueClusterResidual;
-  p.squares_out = squares_out;
-  p.splits = plan.splits;
-  p.bn = plan.bn;
-  p.prefetch_weights = (launch_mode() & B200_LAUNCH_CONSTANT_WEIGHTS) != 0 ? 1 : 0;
-  p.wait_limit = wait_limit();
-  p.drop_loads = drop_loads();
-  // (rings short enough to leave room for the send and receive regions of the reduction)
-  switch (cluster_config(a_rows, plan.bn, ceil_div(ceil_div(k, kBK), plan.splits))) {
-    case ClusterConfig::k32x3: return launch<32, 3, 64, kFormCluster>(p, a_map, b_map, stream);
-    case ClusterConfig::k32x8: return launch<32, 8, 64, kFormCluster>(p, a_map, b_map, stream);
-    case ClusterConfig::k64x4: return launch<64, 4, 64, kFormCluster>(p, a_map, b_map, stream);
-    case ClusterConfig::k64x6: return launch<64, 6, 64, kFormCluster>(p, a_map, b_map, stream);
-    case ClusterConfig::k128x4: return launch<128, 4, 64, kFormCluster>(p, a_map, b_map, stream);
-    case ClusterConfig::k32x6r128: return launch<32, 6, 128, kFormCluster>(p, a_map, b_map, stream);
-    case ClusterConfig::k64x4r128: return launch<64, 4, 128, kFormCluster>(p, a_map, b_map, stream);
-  }
-  return B200_ERR_UNSUPPORTED;
 }
 
 }  // namespace
@@ -1328,28 +1279,38 @@ int linear_splitk_residual_tcgen05(const void* input, const void* weight, const 
   c.squares_out = squares_out;
   c.tile_columns = plan.bn;
   if (takes_few_rows(c)) return linear_few_rows(c, B200_BF16, stream);
-  return launch_cluster_splitk(plan, input, weight, nullptr, residual, output, m, k, n, input_row_stride, status, stream,
-                               squares_out);
-}
-
-// A short prompt against a narrow matrix leaves most SMs idle even in 64-column tiles (whose products take the time of
-// wider ones): K is cut over the CTAs of a cluster as in decoding, from 129 rows on only a long K, where that pays for
-// adding up the tiles. 896 columns, K 4864: 77 rows 27.1 -> 9.6 us, 300 rows 27.9 -> 16.3, 640 rows 28.1 -> 20.9; K
-// 896: 77 rows 7.6 -> 6.5, but 512 rows 8.6 -> 10.3 if it did. For callers that may choose the order of the sums
-// (b200_linear keeps its own: routers behind it choose experts by the last bits). bf16, y = r(r(x W^T + bias) +
-// residual); B200_ERR_UNSUPPORTED: not such a size, use b200_linear.
-int linear_narrow_prompt(const void* input, const void* weight, const void* bias, const void* residual, void* output,
-                         int64_t m, int64_t k, int64_t n, int32_t* status, cudaStream_t stream) {
-  const uintptr_t ends = reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(residual) |
-                         reinterpret_cast<uintptr_t>(bias);
-  if ((launch_mode() & B200_LAUNCH_LINEAR_WARP_LEVEL) != 0 || m <= 64 || m > 65535 || k % 8 != 0 || n % 4 != 0 ||
-      (ends & 7u) != 0 || !aligned16(input) || !aligned16(weight) ||
-      ceil_div(n, static_cast<int64_t>(64)) * ceil_div(m, static_cast<int64_t>(kBM)) >= kNumSMs / 2 ||
-      (m > kBM && ceil_div(k, static_cast<int64_t>(kBK)) < 32))
+  const int a_rows = m <= 64 ? 64 : 128;
+  CUtensorMap a_map, b_map;
+  if (!make_bf16_matrix_map(&a_map, input, m, k, input_row_stride, a_rows) ||
+      !make_bf16_matrix_map(&b_map, weight, n, k, k, plan.bn))
     return B200_ERR_UNSUPPORTED;
-  const PartialPlan plan = plan_cluster(m, k, n);
-  if (plan.splits <= 1) return B200_ERR_UNSUPPORTED;
-  return launch_cluster_splitk(plan, input, weight, bias, residual, output, m, k, n, k, status, stream, nullptr);
+  Tcgen05Params p;
+  p.bias = nullptr;
+  p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.out = static_cast<__nv_bfloat16*>(output);
+  p.partials = nullptr;
+  p.status = status;
+  p.m = static_cast<int>(m);
+  p.k = static_cast<int>(k);
+  p.n = static_cast<int>(n);
+  p.epilogue = kEpilogueClusterResidual;
+  p.squares_out = squares_out;
+  p.splits = plan.splits;
+  p.bn = plan.bn;
+  p.prefetch_weights = (launch_mode() & B200_LAUNCH_CONSTANT_WEIGHTS) != 0 ? 1 : 0;
+  p.wait_limit = wait_limit();
+  p.drop_loads = drop_loads();
+  // (rings short enough to leave room for the send and receive regions of the reduction)
+  switch (cluster_config(a_rows, plan.bn, ceil_div(ceil_div(k, kBK), plan.splits))) {
+    case ClusterConfig::k32x3: return launch<32, 3, 64, kFormCluster>(p, a_map, b_map, stream);
+    case ClusterConfig::k32x8: return launch<32, 8, 64, kFormCluster>(p, a_map, b_map, stream);
+    case ClusterConfig::k64x4: return launch<64, 4, 64, kFormCluster>(p, a_map, b_map, stream);
+    case ClusterConfig::k64x6: return launch<64, 6, 64, kFormCluster>(p, a_map, b_map, stream);
+    case ClusterConfig::k128x4: return launch<128, 4, 64, kFormCluster>(p, a_map, b_map, stream);
+    case ClusterConfig::k32x6r128: return launch<32, 6, 128, kFormCluster>(p, a_map, b_map, stream);
+    case ClusterConfig::k64x4r128: return launch<64, 4, 128, kFormCluster>(p, a_map, b_map, stream);
+  }
+  return B200_ERR_UNSUPPORTED;
 }
 
 // Slices of row sums of squares that the cluster split-K projection leaves (N tiles x K slices);

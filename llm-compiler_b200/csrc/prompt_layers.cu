@@ -32,11 +32,6 @@ extern "C" int b200_qwen2_prompt_layers(const b200_prompt_layer* layers, int64_t
     };
     auto linear = [&](const void* x, const void* weight, const void* bias, const void* residual, void* out, int64_t k,
                       int64_t n, int epilogue) {
-      if (c->dtype == B200_BF16 && epilogue != B200_EPILOGUE_SWIGLU) {
-        const int code = linear_narrow_prompt(x, weight, bias, residual, out, rows, k, n, status,
-                                              static_cast<cudaStream_t>(stream));
-        if (code != B200_ERR_UNSUPPORTED) return code;
-      }
       return b200_linear(x, weight, bias, residual, out, rows, k, n, k, c->dtype, epilogue, c->workspace,
                          c->workspace_bytes, status, stream);
     };

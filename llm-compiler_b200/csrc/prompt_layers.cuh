@@ -12,8 +12,4 @@ int rope_into_cache(const void* qkv, const void* cosine, const void* sine, void*
                     int64_t batch, int64_t tokens, int64_t q_heads, int64_t kv_heads, int64_t head_dim, int64_t capacity,
                     int dtype, cudaStream_t stream);
 
-// linear_tcgen05.cu: a bf16 projection of a short prompt against a narrow matrix, or B200_ERR_UNSUPPORTED.
-int linear_narrow_prompt(const void* input, const void* weight, const void* bias, const void* residual, void* output,
-                         int64_t m, int64_t k, int64_t n, int32_t* status, cudaStream_t stream);
-
 }  // namespace b200

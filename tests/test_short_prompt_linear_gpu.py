@@ -1,5 +1,5 @@
 """Projections of short prompts against the 64-bit product at the lines of the dispatch: too few tiles for the persistent
-kernel, and the row counts around it. (K cut over a cluster is tested with the prompt's layers and the split-K form.)
+kernel, and the row counts around it.
 
 Bound of an element: K 2^-23 sum |x w| for fp32 sums in any order, and half an ulp (at most 2^-8 of a bf16 value, 2^-11
 of an fp16 value) for every rounding: one, or two in front of a residual."""
