@@ -11,9 +11,13 @@
 //
 // fp16 takes this kernel for every mask and mode. Its scores stay in the natural domain (an additive mask may hold
 // the type's lowest value, whose multiple by log2 e would overflow to -inf and turn a uniform row into NaN), and
-// its probabilities, which the CUDA-core kernel holds in fp32, enter P V as the sum of two fp16 numbers: high part
-// and remainder, 22 bits. 2 x 515 tokens, 14 heads of 64: 1851 us on the CUDA-core kernel (one CTA per query row,
-// keys and values re-read by every row) -> 26 us.
+// its probabilities stay fp32 numbers: expf as in the CUDA-core kernel, and 2^15 p enters P V as three fp16 operands with
+// sums of their own, 2^15 p rounded, then 2^11 times what is left, twice: 33 bits, and no probability above 2^-62 of the
+// row's largest is lost (as one fp16 number those below 2^-25 would count in the denominator only). The sums of a key
+// tile are added to the running output in fp32: tensor cores cut an accumulator's last bits off at every step, and a
+// chain through the whole context would show it. Errors against 64 bits at 130 - 4096 tokens are those of the CUDA-core
+// kernel to four digits. 2 x 515 tokens, 14 heads of 64: 1851 us on the CUDA-core kernel (one CTA per
+// query row, keys and values re-read by every row) -> 36 us (26 with one remainder and a chain through the context).
 //
 // fp32 kernel: CUDA cores with IEEE fp32 dots for small full-precision graphs.
 #include <math.h>
@@ -28,6 +32,7 @@ constexpr int kThreads = kWarps * 32;
 constexpr int kBM = 64;  // query rows per CTA
 constexpr int kBN = 64;  // keys per tile
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kHalfScale = 32768.0f, kPartScale = 2048.0f;  // of fp16 probabilities as operands (see above)
 
 template <typename T>
 struct PrefillParams {
@@ -65,7 +70,7 @@ __device__ __forceinline__ uint32_t tile_offset(int row, int chunk) {
 
 // One output row by a whole warp, key by key, touching only the keys that the row sees: what an fp16 row is put right
 // with when its tile product met an infinite or NaN value row of a key that it does not see (0 * inf; fp16
-// activations do overflow). A row that is NaN by itself stays so.
+// activations do overflow). (A row that is NaN by itself, for its scores or for seeing nothing, is left alone.)
 template <typename T, int D>
 __device__ __noinline__ void attend_row(const PrefillParams<T>& p, int b, int hq, int qrow) {
   const int lane = threadIdx.x & 31, kvh = hq / p.groups;
@@ -95,6 +100,7 @@ __device__ __noinline__ void attend_row(const PrefillParams<T>& p, int b, int hq
 template <typename T, int D, int STAGES>
 __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const PrefillParams<T> p) {
   constexpr bool kHalf = IsHalf<T>::value;
+  constexpr int kParts = kHalf ? 3 : 1;
   constexpr int kChunksPerRow = D / 8;
   constexpr int kTileBytes = kBN * D * 2;
   constexpr int kQBytes = kBM * D * 2;
@@ -163,7 +169,7 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
   // scores in the log2 domain (bf16) or the natural one (fp16: see the top of this file)
   constexpr float kUnit = kHalf ? 1.0f : kLog2e;
   const float scale = p.scale * kUnit;
-  auto probability = [](float x) { return fast_exp2(kHalf ? x * kLog2e : x); };
+  auto probability = [](float x) { return kHalf ? expf(x) : fast_exp2(x); };
   const int mat = lane >> 3;
   const int row_lo = q0 + warp * 16 + (lane >> 2);  // this thread's query rows: row_lo, row_lo + 8
 
@@ -241,44 +247,70 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
       m_run[r] = m_new;
       l_run[r] *= alpha[r];
     }
-#pragma unroll
-    for (int i = 0; i < kNTiles; ++i) {
-      oacc[i][0] *= alpha[0];
-      oacc[i][1] *= alpha[0];
-      oacc[i][2] *= alpha[1];
-      oacc[i][3] *= alpha[1];
-    }
+    // P as an operand: bf16, or (fp16) the parts of 2^15 P
+    uint32_t pa[kBN / 16][kParts][4];
+    float l_tile[2] = {kHalf ? 0.0f : l_run[0], kHalf ? 0.0f : l_run[1]};  // (fp16: the denominators by the tile as well)
 #pragma unroll
     for (int kk = 0; kk < kBN / 16; ++kk) {
-      uint32_t pa[4], pa_low[kHalf ? 4 : 1];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int nt = kk * 2 + half;
-        const float p0 = probability(sacc[nt][0] - m_safe[0]);
-        const float p1 = probability(sacc[nt][1] - m_safe[0]);
-        const float p2 = probability(sacc[nt][2] - m_safe[1]);
-        const float p3 = probability(sacc[nt][3] - m_safe[1]);
-        l_run[0] += p0 + p1;
-        l_run[1] += p2 + p3;
-        pa[half * 2] = Elem<T>::pack(p0, p1);
-        pa[half * 2 + 1] = Elem<T>::pack(p2, p3);
+        float p0 = probability(sacc[nt][0] - m_safe[0]);
+        float p1 = probability(sacc[nt][1] - m_safe[0]);
+        float p2 = probability(sacc[nt][2] - m_safe[1]);
+        float p3 = probability(sacc[nt][3] - m_safe[1]);
+        l_tile[0] += p0 + p1;
+        l_tile[1] += p2 + p3;
         if constexpr (kHalf) {
-          pa_low[half * 2] = Elem<T>::pack(p0 - Elem<T>::lo(pa[half * 2]), p1 - Elem<T>::hi(pa[half * 2]));
-          pa_low[half * 2 + 1] = Elem<T>::pack(p2 - Elem<T>::lo(pa[half * 2 + 1]), p3 - Elem<T>::hi(pa[half * 2 + 1]));
+          p0 *= kHalfScale; p1 *= kHalfScale; p2 *= kHalfScale; p3 *= kHalfScale;
+        }
+#pragma unroll
+        for (int part = 0; part < kParts; ++part) {
+          const uint32_t lo = Elem<T>::pack(p0, p1), hi = Elem<T>::pack(p2, p3);
+          pa[kk][part][half * 2] = lo;
+          pa[kk][part][half * 2 + 1] = hi;
+          p0 = (p0 - Elem<T>::lo(lo)) * kPartScale; p1 = (p1 - Elem<T>::hi(lo)) * kPartScale;
+          p2 = (p2 - Elem<T>::lo(hi)) * kPartScale; p3 = (p3 - Elem<T>::hi(hi)) * kPartScale;
         }
       }
+    }
 #pragma unroll
-      for (int np = 0; np < kNTiles / 2; ++np) {
+    for (int r = 0; r < 2; ++r) l_run[r] = kHalf ? l_run[r] + l_tile[r] : l_tile[r];
+#pragma unroll
+    for (int np = 0; np < kNTiles / 2; ++np) {
+      // bf16 adds onto the rescaled output, fp16 sums each part of the tile by itself
+      float sum[kParts][2][4];
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          sum[0][c][e] = kHalf ? 0.0f : oacc[np * 2 + c][e] * alpha[e >> 1];
+#pragma unroll
+          for (int part = 1; part < kParts; ++part) sum[part][c][e] = 0.0f;
+        }
+#pragma unroll
+      for (int kk = 0; kk < kBN / 16; ++kk) {
         uint32_t vb[4];
         const int r = kk * 16 + ((mat & 1) << 3) + (lane & 7);
         ldmatrix_x4_trans(vb, vsm + tile_offset<D>(r, np * 2 + (mat >> 1)));
-        mma_16816<T>(oacc[np * 2], pa, vb[0], vb[1]);
-        mma_16816<T>(oacc[np * 2 + 1], pa, vb[2], vb[3]);
-        if constexpr (kHalf) {
-          mma_16816<T>(oacc[np * 2], pa_low, vb[0], vb[1]);
-          mma_16816<T>(oacc[np * 2 + 1], pa_low, vb[2], vb[3]);
+#pragma unroll
+        for (int part = 0; part < kParts; ++part) {
+          mma_16816<T>(sum[part][0], pa[kk][part], vb[0], vb[1]);
+          mma_16816<T>(sum[part][1], pa[kk][part], vb[2], vb[3]);
         }
       }
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float& out = oacc[np * 2 + c][e];
+          if constexpr (kHalf) {
+            const float tile_sum = fmaf(fmaf(sum[2][c][e], 1.0f / kPartScale, sum[1][c][e]), 1.0f / kPartScale, sum[0][c][e]);
+            out = fmaf(out, alpha[e >> 1], tile_sum);
+          } else {
+            out = sum[0][c][e];
+          }
+        }
     }
   }
   cp_async_wait<0>();
@@ -288,25 +320,27 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
   }
-  bool nan_row[2] = {false, false};
+  bool again[2] = {false, false};  // fp16: NaN, though the row sees a key and its scores are numbers
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int qrow = row_lo + r * 8;
     if (qrow >= tokens) continue;
-    const float inv = 1.0f / l_run[r];  // all-masked row: 0 * inf = NaN, as the oracle
+    // all-masked row: 0 * inf = NaN, as the oracle
+    const float inv = 1.0f / l_run[r];
+    auto quotient = [&](float sum) { return kHalf ? sum * (1.0f / kHalfScale) / l_run[r] : sum * inv; };
     T* orow = p.out + ((static_cast<int64_t>(b) * tokens + qrow) * p.q_heads + hq) * D;
 #pragma unroll
     for (int nt = 0; nt < kNTiles; ++nt) {
       const int col = nt * 8 + (lane & 3) * 2;
-      *reinterpret_cast<uint32_t*>(orow + col) =
-          Elem<T>::pack(oacc[nt][r * 2] * inv, oacc[nt][r * 2 + 1] * inv);
-      nan_row[r] = nan_row[r] || isnan(oacc[nt][r * 2] * inv) || isnan(oacc[nt][r * 2 + 1] * inv);
+      const float y0 = quotient(oacc[nt][r * 2]), y1 = quotient(oacc[nt][r * 2 + 1]);
+      *reinterpret_cast<uint32_t*>(orow + col) = Elem<T>::pack(y0, y1);
+      again[r] = again[r] || (l_run[r] > 0.0f && (isnan(y0) || isnan(y1)));
     }
   }
   if constexpr (kHalf) {
     __syncwarp();  // the rows stored above come before those that are stored again
     for (int i = 0; i < 16; ++i)
-      if (__any_sync(0xffffffffu, (lane >> 2) == (i & 7) && nan_row[i >> 3]))
+      if (__any_sync(0xffffffffu, (lane >> 2) == (i & 7) && again[i >> 3]))
         attend_row<T, D>(p, b, hq, q0 + warp * 16 + i);
   }
 }

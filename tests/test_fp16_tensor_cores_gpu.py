@@ -5,6 +5,8 @@ Tolerance: either kernel sums exact fp16 products in fp32 (order: K x 2^-24 of t
 follows) and rounds a result to 11 bits; a SwiGLU rounds three factors, attention one quotient. 4 x 2^-11 of the
 largest result covers the worst of them."""
 
+import math
+
 import pytest
 import torch
 
@@ -57,6 +59,25 @@ def test_linear_overflow_stays_in_its_row_and_column():
     x[5, 7] = float("inf")
     w[9, 0] = float("nan")
     close(b200.b200_linear(x, w), b200.b200_linear(unaligned(x), w))
+
+
+# Probabilities far below the row's largest count alike in P V and in the denominator: one key 2^-octaves above all others
+# (whose value is zero), so that the result is the others' sum. Its error: the score's and the exponential's (2^-22
+# together), 2 t 2^-24 of the sums, one fp16 rounding.
+@pytest.mark.parametrize("octaves", [14, 20, 25, 30])
+@pytest.mark.parametrize("t,d", [(130, 64), (515, 128), (4096, 64), (4096, 128)])
+def test_prefill_attention_of_a_long_tail(t, d, octaves):
+    q, k, v = (torch.zeros(1, 2, t, d) for _ in range(3))
+    v[:] = 300.0 + torch.randn(1, 2, t, d, generator=torch.Generator().manual_seed(octaves))
+    v[:, :, 0], q[..., 0], k[:, :, 0, 0] = 0.0, 1.0, octaves * 0.6931
+    q, k, v = q.half().cuda(), k.half().cuda(), v.half().cuda()
+    scale = 1.0
+    largest = math.exp(-k[0, 0, 0, 0].double().item())  # of the others, against the first key's
+    others = torch.arange(t, device="cuda").double()[None, None, :, None]
+    expected = v.double().cumsum(2) * largest / (1 + others * largest)
+    out = b200.b200_prefill_attention(q, k, v, None, scale=scale, causal=True).double()
+    bound = (2.0 ** -20 + 2 * t * 2.0 ** -24 + 2.0 ** -11) * expected.abs() + 2.0 ** -25  # (half a subnormal's step)
+    assert ((out - expected).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("mode", ["fast", "pytorch_compatible"])
