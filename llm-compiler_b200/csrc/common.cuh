@@ -313,6 +313,18 @@ struct Elem<__half> {
   }
 };
 
+// silu for a fused SwiGLU epilogue. bf16: x / (1 + 2^(-x log2 e)) on the special-function unit (ex2.approx, rcp.approx:
+// a few ulp of fp32, far below the bf16 rounding that follows). An IEEE expf + division costs ~160 cycles per element on
+// the epilogue's lone warps, which made the epilogue of the gate|up projection longer than its main loop.
+// fp16 keeps expf; x / d is x (1 / d) corrected by its remainder, which after the rounding to fp16 is the IEEE
+// quotient's result for every fp16 x. (Beyond 80 the quotient is x, or rounds to zero; the infinities need no remainder.)
+template <typename T>
+__device__ __forceinline__ float silu_epilogue(float x) {
+  if constexpr (!IsHalf<T>::value) return __fdividef(x, 1.0f + exp2f(-1.4426950408889634f * x));
+  const float d = 1.0f + expf(-x), r = __fdividef(1.0f, d), q = x * r;
+  return fabsf(x) < 80.0f ? fmaf(fmaf(-q, d, x), r, q) : q;
+}
+
 // Calls f(TypeTag<T>{}) with the element type of a dtype code; false for an unknown code.
 template <typename T>
 struct TypeTag { using type = T; };

@@ -53,9 +53,6 @@ struct RowsParams {
   float norm_eps;
 };
 
-// as in linear_tcgen05.cu
-__device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + exp2f(-1.4426950408889634f * x)); }
-
 // x by way of L1: all CTAs of an SM read the same few kilobytes, whose L2 slices would otherwise answer each of them
 __device__ __forceinline__ void copy_through_l1(uint32_t smem_addr, const void* p, int bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr), "l"(p), "r"(bytes));
@@ -240,7 +237,7 @@ __global__ void __launch_bounds__(kMaxSlices * 32) linear_rows16_kernel(const Ro
       for (int e = 0; e < 4; e += 2) {
         if (e >= have) break;
         Elem<T>::round_pair(v[e], v[e + 1]);
-        Elem<T>::store(p.out + static_cast<int64_t>(row) * (p.n / 2) + (n + e) / 2, Elem<T>::round(silu_fast(v[e])) * v[e + 1]);
+        Elem<T>::store(p.out + static_cast<int64_t>(row) * (p.n / 2) + (n + e) / 2, Elem<T>::round(silu_epilogue<T>(v[e])) * v[e + 1]);
       }
       continue;
     }

@@ -89,14 +89,6 @@ struct Tcgen05ParamsOf {
 };
 using Tcgen05Params = Tcgen05ParamsOf<__nv_bfloat16>;
 
-// silu for the fused SwiGLU epilogue: x / (1 + 2^(-x log2 e)) on the special-function unit
-// (ex2.approx, rcp.approx: a few ulp of fp32, far below the bf16 rounding that follows). An
-// IEEE expf + division costs ~160 cycles per element on the epilogue's lone warps, which made
-// the epilogue of the gate|up projection longer than its main loop.
-__device__ __forceinline__ float silu_f32(float x) {
-  return __fdividef(x, 1.0f + exp2f(-1.4426950408889634f * x));
-}
-
 // Bias onto 32 accumulator columns (16-byte loads where all 32 columns exist and are aligned).
 template <typename T>
 __device__ __forceinline__ void add_bias(const Tcgen05ParamsOf<T>& p, int col0, int n_end, float (&v)[32]) {
@@ -154,7 +146,7 @@ __device__ __forceinline__ void swiglu_of_chunk(float (&v)[32], float (&y)[16]) 
   for (int j = 0; j < 16; j += 2) {
     Elem<T>::round_pair(v[2 * j], v[2 * j + 1]);
     Elem<T>::round_pair(v[2 * j + 2], v[2 * j + 3]);
-    float g0 = silu_f32(v[2 * j]), g1 = silu_f32(v[2 * j + 2]);
+    float g0 = silu_epilogue<T>(v[2 * j]), g1 = silu_epilogue<T>(v[2 * j + 2]);
     Elem<T>::round_pair(g0, g1);
     y[j] = g0 * v[2 * j + 1];
     y[j + 1] = g1 * v[2 * j + 3];

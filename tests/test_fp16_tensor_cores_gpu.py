@@ -61,6 +61,18 @@ def test_linear_overflow_stays_in_its_row_and_column():
     close(b200.b200_linear(x, w), b200.b200_linear(unaligned(x), w))
 
 
+@pytest.mark.parametrize("m", [8, 16, 70, 1100])  # streamed rows, warp-level, tcgen05, the persistent kernel
+def test_swiglu_of_every_gate_is_that_of_the_cuda_cores_bit_for_bit(m):
+    gates = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.float16)
+    for part in gates.view(-1, 4096):
+        bias = torch.stack([part, torch.full_like(part, 1.5)], dim=1).flatten().cuda()
+        x, w = torch.zeros(m, 64).half().cuda(), torch.zeros(8192, 64).half().cuda()
+        tensor_cores, cuda_cores = (b200.b200_linear(rows, w, bias, epilogue="swiglu") for rows in (x, unaligned(x)))
+        assert torch.equal(tensor_cores.isnan(), cuda_cores.isnan())
+        assert torch.equal(tensor_cores.nan_to_num(nan=0.0, posinf=7e4, neginf=-7e4),
+                           cuda_cores.nan_to_num(nan=0.0, posinf=7e4, neginf=-7e4))
+
+
 # Probabilities far below the row's largest count alike in P V and in the denominator: one key 2^-octaves above all others
 # (whose value is zero), so that the result is the others' sum. Its error: the score's and the exponential's (2^-22
 # together), 2 t 2^-24 of the sums, one fp16 rounding.
