@@ -61,7 +61,7 @@ __device__ __forceinline__ void epilogue_pair(const LinearParams<T>& p, int m, i
     v0 = __fadd_rn(v0, Elem<T>::load(p.residual + o));
     if (has1) v1 = __fadd_rn(v1, Elem<T>::load(p.residual + o + 1));
   }
-  if (has1 && (o & 1) == 0) {
+  if (has1 && (reinterpret_cast<uintptr_t>(p.out + o) & 3u) == 0) {
     *reinterpret_cast<uint32_t*>(p.out + o) = Elem<T>::pack(v0, v1);
   } else {
     Elem<T>::store(p.out + o, v0);

@@ -12,7 +12,7 @@ import torch
 
 from oracle import serve_ops
 import llm_compiler_b200 as b200
-from llm_compiler_b200 import kernels
+from llm_compiler_b200 import _lib, kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +123,30 @@ def test_prefill_attention_does_not_read_values_that_a_row_does_not_see():
     out = b200.b200_prefill_attention(q, k, v, None, scale=0.125, causal=True)
     assert out[0, 1, :70].isfinite().all() and not out[0, 1, 70:].isfinite().any()
     assert out[0, 0, :90].isfinite().all() and out[0, 0, 90:].isnan().all()
+
+
+# A C caller's output may start on any element. (The warp-level kernel stores pairs, the others up to 16 bytes at once.)
+@pytest.mark.parametrize("variant", [None, "mma.sync"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n", [(1, 896, 896), (8, 72, 130), (16, 72, 130), (33, 136, 64), (64, 136, 2400), (70, 72, 258),
+                                   (1100, 72, 904)])
+def test_linear_output_on_an_odd_element(m, k, n, dtype, variant):
+    g = torch.Generator().manual_seed(m + n)
+    x, w, bias = (torch.randn(*s, generator=g).to(dtype).cuda() for s in ((m, k), (n, k), (n,)))
+    library, code = _lib.load(), {torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}[dtype]
+    for epilogue, columns in ((_lib.EPILOGUE_NONE, n), (_lib.EPILOGUE_RESIDUAL, n), (_lib.EPILOGUE_SWIGLU, n // 2)):
+        residual = torch.randn(m, n, generator=g).to(dtype).cuda()
+        workspace = torch.zeros(library.b200_linear_workspace_bytes(m, k, n, code, epilogue), dtype=torch.uint8, device="cuda")
+        results = []
+        for offset in (0, 1):
+            storage = torch.full((m * columns + 2,), 77.0, dtype=dtype, device="cuda")
+            output = storage[offset:offset + m * columns]
+            with kernels.kernel_variants(linear=variant):
+                assert library.b200_linear(x.data_ptr(), w.data_ptr(), bias.data_ptr(), residual.data_ptr(),
+                                           output.data_ptr(), m, k, n, k, code, epilogue, workspace.data_ptr(),
+                                           workspace.numel(), kernels.runtime().status.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream) == 0
+            assert (storage[:offset] == 77.0).all() and (storage[offset + m * columns:] == 77.0).all()
+            results.append(output.clone())
+        assert torch.equal(*results)
+    kernels.runtime().check_status()
