@@ -283,7 +283,7 @@ class Qwen2Engine(ServingEngine):
         # nothing to hide between launches of 100 us, and waiting CTAs of the next one cost them 1 %: 4 x 4096 tokens of
         # the 0.5B model, some 3000 of the 7B.)
         chained = self.programmatic_launch and batch * tokens * cfg.hidden_size <= 4 << 20
-        with kernels.launch_mode(programmatic=chained, constant_weights=chained):
+        with kernels.launch_mode(programmatic=chained, constant_weights=chained, keep_variants=True):
             x = kernels.b200_qwen2_prompt_layers(
                 x, self.layers, self.state.keys, self.state.values, cosine, sine, self.positions,  # all zero right now
                 q_heads=cfg.num_heads, scale=self.scale, epsilon=cfg.rms_norm_eps, numerical_mode=self.mode,
@@ -377,7 +377,8 @@ class Qwen2Engine(ServingEngine):
         elif self.dtype == torch.bfloat16:
             self._decode_step_separate()
         else:  # (fp32, fp16: the norms, RoPE, attention and projections of few rows wait on the device)
-            with kernels.launch_mode(programmatic=self.programmatic_launch, constant_weights=self.programmatic_launch):
+            with kernels.launch_mode(programmatic=self.programmatic_launch, constant_weights=self.programmatic_launch,
+                                     keep_variants=True):
                 self._decode_step_separate()
 
     def _decode_step_chain(self) -> None:

@@ -109,13 +109,14 @@ def launch_count(device: torch.device | None = None) -> int:
 # ------------------------------------------------------------------------- helpers ----
 @contextlib.contextmanager
 def launch_mode(*, programmatic: bool, constant_weights: bool = False,
-                stable_kv_prefix: bool = False):
+                stable_kv_prefix: bool = False, keep_variants: bool = False):
     """Scope in which the decode-chain kernels are launched with programmatic dependent launch
     (each may become resident while its predecessor still runs and waits on the device before
     touching a tensor). constant_weights promises that no kernel in flight writes a weight
     tensor, which lets the tcgen05 linear fetch weight tiles before that wait; stable_kv_prefix
     promises the same for lengths[] and every KV row below lengths[b] - 1, which lets decode
-    attention fill its pipeline before the wait. The mode belongs to the calling thread (the
+    attention fill its pipeline before the wait. keep_variants leaves the choice of an enclosing
+    kernel_variants scope in force (otherwise the scope runs the library's own). The mode belongs to the calling thread (the
     library keeps it thread-local: engines on other threads are not affected); launches captured
     into a CUDA graph keep the mode they were captured with."""
 
@@ -123,6 +124,8 @@ def launch_mode(*, programmatic: bool, constant_weights: bool = False,
         (_lib.LAUNCH_CONSTANT_WEIGHTS if constant_weights else 0) | \
         (_lib.LAUNCH_STABLE_KV_PREFIX if stable_kv_prefix else 0)
     library = _lib.load()
+    if keep_variants:
+        flags |= library.b200_get_launch_mode() & (_lib.LAUNCH_LINEAR_WARP_LEVEL | _lib.LAUNCH_PREFILL_WARP_LEVEL)
     previous = library.b200_set_launch_mode(flags)
     if previous < 0:
         raise ValueError(f"b200_set_launch_mode: {_lib.error_string(previous)}")

@@ -8,7 +8,7 @@ from pathlib import Path
 
 import pytest
 
-from llm_compiler_b200 import _lib
+from llm_compiler_b200 import _lib, kernels
 
 HEADER = Path(__file__).resolve().parent.parent / "include" / "b200_serve.h"
 
@@ -79,3 +79,17 @@ def test_operands_on_another_gpu_are_refused_before_any_launch(monkeypatch):
     kernels._guard_current_device(torch.device("cuda"))  # no index: the current device
     with pytest.raises(ValueError, match="current device is cuda:0"):
         kernels._guard_current_device(torch.device("cuda", 1))
+
+
+def test_a_launch_mode_scope_can_leave_the_chosen_variants_in_force():
+    library = _lib.load()
+    chosen = _lib.LAUNCH_LINEAR_WARP_LEVEL | _lib.LAUNCH_PREFILL_WARP_LEVEL
+    with kernels.kernel_variants(linear="mma.sync", prefill_attention="mma.sync"):
+        with kernels.launch_mode(programmatic=True, constant_weights=True, keep_variants=True):
+            assert library.b200_get_launch_mode() == chosen | _lib.LAUNCH_PROGRAMMATIC | _lib.LAUNCH_CONSTANT_WEIGHTS
+        with kernels.launch_mode(programmatic=True):
+            assert library.b200_get_launch_mode() == _lib.LAUNCH_PROGRAMMATIC
+        assert library.b200_get_launch_mode() == chosen
+    with kernels.launch_mode(programmatic=True, keep_variants=True):
+        assert library.b200_get_launch_mode() == _lib.LAUNCH_PROGRAMMATIC
+    assert library.b200_get_launch_mode() == 0

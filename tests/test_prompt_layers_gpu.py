@@ -2,10 +2,12 @@
 and KV store in one kernel, whose roundings are the same, so every result is equal bit for bit. Every projection of more
 than 64 rows sums K in one chain, so a prompt's results do not depend on the prompts beside it either."""
 
+import contextlib
+
 import pytest
 import torch
 
-from llm_compiler_b200 import kernels, qwen2
+from llm_compiler_b200 import _lib, kernels, qwen2
 from llm_compiler_b200.engine import Qwen2Engine
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +66,50 @@ def test_a_prompt_is_the_same_bit_for_bit_beside_others(tokens):
     alone = Qwen2Engine(config, weights, batch=1, capacity=320).prefill(ids[:1], all_logits=True)
     beside = Qwen2Engine(config, weights, batch=5, capacity=320).prefill(ids, all_logits=True)
     assert torch.equal(alone[0], beside[0])
+
+
+@pytest.mark.parametrize("switch", ["scope", "environment"])
+@pytest.mark.parametrize("batch,tokens", [(1, 9), (1, 77), (2, 300)])
+def test_named_variants_reach_the_layers(batch, tokens, switch, monkeypatch):
+    config = qwen2.Qwen2Config(hidden_size=896, intermediate_size=2048, num_layers=2, num_heads=14, num_kv_heads=2,
+                               vocab_size=1000)
+    weights = qwen2.make_weights(config, seed=tokens, dtype=torch.bfloat16, device="cuda", reproducible=False)
+    engine = Qwen2Engine(config, weights, batch=batch, capacity=320)
+    ids = torch.randint(0, 1000, (batch, tokens), generator=torch.Generator().manual_seed(batch))
+    own = engine.prefill(ids).clone()
+    scope = contextlib.nullcontext()
+    if switch == "scope":
+        scope = kernels.kernel_variants(linear="mma.sync", prefill_attention="mma.sync")
+    else:
+        monkeypatch.setenv("B200_LINEAR_PATH", "mma.sync")
+        monkeypatch.setenv("B200_PREFILL_ATTENTION_PATH", "mma.sync")
+    with scope:
+        expected, cached = _operator_by_operator(engine, ids)
+        assert torch.equal(engine.prefill(ids), expected)
+        for layer, (keys, values) in enumerate(cached):
+            assert torch.equal(engine.state.keys[layer][:, :tokens], keys)
+            assert torch.equal(engine.state.values[layer][:, :tokens], values)
+    assert not torch.equal(own, expected)  # (the variants sum K in other orders)
+    kernels.runtime().check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_named_variants_reach_the_decode_step(dtype, monkeypatch):
+    config = qwen2.Qwen2Config(hidden_size=256, intermediate_size=512, num_layers=2, num_heads=4, num_kv_heads=2,
+                               vocab_size=1000)
+    weights = qwen2.make_weights(config, seed=4, dtype=dtype, device="cuda", reproducible=False)
+    engine = Qwen2Engine(config, weights, batch=2, capacity=64)
+    engine.prefill(torch.randint(0, 1000, (2, 5), generator=torch.Generator().manual_seed(2)))
+    modes, linear = [], kernels.b200_linear
+
+    def recorded(*args, **options):
+        modes.append(_lib.load().b200_get_launch_mode())
+        return linear(*args, **options)
+
+    monkeypatch.setattr(kernels, "b200_linear", recorded)
+    with kernels.kernel_variants(linear="mma.sync"):
+        engine.decode_step()
+    engine.decode_step()
+    half = len(modes) // 2
+    assert half > 0 and all(mode & _lib.LAUNCH_LINEAR_WARP_LEVEL for mode in modes[:half])
+    assert not any(mode & _lib.LAUNCH_LINEAR_WARP_LEVEL for mode in modes[half:])
