@@ -346,7 +346,7 @@ typedef struct {
   void* attention;             /* [rows, q_heads head_dim] */
   void* gated;                 /* [rows, intermediate] */
   const void *cosine, *sine;   /* [rows, head_dim] */
-  const int64_t* positions;    /* [batch], zeros */
+  const int64_t* positions;    /* [batch], zeros: prompts start at 0 (read where k and v are stored apart from RoPE) */
   const int32_t* block_table;  /* NULL: contiguous caches */
   void* workspace;
   int64_t workspace_bytes, batch, tokens, q_heads, kv_heads, head_dim, hidden, intermediate, capacity;

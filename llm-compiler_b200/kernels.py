@@ -920,18 +920,29 @@ def b200_qwen2_prompt_layers(x: torch.Tensor, layers, keys, values, cosine: torc
     """All layers of a Qwen2 prompt from empty caches, issued by one native call (the operators' own entry points in
     the order of qwen2.py:236-304). x: B x T x hidden, dense, updated in place and returned; layers: the packed weights
     of Qwen2Engine; keys / values: each layer's buffers [B, capacity, kv_heads, head_dim], or with `block_table` its
-    block pools; positions: B zeros."""
+    block pools (`block_table`: int32 B x max_blocks); positions: B zeros, where every prompt starts (only the block
+    pools' store reads them)."""
 
-    device = _require_cuda(x, cosine, sine, positions, block_table, *keys, *values)
+    if not len(layers) == len(keys) == len(values):
+        raise ValueError("every layer needs its weights, its keys and its values")
+    names = ("input_norm", "qkv_w", "qkv_b", "o_w", "post_norm", "gate_up_w", "down_w")
+    device = _require_cuda(x, cosine, sine, positions, block_table, *keys, *values,
+                           *(layer[name] for layer in layers for name in names))
+    if not layers:
+        return x
+    if x.ndim != 3 or keys[0].ndim != 4:
+        raise ValueError("prompt rows must be B x T x hidden and KV buffers of rank 4")
     batch, tokens, hidden = x.shape
     _, capacity, kv_heads, dim = keys[0].shape
     rows, q_size, width = batch * tokens, q_heads * dim, (q_heads + 2 * kv_heads) * dim
     intermediate = layers[0]["down_w"].shape[1]
     pool = [0, 0, 0]
     if block_table is not None:
+        if block_table.dtype != torch.int32 or block_table.ndim != 2 or block_table.shape[0] != batch or \
+                not block_table.is_contiguous():
+            raise ValueError("block_table must be a contiguous int32 B x max_blocks tensor")
         pool = [keys[0].shape[0], capacity, block_table.shape[1]]
         capacity = pool[1] * pool[2]
-    names = ("input_norm", "qkv_w", "qkv_b", "o_w", "post_norm", "gate_up_w", "down_w")
     shapes = dict(input_norm=(hidden,), qkv_w=(width, hidden), qkv_b=(width,), o_w=(hidden, q_size), post_norm=(hidden,),
                   gate_up_w=(2 * intermediate, hidden), down_w=(hidden, intermediate))
     table = (_lib.PromptLayer * len(layers))()
@@ -949,8 +960,9 @@ def b200_qwen2_prompt_layers(x: torch.Tensor, layers, keys, values, cosine: torc
         (entry.input_norm, entry.qkv_weight, entry.qkv_bias, entry.o_weight, entry.post_norm, entry.gate_up_weight,
          entry.down_weight) = (operand.data_ptr() for operand in operands)
         entry.keys, entry.values = layer_keys.data_ptr(), layer_values.data_ptr()
-    if not x.is_contiguous() or tokens > capacity or positions.shape != (batch,) or positions.dtype != torch.int64 or \
-            (block_table is None and keys[0].shape[0] != batch):
+    if positions.shape != (batch,) or positions.dtype != torch.int64 or not positions.is_contiguous():
+        raise ValueError("positions must be a contiguous int64 batch vector")
+    if not x.is_contiguous() or tokens > capacity or (block_table is None and keys[0].shape[0] != batch):
         raise ValueError("prompt rows must be dense and fit the KV buffers")
     if cosine.shape != (batch, tokens, dim) or sine.shape != (batch, tokens, dim) or \
             not (cosine.is_contiguous() and sine.is_contiguous() and cosine.dtype == sine.dtype == x.dtype):

@@ -113,3 +113,37 @@ def test_named_variants_reach_the_decode_step(dtype, monkeypatch):
     half = len(modes) // 2
     assert half > 0 and all(mode & _lib.LAUNCH_LINEAR_WARP_LEVEL for mode in modes[:half])
     assert not any(mode & _lib.LAUNCH_LINEAR_WARP_LEVEL for mode in modes[half:])
+
+
+def _refused(engine, ids, **changed):
+    cfg = engine.config
+    batch, tokens = ids.shape
+    cosine, sine = kernels.b200_rope_table(torch.arange(tokens, device="cuda").repeat(batch, 1), engine.inv_freq, engine.dtype)
+    operands = dict(x=kernels.b200_embedding(engine.embed, ids), layers=engine.layers, keys=engine.state.keys,
+                    values=engine.state.values, cosine=cosine, sine=sine, positions=engine.positions,
+                    block_table=engine.state.block_table if engine.paged else None)
+    operands.update(changed)
+    with pytest.raises(ValueError):
+        kernels.b200_qwen2_prompt_layers(**operands, q_heads=cfg.num_heads, scale=engine.scale, epsilon=cfg.rms_norm_eps)
+
+
+def test_operands_are_checked_before_any_launch():
+    config = qwen2.Qwen2Config(hidden_size=128, intermediate_size=256, num_layers=2, num_heads=2, num_kv_heads=2,
+                               vocab_size=100)
+    weights = qwen2.make_weights(config, seed=1, dtype=torch.bfloat16, device="cuda", reproducible=False)
+    ids = torch.zeros(2, 5, dtype=torch.int64, device="cuda")
+    engine = Qwen2Engine(config, weights, batch=2, capacity=32)
+    for name in ("input_norm", "qkv_w", "qkv_b", "o_w", "post_norm", "gate_up_w", "down_w"):
+        on_host = [engine.layers[0], dict(engine.layers[1], **{name: engine.layers[1][name].cpu()})]
+        _refused(engine, ids, layers=on_host)
+        _refused(engine, ids, layers=[engine.layers[0], dict(engine.layers[1], **{name: engine.layers[1][name][:-1]})])
+    _refused(engine, ids, keys=engine.state.keys[:1])
+    _refused(engine, ids, values=engine.state.values[:1])
+    _refused(engine, ids, layers=engine.layers[:1])
+    _refused(engine, ids, positions=engine.positions.int())
+    _refused(engine, ids, positions=torch.zeros(4, dtype=torch.int64, device="cuda")[::2])
+    _refused(engine, ids, x=kernels.b200_embedding(engine.embed, ids)[0])
+    paged = Qwen2Engine(config, weights, batch=2, capacity=256, kv_layout="paged")
+    table = paged.state.block_table
+    for wrong in (table.long(), table[:1], table[0], table.cpu(), table.repeat(1, 2)[:, ::2]):
+        _refused(paged, ids, block_table=wrong)
