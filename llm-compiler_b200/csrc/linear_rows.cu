@@ -339,8 +339,14 @@ bool takes_few_rows(const FewRowsCall& c) {
   }();
   if (c.m > limit || c.m > kRows || c.splits < 1) return false;
   // A launch that is a chain of latencies. A larger matrix is a stream, which the tcgen05 kernels' TMA rings keep fuller
-  // than one warp a slice can: 151936 x 896 56 against 82 us on 1 row, four layers of Qwen2-7B 688 against 955.
-  if (c.n * c.k > (10 << 20)) return false;
+  // than one warp a slice can: 151936 x 896 56 against 82 us on 1 row, four layers of Qwen2-7B 688 against 955. The line
+  // lies where the first form loses. us in a chain of launches, tcgen05 -> here, 1 and 8 rows, N x K in Mi elements:
+  //    2.2, 1536 x 1536:   residual 6.3, 6.3 -> 4.3, 4.6; fp32 sums 3.7, 3.9 -> 2.9, 3.1; norm + SwiGLU 10.4 -> 7.2, 7.4
+  //    9.0, 3072 x 3072:   residual 9.4, 9.6 -> 6.7, 8.1; fp32 sums 6.5, 6.6 -> 6.2, 5.6; norm + SwiGLU 20.6, 18.9 -> 15.1
+  //    9.0, 6144 x 1536:   residual 12.1, 12.2 -> 7.9, 8.9; fp32 sums 6.8, 6.8 -> 6.2, 5.6
+  //   10.0, 10240 x 1024:  residual 10.4, 10.6 -> 6.8, 7.1; fp32 sums 7.3, 7.2 -> 6.4, 8.6; norm + SwiGLU 11.2 -> 12.9 (8 rows)
+  //   12.3, 3584 x 3584:   residual 11.7, 11.7 -> 8.3, 13.9
+  if (c.n * c.k > (9 << 20)) return false;
   if (c.sums == nullptr && c.splits > kMaxSlices) return false;
   if (c.row_squares != nullptr && blocks_per_slice(c) > x_ring(kLongRing)) return false;  // the helper reads the whole slice
   if (c.squares_out != nullptr && c.tile_columns > kColumns * kMaxSlices) return false;
