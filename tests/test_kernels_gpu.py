@@ -206,6 +206,21 @@ def test_rms_norm_3d_and_strided_rows():
         (exact if mode == "pytorch_compatible" else lambda a, e: close(a, e, BF16_TOL))(out, ref)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hidden", [896, 3584, 5408, 8192, 16384, 33000])
+def test_rms_norm_of_wide_rows(hidden, dtype):
+    """Up to 1024 threads a row, each with up to four pieces in registers, and rows beyond them. Two roundings, and fp32
+    sums of at most hidden / 128 terms a thread."""
+
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    x, w = (torch.randn(*s, generator=g, device="cuda").to(dtype) for s in ((3, hidden), (hidden,)))
+    expected = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    out = b200.b200_rms_norm(x, w, epsilon=1e-6, round_before_weight=True, numerical_mode="fast")
+    half = {torch.float32: 2.0 ** -24, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    bound = (2.02 * half + (hidden / 128 + 16) * 2.0 ** -24) * expected.abs() + 2.0 ** -23  # (fp16 subnormals)
+    assert ((out.double() - expected).abs() <= bound).all()
+
+
 # ---------------------------------------------------------------- decode attention ----
 @pytest.fixture(params=["tma", "cp.async"])
 def decode_loads(request, monkeypatch):
