@@ -1096,11 +1096,13 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
           bn = candidate;
         }
       }
-      // ... unless its tiles would not fill the SMs once (1030 rows x 896 columns: 36 of 148 have work; K 896 10.0 ->
-      // 9.0 us, K 4864 31.2 -> 28.3)
-      if (ceil_div(n, bn) * tiles_m < kNumSMs * 3 / 4) {
+      // ... unless so few tiles leave SMs idle that only 64-column ones fill them: all of these are resident at once.
+      // 1030 and 1800 rows x 896 columns: K 896 12.7 -> 9.9 and 13.1 -> 12.1 us, K 4864 34.3 -> 29.6 and 34.9 -> 32.3.
+      // (128-column tiles, which is what more rows would take, lose by their second wave or their shorter ring: 3000
+      // rows x 896 columns, K 4864 35.9 -> 39.6; 1200 x 1536, K 8960 56.9 -> 60.0.)
+      if (ceil_div(n, bn) * tiles_m < kNumSMs * 3 / 4 && filling_width() == 64) {
         persistent = false;
-        bn = filling_width();
+        bn = 64;
       }
     }
   } else {
