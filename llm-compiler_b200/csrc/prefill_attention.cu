@@ -100,7 +100,6 @@ __device__ __noinline__ void attend_row(const PrefillParams<T>& p, int b, int hq
 template <typename T, int D, int STAGES>
 __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const PrefillParams<T> p) {
   constexpr bool kHalf = IsHalf<T>::value;
-  constexpr int kParts = kHalf ? 3 : 1;
   constexpr int kChunksPerRow = D / 8;
   constexpr int kTileBytes = kBN * D * 2;
   constexpr int kQBytes = kBM * D * 2;
@@ -247,70 +246,89 @@ __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const Prefi
       m_run[r] = m_new;
       l_run[r] *= alpha[r];
     }
-    // P as an operand: bf16, or (fp16) the parts of 2^15 P
-    uint32_t pa[kBN / 16][kParts][4];
-    float l_tile[2] = {kHalf ? 0.0f : l_run[0], kHalf ? 0.0f : l_run[1]};  // (fp16: the denominators by the tile as well)
-#pragma unroll
-    for (int kk = 0; kk < kBN / 16; ++kk) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int nt = kk * 2 + half;
-        float p0 = probability(sacc[nt][0] - m_safe[0]);
-        float p1 = probability(sacc[nt][1] - m_safe[0]);
-        float p2 = probability(sacc[nt][2] - m_safe[1]);
-        float p3 = probability(sacc[nt][3] - m_safe[1]);
-        l_tile[0] += p0 + p1;
-        l_tile[1] += p2 + p3;
-        if constexpr (kHalf) {
-          p0 *= kHalfScale; p1 *= kHalfScale; p2 *= kHalfScale; p3 *= kHalfScale;
-        }
-#pragma unroll
-        for (int part = 0; part < kParts; ++part) {
-          const uint32_t lo = Elem<T>::pack(p0, p1), hi = Elem<T>::pack(p2, p3);
-          pa[kk][part][half * 2] = lo;
-          pa[kk][part][half * 2 + 1] = hi;
-          p0 = (p0 - Elem<T>::lo(lo)) * kPartScale; p1 = (p1 - Elem<T>::hi(lo)) * kPartScale;
-          p2 = (p2 - Elem<T>::lo(hi)) * kPartScale; p3 = (p3 - Elem<T>::hi(hi)) * kPartScale;
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r) l_run[r] = kHalf ? l_run[r] + l_tile[r] : l_tile[r];
-#pragma unroll
-    for (int np = 0; np < kNTiles / 2; ++np) {
-      // bf16 adds onto the rescaled output, fp16 sums each part of the tile by itself
-      float sum[kParts][2][4];
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          sum[0][c][e] = kHalf ? 0.0f : oacc[np * 2 + c][e] * alpha[e >> 1];
-#pragma unroll
-          for (int part = 1; part < kParts; ++part) sum[part][c][e] = 0.0f;
-        }
+    if constexpr (kHalf) {
+      // the parts of 2^15 P, and the tile's part of the denominators
+      uint32_t pa[kBN / 16][3][4];
+      float l_tile[2] = {0.0f, 0.0f};
 #pragma unroll
       for (int kk = 0; kk < kBN / 16; ++kk) {
-        uint32_t vb[4];
-        const int r = kk * 16 + ((mat & 1) << 3) + (lane & 7);
-        ldmatrix_x4_trans(vb, vsm + tile_offset<D>(r, np * 2 + (mat >> 1)));
 #pragma unroll
-        for (int part = 0; part < kParts; ++part) {
-          mma_16816<T>(sum[part][0], pa[kk][part], vb[0], vb[1]);
-          mma_16816<T>(sum[part][1], pa[kk][part], vb[2], vb[3]);
-        }
-      }
+        for (int half = 0; half < 2; ++half) {
+          float pr[4];
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+          for (int e = 0; e < 4; ++e) {
+            pr[e] = probability(sacc[kk * 2 + half][e] - m_safe[e >> 1]);
+            l_tile[e >> 1] += pr[e];
+            pr[e] *= kHalfScale;
+          }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float& out = oacc[np * 2 + c][e];
-          if constexpr (kHalf) {
-            const float tile_sum = fmaf(fmaf(sum[2][c][e], 1.0f / kPartScale, sum[1][c][e]), 1.0f / kPartScale, sum[0][c][e]);
-            out = fmaf(out, alpha[e >> 1], tile_sum);
-          } else {
-            out = sum[0][c][e];
+          for (int part = 0; part < 3; ++part) {
+            const uint32_t lo = Elem<T>::pack(pr[0], pr[1]), hi = Elem<T>::pack(pr[2], pr[3]);
+            pa[kk][part][half * 2] = lo;
+            pa[kk][part][half * 2 + 1] = hi;
+            pr[0] = (pr[0] - Elem<T>::lo(lo)) * kPartScale;
+            pr[1] = (pr[1] - Elem<T>::hi(lo)) * kPartScale;
+            pr[2] = (pr[2] - Elem<T>::lo(hi)) * kPartScale;
+            pr[3] = (pr[3] - Elem<T>::hi(hi)) * kPartScale;
           }
         }
+      }
+      l_run[0] += l_tile[0];
+      l_run[1] += l_tile[1];
+#pragma unroll
+      for (int np = 0; np < kNTiles / 2; ++np) {
+        float sum[3][2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < kBN / 16; ++kk) {
+          uint32_t vb[4];
+          const int r = kk * 16 + ((mat & 1) << 3) + (lane & 7);
+          ldmatrix_x4_trans(vb, vsm + tile_offset<D>(r, np * 2 + (mat >> 1)));
+#pragma unroll
+          for (int part = 0; part < 3; ++part) {
+            mma_16816<T>(sum[part][0], pa[kk][part], vb[0], vb[1]);
+            mma_16816<T>(sum[part][1], pa[kk][part], vb[2], vb[3]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float tile_sum = fmaf(fmaf(sum[2][c][e], 1.0f / kPartScale, sum[1][c][e]), 1.0f / kPartScale, sum[0][c][e]);
+            oacc[np * 2 + c][e] = fmaf(oacc[np * 2 + c][e], alpha[e >> 1], tile_sum);
+          }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kNTiles; ++i) {
+        oacc[i][0] *= alpha[0];
+        oacc[i][1] *= alpha[0];
+        oacc[i][2] *= alpha[1];
+        oacc[i][3] *= alpha[1];
+      }
+#pragma unroll
+      for (int kk = 0; kk < kBN / 16; ++kk) {
+        uint32_t pa[4];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int nt = kk * 2 + half;
+          const float p0 = probability(sacc[nt][0] - m_safe[0]);
+          const float p1 = probability(sacc[nt][1] - m_safe[0]);
+          const float p2 = probability(sacc[nt][2] - m_safe[1]);
+          const float p3 = probability(sacc[nt][3] - m_safe[1]);
+          l_run[0] += p0 + p1;
+          l_run[1] += p2 + p3;
+          pa[half * 2] = Elem<T>::pack(p0, p1);
+          pa[half * 2 + 1] = Elem<T>::pack(p2, p3);
+        }
+#pragma unroll
+        for (int np = 0; np < kNTiles / 2; ++np) {
+          uint32_t vb[4];
+          const int r = kk * 16 + ((mat & 1) << 3) + (lane & 7);
+          ldmatrix_x4_trans(vb, vsm + tile_offset<D>(r, np * 2 + (mat >> 1)));
+          mma_16816<T>(oacc[np * 2], pa, vb[0], vb[1]);
+          mma_16816<T>(oacc[np * 2 + 1], pa, vb[2], vb[3]);
+        }
+      }
     }
   }
   cp_async_wait<0>();
