@@ -566,9 +566,21 @@ extern "C" int64_t b200_linear_workspace_bytes(int64_t m, int64_t k, int64_t n, 
 }
 
 // Rows up to which W is streamed (linear_rows_kernel, whose time grows with every 8 rows) instead of multiplied in tiles
-// (the same time for 1 to 64 rows). 9728 x 896: 11.7, 18.0, 33.1, 40.7 us for 8, 16, 32,
-// 40 rows, 58 us in tiles; 896 x 4864: 7.7, 14.5, 24.4, 25.5 against 45 us.
+// (the same time for 1 to 64 rows). 8, 16, 32, 40 rows against tiles, us in a chain of launches: 9728 x 896 12.0, 18.6,
+// 33.6, 41.3 against 58; 896 x 4864 7.8, 14.5, 24.8, 25.6 against 45. Matrices beyond L2, which every 8 rows read again:
+// 37888 x 3584 126, 246, 473, 590 against 856; 3584 x 18944 79, 144, 247, 298 against 576; LM head 151936 x 896 125, 244,
+// 479, 597 against 646.
 constexpr int64_t kRowsLimit = 40;
+// A short K leaves most of a CTA's 4 x 128 k idle, so that every 8 rows more cost as much as with a long one, while tiles
+// cost in proportion to K. 12000 columns, K 128, 384, 768: 16 rows 13.0, 15.5, 21.0 us against 13.5, 24.7, 44.2 in tiles,
+// 24 rows 18.1, 22.0, 30.2 against 14.0, 25.1, 44.9, 40 rows 28.3, 34.5, 46.9 against 14.1, 25.9, 45.7. As long as the
+// CTAs are few (1024 columns, 40 rows, K 128: 5.3 against 10.4; 4096 columns, 24 rows, K 128: 7.9 against 10.3) this
+// does not show.
+static bool streams_rows(int64_t m, int64_t k, int64_t n) {
+  const int64_t tall = ceil_div(m, static_cast<int64_t>(kRowsOfX));
+  return m <= kRowsLimit && (tall == 1 || ceil_div(n, static_cast<int64_t>(kRowsColumns)) * tall <= 16 * kNumSMs ||
+                             k >= 192 * (tall - 1));
+}
 
 template <int ROWS>
 static int launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
@@ -607,7 +619,7 @@ static int linear_generic(const void* input, const void* weight, const void* bia
   bool vec = false;
   if constexpr (sizeof(T) == 4) {
     vec = k % 4 == 0 && input_row_stride % 4 == 0 && aligned16(input) && aligned16(weight);
-    if (vec && m <= kRowsLimit) return m <= 4 ? launch_rows<4>(p, s) : launch_rows<8>(p, s);
+    if (vec && streams_rows(m, k, n)) return m <= 4 ? launch_rows<4>(p, s) : launch_rows<8>(p, s);
   }
   const int64_t tiles_m = ceil_div(m, kTile), tiles_n = ceil_div(n, kTile);
   if (tiles_m > 65535) return B200_ERR_TOO_LARGE;
