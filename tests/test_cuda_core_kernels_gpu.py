@@ -112,7 +112,7 @@ def test_decode_attention(dtype, d, groups):
 
 @pytest.mark.parametrize("dtype,d", [(torch.float32, 64), (torch.float32, 128), (torch.bfloat16, 16),
                                      (torch.float16, 32), (torch.float32, 256), (torch.bfloat16, 256)])
-@pytest.mark.parametrize("t", [1, 63, 65, 200])
+@pytest.mark.parametrize("t", [1, 16, 32, 33, 63, 65, 200])
 def test_prefill_attention(t, dtype, d):
     g = torch.Generator(device="cuda").manual_seed(d + t)
     batch, heads, kv_heads, scale = 2, 4, 2, d ** -0.5

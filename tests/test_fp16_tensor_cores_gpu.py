@@ -94,7 +94,7 @@ def test_prefill_attention_of_a_long_tail(t, d, octaves):
 
 @pytest.mark.parametrize("mode", ["fast", "pytorch_compatible"])
 @pytest.mark.parametrize("d", [64, 128])
-@pytest.mark.parametrize("t", [1, 15, 64, 65, 130])
+@pytest.mark.parametrize("t", [1, 8, 9, 15, 64, 65, 130])
 def test_prefill_attention(t, d, mode):
     g = torch.Generator().manual_seed(t + d)
     batch, heads, kv_heads = 2, 6, 2
