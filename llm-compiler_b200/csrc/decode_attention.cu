@@ -1114,9 +1114,14 @@ __global__ void __launch_bounds__(kSplitThreads) decode_attention_split_kernel(c
     }
     __syncthreads();
     if (tile + 1 < last) fetch(tile + 1);
+    const int here = static_cast<int>(min(static_cast<int64_t>(kTile), len - static_cast<int64_t>(tile) * kTile));
     for (int item = threadIdx.x; item < kSplitHeads * kTile; item += kSplitThreads) {
       const int h = item / kTile, t = item % kTile;
       const int64_t token = static_cast<int64_t>(tile) * kTile + t;
+      if (t >= here || h >= heads) {
+        sp[h][t] = -INFINITY;
+        continue;
+      }
       float s = 0.0f;
 #pragma unroll 8
       for (int d = 0; d < D; d += 4) {
@@ -1124,8 +1129,7 @@ __global__ void __launch_bounds__(kSplitThreads) decode_attention_split_kernel(c
         s = fmaf(q4.x, k4.x, s); s = fmaf(q4.y, k4.y, s); s = fmaf(q4.z, k4.z, s); s = fmaf(q4.w, k4.w, s);
       }
       s = p.compat ? Elem<T>::round(Elem<T>::round(s) * p.scale) : s * p.scale;
-      if (token >= len) s = -INFINITY;
-      else if (p.mask != nullptr) s += load_mask(p.mask, p.mask_dtype, b * p.mask_batch_stride + token);
+      if (p.mask != nullptr) s += load_mask(p.mask, p.mask_dtype, b * p.mask_batch_stride + token);
       sp[h][t] = s;
     }
     __syncthreads();
@@ -1156,7 +1160,7 @@ __global__ void __launch_bounds__(kSplitThreads) decode_attention_split_kernel(c
     if (group < kGroups) {
       float part[kEach] = {};
 #pragma unroll 4
-      for (int t = 0; t < kTile; t += 4) {
+      for (int t = 0; t < here; t += 4) {  // (tokens behind the last one have weight 0 and value 0)
         float v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = sv[t + j][column];
