@@ -36,7 +36,7 @@ __device__ __forceinline__ float sum_slices(const float* first, int64_t slice, i
 // With B200_LAUNCH_PROGRAMMATIC set (b200_set_launch_mode) the kernels of the decode chain are
 // launched with programmatic stream serialisation: a kernel may become resident while its
 // predecessor in the stream still runs. Every such kernel signals its own dependents at its
-// top and executes grid_dependency_wait() before its first access to memory that another
+// top (norms and RoPE: behind their wait) and executes grid_dependency_wait() before its first access to memory that another
 // kernel writes, and before its first write; only set-up (mbarriers, tensor memory) and, with
 // B200_LAUNCH_CONSTANT_WEIGHTS, loads of weight operands come before the wait. Completion is
 // transitive: the wait returns once the predecessor has finished, and the predecessor could

@@ -256,6 +256,7 @@ grouped_linear_tcgen05_kernel(const Params p, const __grid_constant__ CUtensorMa
 template <int TILE>
 int launch(const Params& p, const CUtensorMap& w_map, const CUtensorMap& x_map, cudaStream_t stream) {
   static_assert(Shape<TILE>::kSmem <= 227 * 1024, "stage ring exceeds shared memory");
+  static_assert(tensor_memory_fits(2 * Shape<TILE>::kColumns, Shape<TILE>::kSmem), "columns without room");
   auto kernel = grouped_linear_tcgen05_kernel<TILE>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<TILE>::kSmem) != cudaSuccess)
     return B200_ERR_LAUNCH;

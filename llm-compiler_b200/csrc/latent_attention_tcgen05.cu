@@ -389,7 +389,7 @@ LatentTcPlan plan_latent_tcgen05(int64_t sequences, int64_t longest, int64_t hea
     if ((plan.ring >= plan.pairs && (plan.pairs + 2) * 2 * n <= 512) || n == 32) break;
   }
   if (plan.ring > kMaxRing) plan.ring = kMaxRing;
-  if (plan.ring < plan.pairs) return plan;
+  if (plan.ring < plan.pairs || !tensor_memory_fits(512, fixed + plan.ring * kPairBytes)) return plan;
   plan.n = n;
   plan.smem = fixed + plan.ring * kPairBytes;
   plan.row_blocks = static_cast<int>(ceil_div(rows, n));

@@ -822,6 +822,7 @@ int launch_persistent(const Tcgen05ParamsOf<T>& p, const CUtensorMap& a_map, con
   // the stage ring, 4 KB of store staging per epilogue warp, alignment slack
   constexpr int smem = kPersistentStages * (kBM + kPersistentBN) * 128 + 4 * 4096 + 1024;
   static_assert(smem <= 227 * 1024, "stage ring exceeds shared memory");
+  static_assert(tensor_memory_fits(512, smem), "columns without room");
   auto kernel = linear_tcgen05_persistent_kernel<T>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return B200_ERR_LAUNCH;
@@ -861,6 +862,7 @@ int launch(const Tcgen05ParamsOf<T>& p, const CUtensorMap& a_map, const CUtensor
   // slack: the last stage's 64-row x box is followed by up to 8 KB that the 128-row MMA reads past
   constexpr int ring = STAGES * (A_ROWS + BN) * 128 + 9216;
   static_assert(ring <= 227 * 1024, "stage ring exceeds shared memory");
+  static_assert(tensor_memory_fits(BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256, ring), "columns without room");
   if (p.bn <= 0 || p.bn > BN || p.bn % 16 != 0) return B200_ERR_BAD_ARGUMENT;
   // cluster split-K: behind the ring, room for every slice's copy of the units this CTA owns
   int smem = ring;

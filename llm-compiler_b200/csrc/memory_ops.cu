@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kThreads)
 rope_into_cache_kernel(const T* qkv, const T* cosine, const T* sine, T* q_out, T* keys, T* values, uint32_t total,
                        uint32_t tokens, uint32_t q_heads, uint32_t kv_heads, uint32_t dim, int64_t capacity) {
   constexpr uint32_t per = Elem<T>::kPerVec;
-  // What follows may start once the kernel in front has finished: it may take tensor memory that one still needs.
+  // What follows may start once the kernel in front has finished: earlier, its CTAs would only wait where that one's run.
   // (No __restrict__: nothing may be read ahead of the wait.)
   grid_dependency_wait();
   grid_launch_dependents();

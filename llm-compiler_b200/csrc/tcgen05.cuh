@@ -7,6 +7,18 @@
 
 namespace b200 {
 
+// Tensor memory under programmatic launches. A kernel signals its dependents at its top and allocates its columns behind
+// that, so a successor's CTA, with several kernels between them too, may allocate first and hold its columns while it
+// waits for the very kernel that has yet to get its own. That cannot deadlock, because shared memory lets no more CTAs
+// onto an SM (228 KB, 1 KB of it per CTA) than 512 columns serve: a kernel with tensor memory
+//   takes so much that no other such kernel fits beside it (the smallest uses 45 KB),
+//   or holds at most 256 columns and takes 105 KB, so that there are two of them, or one beside 122 KB of the rest,
+//   or holds at most 128 columns per 105 KB: 276 on an SM, 148 in 122 KB.
+constexpr bool tensor_memory_fits(int columns, int smem) {
+  return smem >= 45 * 1024 && (smem > 182 * 1024 || (columns <= 256 && smem >= 105 * 1024) ||
+                               columns * 105 <= 128 * (smem / 1024));
+}
+
 // Shared-memory matrix descriptor of a K-major tile of 128-byte swizzled rows: start address,
 // leading byte offset 16 B (unused by swizzled K-major layouts), stride byte offset 1024 B
 // (8 rows of 128 B per swizzle atom), descriptor version 1 (Blackwell), layout SWIZZLE_128B.
