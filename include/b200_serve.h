@@ -32,8 +32,8 @@ extern "C" {
 /* element types */
 #define B200_F32 0
 #define B200_BF16 1
-#define B200_F16 2 /* generic (non-tensor-core) kernels only; the reference's kernels accept it:
-                      backends/triton_linear.py:100-105 */
+#define B200_F16 2 /* the reference's kernels accept it: backends/triton_linear.py:100-105. Projections and prompt
+                      attention on the tensor cores where rows allow 16-byte loads, the rest on the CUDA cores */
 
 /* numerical modes: lowering.py:24-37 (_NUMERICAL_LOWERINGS) */
 #define B200_MODE_FAST 0
@@ -62,9 +62,10 @@ extern "C" {
 #define B200_LAUNCH_LINEAR_WARP_LEVEL 8    /* b200_linear: warp-level kernel, not tcgen05       */
 #define B200_LAUNCH_PREFILL_WARP_LEVEL 16  /* b200_prefill_attention: warp-level kernel         */
 
-/* Launch mode of the CALLING THREAD for the decode-chain kernels (linear on tcgen05 incl. the
- * partial-sum, folded-norm and cluster split-K forms, the two reduce_* consumers, decode
- * attention; every other kernel, advance_lengths / embedding / rope table among them, is always
+/* Launch mode of the CALLING THREAD for the kernels that can wait on the device (linear on tcgen05 incl. the
+ * partial-sum, folded-norm and cluster split-K forms, projections of a few rows, the two reduce_* consumers, decode
+ * attention, RMS norms, RoPE with the KV store, the hybrid layers' steps; every other kernel, advance_lengths /
+ * embedding / rope table among them, is always
  * launched fully serialised, which is what makes lengths[] stable before the attention's wait).
  * Thread-local: two engines driven from two threads do not see each other's promises; launches
  * captured into a CUDA graph keep the mode they were captured with. No counterpart in the
@@ -84,6 +85,10 @@ extern "C" {
  * B200_ERR_BAD_ARGUMENT for unknown bits. Default 0. */
 int b200_set_launch_mode(int flags);
 int b200_get_launch_mode(void);
+
+/* Identifies the capture into a CUDA graph that `stream` takes part in; 0: none. (No counterpart in the reference,
+ * which captures nothing.) Scratch that is kept from call to call must not be shared by two graphs. */
+int64_t b200_capture_id(void* stream);
 
 /* Debug control of the bounded in-kernel waits (no counterpart in the reference, whose kernels
  * have no waits to bound). Every mbarrier wait of the TMA / tcgen05 kernels gives up after
@@ -167,7 +172,7 @@ int b200_rms_norm(const void* input, const void* weight, void* output, int64_t r
  *  split_tokens  tokens per split (0 = library default); max_length_hint: an upper
  *                bound on lengths[] known to the host (0 = mask_len / capacity).
  * bf16 with head_dim 64 / 128 runs the tensor-core kernel; fp32, fp16 and head_dim 16 / 32 /
- * 256 (any dtype) a generic one without scratch.
+ * 256 (any dtype) a CUDA-core one without scratch.
  * Workspace: b200_decode_attention_workspace_bytes(...) bytes, 256-byte aligned. */
 int64_t b200_decode_attention_workspace_bytes(int64_t batch, int64_t q_heads, int64_t kv_heads,
                                               int64_t head_dim, int64_t max_length,
@@ -276,8 +281,9 @@ int b200_paged_qkv_decode_attention(
  * and a workspace of b200_prefill_attention_workspace_bytes(batch, tokens) is given; a pre-pass
  * then classifies the mask's 128 x 128 tiles (all zero / all -inf / mixed) so that tiles that
  * are all -inf at either end of a row block are never touched and all-zero tiles read no mask.
- * Other masked calls and the pytorch_compatible mode use the warp-level kernel; fp32, fp16 and
- * head_dim 16 / 32 / 256 (any dtype) a generic CUDA-core kernel (workspace may be NULL). status (may be NULL) receives B200_STATUS_WAIT_TIMEOUT. */
+ * Other masked calls and the pytorch_compatible mode use the warp-level kernel, and so does fp16 with
+ * head_dim 64 / 128 and 16-byte rows; fp32, other fp16 calls and head_dim 16 / 32 / 256 (any dtype) run on the
+ * CUDA cores (workspace may be NULL). status (may be NULL) receives B200_STATUS_WAIT_TIMEOUT. */
 int64_t b200_prefill_attention_workspace_bytes(int64_t batch, int64_t tokens);
 int b200_prefill_attention(const void* query, const void* key, const void* value,
                            const void* mask, void* output, int64_t batch, int64_t q_heads,
@@ -309,11 +315,13 @@ int b200_context_attention(const void* query, const void* key, const void* value
  * aten.add.Tensor that follows o_proj / down_proj, qwen2.py:299-304); 2 SwiGLU over
  * row-interleaved gate/up weights: W holds n rows (gate_j, up_j alternating), the output is
  * [M, n/2] and y[m,j] = r(r(silu(r(gate_j))) * r(up_j)) (qwen2.py:262-264).
- * bf16 problems run on tcgen05 tensor cores (TMEM accumulator, TMA-fed stage ring): 64-row
+ * bf16 and fp16 problems run on tcgen05 tensor cores (TMEM accumulator, TMA-fed stage ring): 64-row
  * activation boxes and a tile width chosen at run time at decode sizes, 128 x 64..256 tiles
  * beyond, a persistent two-accumulator kernel from 1024 rows on. Decode-size calls with too
  * few N tiles to fill the GPU and operands no tensor map can describe run on the warp-level
- * kernel with deterministic split-K, fp32 and fp16 on a generic CUDA-core kernel. Workspace (split-K partial sums + tile counters):
+ * kernel with deterministic split-K; up to 8 rows against at most 9 Mi weights on a kernel that streams W. fp32, and fp16
+ * whose K, rows or workspace these do not allow, run on the CUDA cores. Outputs may start on any element. Workspace
+ * (split-K partial sums + tile counters):
  * b200_linear_workspace_bytes. `status` receives B200_STATUS_WAIT_TIMEOUT if a bounded
  * in-kernel wait gives up. */
 #define B200_EPILOGUE_NONE 0

@@ -127,6 +127,7 @@ SIGNATURES = {
     "b200_debug_set_waits": (c_int64, [c_int64, c_int]),
     "b200_set_launch_mode": (c_int, [c_int]),
     "b200_get_launch_mode": (c_int, []),
+    "b200_capture_id": (c_int64, [c_void_p]),
     "b200_kv_store": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64,
                               c_int64, c_int64, c_int64, _I64P, _I64P, c_int, c_void_p, c_void_p]),
     "b200_rope": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,

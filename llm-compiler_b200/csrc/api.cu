@@ -40,6 +40,16 @@ extern "C" int b200_set_launch_mode(int flags) {
 
 extern "C" int b200_get_launch_mode(void) { return b200::launch_mode(); }
 
+extern "C" int64_t b200_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
+    (void)cudaGetLastError();  // the legacy stream beside another thread's capture
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? static_cast<int64_t>(id) : 0;
+}
+
 extern "C" const char* b200_error_string(int code) {
   switch (code) {
     case B200_OK: return "ok";

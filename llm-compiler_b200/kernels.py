@@ -48,6 +48,9 @@ class DeviceRuntime:
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self._workspaces: dict[str, torch.Tensor] = {}
         self._retired: list[torch.Tensor] = []
+        self._of_streams: dict[tuple[str, int], torch.Tensor] = {}
+        self._of_capture: dict[tuple[str, int], torch.Tensor] = {}  # (of the latest capture's streams)
+        self._capture = 0
         self.launches = 0
 
     def workspace(self, name: str, nbytes: int) -> Optional[torch.Tensor]:
@@ -60,6 +63,25 @@ class DeviceRuntime:
                 nbytes = max(int(nbytes), 2 * current.numel())
             current = torch.zeros(int(nbytes), dtype=torch.uint8, device=self.device)
             self._workspaces[name] = current
+        return current
+
+    def own_workspace(self, name: str, nbytes: int) -> Optional[torch.Tensor]:
+        """A workspace (zero-filled as above) of the current stream alone, or of the graph that is being captured on
+        it: for operators that calls on several streams, or graphs replayed side by side, may run at the same time. A
+        stream's workspace only its own later calls use, so one that is outgrown is freed in stream order; a graph's
+        lives in the graph's pool."""
+
+        if nbytes <= 0:
+            return None
+        stream = _stream()
+        capture = int(_lib.load().b200_capture_id(stream))
+        if capture and capture != self._capture:
+            self._of_capture, self._capture = {}, capture
+        kept = self._of_capture if capture else self._of_streams
+        current = kept.get((name, stream))
+        if current is None or current.numel() < nbytes:
+            grown = 0 if current is None else 2 * current.numel()
+            current = kept[name, stream] = torch.zeros(max(int(nbytes), grown), dtype=torch.uint8, device=self.device)
         return current
 
     def reserve(self, name: str, nbytes: int) -> None:
@@ -857,6 +879,12 @@ def linear_workspace_bytes(m: int, k: int, n: int, dtype: torch.dtype,
                                                        _EPILOGUES[epilogue]))
 
 
+def _linear_workspace(rt: DeviceRuntime, nbytes: int, dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """fp16 projections took no workspace, and could run on several streams at once, before split K came to them."""
+
+    return rt.own_workspace("linear", nbytes) if dtype == torch.float16 else rt.workspace("linear", nbytes)
+
+
 def b200_linear(tensor: torch.Tensor, weight: torch.Tensor,
                 bias: Optional[torch.Tensor] = None, *, residual: Optional[torch.Tensor] = None,
                 epilogue: str = "none") -> torch.Tensor:
@@ -905,7 +933,7 @@ def b200_linear(tensor: torch.Tensor, weight: torch.Tensor,
     library = _lib.load()
     code_dtype = _code(tensor.dtype)
     need = int(library.b200_linear_workspace_bytes(m, k, n, code_dtype, _EPILOGUES[epilogue]))
-    workspace = rt.workspace("linear", need)
+    workspace = _linear_workspace(rt, need, tensor.dtype)
     code = library.b200_linear(source.data_ptr(), weight.data_ptr(), _ptr(bias), _ptr(residual),
                                output.data_ptr(), m, k, n, row_stride, code_dtype,
                                _EPILOGUES[epilogue], _ptr(workspace), need, rt.status.data_ptr(), _stream())
@@ -975,7 +1003,7 @@ def b200_qwen2_prompt_layers(x: torch.Tensor, layers, keys, values, cosine: torc
                for columns in (hidden, hidden, width, q_size, kv_heads * dim, q_size, intermediate)]
     call = _lib.PromptCall(
         x.data_ptr(), *(buffer.data_ptr() for buffer in scratch), cosine.data_ptr(), sine.data_ptr(),
-        positions.data_ptr(), _ptr(block_table), _ptr(rt.workspace("linear", need)), need, batch, tokens, q_heads, kv_heads,
+        positions.data_ptr(), _ptr(block_table), _ptr(_linear_workspace(rt, need, x.dtype)), need, batch, tokens, q_heads, kv_heads,
         dim, hidden, intermediate, capacity, *pool, float(epsilon), float(scale), code_dtype, _mode(numerical_mode))
     code = library.b200_qwen2_prompt_layers(table, len(layers), ctypes.byref(call), rt.status.data_ptr(), _stream())
     _check(code, "b200_qwen2_prompt_layers")

@@ -150,3 +150,39 @@ def test_linear_output_on_an_odd_element(m, k, n, dtype, variant):
             results.append(output.clone())
         assert torch.equal(*results)
     kernels.runtime().check_status()
+
+
+def test_linear_on_several_streams_at_once():
+    """Sizes that split K through a workspace: every stream, and every captured graph, has its own."""
+
+    g = torch.Generator().manual_seed(5)
+    x = [torch.randn(48, 4864, generator=g).half().cuda() for _ in range(3)]
+    w = (0.02 * torch.randn(896, 4864, generator=g)).half().cuda()
+    expected = [b200.b200_linear(rows, w) for rows in x]
+    assert kernels.linear_workspace_bytes(48, 4864, 896, torch.float16) > 0
+    torch.cuda.synchronize()
+    streams, graphs, outputs = [torch.cuda.Stream() for _ in x], [], []
+    for rows, stream in zip(x, streams):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            outputs.append([b200.b200_linear(rows, w) for _ in range(20)])
+        graphs.append(graph)
+    for _ in range(5):
+        for graph, stream in zip(graphs, streams):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        eager = []
+        for rows, stream in zip(x, streams):
+            with torch.cuda.stream(stream):
+                eager.append([b200.b200_linear(rows, w) for _ in range(20)])
+        torch.cuda.synchronize()
+        for results in (*zip(outputs, expected), *zip(eager, expected)):
+            assert all(torch.equal(result, results[1]) for result in results[0])
+    rt = kernels.runtime()
+    addresses = []
+    for stream in streams:
+        with torch.cuda.stream(stream):
+            addresses.append(rt.own_workspace("linear", 64).data_ptr())
+            assert rt.own_workspace("linear", 64).data_ptr() == addresses[-1]
+    assert len(set(addresses)) == len(streams)
+    torch.cuda.synchronize()
