@@ -26,11 +26,11 @@ def unaligned(tensor):
     return view
 
 
-# the streaming kernel's row tiles (8, up to 40 rows) and K splits, the tiled kernel's 64 x 64 x 16 tiles, with and
+# the streaming kernel's row tiles (8, up to 40 rows), K splits and shortest K for many columns, the tiled kernel's 64 x 64 x 16 tiles, with and
 # without a cluster over K, vector and scalar loads
 @pytest.mark.parametrize("epilogue", ["none", "residual", "swiglu"])
 @pytest.mark.parametrize("m,k,n", [(1, 4, 2), (1, 896, 896), (4, 4864, 896), (8, 260, 130), (9, 1028, 6), (16, 520, 9728), (4, 3588, 34),
-                                   (40, 4864, 900), (41, 4864, 900),
+                                   (40, 4864, 900), (41, 4864, 900), (17, 380, 9728), (17, 384, 9728), (40, 132, 9728),
                                    (17, 896, 1152), (64, 7, 66), (65, 4864, 130), (200, 270, 62), (300, 4864, 896)])
 def test_linear_fp32(m, k, n, epilogue):
     g = torch.Generator(device="cuda").manual_seed(m + k + n)

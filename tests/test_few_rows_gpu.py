@@ -90,7 +90,8 @@ def test_forms_of_the_decode_chain(m, k, n):
 # the sizes above whose rows take few blocks, the projections of a Qwen2-0.5B layer, longer K, more
 # column tiles than the GPU holds at once, and one matrix over the limit
 CHAIN = [(1, 896, 1152), (8, 896, 896), (3, 4864, 896), (5, 904, 1092), (2, 3584, 2308), (7, 3584, 2800), (4, 18944, 512),
-         (6, 896, 9728), (2, 264, 30000), (8, 72, 2500), (1, 896, 12000)]
+         (6, 896, 9728), (2, 264, 30000), (8, 72, 2500), (1, 896, 12000),
+         (8, 3072, 3072), (8, 3072, 3076)]  # (on both sides of the largest matrix)
 
 
 @pytest.mark.parametrize("early", [False, True])
