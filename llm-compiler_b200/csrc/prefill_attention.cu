@@ -476,8 +476,9 @@ __global__ void __launch_bounds__(256) prefill_attention_tiled_kernel(const Pref
     float part[4][kColumns] = {};
     const int keys = min(64, key_end - k0);
     auto add_keys = [&](auto masked) {
+      const int end = decltype(masked)::value ? keys : 64;  // (a tile that every row sees whole has them all)
 #pragma unroll 4
-      for (int key = 0; key < keys; ++key) {
+      for (int key = 0; key < end; ++key) {
         const float4 w = *reinterpret_cast<const float4*>(p_sm + key * kPitch + ty * 4);
         const float wv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
