@@ -122,9 +122,10 @@ grouped_linear_tcgen05_kernel(const Params p, const __grid_constant__ CUtensorMa
       for (int r = round < STAGES ? 0 : round - STAGES; r < round; ++r)
         mbarrier_wait_bounded(smem_u32(&full_bar[r % STAGES]), (r / STAGES) & 1, min(p.wait_limit, 100000u));
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == 5) {
     // ---- MMA issuer ----
     grid_dependency_wait();
+    const uint32_t leader = elect_one();
     int round = 0, local = 0;
     bool ok = true;
     for (int item = blockIdx.x; ok && item < items; item += gridDim.x, ++local) {
@@ -132,7 +133,7 @@ grouped_linear_tcgen05_kernel(const Params p, const __grid_constant__ CUtensorMa
       if (expert < 0 || expert >= p.experts) break;
       const uint32_t idesc = instruction_descriptor(kFeatures, ((all_rows > 0 ? all_rows : held) + 15) / 16 * 16);
       const int acc = local & 1;
-      if (local >= 2 && !mbarrier_wait_bounded(smem_u32(&acc_empty[acc]), ((local >> 1) - 1) & 1, p.wait_limit)) {
+      if (local >= 2 && !mbarrier_wait_warp(smem_u32(&acc_empty[acc]), ((local >> 1) - 1) & 1, p.wait_limit)) {
         ok = false;
         break;
       }
@@ -140,20 +141,20 @@ grouped_linear_tcgen05_kernel(const Params p, const __grid_constant__ CUtensorMa
       const uint32_t d_tmem = tmem_base + acc * S::kColumns;
       for (int kb = 0; kb < nkb; ++kb, ++round) {
         const int s = round % STAGES;
-        if (!mbarrier_wait_bounded(smem_u32(&full_bar[s]), (round / STAGES) & 1, p.wait_limit)) {
+        if (!mbarrier_wait_warp(smem_u32(&full_bar[s]), (round / STAGES) & 1, p.wait_limit)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t w_addr = smem_base + s * S::kStageBytes;
-        const uint32_t x_addr = w_addr + S::kWeightBytes;
+        const uint64_t w_desc = smem_descriptor(smem_base + s * S::kStageBytes);
+        const uint64_t x_desc = descriptor_advance(w_desc, S::kWeightBytes);
 #pragma unroll
         for (int j = 0; j < kDepth / 16; ++j)
-          umma_bf16(d_tmem, smem_descriptor(w_addr + j * 32), smem_descriptor(x_addr + j * 32), idesc,
-                    (kb > 0 || j > 0) ? 1u : 0u);
-        umma_commit(smem_u32(&empty_bar[s]));
+          umma_bf16_if(leader, d_tmem, descriptor_advance(w_desc, j * 32), descriptor_advance(x_desc, j * 32), idesc,
+                       (kb > 0 || j > 0) ? 1u : 0u);
+        umma_commit_if(leader, smem_u32(&empty_bar[s]));
       }
-      if (ok) umma_commit(smem_u32(&acc_full[acc]));
+      if (ok) umma_commit_if(leader, smem_u32(&acc_full[acc]));
     }
     if (!ok) failed = 1;
   } else if (warp < 4) {

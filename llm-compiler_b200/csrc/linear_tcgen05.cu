@@ -401,25 +401,25 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
       row_scale[row] = rsqrtf(ss / static_cast<float>(p.k) + p.norm_eps);
     }
   }
-  if (warp == 1 && lane == 0) {
+  if (warp == 1) {
     // ---- MMA issuer ----
+    const uint32_t leader = elect_one();
+    bool fine = true;
     for (int kb = 0; kb < nkb; ++kb) {
       const int s = kb % STAGES;
-      if (!mbarrier_wait_bounded(smem_u32(&full_bar[s]), (kb / STAGES) & 1, p.wait_limit)) {
-        failed = 1;
-        break;
-      }
-
+      fine = mbarrier_wait_warp(smem_u32(&full_bar[s]), (kb / STAGES) & 1, p.wait_limit);
+      if (!fine) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_addr = smem_base + s * kStageBytes;
-      const uint32_t b_addr = a_addr + kABytes;
+      const uint64_t a_desc = smem_descriptor(smem_base + s * kStageBytes);
+      const uint64_t b_desc = descriptor_advance(a_desc, kABytes);
 #pragma unroll
       for (int j = 0; j < kBK / 16; ++j)
-        umma_bf16(tmem_base, smem_descriptor(a_addr + j * 32), smem_descriptor(b_addr + j * 32),
-                  idesc, (kb > 0 || j > 0) ? 1u : 0u);
-      umma_commit(smem_u32(&empty_bar[s]));  // the stage is free once these MMAs have read it
+        umma_bf16_if(leader, tmem_base, descriptor_advance(a_desc, j * 32), descriptor_advance(b_desc, j * 32),
+                     idesc, (kb > 0 || j > 0) ? 1u : 0u);
+      umma_commit_if(leader, smem_u32(&empty_bar[s]));  // the stage is free once these MMAs have read it
     }
-    umma_commit(smem_u32(&accum_bar));  // the accumulator is complete once all MMAs retired
+    if (!fine) failed = 1;
+    umma_commit_if(leader, smem_u32(&accum_bar));  // the accumulator is complete once all MMAs retired
   }
   __syncwarp();
 
@@ -603,7 +603,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
 // main loop of the next. With K = 896 (14 k-blocks) the epilogue of a 128 x 256 tile is about a
 // third of its main loop; unhidden it capped these GEMMs near 0.45 of the tensor peak.
 // Roles: warps 0-3 epilogue (warp w reads TMEM lanes 32 w ..), warp 4 (one lane) TMA producer,
-// warp 5 (one lane) MMA issuer and owner of the 512 TMEM columns. The stage ring runs on across
+// warp 5 (an elected lane) MMA issuer and owner of the 512 TMEM columns. The stage ring runs on across
 // tile boundaries: the producer is already fetching the next tile while the last k-blocks of
 // the current one are multiplied. Tiles are taken round-robin with N fastest, so the CTAs that
 // run at the same time share their rows of x and the (small) W in L2.
@@ -681,15 +681,16 @@ linear_tcgen05_persistent_kernel(const Tcgen05ParamsOf<T> p, const __grid_consta
       }
     }
     if (!ok) failed = 1;
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == 5) {
     // ---- MMA issuer ----
     grid_dependency_wait();
+    const uint32_t leader = elect_one();
     int round = 0, local = 0;
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, ++local) {
       const int acc = local & 1;
       // the epilogue must have read this accumulator's previous tile
-      if (local >= 2 && !mbarrier_wait_bounded(smem_u32(&acc_empty[acc]), ((local >> 1) - 1) & 1, p.wait_limit)) {
+      if (local >= 2 && !mbarrier_wait_warp(smem_u32(&acc_empty[acc]), ((local >> 1) - 1) & 1, p.wait_limit)) {
         ok = false;
         break;
       }
@@ -697,20 +698,20 @@ linear_tcgen05_persistent_kernel(const Tcgen05ParamsOf<T> p, const __grid_consta
       const uint32_t d_tmem = tmem_base + acc * kPersistentBN;
       for (int kb = 0; kb < nkb; ++kb, ++round) {
         const int s = round % STAGES;
-        if (!mbarrier_wait_bounded(smem_u32(&full_bar[s]), (round / STAGES) & 1, p.wait_limit)) {
+        if (!mbarrier_wait_warp(smem_u32(&full_bar[s]), (round / STAGES) & 1, p.wait_limit)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_addr = smem_base + s * kStageBytes;
-        const uint32_t b_addr = a_addr + kABytes;
+        const uint64_t a_desc = smem_descriptor(smem_base + s * kStageBytes);
+        const uint64_t b_desc = descriptor_advance(a_desc, kABytes);
 #pragma unroll
         for (int j = 0; j < kBK / 16; ++j)
-          umma_bf16(d_tmem, smem_descriptor(a_addr + j * 32), smem_descriptor(b_addr + j * 32), idesc,
-                    (kb > 0 || j > 0) ? 1u : 0u);
-        umma_commit(smem_u32(&empty_bar[s]));  // the stage is free once these MMAs have read it
+          umma_bf16_if(leader, d_tmem, descriptor_advance(a_desc, j * 32), descriptor_advance(b_desc, j * 32), idesc,
+                       (kb > 0 || j > 0) ? 1u : 0u);
+        umma_commit_if(leader, smem_u32(&empty_bar[s]));  // the stage is free once these MMAs have read it
       }
-      if (ok) umma_commit(smem_u32(&acc_full[acc]));  // the tile's accumulator is complete
+      if (ok) umma_commit_if(leader, smem_u32(&acc_full[acc]));  // the tile's accumulator is complete
     }
     if (!ok) failed = 1;
   } else if (warp < 4) {

@@ -20,7 +20,7 @@
 // With the row in registers a group's next S is computed during its current softmax, and the
 // tensor core works for one group while the other group's warps are in their exponentials.
 // Roles: warps 0-7 and 8-15 softmax groups, warp 16 (one lane) TMA producer (two K buffers, two
-// V buffers at D = 64, one at D = 128; K one tile ahead of V), warp 17 (one lane) MMA issuer and
+// V buffers at D = 64, one at D = 128; K one tile ahead of V), warp 17 (an elected lane) MMA issuer and
 // owner of the 512 TMEM columns (S at 0 and 128, O behind them). Every mbarrier wait is bounded:
 // a wait that gives up sets B200_STATUS_WAIT_TIMEOUT, tensor memory is freed and the CTA
 // returns. Query blocks are handed out heaviest first across all heads and sequences.
@@ -110,7 +110,7 @@ constexpr int kGroups = 2;
 constexpr int kSoftmaxWarps = 8 * kGroups;  // two warps per 32 query rows
 constexpr int kThreads = (kSoftmaxWarps + 2) * 32;  // + TMA warp + MMA warp
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain
-constexpr uint32_t kSpinLimit = 2000000u;   // polls of an MMA thread before it gives up (about 0.1 s)
+constexpr uint32_t kSpinLimit = 2000000u;   // polls of the MMA warp before it gives up (about 0.1 s)
 
 // 18 warps: five on one of the four 16 K-register sub-partitions, so at most 96 registers each.
 template <int D, bool MASKED, bool CHUNKED = false>
@@ -121,7 +121,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
   constexpr int G = kGroups;
   constexpr int kVStages = D == 64 ? 2 : 1;               // 227 KB hold one V tile at D = 128
   // With two V buffers V_j has long landed when P_j is written and a softmax warp vouches for it;
-  // a single buffer is refilled late, and only the MMA thread should wait for that.
+  // a single buffer is refilled late, and only the MMA warp should wait for that.
   constexpr bool kSoftmaxChecksV = kVStages > 1;
   constexpr int kPanels = D / 64;                         // 64-wide (128-byte) panels along D
   constexpr uint32_t kPanelBytes = kTile * 128;           // 128 rows x 128 B
@@ -256,11 +256,11 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
                  panel * 64, (lo + j) * kTile, kvh, b, p.v_token_dim1);
     }
     if (!ok) failed = 1;
-  } else if (warp == kMmaWarp && lane == 0) {
+  } else if (warp == kMmaWarp) {
     // ---- MMA issuer ----
-    // A poll that follows a tcgen05.commit of the same thread takes a few hundred cycles, so this
-    // thread polls as little as it can: that a K or V tile has landed is checked by a softmax
+    // This warp polls as little as it can: that a K or V tile has landed is checked by a softmax
     // warp before it reports S read or P written.
+    const uint32_t leader = elect_one();
     constexpr uint32_t idesc_s = instruction_descriptor(kTile, kTile);
     constexpr uint32_t idesc_o = instruction_descriptor(kTile, D, true);  // V: MN-major B operand
     const uint64_t q_desc = smem_descriptor(q_smem), k_desc = smem_descriptor(k_smem);
@@ -272,10 +272,10 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
         const uint32_t offset = (ks / 4) * kPanelBytes + (ks % 4) * 32;
-        umma_bf16(s_column(g), descriptor_advance(a, offset), descriptor_advance(bd, offset), idesc_s,
+        umma_bf16_if(leader, s_column(g), descriptor_advance(a, offset), descriptor_advance(bd, offset), idesc_s,
                   ks > 0 ? 1u : 0u);
       }
-      umma_commit(smem_u32(&s_full[g]));
+      umma_commit_if(leader, smem_u32(&s_full[g]));
     };
     auto issue_o = [&](int g, int j) {  // O_g (+)= P_g V_j, K = 128 keys
       const uint64_t a = descriptor_advance(p_desc, g * kPBytes);
@@ -283,18 +283,18 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
 #pragma unroll
       for (int ks = 0; ks < kTile / 16; ++ks) {
         const uint32_t p_offset = (ks / 4) * kPanelBytes + (ks % 4) * 32;
-        umma_bf16(o_column(g), descriptor_advance(a, p_offset), descriptor_advance(bd, ks * 2048),
+        umma_bf16_if(leader, o_column(g), descriptor_advance(a, p_offset), descriptor_advance(bd, ks * 2048),
                   idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
       }
-      umma_commit(smem_u32(&o_done[g]));
+      umma_commit_if(leader, smem_u32(&o_done[g]));
     };
-    bool ok = mbarrier_spin_bounded(smem_u32(&q_full), 0, p.spin_limit) &&
-              mbarrier_spin_bounded(smem_u32(&k_full[0]), 0, p.spin_limit);
+    bool ok = mbarrier_spin_warp(smem_u32(&q_full), 0, p.spin_limit) &&
+              mbarrier_spin_warp(smem_u32(&k_full[0]), 0, p.spin_limit);
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int g = 0; g < G; ++g) issue_s(g, 0);  // every group has key tile 0
-      umma_commit(smem_u32(&k_empty[0]));
+      umma_commit_if(leader, smem_u32(&k_empty[0]));
     }
     for (int j = 0; ok && j < n_tiles; ++j) {
       // S of the next key tile as soon as a group holds its current row of S in registers (its
@@ -303,22 +303,22 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         if (ok && more && j + 1 < tiles_of(g)) {
-          ok = mbarrier_spin_bounded(smem_u32(&s_free[g]), j & 1, p.spin_limit);
+          ok = mbarrier_spin_warp(smem_u32(&s_free[g]), j & 1, p.spin_limit);
           if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             issue_s(g, j + 1);
           }
         }
       }
-      if (ok && more) umma_commit(smem_u32(&k_empty[(j + 1) % kKStages]));  // K_{j+1}: all S issued
+      if (ok && more) umma_commit_if(leader, smem_u32(&k_empty[(j + 1) % kKStages]));  // K_{j+1}: all S issued
       // ... and O += P V once the group has written its probabilities (and has seen V_j land)
       bool v_landed = kSoftmaxChecksV;
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         if (ok && j < tiles_of(g)) {
-          ok = mbarrier_spin_bounded(smem_u32(&p_full[g]), j & 1, p.spin_limit) &&
+          ok = mbarrier_spin_warp(smem_u32(&p_full[g]), j & 1, p.spin_limit) &&
                (v_landed ||
-                mbarrier_spin_bounded(smem_u32(&v_full[j % kVStages]), (j / kVStages) & 1, p.spin_limit));
+                mbarrier_spin_warp(smem_u32(&v_full[j % kVStages]), (j / kVStages) & 1, p.spin_limit));
           v_landed = true;
           if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -326,7 +326,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
           }
         }
       }
-      if (ok) umma_commit(smem_u32(&v_empty[j % kVStages]));  // V_j is free once its last reader retires
+      if (ok) umma_commit_if(leader, smem_u32(&v_empty[j % kVStages]));  // V_j is free once its last reader retires
     }
     if (!ok) failed = 1;
   } else if (warp < kSoftmaxWarps) {

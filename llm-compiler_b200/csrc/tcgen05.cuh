@@ -46,23 +46,13 @@ __host__ __device__ constexpr uint32_t instruction_descriptor(int m, int n, bool
          (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-               ::"r"(bar) : "memory");
-}
-
-// The same for a warp that walks its loops as a whole: only the lane that passes a leader other than 0 issues
-// (always the same one: a commit covers its own thread's products).
+// One product of 16 along K (M and N from the instruction descriptor). The issuing warp walks its loops as a whole, so
+// that descriptors stay in uniform registers, and the one lane that passes a leader other than 0 issues (elect_one;
+// always the same lane: a commit covers its own thread's products). A product of M 128 x N takes N / 2 cycles, 48 at
+// least at N 64, 39 at N 16, dependent on the one before or not. A lone thread in a branch of its own could not issue
+// that fast: 46 cycles a product, 57 with a commit behind every fourth, and its polls waited behind them. Projections on
+// 128 rows x 64 columns a CTA, K 4864, 515 rows: 27.8 -> 24.4 us, 16 rows x 3584 x 3584 22.1 -> 17.3; 16384 rows, 128 x
+// 256 columns a CTA, 234 -> 216 (9728 x 896).
 __device__ __forceinline__ void umma_bf16_if(uint32_t leader, uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -77,6 +67,20 @@ __device__ __forceinline__ void umma_commit_if(uint32_t leader, uint32_t bar) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
                "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
                ::"r"(bar), "r"(leader) : "memory");
+}
+
+// 1 on one lane of a whole warp, 0 on the others: the lane that issues.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t leader;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+  return leader;
+}
+// A bounded wait of a whole warp, whose outcome is the same on all lanes.
+__device__ __forceinline__ bool mbarrier_wait_warp(uint32_t bar, uint32_t parity, uint32_t limit) {
+  return __all_sync(0xffffffffu, mbarrier_wait_ready_first(bar, parity, limit));
+}
+__device__ __forceinline__ bool mbarrier_spin_warp(uint32_t bar, uint32_t parity, uint32_t limit) {
+  return __all_sync(0xffffffffu, mbarrier_spin_bounded(bar, parity, limit));
 }
 
 __device__ __forceinline__ void tmem_load_32x32(uint32_t taddr, float (&v)[32]) {
