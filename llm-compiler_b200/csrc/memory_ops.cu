@@ -536,67 +536,55 @@ __global__ void classify_causal_mask_kernel(const T* __restrict__ mask, int64_t 
   if (__syncthreads_or(!ok) && threadIdx.x == 0) atomicAnd(flag, 0);
 }
 
-constexpr int kArgmaxThreads = 1024;
+constexpr int kArgmaxThreads = 1024, kArgmaxParts = 8;
+constexpr int64_t kArgmaxClusterRows = 96;
 
-template <typename T>
-__global__ void argmax_kernel(const T* __restrict__ logits, int64_t* __restrict__ ids,
-                              int64_t vocab, int64_t row_stride, bool vector_ok) {
-  constexpr int per = Elem<T>::kPerVec;
-  const T* row = logits + blockIdx.x * row_stride;
-  float best = -INFINITY;
-  int64_t best_idx = INT64_MAX;
-  if (vector_ok) {
-    const int64_t chunks = vocab / per;
-    for (int64_t c = threadIdx.x; c < chunks; c += blockDim.x) {
-      Vec16<T> x;
-      x.load(row + c * per);
-#pragma unroll
-      for (int i = 0; i < per; ++i) {
-        // strictly greater keeps the lowest index inside one thread's ascending scan
-        if (x.v[i] > best || best_idx == INT64_MAX) {
-          best = x.v[i];
-          best_idx = c * per + i;
-        }
-      }
-    }
-    for (int64_t i = chunks * per + threadIdx.x; i < vocab; i += blockDim.x) {
-      const float v = Elem<T>::load(row + i);
-      if (v > best || best_idx == INT64_MAX) {
-        best = v;
-        best_idx = i;
-      }
-    }
-  } else {
-    for (int64_t i = threadIdx.x; i < vocab; i += blockDim.x) {
-      const float v = Elem<T>::load(row + i);
-      if (v > best || best_idx == INT64_MAX) {
-        best = v;
-        best_idx = i;
-      }
-    }
-  }
-  // warp then block reduction on (value, index): larger value wins, lower index on ties
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int64_t oi = __shfl_xor_sync(0xffffffffu, best_idx, o);
-    if (ov > best || (ov == best && oi < best_idx)) {
-      best = ov;
-      best_idx = oi;
-    }
-  }
+// A few rows (the last launch of a decode step but one) are bound by the latency of their loads: a row is shared by the
+// CTAs of a cluster, 1024 threads together, each with four loads in flight. 151936 bf16, one CTA per row -> a cluster:
+// 1 row 10.2 -> 5.5 us, 64 rows 10.5 -> 8.8; 32 rows of 32768 4.3 -> 3.2. Rows that fill the GPU by themselves keep a CTA
+// each (593 rows: 47 us, 66 with four loads a thread).
+// (Which thread looks at which element, and the order of the comparisons, are the same in both forms.)
+template <typename T, int parts>
+__global__ void __launch_bounds__(kArgmaxThreads / parts)
+argmax_kernel(const T* __restrict__ logits, int64_t* __restrict__ ids, int64_t vocab, int64_t row_stride,
+              bool vector_ok) {
+  constexpr int per = Elem<T>::kPerVec, kAhead = parts > 1 ? 4 : 1;
   __shared__ float s_val[32];
   __shared__ int64_t s_idx[32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    s_val[warp] = best;
-    s_idx[warp] = best_idx;
+  const int rank = parts > 1 ? cluster_cta_rank() : 0;
+  if (parts > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (started: its memory may be written)
+  grid_dependency_wait();
+  const int thread = rank * blockDim.x + threadIdx.x, row_index = blockIdx.x / parts;
+  const T* row = logits + static_cast<int64_t>(row_index) * row_stride;
+  float best = -INFINITY;
+  int64_t best_idx = INT64_MAX;
+  auto consider = [&](float v, int64_t i) {
+    // strictly greater keeps the lowest index inside one thread's ascending scan
+    if (v > best || best_idx == INT64_MAX) {
+      best = v;
+      best_idx = i;
+    }
+  };
+  int64_t scanned = 0;
+  if (vector_ok) {
+    const int64_t chunks = vocab / per;
+    for (int64_t c = thread; c < chunks; c += kArgmaxThreads * kAhead) {
+      Vec16<T> x[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (c + u * kArgmaxThreads < chunks) x[u].load(row + (c + u * kArgmaxThreads) * per);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        if (c + u * kArgmaxThreads >= chunks) break;
+#pragma unroll
+        for (int i = 0; i < per; ++i) consider(x[u].v[i], (c + u * kArgmaxThreads) * per + i);
+      }
+    }
+    scanned = chunks * per;
   }
-  __syncthreads();
-  if (warp == 0) {
-    const int warps = blockDim.x >> 5;
-    best = lane < warps ? s_val[lane] : -INFINITY;
-    best_idx = lane < warps ? s_idx[lane] : INT64_MAX;
+  for (int64_t i = scanned + thread; i < vocab; i += kArgmaxThreads) consider(Elem<T>::load(row + i), i);
+  // warp then block reduction on (value, index): larger value wins, lower index on ties
+  auto reduce = [&] {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -606,7 +594,31 @@ __global__ void argmax_kernel(const T* __restrict__ logits, int64_t* __restrict_
         best_idx = oi;
       }
     }
-    if (lane == 0) ids[blockIdx.x] = best_idx == INT64_MAX ? 0 : best_idx;
+  };
+  reduce();
+  const int warp = thread >> 5, lane = threadIdx.x & 31;
+  if (parts > 1) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (lane == 0) {  // into the first CTA's memory
+      uint32_t value_at, index_at;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(value_at) : "r"(smem_u32(&s_val[warp])), "r"(0));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(index_at) : "r"(smem_u32(&s_idx[warp])), "r"(0));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(value_at), "f"(best) : "memory");
+      asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(index_at), "l"(best_idx) : "memory");
+    }
+    cluster_sync();
+  } else {
+    if (lane == 0) {
+      s_val[warp] = best;
+      s_idx[warp] = best_idx;
+    }
+    __syncthreads();
+  }
+  if (warp == 0) {
+    best = s_val[lane];
+    best_idx = s_idx[lane];
+    reduce();
+    if (lane == 0) ids[row_index] = best_idx == INT64_MAX ? 0 : best_idx;
   }
 }
 
@@ -919,11 +931,18 @@ int b200_argmax(const void* logits, int64_t* ids, int64_t rows, int64_t vocab,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t elt = dtype_bytes(dtype);
   const bool vec = aligned16(logits) && (row_stride * static_cast<int64_t>(elt)) % 16 == 0;
+  bool launched = true;
   const bool known = with_element_type(dtype, [&](auto tag) {
     using T = typename decltype(tag)::type;
-    argmax_kernel<T><<<static_cast<int>(rows), kArgmaxThreads, 0, s>>>(
-        static_cast<const T*>(logits), ids, vocab, row_stride, vec);
+    const T* from = static_cast<const T*>(logits);
+    if (rows > kArgmaxClusterRows)
+      argmax_kernel<T, 1><<<static_cast<unsigned>(rows), kArgmaxThreads, 0, s>>>(from, ids, vocab, row_stride, vec);
+    else
+      launched = launch_chained_cluster(argmax_kernel<T, kArgmaxParts>, dim3(static_cast<unsigned>(rows * kArgmaxParts)),
+                                        dim3(kArgmaxThreads / kArgmaxParts), 0, s, kArgmaxParts, from, ids, vocab,
+                                        row_stride, vec) == cudaSuccess;
   });
+  if (!launched) return B200_ERR_LAUNCH;
   return known ? launch_status() : B200_ERR_UNSUPPORTED;
 }
 
