@@ -451,6 +451,12 @@ int b200_linear_rms_input(const void* input, const void* folded_weight, const vo
                           void* output, const void* row_squares, int64_t row_square_slices,
                           int64_t m, int64_t k, int64_t n, int64_t input_row_stride,
                           double epsilon, int epilogue, int32_t* status, void* stream);
+/* serve.rms_norm + serve.linear (+ bias, + SwiGLU epilogue) of fp32 rows in one launch, norm weight [k] and weight as
+ * they are: y = rsqrt(mean(x^2) + eps) * ((x * w_norm) W^T). Fast mode only. For the rows whose projection streams W
+ * (b200_linear in fp32: up to 40) with 16-byte rows; B200_ERR_UNSUPPORTED otherwise. */
+int b200_rms_norm_linear(const void* input, const void* norm_weight, const void* weight, const void* bias,
+                         void* output, int64_t m, int64_t k, int64_t n, int64_t input_row_stride,
+                         double epsilon, int dtype, int epilogue, void* stream);
 int64_t b200_linear_splitk_slices(int64_t m, int64_t k, int64_t n);
 int b200_linear_splitk_residual(const void* input, const void* weight, const void* residual,
                                 void* output, void* row_squares_out, int64_t m, int64_t k,

@@ -220,6 +220,9 @@ struct LinearParamsGeneric {
   T* out;
   int64_t x_row_stride;
   int m, k, n, epilogue;
+  // RMS norm in front of the projection (linear_rows_kernel): x is the row before the norm
+  const T* norm_weight = nullptr;
+  float norm_eps = 0.0f;
 };
 
 // One output, or with SwiGLU the output of the column pair (n, n + 1): v0 is column n's sum, v1 column n + 1's.
@@ -264,13 +267,21 @@ __device__ __forceinline__ float sum_transposed(float (&v)[32], int lane) {
   return v[0];
 }
 
+//
+// NORM: the RMS norm in front of the projection as well. A row's factor rsqrt(mean(x^2) + eps) does not depend on k, so
+// the products take x times the norm's weight, every CTA adds the squares of the x that it reads anyway, and the factor
+// scales the sums: no launch for the norm, and none of its round trips. A decode step of Qwen2-0.5B in fp32, 4 sequences x
+// 600 tokens: 1028 -> 983 us (with the faster choice of tokens; the norms alone were 49 launches of some 2 us each).
+//
 // ROWS: rows of x a CTA takes (4 or 8)
-template <int ROWS>
+template <int ROWS, bool NORM>
 __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearParamsGeneric<float> p, int slots, int early) {
   extern __shared__ __align__(16) unsigned char rows_ring[];  // [warp][chunk][column][lane]
   constexpr int kOutputs = ROWS * kRowsColumns;
   __shared__ float part[kRowsWarps][kOutputs];
   __shared__ float total[kOutputs];
+  __shared__ float part_squares[kRowsWarps][ROWS];
+  __shared__ float total_squares[ROWS];
   grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kRowsColumns, m0 = blockIdx.y * ROWS, rows = min(ROWS, p.m - m0);
@@ -298,6 +309,7 @@ __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearP
   if (early) grid_dependency_wait();
 
   float acc[ROWS][kRowsColumns] = {};
+  float squares[ROWS] = {};
   const float* x = p.x + m0 * p.x_row_stride;
   for (int c = 0; c < count; ++c) {
     const int k = (first + c) * kRowsChunk + lane * 4;
@@ -308,6 +320,14 @@ __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearP
       if (i < rows && k < p.k)
         asm volatile("ld.global.ca.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(xv[i].x), "=f"(xv[i].y), "=f"(xv[i].z), "=f"(xv[i].w)
                      : "l"(x + i * p.x_row_stride + k) : "memory");
+    }
+    if (NORM) {
+      const float4 scale = k < p.k ? __ldg(reinterpret_cast<const float4*>(p.norm_weight + k)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        squares[i] = fmaf(xv[i].w, xv[i].w, fmaf(xv[i].z, xv[i].z, fmaf(xv[i].y, xv[i].y, fmaf(xv[i].x, xv[i].x, squares[i]))));
+        xv[i].x *= scale.x; xv[i].y *= scale.y; xv[i].z *= scale.z; xv[i].w *= scale.w;
+      }
     }
     cp_async_wait<kRowsRing - 1>();
     const uint32_t at = base + c % kRowsRing * kRowsChunkBytes;
@@ -331,8 +351,21 @@ __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearP
     for (int i = 0; i < 32; ++i) v[i] = acc[(h * 32 + i) / kRowsColumns][i % kRowsColumns];
     part[warp][h * 32 + lane] = sum_transposed(v, lane);
   }
+  if (NORM) {
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const float sum = warp_sum(squares[i]);
+      if (lane == 0) part_squares[warp][i] = sum;
+    }
+  }
   __syncthreads();
   if (splits > 1) {
+    if (NORM && threadIdx.x < ROWS) {
+      float sum = 0.0f;
+#pragma unroll
+      for (int s = 0; s < kRowsWarps; ++s) sum += part_squares[s][threadIdx.x];
+      total_squares[threadIdx.x] = sum;
+    }
     if (threadIdx.x < kOutputs) {
       float sum = 0.0f;
 #pragma unroll
@@ -357,6 +390,18 @@ __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearP
         v0 += part[s][at];
         v1 += part[s][at + 1];
       }
+    }
+    if (NORM) {
+      float sum = 0.0f;
+      if (splits > 1) {
+        for (int s = 0; s < splits; ++s) sum += load_cluster_f32(smem_u32(&total_squares[i]), s);
+      } else {
+#pragma unroll
+        for (int s = 0; s < kRowsWarps; ++s) sum += part_squares[s][i];
+      }
+      const float factor = rsqrtf(sum / static_cast<float>(p.k) + p.norm_eps);
+      v0 *= factor;
+      v1 *= factor;
     }
     epilogue_generic(p, m0 + i, n0 + c, v0, v1);
     epilogue_generic(p, m0 + i, n0 + c + 1, v1, 0.0f);
@@ -582,8 +627,8 @@ static bool streams_rows(int64_t m, int64_t k, int64_t n) {
                              k >= 192 * (tall - 1));
 }
 
-template <int ROWS>
-static int launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
+template <int ROWS, bool NORM>
+static int launch_rows_of(const LinearParamsGeneric<float>& p, cudaStream_t s) {
   // with few columns as many CTAs of a cluster along K as it takes to hold W in one ring each, up to some eight an SM
   const int64_t groups = ceil_div(p.n, kRowsColumns), tall = ceil_div(p.m, ROWS), chunks = ceil_div(p.k, kRowsChunk);
   int64_t splits = ceil_div(chunks, kRowsWarps * kRowsRing);
@@ -592,14 +637,18 @@ static int launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
   if (splits < 1) splits = 1;
   const int64_t most = ceil_div(chunks, kRowsWarps * splits);
   const int slots = static_cast<int>(most < kRowsRing ? most : kRowsRing), smem = kRowsWarps * slots * kRowsChunkBytes;
-  if (cudaFuncSetAttribute(linear_rows_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute((linear_rows_kernel<ROWS, NORM>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kRowsWarps * kRowsRing * kRowsChunkBytes) != cudaSuccess)
     return B200_ERR_LAUNCH;
   const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(tall), static_cast<unsigned>(splits));
   const int early = (launch_mode() & B200_LAUNCH_CONSTANT_WEIGHTS) != 0 ? 1 : 0;
-  return launch_chained_cluster_xz(linear_rows_kernel<ROWS>, grid, dim3(kRowsThreads), static_cast<size_t>(smem), s, 1u,
+  return launch_chained_cluster_xz(linear_rows_kernel<ROWS, NORM>, grid, dim3(kRowsThreads), static_cast<size_t>(smem), s, 1u,
                                    static_cast<unsigned>(splits), p, slots, early) == cudaSuccess
              ? launch_status() : B200_ERR_LAUNCH;
+}
+template <bool NORM>
+static int launch_rows(const LinearParamsGeneric<float>& p, cudaStream_t s) {
+  return p.m <= 4 ? launch_rows_of<4, NORM>(p, s) : launch_rows_of<8, NORM>(p, s);
 }
 
 template <typename T>
@@ -619,7 +668,7 @@ static int linear_generic(const void* input, const void* weight, const void* bia
   bool vec = false;
   if constexpr (sizeof(T) == 4) {
     vec = k % 4 == 0 && input_row_stride % 4 == 0 && aligned16(input) && aligned16(weight);
-    if (vec && streams_rows(m, k, n)) return m <= 4 ? launch_rows<4>(p, s) : launch_rows<8>(p, s);
+    if (vec && streams_rows(m, k, n)) return launch_rows<false>(p, s);
   }
   const int64_t tiles_m = ceil_div(m, kTile), tiles_n = ceil_div(n, kTile);
   if (tiles_m > 65535) return B200_ERR_TOO_LARGE;
@@ -711,4 +760,32 @@ extern "C" int b200_linear(const void* input, const void* weight, const void* bi
   if (!aligned16(input) || !aligned16(weight)) return B200_ERR_ALIGNMENT;
   return linear_tensor_core<__nv_bfloat16>(input, weight, bias, residual, output, m, k, n, input_row_stride, dtype,
                                            epilogue, workspace, workspace_bytes, status, s);
+}
+
+extern "C" int b200_rms_norm_linear(const void* input, const void* norm_weight, const void* weight, const void* bias,
+                                    void* output, int64_t m, int64_t k, int64_t n, int64_t input_row_stride,
+                                    double epsilon, int dtype, int epilogue, void* stream) {
+  if (!input || !norm_weight || !weight || !output || m < 0 || k <= 0 || n <= 0 || input_row_stride < k || !(epsilon >= 0.0))
+    return B200_ERR_BAD_ARGUMENT;
+  if (epilogue != B200_EPILOGUE_NONE && epilogue != B200_EPILOGUE_SWIGLU) return B200_ERR_BAD_ARGUMENT;
+  if (epilogue == B200_EPILOGUE_SWIGLU && n % 2 != 0) return B200_ERR_BAD_ARGUMENT;
+  if (m == 0) return B200_OK;
+  if (m > INT32_MAX || k > INT32_MAX || n > INT32_MAX) return B200_ERR_TOO_LARGE;
+  if (dtype != B200_F32 || k % 4 != 0 || input_row_stride % 4 != 0 || !aligned16(input) || !aligned16(norm_weight) ||
+      !aligned16(weight) || !streams_rows(m, k, n))
+    return B200_ERR_UNSUPPORTED;
+  LinearParamsGeneric<float> p;
+  p.x = static_cast<const float*>(input);
+  p.w = static_cast<const float*>(weight);
+  p.bias = static_cast<const float*>(bias);
+  p.residual = nullptr;
+  p.out = static_cast<float*>(output);
+  p.x_row_stride = input_row_stride;
+  p.m = static_cast<int>(m);
+  p.k = static_cast<int>(k);
+  p.n = static_cast<int>(n);
+  p.epilogue = epilogue;
+  p.norm_weight = static_cast<const float*>(norm_weight);
+  p.norm_eps = static_cast<float>(epsilon);
+  return launch_rows<true>(p, static_cast<cudaStream_t>(stream));
 }

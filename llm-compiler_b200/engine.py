@@ -486,10 +486,22 @@ class Qwen2Engine(ServingEngine):
         cosine, sine = kernels.b200_rope_table(self.positions.view(batch, 1), self.inv_freq,
                                                self.dtype)
         q_size, kv_size = cfg.q_size, cfg.kv_size
+
+        def normed_linear(x, norm_weight, weight, bias=None, epilogue="none"):
+            """The norm and the projection behind it: one launch for a few fp32 rows, else two."""
+
+            y = None
+            if self.dtype == torch.float32 and self.mode == "fast":
+                y = kernels.b200_rms_norm_linear(x, norm_weight, weight, bias, epsilon=cfg.rms_norm_eps,
+                                                 epilogue=epilogue)
+            if y is None:
+                h = kernels.b200_rms_norm(x, norm_weight, epsilon=cfg.rms_norm_eps, round_before_weight=True,
+                                          numerical_mode=self.mode)
+                y = kernels.b200_linear(h, weight, bias, epilogue=epilogue)
+            return y
+
         for index, layer in enumerate(self.layers):
-            h = kernels.b200_rms_norm(x, layer["input_norm"], epsilon=cfg.rms_norm_eps,
-                                      round_before_weight=True, numerical_mode=self.mode)
-            qkv = kernels.b200_linear(h, layer["qkv_w"], layer["qkv_b"])
+            qkv = normed_linear(x, layer["input_norm"], layer["qkv_w"], layer["qkv_b"])
             q = qkv[:, :q_size].view(batch, cfg.num_heads, cfg.head_dim)
             k = qkv[:, q_size:q_size + kv_size].view(batch, cfg.num_kv_heads, cfg.head_dim)
             v = qkv[:, q_size + kv_size:].view(batch, cfg.num_kv_heads, cfg.head_dim)
@@ -517,9 +529,7 @@ class Qwen2Engine(ServingEngine):
             else:
                 x = kernels.b200_linear(attn.view(batch, q_size), layer["o_w"], residual=x,
                                         epilogue="residual")
-            h = kernels.b200_rms_norm(x, layer["post_norm"], epsilon=cfg.rms_norm_eps,
-                                      round_before_weight=True, numerical_mode=self.mode)
-            a = kernels.b200_linear(h, layer["gate_up_w"], epilogue="swiglu")
+            a = normed_linear(x, layer["post_norm"], layer["gate_up_w"], epilogue="swiglu")
             if splitk:
                 x = kernels.b200_linear_splitk_residual(a, layer["down_w"], x)
             else:

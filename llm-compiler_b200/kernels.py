@@ -1288,6 +1288,37 @@ def b200_linear_rms_input(tensor: torch.Tensor, folded_weight: torch.Tensor,
     return output
 
 
+def b200_rms_norm_linear(tensor: torch.Tensor, norm_weight: torch.Tensor, weight: torch.Tensor,
+                         bias: Optional[torch.Tensor] = None, *, epsilon: float,
+                         epilogue: str = "none") -> Optional[torch.Tensor]:
+    """serve.rms_norm + serve.linear of a few fp32 rows in one launch (fast mode), or None where the rows are
+    too many or not laid out for it: the two operators then run one after the other."""
+
+    device = _require_cuda(tensor, norm_weight, weight, bias)
+    if tensor.ndim != 2 or weight.ndim != 2 or tensor.shape[1] != weight.shape[1] or \
+            norm_weight.shape != (weight.shape[1],):
+        raise ValueError("input must be M x K, the norm weight a vector of K and the weight N x K")
+    m, k = tensor.shape
+    n = weight.shape[0]
+    if not (tensor.dtype == weight.dtype == norm_weight.dtype) or \
+            (bias is not None and (bias.shape != (n,) or bias.dtype != tensor.dtype)):
+        raise ValueError("input, weights and a bias of N elements must share one dtype")
+    if epilogue not in ("none", "swiglu"):
+        raise ValueError(f"unsupported epilogue {epilogue!r}")
+    if tensor.dtype != torch.float32 or tensor.stride(1) != 1 or tensor.stride(0) < k or \
+            not all(t is None or t.is_contiguous() for t in (weight, norm_weight, bias)):
+        return None
+    output = torch.empty((m, n // 2 if epilogue == "swiglu" else n), dtype=tensor.dtype, device=device)
+    code = _lib.load().b200_rms_norm_linear(
+        tensor.data_ptr(), norm_weight.data_ptr(), weight.data_ptr(), _ptr(bias), output.data_ptr(), m, k, n,
+        tensor.stride(0), float(epsilon), _code(tensor.dtype), _EPILOGUES[epilogue], _stream())
+    if code == _lib.ERR_UNSUPPORTED:
+        return None
+    _check(code, "b200_rms_norm_linear")
+    _count(runtime(device))
+    return output
+
+
 def b200_linear_splitk_residual(tensor: torch.Tensor, weight: torch.Tensor,
                                 residual: torch.Tensor, *, row_squares: bool = False):
     """serve.linear + aten.add in one launch at decode sizes (bf16, at most 256 rows):
