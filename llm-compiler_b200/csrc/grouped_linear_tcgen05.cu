@@ -91,9 +91,10 @@ grouped_linear_tcgen05_kernel(const Params p, const __grid_constant__ CUtensorMa
 
   const int all_rows = p.index != nullptr ? p.x_rows : 0;  // 0: x is sorted
 
-  if (warp == 4 && lane == 0 && !p.drop_loads) {
+  if (warp == 4 && !p.drop_loads) {
     // ---- TMA producer ----
     grid_dependency_wait();
+    const uint32_t leader = elect_one();
     int round = 0;
     bool ok = true;
     for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
@@ -105,16 +106,16 @@ grouped_linear_tcgen05_kernel(const Params p, const __grid_constant__ CUtensorMa
       for (int kb = 0; kb < nkb; ++kb, ++round) {
         const int s = round % STAGES;
         if (round >= STAGES &&
-            !mbarrier_wait_bounded(smem_u32(&empty_bar[s]), ((round / STAGES) - 1) & 1, p.wait_limit)) {
+            !mbarrier_wait_warp(smem_u32(&empty_bar[s]), ((round / STAGES) - 1) & 1, p.wait_limit)) {
           ok = false;
           break;
         }
         const uint32_t bar = smem_u32(&full_bar[s]);
         const uint32_t w_dst = smem_base + s * S::kStageBytes;
-        mbarrier_arrive_expect_tx(bar, static_cast<uint32_t>(S::kWeightBytes + boxes * S::kBox * 128));
-        tma_load_3d(w_dst, &w_map, bar, kb * kDepth, feature, expert);
+        mbarrier_arrive_expect_tx_if(leader, bar, static_cast<uint32_t>(S::kWeightBytes + boxes * S::kBox * 128));
+        tma_load_3d_if(leader, w_dst, &w_map, bar, kb * kDepth, feature, expert);
         for (int box = 0; box < boxes; ++box)
-          tma_load_2d(w_dst + S::kWeightBytes + box * S::kBox * 128, &x_map, bar, kb * kDepth, first + box * S::kBox);
+          tma_load_2d_if(leader, w_dst + S::kWeightBytes + box * S::kBox * 128, &x_map, bar, kb * kDepth, first + box * S::kBox);
       }
     }
     if (!ok) {  // the copies still in flight get a bounded chance to land before the CTA retires

@@ -284,40 +284,37 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
       mbarrier_arrive_expect_tx(smem_u32(&reduce_bar), static_cast<uint32_t>(p.splits * reduce_owned * 16));
   }
 
-  if (warp == 0 && lane == 0 && !p.drop_loads) {
+  if (warp == 0 && !p.drop_loads) {
     // ---- TMA producer ----
     // The first ring of W tiles does not depend on the kernel before this one: fetch it
     // before waiting for that kernel (the transaction bytes are announced without arriving,
     // so a stage cannot complete before its x box has been requested as well).
+    const uint32_t leader = elect_one();
     const int early = p.prefetch_weights ? min(nkb, STAGES) : 0;
     auto k_of = [&](int kb) { return (kb_first + kb) * kBK; };  // element offset of the kb-th k-block
     for (int kb = 0; kb < early; ++kb) {
       const uint32_t bar = smem_u32(&full_bar[kb]);
-      mbarrier_expect_tx(bar, static_cast<uint32_t>(bn * 128));
-      tma_load_2d(smem_base + kb * kStageBytes + kABytes, &b_map, bar, k_of(kb), tile_n * bn);
+      if (leader) mbarrier_expect_tx(bar, static_cast<uint32_t>(bn * 128));
+      tma_load_2d_if(leader, smem_base + kb * kStageBytes + kABytes, &b_map, bar, k_of(kb), tile_n * bn);
     }
-    if (p.prefetch_l2)
+    if (p.prefetch_l2 && leader)
       for (int kb = early; kb < nkb; ++kb) tma_prefetch_l2_2d(&b_map, k_of(kb), tile_n * bn);
+    __syncwarp();
     grid_dependency_wait();
     trace.mark(0);
     for (int kb = 0; kb < nkb; ++kb) {
       const int s = kb % STAGES;
-      if (kb >= STAGES &&
-          !mbarrier_wait_bounded(smem_u32(&empty_bar[s]), ((kb / STAGES) - 1) & 1, p.wait_limit)) {
+      if (kb >= STAGES && !mbarrier_wait_warp(smem_u32(&empty_bar[s]), ((kb / STAGES) - 1) & 1, p.wait_limit)) {
         failed = 1;
         break;
       }
       const uint32_t bar = smem_u32(&full_bar[s]);
       const uint32_t a_dst = smem_base + s * kStageBytes;
-      if (kb < early) {
-        mbarrier_arrive_expect_tx(bar, static_cast<uint32_t>(kABytes));
-        tma_load_2d(a_dst, &a_map, bar, k_of(kb), tile_m * kBM);
-      } else {
-        mbarrier_arrive_expect_tx(bar, stage_tx_bytes);
-        tma_load_2d(a_dst, &a_map, bar, k_of(kb), tile_m * kBM);
-        tma_load_2d(a_dst + kABytes, &b_map, bar, k_of(kb), tile_n * bn);
-      }
+      mbarrier_arrive_expect_tx_if(leader, bar, kb < early ? static_cast<uint32_t>(kABytes) : stage_tx_bytes);
+      tma_load_2d_if(leader, a_dst, &a_map, bar, k_of(kb), tile_m * kBM);
+      if (kb >= early) tma_load_2d_if(leader, a_dst + kABytes, &b_map, bar, k_of(kb), tile_n * bn);
     }
+    __syncwarp();
   } else if (warp == 1 && lane == 0) {
     // The MMA issuer waits too (a K slice without k-blocks has no TMA copy to order it after
     // the producer's wait). The other threads only ever act on what these three hand them
@@ -602,7 +599,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
 // 256), with two accumulators in tensor memory so that the epilogue of one tile runs under the
 // main loop of the next. With K = 896 (14 k-blocks) the epilogue of a 128 x 256 tile is about a
 // third of its main loop; unhidden it capped these GEMMs near 0.45 of the tensor peak.
-// Roles: warps 0-3 epilogue (warp w reads TMEM lanes 32 w ..), warp 4 (one lane) TMA producer,
+// Roles: warps 0-3 epilogue (warp w reads TMEM lanes 32 w ..), warp 4 (an elected lane) TMA producer,
 // warp 5 (an elected lane) MMA issuer and owner of the 512 TMEM columns. The stage ring runs on across
 // tile boundaries: the producer is already fetching the next tile while the last k-blocks of
 // the current one are multiplied. Tiles are taken round-robin with N fastest, so the CTAs that
@@ -659,9 +656,10 @@ linear_tcgen05_persistent_kernel(const Tcgen05ParamsOf<T> p, const __grid_consta
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_base_slot;
 
-  if (warp == 4 && lane == 0 && !p.drop_loads) {
+  if (warp == 4 && !p.drop_loads) {
     // ---- TMA producer ----
     grid_dependency_wait();
+    const uint32_t leader = elect_one();
     int round = 0;  // k-blocks issued so far, over all tiles
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
@@ -669,15 +667,15 @@ linear_tcgen05_persistent_kernel(const Tcgen05ParamsOf<T> p, const __grid_consta
       for (int kb = 0; kb < nkb; ++kb, ++round) {
         const int s = round % STAGES;
         if (round >= STAGES &&
-            !mbarrier_wait_bounded(smem_u32(&empty_bar[s]), ((round / STAGES) - 1) & 1, p.wait_limit)) {
+            !mbarrier_wait_warp(smem_u32(&empty_bar[s]), ((round / STAGES) - 1) & 1, p.wait_limit)) {
           ok = false;
           break;
         }
         const uint32_t bar = smem_u32(&full_bar[s]);
         const uint32_t a_dst = smem_base + s * kStageBytes;
-        mbarrier_arrive_expect_tx(bar, stage_tx_bytes);
-        tma_load_2d(a_dst, &a_map, bar, kb * kBK, tile_m * kBM);
-        tma_load_2d(a_dst + kABytes, &b_map, bar, kb * kBK, tile_n * bn);
+        mbarrier_arrive_expect_tx_if(leader, bar, stage_tx_bytes);
+        tma_load_2d_if(leader, a_dst, &a_map, bar, kb * kBK, tile_m * kBM);
+        tma_load_2d_if(leader, a_dst + kABytes, &b_map, bar, kb * kBK, tile_n * bn);
       }
     }
     if (!ok) failed = 1;
