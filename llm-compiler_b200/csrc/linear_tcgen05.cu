@@ -1195,8 +1195,15 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
   }
   if (persistent) return launch_persistent(p, a_map, b_map, stream);
   if (bn == 256) return launch_linear<256, 4, 128>(p, a_map, b_map, stream);
-  if (bn == 128) return launch_linear<128, 3, 128>(p, a_map, b_map, stream);
-  return launch_linear<64, 4, 128>(p, a_map, b_map, stream);
+  // Two CTAs an SM hide one another's latencies behind short rings. Tiles that do not fill the GPU once have an SM each,
+  // which hides them behind a ring of all its shared memory: W comes from HBM, 1 us away, and a stage of 64 columns is
+  // multiplied in 0.1. 77 and 515 rows, 4 -> 8 stages: 4864 x 896 24.0 -> 17.7 and 23.1 -> 18.2 us, 896 x 896 7.2 -> 6.4
+  // and 7.7 -> 7.0, 3584 x 3584 on 77 rows 19.2 -> 14.7; 128 columns, 3 -> 6 stages, 515 rows x 3584 x 3584 24.5 -> 17.8,
+  // 18944 x 3584 110 -> 73. With more tiles than SMs: 896 x 9728 on 77 rows 8.7 us in two short rings, 11.7 in a long one.
+  const bool alone = ceil_div(n, bn) * ceil_div(m, kBM) <= kNumSMs;
+  if (bn == 128)
+    return alone ? launch_linear<128, 6, 128>(p, a_map, b_map, stream) : launch_linear<128, 3, 128>(p, a_map, b_map, stream);
+  return alone ? launch_linear<64, 8, 128>(p, a_map, b_map, stream) : launch_linear<64, 4, 128>(p, a_map, b_map, stream);
 }
 
 int linear_tcgen05(const void* input, const void* weight, const void* bias, const void* residual,

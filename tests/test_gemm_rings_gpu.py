@@ -1,0 +1,32 @@
+"""Projections of 65 rows and more in 64- and 128-column tiles, on both sides of the line between short rings and long ones
+(148 tiles), K in fewer blocks than a ring has stages and in more: a tile's sums do not depend on the ring, so every row
+and column equals that of a call on the other side of the line bit for bit."""
+
+import pytest
+import torch
+
+from llm_compiler_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("epilogue", ["none", "residual", "swiglu"])
+# tiles: 2 x 74 and 2 x 75 of 64 columns; 1 x 148 and 1 x 149 of 64; 5 x 28 and 5 x 30 of 128; ragged rows and columns
+@pytest.mark.parametrize("m,k,n,fewer", [(130, 896, 4800, 4736), (77, 64, 9500, 9470), (128, 456, 9536, 9472),
+                                         (515, 1032, 3840, 3584), (600, 8, 3840, 3520)])
+def test_sums_do_not_depend_on_the_ring(m, k, n, fewer, epilogue, dtype):
+    g = torch.Generator(device="cuda").manual_seed(m + k + n)
+    x, w = ((torch.randn(*s, generator=g, device="cuda") * k ** -0.25).to(dtype) for s in ((m, k), (n, k)))
+    bias = torch.randn(n, generator=g, device="cuda").to(dtype)
+    residual = torch.randn(m, n, generator=g, device="cuda").to(dtype) if epilogue == "residual" else None
+    full = kernels.b200_linear(x, w, bias, residual=residual, epilogue=epilogue)
+    part = kernels.b200_linear(x, w[:fewer], bias[:fewer], epilogue=epilogue,
+                               residual=None if residual is None else residual[:, :fewer].contiguous())
+    assert torch.equal(full[:, :part.shape[1]], part)
+    if epilogue == "none":
+        exact = x.double() @ w.double().T + bias.double()
+        # one rounding of the result, and sums in fp32 in one chain of K / 16 products
+        bound = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * exact.abs() + \
+            (k / 16 + 8) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + 1e-6
+        assert ((full.double() - exact).abs() <= bound).all()
