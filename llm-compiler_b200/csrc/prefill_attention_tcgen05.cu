@@ -10,7 +10,8 @@
 //                 lanes, so warps w and w + 4 share 32 rows and split the keys in halves): the
 //                 half row of S is read into registers once, which frees S for the next product
 //                 at once; the halves exchange their maxima through shared memory; exp2; bf16
-//                 probabilities written as the K-major A operand P
+//                 probabilities written as the A operand P: into tensor memory at D 64 (64
+//                 columns a group are left beside S and O), into K-major shared memory at D 128
 //   O += P V      tcgen05.mma M 128 x N D accumulating in the group's D TMEM columns; V is used
 //                 as it lies in memory (an MN-major B operand: no transpose pass)
 // The running maximum is lazy: probabilities are taken against a reference maximum that is moved
@@ -18,7 +19,13 @@
 // tile raises a row's maximum by more than 8 in the log2 domain, so probabilities stay below 2^8
 // and most tiles touch O only through the tensor core. The result is O / row sum.
 // With the row in registers a group's next S is computed during its current softmax, and the
-// tensor core works for one group while the other group's warps are in their exponentials.
+// tensor core works for one group while the other group's warps are in their exponentials: the
+// products are issued group by group (S and O of one, then of the other), so that the second group
+// falls half a tile behind the first. Both S first, then both O, kept the groups in step, all warps
+// in their loads and then all in their exponentials. 4 sequences x 14 heads x 4096 tokens, D 64:
+// 240 -> 224 us with P in tensor memory, 205 in this order; 28 heads x 4096, D 128: 135 -> 128 us in this order. (Bound by neither unit:
+// the exponentials take 110 us, the products 55. exp2 by a polynomial on every fourth key, or a second
+// buffer of P, made it slower.)
 // Roles: warps 0-7 and 8-15 softmax groups, warp 16 (one lane) TMA producer (two K buffers, two
 // V buffers at D = 64, one at D = 128; K one tile ahead of V), warp 17 (an elected lane) MMA issuer and
 // owner of the 512 TMEM columns (S at 0 and 128, O behind them). Every mbarrier wait is bounded:
@@ -123,6 +130,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
   // With two V buffers V_j has long landed when P_j is written and a softmax warp vouches for it;
   // a single buffer is refilled late, and only the MMA warp should wait for that.
   constexpr bool kSoftmaxChecksV = kVStages > 1;
+  constexpr bool kPInTmem = D == 64;
   constexpr int kPanels = D / 64;                         // 64-wide (128-byte) panels along D
   constexpr uint32_t kPanelBytes = kTile * 128;           // 128 rows x 128 B
   constexpr uint32_t kTileBytes = kPanels * kPanelBytes;  // one of Q, K, V
@@ -188,7 +196,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
   const uint32_t q_smem = smem_u32(smem);                   // G tiles
   const uint32_t k_smem = q_smem + G * kTileBytes;          // two buffers
   const uint32_t v_smem = k_smem + kKStages * kTileBytes;   // one or two buffers
-  const uint32_t p_smem = v_smem + kVStages * kTileBytes;   // G x [2 panels][128 rows][128 B]
+  const uint32_t p_smem = v_smem + kVStages * kTileBytes;   // G x [2 panels][128 rows][128 B] (not kPInTmem)
 
   if (threadIdx.x == 0) {
     failed = 0;
@@ -220,6 +228,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
   const uint32_t tmem_base = tmem_base_slot;
   auto s_column = [&](int g) { return tmem_base + g * kTile; };
   auto o_column = [&](int g) { return tmem_base + G * kTile + g * D; };
+  auto p_column = [&](int g) { return tmem_base + G * (kTile + D) + g * (kTile / 2); };  // kPInTmem
 
   if (warp == kTmaWarp && lane == 0 && !p.drop_loads) {
     // ---- TMA producer ----
@@ -282,9 +291,10 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
       const uint64_t bd = descriptor_advance(v_desc, (j % kVStages) * kTileBytes);
 #pragma unroll
       for (int ks = 0; ks < kTile / 16; ++ks) {
-        const uint32_t p_offset = (ks / 4) * kPanelBytes + (ks % 4) * 32;
-        umma_bf16_if(leader, o_column(g), descriptor_advance(a, p_offset), descriptor_advance(bd, ks * 2048),
-                  idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+        const uint32_t p_offset = (ks / 4) * kPanelBytes + (ks % 4) * 32, accumulate = j > 0 || ks > 0 ? 1u : 0u;
+        const uint64_t b = descriptor_advance(bd, ks * 2048);
+        if (kPInTmem) umma_bf16_tmem_if(leader, o_column(g), p_column(g) + ks * 8, b, idesc_o, accumulate);
+        else umma_bf16_if(leader, o_column(g), descriptor_advance(a, p_offset), b, idesc_o, accumulate);
       }
       umma_commit_if(leader, smem_u32(&o_done[g]));
     };
@@ -296,36 +306,30 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
       for (int g = 0; g < G; ++g) issue_s(g, 0);  // every group has key tile 0
       umma_commit_if(leader, smem_u32(&k_empty[0]));
     }
+    // S of a group's next key tile as soon as it holds its current row of S in registers (its report also says
+    // that K_{j+1} has landed) ...
+    auto next_s = [&](int g, int j) {
+      if (!ok || j + 1 >= tiles_of(g)) return;
+      ok = mbarrier_spin_warp(smem_u32(&s_free[g]), j & 1, p.spin_limit);
+      if (!ok) return;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      issue_s(g, j + 1);
+    };
+    // ... and O += P V once it has written its probabilities (and has seen V_j land)
+    auto next_o = [&](int g, int j) {
+      if (!ok || j >= tiles_of(g)) return;
+      ok = mbarrier_spin_warp(smem_u32(&p_full[g]), j & 1, p.spin_limit) &&
+           (kSoftmaxChecksV || mbarrier_spin_warp(smem_u32(&v_full[j % kVStages]), (j / kVStages) & 1, p.spin_limit));
+      if (!ok) return;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      issue_o(g, j);
+    };
     for (int j = 0; ok && j < n_tiles; ++j) {
-      // S of the next key tile as soon as a group holds its current row of S in registers (its
-      // report also says that K_{j+1} has landed) ...
-      const bool more = j + 1 < n_tiles;
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        if (ok && more && j + 1 < tiles_of(g)) {
-          ok = mbarrier_spin_warp(smem_u32(&s_free[g]), j & 1, p.spin_limit);
-          if (ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_s(g, j + 1);
-          }
-        }
-      }
-      if (ok && more) umma_commit_if(leader, smem_u32(&k_empty[(j + 1) % kKStages]));  // K_{j+1}: all S issued
-      // ... and O += P V once the group has written its probabilities (and has seen V_j land)
-      bool v_landed = kSoftmaxChecksV;
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        if (ok && j < tiles_of(g)) {
-          ok = mbarrier_spin_warp(smem_u32(&p_full[g]), j & 1, p.spin_limit) &&
-               (v_landed ||
-                mbarrier_spin_warp(smem_u32(&v_full[j % kVStages]), (j / kVStages) & 1, p.spin_limit));
-          v_landed = true;
-          if (ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_o(g, j);
-          }
-        }
-      }
+      next_s(0, j);
+      next_o(0, j);
+      next_s(1, j);
+      if (ok && j + 1 < n_tiles) umma_commit_if(leader, smem_u32(&k_empty[(j + 1) % kKStages]));  // K_{j+1}: all S issued
+      next_o(1, j);
       if (ok) umma_commit_if(leader, smem_u32(&v_empty[j % kVStages]));  // V_j is free once its last reader retires
     }
     if (!ok) failed = 1;
@@ -343,6 +347,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t s_taddr = s_column(g) + lane_base + half * 64;
     const uint32_t o_taddr = o_column(g) + lane_base + half * (D / 2);
+    const uint32_t p_taddr = p_column(g) + lane_base + half * 32;  // two keys a column
     const uint32_t p_row = p_smem + g * kPBytes + half * kPanelBytes + row * 128;  // panel = 64 keys
     const uint32_t swizzle = row & 7;
     const int key0 = half * 64;               // first key column of this thread inside a tile
@@ -421,7 +426,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) {
-          // the group's first warp vouches for K_{j+1}: the MMA thread then needs one poll, not two
+          // the group's first warp vouches for K_{j+1}: the MMA warp then needs one poll, not two
           bool landed = true;
           if ((warp & 7) == 0 && j + 1 < my_tiles)
             landed = mbarrier_wait_ready_first(smem_u32(&k_full[(j + 1) % kKStages]), ((j + 1) / kKStages) & 1,
@@ -504,9 +509,10 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
           sum1 += p1;
           packed[i / 2] = pack_bf16x2(p0, p1);
         }
+        if constexpr (kPInTmem) tmem_store_32x16(p_taddr + c0 / 2, packed);
         // K-major A operand: row = query, 16-byte chunks of the 128-byte row XOR-swizzled by row % 8
 #pragma unroll
-        for (int chunk = 0; chunk < 4; ++chunk) {
+        for (int chunk = 0; !kPInTmem && chunk < 4; ++chunk) {
           const uint32_t logical = c0 / 8 + chunk;
           const uint32_t address = p_row + ((logical ^ swizzle) << 4);
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(address),
@@ -517,8 +523,9 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
       emit(s0, 0);
       emit(s1, 32);
       l_run += sum0 + sum1;
+      if (kPInTmem) tmem_store_wait();
       // generic-proxy writes of P must be visible to the tensor core (async proxy)
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      else asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
@@ -533,10 +540,10 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
     }
     if (ok && my_tiles > 0)
       ok = __all_sync(0xffffffffu, mbarrier_wait_ready_first(smem_u32(&o_done[g]), (my_tiles - 1) & 1, p.wait_limit));
-    // The row sum is the sum of the two halves (both took the same reference maximum); they meet
-    // in the first K buffer, which nothing reads any more once the last product has completed
-    // (on the failure path the sums are not used).
-    float* row_sum_slot = reinterpret_cast<float*>(smem + G * kTileBytes) + g * 2 * kTile;
+    // The row sum is the sum of the two halves (both took the same reference maximum); they meet in the group's own
+    // tile of Q, which nothing reads any more once its last product has completed (K may still serve the other group;
+    // on the failure path the sums are not used).
+    float* row_sum_slot = reinterpret_cast<float*>(smem + g * kTileBytes);
     row_sum_slot[half * kTile + row] = l_run;
     asm volatile("bar.sync %0, 256;" ::"r"(group_barrier) : "memory");
     const int q_row = q0 + g * kTile + row;
@@ -654,8 +661,12 @@ int prefill_attention_tcgen05(const void* query, const void* key, const void* va
   dim3 grid(static_cast<unsigned>(q_heads), static_cast<unsigned>(batch), static_cast<unsigned>(q_blocks));
   const int tile_bytes = static_cast<int>(head_dim) * kTile * 2;
   const int v_stages = head_dim == 64 ? 2 : 1;
-  // the pair of Q tiles, two K tiles, one or two V tiles, the pair of probability tiles
-  const int smem = tile_bytes * (kGroups + kKStages + v_stages) + kGroups * kTile * kTile * 2;
+  // the pair of Q tiles, two K tiles, one or two V tiles, at D 128 the pair of probability tiles; at least what leaves
+  // no other kernel with tensor memory room beside all 512 columns
+  constexpr int kAlone = 184 * 1024;
+  static_assert(tensor_memory_fits(512, kAlone), "columns without room");
+  const int tiles_bytes = tile_bytes * (kGroups + kKStages + v_stages) + (head_dim == 64 ? 0 : kGroups * kTile * kTile * 2);
+  const int smem = tiles_bytes > kAlone ? tiles_bytes : kAlone;
   auto launch = [&](auto kernel) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return false;
