@@ -1126,14 +1126,6 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
       }
     }
     if (best < 0.5 && !fold_norm) return B200_ERR_UNSUPPORTED;
-    // A folded-norm projection at decode sizes (gate|up: 17 MB of weights) is a chain of
-    // latencies, not a stream: 64-column tiles with short rings put two or three CTAs on an SM,
-    // whose ring round trips and two-warp SwiGLU epilogues overlap. Measured on the Qwen2-0.5B
-    // step: 1.389 ms with 152 x 64 columns against 1.449 ms with 122 x 80 (one CTA per SM).
-    if (fold_norm && small_rings()) {
-      const int64_t tiles64 = ceil_div(n, 64);
-      if (tiles64 >= kNumSMs - 28 && tiles64 <= 3 * kNumSMs) bn = 64;
-    }
     if (fold_norm) {  // B200_FOLD_BN: tile width of the folded-norm projection (experiments only)
       static const int forced = [] {
         const char* text = getenv("B200_FOLD_BN");
@@ -1184,13 +1176,9 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
   if (m <= 64) {
     if (bn == 192 && ceil_div(n, 192) >= 4 * kNumSMs) return launch_linear<192, 3, 64>(p, a_map, b_map, stream);
     if (bn > 128) return launch_linear<256, 5, 64>(p, a_map, b_map, stream);
-    if (bn > 64)
-      return small_rings() && fold_norm ? launch_linear<128, 4, 64>(p, a_map, b_map, stream)
-                                        : launch_linear<128, 8, 64>(p, a_map, b_map, stream);
-    // narrow tiles of a folded-norm projection: short rings, three CTAs per SM
-    // (4-stage rings measured best: 3 stages -4 %, 6 stages -2 %, 12 stages -17 % of the decode step)
-    if (small_rings() && fold_norm)
-      return bn > 32 ? launch_linear<64, 4, 64>(p, a_map, b_map, stream) : launch_linear<32, 4, 64>(p, a_map, b_map, stream);
+    // (a folded norm, too: 152 tiles of 64 columns in short rings, three of them an SM, were the better form while a lone
+    // thread issued their products; a Qwen2-0.5B step of 16 sequences 931 -> 863 us, of 23 1124 -> 1097, of 64 the same)
+    if (bn > 64) return launch_linear<128, 8, 64>(p, a_map, b_map, stream);
     return launch_linear<64, 12, 64>(p, a_map, b_map, stream);
   }
   if (persistent) return launch_persistent(p, a_map, b_map, stream);
@@ -1306,7 +1294,12 @@ int linear_splitk_residual_tcgen05(const void* input, const void* weight, const 
   switch (cluster_config(a_rows, plan.bn, ceil_div(ceil_div(k, kBK), plan.splits))) {
     case ClusterConfig::k32x3: return launch<32, 3, 64, kFormCluster>(p, a_map, b_map, stream);
     case ClusterConfig::k32x8: return launch<32, 8, 64, kFormCluster>(p, a_map, b_map, stream);
-    case ClusterConfig::k64x4: return launch<64, 4, 64, kFormCluster>(p, a_map, b_map, stream);
+    case ClusterConfig::k64x4:
+      // 6 stages where all clusters are resident with them as well (K slices, and so the sums, are the plan's): a whole
+      // step of 16 sequences 931 -> 881 us
+      if (resident_clusters_of(ClusterConfig::k64x6, plan.bn, plan.splits) >= ceil_div(n, static_cast<int64_t>(plan.bn)))
+        return launch<64, 6, 64, kFormCluster>(p, a_map, b_map, stream);
+      return launch<64, 4, 64, kFormCluster>(p, a_map, b_map, stream);
     case ClusterConfig::k64x6: return launch<64, 6, 64, kFormCluster>(p, a_map, b_map, stream);
     case ClusterConfig::k128x4: return launch<128, 4, 64, kFormCluster>(p, a_map, b_map, stream);
     case ClusterConfig::k32x6r128: return launch<32, 6, 128, kFormCluster>(p, a_map, b_map, stream);
