@@ -9,7 +9,8 @@
 // stream through a ring. Where the ring holds two tiles, a tile's pairs stay until its output product has
 // read them. Where it does not (rank above 256), every pair is fetched twice, once per product (the second
 // time from L2, a few microseconds later), so that the stream never waits for a softmax: the scores of tile
-// j + 1 are computed before the output of tile j. One thread issues the TMA boxes, one the MMAs; four warps
+// j + 1 are computed before the output of tile j. A warp issues the TMA boxes, another the MMAs (an elected lane of each:
+// from a lone thread with suspending polls, the stream of 32 x 4096 latents of rank 512 took 52.6 us, 43.6 now); four warps
 // hold a key per thread, take the column maxima with warp reductions, and write the probabilities as two
 // bf16 numbers whose sum keeps 16 bits of mantissa: both are rows of one operand (2 N columns of O^T, added at
 // the end), because a product of this shape costs what reading its M operand costs. The reference maximum is lazy: O^T is rescaled in tensor memory only when a row's
@@ -124,23 +125,27 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
     if (slot >= 0 && row0 < rows)
       for (int r = threadIdx.x; r <= last_row - row0; r += kThreads)
         p.partial_stats[(unit0 + r) * p.splits + split] = make_float2(-INFINITY, 0.0f);
-  } else if (warp == kTmaWarp && lane == 0 && !p.drop_loads) {
-    // ---- TMA producer ----
-    mbarrier_arrive_expect_tx(smem_u32(&q_full), 2 * p.pairs * kQPanel);
+  } else if (warp == kTmaWarp && !p.drop_loads) {
+    // ---- TMA producer (the whole warp walks the loops, one lane issues) ----
+    const uint32_t leader = elect_one();
+    mbarrier_arrive_expect_tx_if(leader, smem_u32(&q_full), 2 * p.pairs * kQPanel);
     for (int panel = 0; panel < 2 * p.pairs; ++panel)
-      tma_load_2d(q_smem + panel * kQPanel, &q_map, smem_u32(&q_full), panel * 64, static_cast<int>(unit0));
+      tma_load_2d_if(leader, q_smem + panel * kQPanel, &q_map, smem_u32(&q_full), panel * 64, static_cast<int>(unit0));
     bool ok = true;
-    int index = 0;  // pairs fetched so far
+    int index = 0, place = 0, use = 0;  // pairs fetched so far; index % ring, index / ring
     auto push = [&](int j) {
       for (int m = 0; ok && m < p.pairs; ++m) {
-        const int place = index % p.ring, use = index / p.ring;
-        ok = use == 0 || mbarrier_wait_bounded(smem_u32(&pair_empty[place]), (use - 1) & 1, p.wait_limit);
+        ok = use == 0 || mbarrier_wait_warp(smem_u32(&pair_empty[place]), (use - 1) & 1, p.wait_limit);
         if (!ok) return;
-        mbarrier_arrive_expect_tx(smem_u32(&pair_full[place]), kPairBytes);
+        mbarrier_arrive_expect_tx_if(leader, smem_u32(&pair_full[place]), kPairBytes);
         for (int half = 0; half < 2; ++half)
-          tma_load_3d(ring_smem + place * kPairBytes + half * kPanelBytes, &c_map, smem_u32(&pair_full[place]),
-                      m * 128 + half * 64, static_cast<int>(begin) + j * kTileKeys, slot);
+          tma_load_3d_if(leader, ring_smem + place * kPairBytes + half * kPanelBytes, &c_map, smem_u32(&pair_full[place]),
+                         m * 128 + half * 64, static_cast<int>(begin) + j * kTileKeys, slot);
         ++index;
+        if (++place == p.ring) {
+          place = 0;
+          ++use;
+        }
       }
     };
     push(0);
@@ -155,7 +160,7 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
       mbarrier_wait_bounded(smem_u32(&pair_full[i % p.ring]), (i / p.ring) & 1, p.wait_limit);
   } else if (warp == kMmaWarp) {
     // ---- MMA issuer: the whole warp walks the loops (the descriptors stay in uniform registers), one lane issues ----
-    const uint32_t leader = lane == 0 ? 1u : 0u;
+    const uint32_t leader = elect_one();
     constexpr uint32_t idesc_s = instruction_descriptor(128, N);
     constexpr uint32_t idesc_o = instruction_descriptor(128, 2 * N, false, true);
     const uint64_t q_desc = smem_descriptor(q_smem), p_desc = smem_descriptor(p_smem);
@@ -163,7 +168,7 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
     int index = 0;  // pairs taken so far (refetch)
     auto next_pair = [&](int j, int m) { return p.refetch ? index++ : j * p.pairs + m; };
     auto landed = [&](int pair) {
-      ok = __all_sync(0xffffffffu, mbarrier_wait_bounded(smem_u32(&pair_full[pair % p.ring]), (pair / p.ring) & 1, p.wait_limit));
+      ok = mbarrier_wait_warp(smem_u32(&pair_full[pair % p.ring]), (pair / p.ring) & 1, p.wait_limit);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       return ok;
     };
@@ -184,7 +189,7 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
     if (ok) issue_scores(0);
     for (int j = 0; ok && j < tiles; ++j) {
       if (j + 1 < tiles) issue_scores(j + 1);  // (its buffer's scores, of tile j - 1, were read before p_full of j - 1)
-      ok = ok && __all_sync(0xffffffffu, mbarrier_wait_bounded(smem_u32(&p_full), j & 1, p.wait_limit));
+      ok = ok && mbarrier_wait_warp(smem_u32(&p_full), j & 1, p.wait_limit);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // Products with one accumulator follow one another at the latency of a product: two blocks of O^T
