@@ -1,6 +1,6 @@
 // Latent attention over cached latents on the 5th-generation tensor cores, transposed: the 128 keys of a
 // tile are the M rows of the score product and the rank is the M extent of the output product, so that
-// both run at full width however few (token, head) rows a decode step has; those rows are N (32 or 64).
+// both run at full width however few (token, head) rows a decode step has; those rows are N (16, 32 or 64).
 //
 //   S^T [128 keys x N]       = C Q^T        C tile K-major (as TMA lays it down), Q K-major
 //   O^T [128 rank x N] each  = C^T P^T      the same C tile read MN-major, P [N x 128 keys] K-major
@@ -59,7 +59,7 @@ template <int N>
 __global__ void __launch_bounds__(kThreads, 1)
 latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ CUtensorMap q_map,
                                 const __grid_constant__ CUtensorMap c_map) {
-  constexpr int kGroups = N / 32;                        // 32-column groups of a row of S^T
+  constexpr int W = N < 32 ? N : 32, kGroups = N / W;    // columns of a group, groups of a row of S^T
   constexpr uint32_t kQPanel = N * 128, kPPanel = 2 * N * 128, kPLow = N * 128;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t q_full, s_full[2], p_full, o_done, pair_full[kMaxRing], pair_empty[kMaxRing];
@@ -218,7 +218,7 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
     // ---- softmax: one key a thread ----
     const int row = warp * 32 + lane;                               // key of the tile, lane of tensor memory
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    float reference[kGroups];                                       // of row 32 g + lane
+    float reference[kGroups];                                       // of row W g + lane
     float sums[N];                                                  // over this thread's keys
 #pragma unroll
     for (int g = 0; g < kGroups; ++g) reference[g] = -INFINITY;
@@ -237,11 +237,11 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
-          float t[32], u[32];  // the sums over even and odd k-steps
-          tmem_load_32x32(tmem + (j & 1) * 2 * N + lane_base + g * 32, t);
-          tmem_load_32x32(tmem + (j & 1) * 2 * N + N + lane_base + g * 32, u);
+          float t[W], u[W];  // the sums over even and odd k-steps
+          tmem_load_32x32(tmem + (j & 1) * 2 * N + lane_base + g * W, t);
+          tmem_load_32x32(tmem + (j & 1) * 2 * N + N + lane_base + g * W, u);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) s[g * 32 + i] = (t[i] + u[i]) * p.scale_log2;
+          for (int i = 0; i < W; ++i) s[g * W + i] = (t[i] + u[i]) * p.scale_log2;
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         if ((j + 1) * kTileKeys > seen_by_all) {
@@ -253,11 +253,11 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
         for (int g = 0; g < kGroups; ++g) {
           float top = 0.0f;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float t = warp_max_redux(s[g * 32 + i]);
+          for (int i = 0; i < W; ++i) {
+            const float t = warp_max_redux(s[g * W + i]);
             if (lane == i) top = t;
           }
-          warp_tops[j & 1][warp][g * 32 + lane] = top;
+          if (lane < W) warp_tops[j & 1][warp][g * W + lane] = top;
         }
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -267,9 +267,10 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
       bool raise = false;
 #pragma unroll
       for (int g = 0; g < kGroups; ++g) {
-        float top = warp_tops[j & 1][0][g * 32 + lane];
+        const int place = g * W + min(lane, W - 1);
+        float top = warp_tops[j & 1][0][place];
 #pragma unroll
-        for (int w = 1; w < kSoftmaxWarps; ++w) top = fmaxf(top, warp_tops[j & 1][w][g * 32 + lane]);
+        for (int w = 1; w < kSoftmaxWarps; ++w) top = fmaxf(top, warp_tops[j & 1][w][place]);
         const bool move = top > reference[g] + kRaise || (reference[g] == -INFINITY && top > -INFINITY);
         factor[g] = move ? exp2_fast(reference[g] - top) : 1.0f;  // (0 where nothing had been seen)
         if (move) reference[g] = top;
@@ -283,25 +284,25 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
-          float f[32];
+          float f[W];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < W; ++i) {
             f[i] = __shfl_sync(0xffffffffu, factor[g], i);
-            sums[g * 32 + i] *= f[i];
+            sums[g * W + i] *= f[i];
           }
           for (int m = 0; m < 2 * p.pairs; ++m) {  // high and low parts
-            float t[32];
-            tmem_load_32x32(o_column + m * N + lane_base + g * 32, t);
+            float t[W];
+            tmem_load_32x32(o_column + m * N + lane_base + g * W, t);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) t[i] *= f[i];
-            tmem_store_32x32(o_column + m * N + lane_base + g * 32, t);
+            for (int i = 0; i < W; ++i) t[i] *= f[i];
+            tmem_store_32x32(o_column + m * N + lane_base + g * W, t);
           }
         }
         tmem_store_wait();
       }
 #pragma unroll
       for (int n = 0; n < N; ++n) {
-        const float r = __shfl_sync(0xffffffffu, reference[n / 32], n % 32);
+        const float r = __shfl_sync(0xffffffffu, reference[n / W], n % W);
         const float value = exp2_fast(s[n] - (r == -INFINITY ? 0.0f : r));
         sums[n] += value;
         const uint16_t high = f32_to_bf16_bits(value), low = f32_to_bf16_bits(value - bf16_to_f32(high));
@@ -338,14 +339,14 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
       for (int m = 0; m < p.pairs; ++m)
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
-          float t[32], low[32];
-          tmem_load_32x32(o_column + m * 2 * N + lane_base + g * 32, t);
-          tmem_load_32x32(o_column + m * 2 * N + N + lane_base + g * 32, low);
+          float t[W], low[W];
+          tmem_load_32x32(o_column + m * 2 * N + lane_base + g * W, t);
+          tmem_load_32x32(o_column + m * 2 * N + N + lane_base + g * W, low);
           if (m * 128 + row < p.rank) {
-            float* out = p.partial + ((unit0 + g * 32) * p.splits + split) * p.rank + m * 128 + row;
+            float* out = p.partial + ((unit0 + g * W) * p.splits + split) * p.rank + m * 128 + row;
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (row0 + g * 32 + i <= last_row) out[static_cast<int64_t>(i) * p.splits * p.rank] = t[i] + low[i];
+            for (int i = 0; i < W; ++i)
+              if (row0 + g * W + i <= last_row) out[static_cast<int64_t>(i) * p.splits * p.rank] = t[i] + low[i];
           }
         }
     }
@@ -354,11 +355,11 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
     for (int g = 0; g < kGroups; ++g) {
       float total = 0.0f;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float t = warp_sum(sums[g * 32 + i]);
+      for (int i = 0; i < W; ++i) {
+        const float t = warp_sum(sums[g * W + i]);
         if (lane == i) total = t;
       }
-      warp_tops[tiles & 1][warp][g * 32 + lane] = total;
+      if (lane < W) warp_tops[tiles & 1][warp][g * W + lane] = total;
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");
     if (warp == 0 && ok) {
@@ -366,9 +367,9 @@ latent_attention_tcgen05_kernel(const LatentTcParams p, const __grid_constant__ 
       for (int g = 0; g < kGroups; ++g) {
         float total = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kSoftmaxWarps; ++w) total += warp_tops[tiles & 1][w][g * 32 + lane];
-        if (row0 + g * 32 + lane <= last_row)
-          p.partial_stats[(unit0 + g * 32 + lane) * p.splits + split] = make_float2(reference[g], total);
+        for (int w = 0; w < kSoftmaxWarps; ++w) total += warp_tops[tiles & 1][w][g * W + min(lane, W - 1)];
+        if (lane < W && row0 + g * W + lane <= last_row)
+          p.partial_stats[(unit0 + g * W + lane) * p.splits + split] = make_float2(reference[g], total);
       }
     }
   }
@@ -387,11 +388,13 @@ LatentTcPlan plan_latent_tcgen05(int64_t sequences, int64_t longest, int64_t hea
   if (rank % 16 != 0 || rank > 512) return plan;
   const int64_t rows = longest * heads;
   plan.pairs = static_cast<int>(ceil_div(rank, 128));
-  int n = rows <= 32 ? 32 : 64, fixed = 0;
+  // (up to 16 rows, a decode step of 14 or 16 heads: 32 columns would double the softmax's work for rows that are not
+  // there; 32 x 4096, 16 heads x rank 512 43.5 -> 39.6 us)
+  int n = rows <= 16 ? 16 : rows <= 32 ? 32 : 64, fixed = 0;
   for (;; n = 32) {  // 64 rows where a whole tile fits beside them, and the output in tensor memory
     fixed = 2 * plan.pairs * n * 128 + 4 * n * 128;  // Q, P
     plan.ring = (222 * 1024 - fixed) / kPairBytes;
-    if ((plan.ring >= plan.pairs && (plan.pairs + 2) * 2 * n <= 512) || n == 32) break;
+    if ((plan.ring >= plan.pairs && (plan.pairs + 2) * 2 * n <= 512) || n <= 32) break;
   }
   if (plan.ring > kMaxRing) plan.ring = kMaxRing;
   if (plan.ring < plan.pairs || !tensor_memory_fits(512, fixed + plan.ring * kPairBytes)) return plan;
@@ -429,7 +432,11 @@ int latent_attention_tcgen05(const LatentTcPlan& plan, const void* q, const void
     return launch_chained(kernel, grid, dim3(kThreads), plan.smem, stream, p, q_map, c_map) == cudaSuccess
                ? B200_OK : B200_ERR_LAUNCH;
   };
-  return plan.n == 32 ? go(latent_attention_tcgen05_kernel<32>) : go(latent_attention_tcgen05_kernel<64>);
+  switch (plan.n) {
+    case 16: return go(latent_attention_tcgen05_kernel<16>);
+    case 32: return go(latent_attention_tcgen05_kernel<32>);
+    default: return go(latent_attention_tcgen05_kernel<64>);
+  }
 }
 
 }  // namespace b200
