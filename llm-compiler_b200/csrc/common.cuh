@@ -59,6 +59,10 @@ __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The line that holds `p`, requested into L2: for constants that are read late in a kernel (a norm's weight behind its
+// sum). L2 is coherent, so the request may be made before the dependency wait, whoever writes the line.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Thread-block cluster helpers: a barrier over all threads of the cluster (release / acquire,
 // so shared-memory writes before it are visible to the other CTAs after it) and a load from
 // the shared memory of the cluster's CTA `rank` at the offset of a local address.

@@ -119,7 +119,18 @@ __global__ void __launch_bounds__(Q == 1 ? 1024 : 512) residual_norm_quads_kerne
   float* x = p.x + row * p.width;
   const T* post = static_cast<const T*>(p.w_post);
   const T* next = static_cast<const T*>(p.w_next);
+  // The weights come from HBM in a model larger than L2, and are wanted one after the other, each behind a sum.
+  const int line = threadIdx.x * (128 / static_cast<int>(sizeof(T)));
+  if (line < p.width) {
+    if (post != nullptr) prefetch_l2(post + line);
+    if (next != nullptr) prefetch_l2(next + line);
+  }
   grid_dependency_wait_cta();
+  float4 post_weight = make_float4(0.0f, 0.0f, 0.0f, 0.0f), next_weight = post_weight;  // Q 1: beside the row's loads
+  if (Q == 1 && static_cast<int>(threadIdx.x) < quads) {
+    if (p.adds()) post_weight = load_quad<T>(post + threadIdx.x * 4);
+    if (next != nullptr) next_weight = load_quad<T>(next + threadIdx.x * 4);
+  }
   float4 v[Q], y[Q];
   float sum = 0.0f;
 #pragma unroll
@@ -137,14 +148,16 @@ __global__ void __launch_bounds__(Q == 1 ? 1024 : 512) residual_norm_quads_kerne
       for (int i = 0; i < Q; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
         if (c >= quads) continue;
-        for (int s0 = 0; s0 < p.splits; s0 += 4) {
-          float4 t[4];
+        constexpr int kAhead = Q == 1 ? 6 : 4;
+        for (int s0 = 0; s0 < p.splits; s0 += kAhead) {
+          float4 t[kAhead];
 #pragma unroll
-          for (int s = 0; s < 4; ++s)
+          for (int s = 0; s < kAhead; ++s)
             t[s] = s0 + s < p.splits ? __ldcg(reinterpret_cast<const float4*>(partial + (s0 + s) * slice + c * 4))
                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-          for (int s = 0; s < 4; ++s) {
+          for (int s = 0; s < kAhead; ++s) {
+            if (s0 + s >= p.splits) break;
             y[i].x += t[s].x; y[i].y += t[s].y; y[i].z += t[s].z; y[i].w += t[s].w;
           }
         }
@@ -184,7 +197,7 @@ __global__ void __launch_bounds__(Q == 1 ? 1024 : 512) residual_norm_quads_kerne
     for (int i = 0; i < Q; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
       if (c >= quads) continue;
-      const float4 w = load_quad<T>(post + c * 4);
+      const float4 w = Q == 1 ? post_weight : load_quad<T>(post + c * 4);
       v[i].x += y[i].x * factor * (p.weight_offset + w.x);
       v[i].y += y[i].y * factor * (p.weight_offset + w.y);
       v[i].z += y[i].z * factor * (p.weight_offset + w.z);
@@ -211,7 +224,7 @@ __global__ void __launch_bounds__(Q == 1 ? 1024 : 512) residual_norm_quads_kerne
   for (int i = 0; i < Q; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     if (c >= quads) continue;
-    const float4 w = load_quad<T>(next + c * 4);
+    const float4 w = Q == 1 ? next_weight : load_quad<T>(next + c * 4);
     store_quad<T>(h + c * 4, make_float4(v[i].x * factor * (p.weight_offset + w.x), v[i].y * factor * (p.weight_offset + w.y),
                                          v[i].z * factor * (p.weight_offset + w.z), v[i].w * factor * (p.weight_offset + w.w)));
   }
