@@ -99,6 +99,8 @@ __device__ __noinline__ void attend_row(const PrefillParams<T>& p, int b, int hq
 
 template <typename T, int D, int STAGES>
 __global__ void __launch_bounds__(kThreads) prefill_attention_kernel(const PrefillParams<T> p) {
+  grid_launch_dependents();
+  grid_dependency_wait();
   constexpr bool kHalf = IsHalf<T>::value;
   constexpr int kChunksPerRow = D / 8;
   constexpr int kTileBytes = kBN * D * 2;
@@ -584,8 +586,7 @@ int launch_warp_level(const PrefillParams<T>& p, cudaStream_t stream) {
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return B200_ERR_LAUNCH;
   dim3 grid((p.tokens + kBM - 1) / kBM, p.q_heads, p.batch);
-  kernel<<<grid, kThreads, smem, stream>>>(p);
-  return launch_status();
+  return launch_chained(kernel, grid, dim3(kThreads), smem, stream, p) == cudaSuccess ? launch_status() : B200_ERR_LAUNCH;
 }
 
 }  // namespace

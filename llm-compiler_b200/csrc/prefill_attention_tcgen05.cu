@@ -147,6 +147,10 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
   __shared__ int failed;
 
   TraceScope trace(8);
+  // (Programmatic launches: the set-up runs under the kernel before this one, whose results the copies alone read; the
+  // tile classes of a mask are read at once.)
+  grid_launch_dependents();
+  if (MASKED) grid_dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Blocks are handed out with z slowest: every (batch, head) gets its heaviest query block (the
   // last: most key tiles) before any gets a lighter one, so the lightest blocks fill the tail.
@@ -232,6 +236,7 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
 
   if (warp == kTmaWarp && lane == 0 && !p.drop_loads) {
     // ---- TMA producer ----
+    if (!MASKED) grid_dependency_wait();
     mbarrier_arrive_expect_tx(smem_u32(&q_full), G * kTileBytes);
 #pragma unroll
     for (int g = 0; g < G; ++g)
@@ -670,8 +675,7 @@ int prefill_attention_tcgen05(const void* query, const void* key, const void* va
   auto launch = [&](auto kernel) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return false;
-    kernel<<<grid, kThreads, smem, stream>>>(p, q_map, k_map, v_map);
-    return true;
+    return launch_chained(kernel, grid, dim3(kThreads), smem, stream, p, q_map, k_map, v_map) == cudaSuccess;
   };
   bool launched;
   if (mask != nullptr)
