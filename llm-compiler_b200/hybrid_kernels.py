@@ -161,7 +161,7 @@ def residual_norm(x: torch.Tensor, y, post_weight: Optional[torch.Tensor],
     if next_weight is not None or narrow:
         if next_weight is not None and (next_weight.shape != (width,) or next_weight.dtype != dtype):
             raise ValueError("the norm weight must be a vector of the residual's width")
-        h = torch.empty((rows, pad8(width)), dtype=dtype, device=device)
+        h = x.new_empty((rows, pad8(width)), dtype=dtype) if next_weight is None else next_weight.new_empty((rows, pad8(width)))
     rt = runtime(device)
     code = _lib.load().b200_residual_norm(
         x.data_ptr(), _ptr(y), _ptr(parts.bias), _ptr(post_weight), _ptr(next_weight), _ptr(h), _ptr(parts.rows),
@@ -186,7 +186,7 @@ def latent_norm(projected: torch.Tensor, q_weight: torch.Tensor, kv_weight: Opti
     if projected.dtype != q_weight.dtype or (kv_weight is not None and (
             cache is None or cache.dtype != projected.dtype or not cache.is_contiguous())):
         raise ValueError("projection, weights and cache must share one dtype")
-    q_out = torch.empty((rows, pad8(q_rank)), dtype=projected.dtype, device=device)
+    q_out = projected.new_empty((rows, pad8(q_rank)))
     kv_rank = kv_weight.shape[0] if kv_weight is not None else 0
     row = cache.shape[2] if kv_weight is not None else 0
     dense_out = torch.empty((rows, row), dtype=projected.dtype, device=device) \
@@ -212,7 +212,7 @@ def gated_head_norm(read_out: torch.Tensor, weight: Optional[torch.Tensor], gate
     _require_rows(gate, "the gate")
     if read_out.dtype != torch.float32 or not read_out.is_contiguous() or gate.shape[0] != rows:
         raise ValueError("the read-out must be contiguous fp32 and match the gate")
-    output = torch.empty((rows, pad8(heads * vdim)), dtype=gate.dtype, device=device)
+    output = gate.new_empty((rows, pad8(heads * vdim)))
     rt = runtime(device)
     code = _lib.load().b200_gated_head_norm(
         read_out.data_ptr(), _ptr(weight), gate.data_ptr(), output.data_ptr(), rows, heads, vdim, gate.stride(0),
@@ -339,7 +339,7 @@ def recurrence_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Opt
     if state.dtype != torch.float32 or state.ndim != 4 or not state.is_contiguous() or \
             state.shape[1] != heads or state.shape[2] != dim or state.shape[3] < vdim:
         raise ValueError("the state must be contiguous fp32 [slots, heads, dim, >= vdim]")
-    output = torch.empty((rows, heads, vdim), dtype=torch.float32, device=device)
+    output = v.new_empty((rows, heads, vdim))
     rt = runtime(device)
     code = _lib.load().b200_recurrence_scan(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(beta), decay.data_ptr(), state.data_ptr(), output.data_ptr(),
@@ -365,7 +365,7 @@ def recurrence_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: 
     need = int(library.b200_recurrence_chunked_workspace_bytes(chunks, heads, dim, vdim, int(beta is not None)))
     if need == 0:
         return None
-    output = torch.empty((rows, heads, vdim), dtype=torch.float32, device=device)
+    output = v.new_empty((rows, heads, vdim))
     rt = runtime(device)
     workspace = rt.workspace("recurrence_chunked", need)
     code = library.b200_recurrence_chunked(
@@ -397,7 +397,7 @@ def head_linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tenso
         raise ValueError("head_linear needs x [rows, heads, k] and a contiguous weight [heads, n, k]")
     n = weight.shape[1]
     if out is None:
-        out = torch.empty((rows, heads, n), dtype=x.dtype, device=device)
+        out = x.new_empty((rows, heads, n))
     rt = runtime(device)
     code = _lib.load().b200_head_linear(x.data_ptr(), weight.data_ptr(), out.data_ptr(), rows, heads, k, n,
                                         x.stride(0), x.stride(1), out.stride(0), out.stride(1), _code(x.dtype),
@@ -481,7 +481,7 @@ def attention_prep(projected: torch.Tensor, bias: Optional[torch.Tensor], q_weig
                                  not (keys.is_contiguous() and values.is_contiguous())):
         raise ValueError("caches must be contiguous [slots, capacity, kv_heads, row_size] in the weights' dtype")
     own = k_weight is not None
-    q = torch.empty((rows, heads, row_size), dtype=q_weight.dtype, device=device)
+    q = q_weight.new_empty((rows, heads, row_size))
     inputs = _lib.AttentionPrepInputs(
         projected.data_ptr(), _ptr(bias), q_weight.data_ptr(), _ptr(k_weight), turns.data_ptr(), q.data_ptr(),
         _ptr(keys) if own else None, _ptr(values) if own else None, *batch.pointers(), rows, heads, kv_heads, dim, vdim,
@@ -607,7 +607,7 @@ def expert_route(logits: torch.Tensor, h: torch.Tensor, counters: torch.Tensor, 
     if logits.dtype != torch.float32 or not logits.is_contiguous() or h.shape[0] != rows:
         raise ValueError("the router's logits are contiguous fp32, a row for every row of h")
     order, block = _expert_order(rows, counters, top, always, tile)
-    ordered = torch.empty((order.index.shape[0], h.shape[1]), dtype=h.dtype, device=device)
+    ordered = h.new_empty((order.index.shape[0], h.shape[1]))
     rt = runtime(device)
     library = _lib.load()
     _check(library.b200_expert_route(logits.data_ptr(), byref(block), rows, logits.shape[0] if logits.ndim == 3 else 1,
@@ -630,7 +630,7 @@ def grouped_linear(x: torch.Tensor, weight: torch.Tensor, order: ExpertOrder, *,
     if not (x.is_contiguous() and weight.is_contiguous()) or x.ndim != 2 or x.shape[1] != k or x.dtype != weight.dtype or \
             x.shape[0] != (order.places.shape[0] if gather else sorted_rows):
         raise ValueError("grouped_linear needs contiguous rows and weights [experts, n, k] of one dtype")
-    output = torch.empty((sorted_rows, n // 2 if swiglu else n), dtype=x.dtype, device=device)
+    output = x.new_empty((sorted_rows, n // 2 if swiglu else n))
     rt = runtime(device)
     code = _lib.load().b200_grouped_linear(
         x.data_ptr(), weight.data_ptr(), order.tiles.data_ptr(), order.index.data_ptr() if gather else None,

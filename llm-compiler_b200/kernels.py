@@ -11,6 +11,7 @@ libb200serve.so, and a missing library or a CPU tensor is an error, never a fall
 from __future__ import annotations
 
 import contextlib
+import functools
 import ctypes
 import math
 from typing import Optional, Tuple
@@ -193,18 +194,20 @@ def _guard_current_device(device: torch.device) -> None:
 
 
 def _require_cuda(*tensors: torch.Tensor) -> torch.device:
-    device = None
+    index, device = -1, None
     for tensor in tensors:
         if tensor is None:
             continue
         if not isinstance(tensor, torch.Tensor) or not tensor.is_cuda:
             raise ValueError("the B200 backend only runs CUDA tensors (there is no CPU fallback)")
-        if device is None:
-            device = tensor.device
-        elif tensor.device != device:
+        own = tensor.get_device()
+        if index < 0:
+            index, device = own, tensor.device
+        elif own != index:
             raise ValueError("all operands must live on the same CUDA device")
     assert device is not None
-    _guard_current_device(device)
+    if index != torch._C._cuda_getDevice():  # (there are CUDA tensors: no need to ask whether CUDA is initialised)
+        _guard_current_device(device)
     return device
 
 
@@ -224,7 +227,7 @@ def _mode(numerical_mode: str) -> int:
 
 def _stream() -> int:
     # (the raw handle: building a torch.cuda.Stream around it costs 3 us a launch)
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _check(code: int, what: str) -> None:
@@ -879,6 +882,13 @@ def linear_workspace_bytes(m: int, k: int, n: int, dtype: torch.dtype,
                                                        _EPILOGUES[epilogue]))
 
 
+@functools.lru_cache(maxsize=4096)
+def _linear_need(m: int, k: int, n: int, dtype: int, epilogue: int) -> int:
+    """Workspace bytes of a projection: sizes in, bytes out, so every size asks the library once."""
+
+    return int(_lib.load().b200_linear_workspace_bytes(m, k, n, dtype, epilogue))
+
+
 def _linear_workspace(rt: DeviceRuntime, nbytes: int, dtype: torch.dtype) -> Optional[torch.Tensor]:
     """fp16 projections took no workspace, and could run on several streams at once, before split K came to them."""
 
@@ -900,29 +910,29 @@ def b200_linear(tensor: torch.Tensor, weight: torch.Tensor,
     if weight.ndim != 2:
         raise ValueError("weight must be N x K")
     n, k = weight.shape
-    if tensor.ndim < 1 or tensor.shape[-1] != k:
+    shape, dtype = tensor.shape, tensor.dtype
+    if not shape or shape[-1] != k:
         raise ValueError("the last input dimension must equal the weight's K")
-    if tensor.dtype != weight.dtype:
+    if dtype != weight.dtype:
         raise ValueError("input and weight must share one dtype")
-    if bias is not None and (bias.shape != (n,) or bias.dtype != tensor.dtype):
+    if bias is not None and (bias.shape != (n,) or bias.dtype != dtype):
         raise ValueError("bias must be a vector of N elements in the input dtype")
     if epilogue not in _EPILOGUES:
         raise ValueError(f"unknown epilogue {epilogue!r}")
     weight = _dense(weight)
-    row_stride = k
-    if tensor.ndim == 2 and tensor.stride(1) == 1 and tensor.stride(0) >= k and (
-            tensor.dtype != torch.bfloat16 or
-            (tensor.stride(0) % 8 == 0 and tensor.data_ptr() % 16 == 0)):
-        source, row_stride = tensor, tensor.stride(0)  # a column slice of a wider matrix
-    else:
-        source = _dense(tensor) if tensor.ndim <= 4 else tensor
+    source, row_stride, matrix = tensor, k, len(shape) == 2
+    if not (matrix and tensor.stride(1) == 1 and tensor.stride(0) >= k and (
+            dtype != torch.bfloat16 or (tensor.stride(0) % 8 == 0 and tensor.data_ptr() % 16 == 0))):
+        source = _dense(tensor) if len(shape) <= 4 else tensor
         if not source.is_contiguous():
             raise ValueError("inputs of rank > 4 must be contiguous")
-    m = source.numel() // k
+    else:
+        row_stride = tensor.stride(0)  # a column slice of a wider matrix
+    m = shape[0] if matrix else source.numel() // k
     out_features = n // 2 if epilogue == "swiglu" else n
-    output = torch.empty((*tensor.shape[:-1], out_features), dtype=tensor.dtype, device=device)
+    output = tensor.new_empty((m, out_features) if matrix else (*shape[:-1], out_features))
     if epilogue == "residual":
-        if residual is None or residual.shape != output.shape or residual.dtype != tensor.dtype:
+        if residual is None or residual.shape != output.shape or residual.dtype != dtype:
             raise ValueError("residual must match the output shape and dtype")
         residual = _dense(residual)
     elif residual is not None:
@@ -930,13 +940,12 @@ def b200_linear(tensor: torch.Tensor, weight: torch.Tensor,
     if bias is not None:
         bias = _dense(bias)
     rt = runtime(device)
-    library = _lib.load()
-    code_dtype = _code(tensor.dtype)
-    need = int(library.b200_linear_workspace_bytes(m, k, n, code_dtype, _EPILOGUES[epilogue]))
-    workspace = _linear_workspace(rt, need, tensor.dtype)
-    code = library.b200_linear(source.data_ptr(), weight.data_ptr(), _ptr(bias), _ptr(residual),
-                               output.data_ptr(), m, k, n, row_stride, code_dtype,
-                               _EPILOGUES[epilogue], _ptr(workspace), need, rt.status.data_ptr(), _stream())
+    code_dtype, code_epilogue = _code(dtype), _EPILOGUES[epilogue]
+    need = _linear_need(m, k, n, code_dtype, code_epilogue)
+    workspace = _linear_workspace(rt, need, dtype) if need else None
+    code = _lib.load().b200_linear(source.data_ptr(), weight.data_ptr(), _ptr(bias), _ptr(residual),
+                                   output.data_ptr(), m, k, n, row_stride, code_dtype,
+                                   code_epilogue, _ptr(workspace), need, rt.status.data_ptr(), _stream())
     _check(code, "b200_linear")
     _count(rt)
     return output
