@@ -297,7 +297,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
       if (leader) mbarrier_expect_tx(bar, static_cast<uint32_t>(bn * 128));
       tma_load_2d_if(leader, smem_base + kb * kStageBytes + kABytes, &b_map, bar, k_of(kb), tile_n * bn);
     }
-    if (p.prefetch_l2 && leader)
+    if (p.prefetch_l2 && tile_m == 0 && leader)
       for (int kb = early; kb < nkb; ++kb) tma_prefetch_l2_2d(&b_map, k_of(kb), tile_n * bn);
     __syncwarp();
     grid_dependency_wait();
@@ -311,7 +311,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
       const uint32_t bar = smem_u32(&full_bar[s]);
       const uint32_t a_dst = smem_base + s * kStageBytes;
       mbarrier_arrive_expect_tx_if(leader, bar, kb < early ? static_cast<uint32_t>(kABytes) : stage_tx_bytes);
-      tma_load_2d_if(leader, a_dst, &a_map, bar, k_of(kb), tile_m * kBM);
+      tma_load_2d_if(leader, a_dst, &a_map, bar, k_of(kb), tile_m * A_ROWS);
       if (kb >= early) tma_load_2d_if(leader, a_dst + kABytes, &b_map, bar, k_of(kb), tile_n * bn);
     }
     __syncwarp();
@@ -366,8 +366,8 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
       const int row = r + 64 * h;
       if (kNorm)
         row_scale[row] = rsqrtf(ss[h] / static_cast<float>(p.k) + p.norm_eps);
-      else if (tile_m * kBM + row < p.m)
-        p.row_squares[static_cast<int64_t>(split) * p.m + tile_m * kBM + row] = fine ? ss[h] : 0.0f;
+      else if (tile_m * A_ROWS + row < p.m)
+        p.row_squares[static_cast<int64_t>(split) * p.m + tile_m * A_ROWS + row] = fine ? ss[h] : 0.0f;
     }
   }
   if (kNorm && warp >= 2 && p.norm_squares != nullptr) {
@@ -379,7 +379,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
     __syncwarp();
 #pragma unroll 1
     for (int row = (warp - 2) * 32 + lane; row < A_ROWS; row += 64) {
-      const int global_row = tile_m * kBM + row;
+      const int global_row = tile_m * A_ROWS + row;
       float ss = 0.0f;
       if (global_row < p.m) {
         const float* src = p.norm_squares + global_row;
@@ -440,7 +440,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
     // send region have landed. A CTA whose waits gave up still ships (zeros) and arrives.
     // (The code is kept small on purpose -- one division per thread, rolled loops: a kernel this
     // short pays for every instruction-cache line it touches for the first time.)
-    const int rows = min(A_ROWS, p.m - tile_m * kBM);
+    const int rows = min(A_ROWS, p.m - tile_m * A_ROWS);
     const int unit_shift = 31 - __clz(bn / 4);  // bn is 32, 64 or 128 here: 8, 16 or 32 units a row
     const int owned = reduce_owned;
     const uint32_t chunk_bytes = static_cast<uint32_t>(owned * 16);
@@ -489,7 +489,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
     const int first_item = threadIdx.x * p.splits + rank;
     const int first_row = first_item >> unit_shift, first_col = tile_n * bn + (first_item & ((bn / 4) - 1)) * 4;
     const bool first_valid = threadIdx.x < owned && first_row < rows && first_col < n_end;
-    const int64_t first_offset = static_cast<int64_t>(tile_m * kBM + first_row) * p.n + first_col;
+    const int64_t first_offset = static_cast<int64_t>(tile_m * A_ROWS + first_row) * p.n + first_col;
     uint2 res = first_valid ? *reinterpret_cast<const uint2*>(p.residual + first_offset) : make_uint2(0u, 0u);
     const bool landed = mbarrier_wait_bounded(smem_u32(&reduce_bar), 0, p.wait_limit);
     trace.stamp(4);
@@ -503,7 +503,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
           asm volatile("st.shared.f32 [%0], %1;" ::"r"(recv_base + local * 16), "f"(0.0f) : "memory");
         continue;
       }
-      const int64_t o = static_cast<int64_t>(tile_m * kBM + r) * p.n + col;  // n % 4 == 0
+      const int64_t o = static_cast<int64_t>(tile_m * A_ROWS + r) * p.n + col;  // n % 4 == 0
       if (local != threadIdx.x) res = *reinterpret_cast<const uint2*>(p.residual + o);
       float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       float4 t[8];
@@ -541,7 +541,7 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
           asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sq) : "r"(recv_base + (i / p.splits) * 16) : "memory");
           ss += sq;
         }
-        p.squares_out[static_cast<int64_t>(tile_n * p.splits + rank) * p.m + tile_m * kBM + r] = ss;
+        p.squares_out[static_cast<int64_t>(tile_n * p.splits + rank) * p.m + tile_m * A_ROWS + r] = ss;
       }
     }
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -549,7 +549,8 @@ linear_tcgen05_kernel(const Tcgen05ParamsOf<T> p, const __grid_constant__ CUtens
     trace.stamp(6);
     if (!ok && threadIdx.x == 0 && p.status != nullptr) atomicOr(p.status, B200_STATUS_WAIT_TIMEOUT);
   } else if (ok) {
-    const int row = tile_m * kBM + warp * 32 + lane;
+    // (the accumulator's lanes behind a tile of 64 rows hold junk)
+    const int row = warp * 32 + lane < A_ROWS ? tile_m * A_ROWS + warp * 32 + lane : p.m;
     const float scale = kNorm ? row_scale[(warp * 32 + lane) % kBM] : 1.0f;
     const int n_end = min(p.n, (tile_n + 1) * bn);  // columns of this tile
 #pragma unroll 1
@@ -874,7 +875,7 @@ int launch(const Tcgen05ParamsOf<T>& p, const CUtensorMap& a_map, const CUtensor
   auto kernel = linear_tcgen05_kernel<BN, STAGES, A_ROWS, FORM, T>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return B200_ERR_LAUNCH;
-  const int64_t tiles_n = ceil_div(p.n, p.bn), tiles_m = ceil_div(p.m, kBM);
+  const int64_t tiles_n = ceil_div(p.n, p.bn), tiles_m = ceil_div(p.m, A_ROWS);
   Tcgen05ParamsOf<T> q = p;
   static const bool n_fastest_always = [] {  // B200_TILE_ORDER=n: the comparison run
     const char* text = getenv("B200_TILE_ORDER");
@@ -1147,8 +1148,20 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
     c.norm_eps = norm_eps;
     if (takes_few_rows(c)) return linear_few_rows(c, IsHalf<T>::value ? B200_F16 : B200_BF16, stream);
   }
+  // Short prompts against narrow matrices: the smallest tiles that have an SM each. What a CTA waits for is its ring (W is
+  // 1 us away), and a stage of 64 rows and 32 columns is half the bytes, so that twice as many are under way; the products
+  // of a K 16 step take 40 cycles against 48. 77 rows, 128 x 64 -> 64 x 32: 4864 x 896 17.8 -> 16.6 us, 896 x 896 6.4 -> 6.0,
+  // 300 rows (64 x 32) 18.2 -> 16.7 and 6.9 -> 6.0, 515 rows (64 x 64) 18.2 -> 17.4 and 7.0 -> 6.5.
+  int a_rows = m <= 64 ? 64 : kBM;
+  if (m > 64 && !persistent && !fold_norm && bn == 64) {
+    for (int columns : {32, 64})
+      if (a_rows == kBM && ceil_div(n, static_cast<int64_t>(columns)) * ceil_div(m, static_cast<int64_t>(64)) <= kNumSMs) {
+        a_rows = 64;
+        bn = columns;
+      }
+  }
   CUtensorMap a_map, b_map;
-  if (!make_bf16_matrix_map(&a_map, input, m, k, input_row_stride, m <= 64 ? 64 : kBM) ||
+  if (!make_bf16_matrix_map(&a_map, input, m, k, input_row_stride, a_rows) ||
       !make_bf16_matrix_map(&b_map, weight, n, k, k, bn))
     return B200_ERR_UNSUPPORTED;
   Tcgen05ParamsOf<T> p;
@@ -1182,6 +1195,8 @@ int linear_tcgen05_of(const void* input, const void* weight, const void* bias, c
     return launch_linear<64, 12, 64>(p, a_map, b_map, stream);
   }
   if (persistent) return launch_persistent(p, a_map, b_map, stream);
+  if (a_rows == 64)
+    return bn == 32 ? launch<32, 16, 64, kFormPlain>(p, a_map, b_map, stream) : launch<64, 12, 64, kFormPlain>(p, a_map, b_map, stream);
   if (bn == 256) return launch_linear<256, 4, 128>(p, a_map, b_map, stream);
   // Two CTAs an SM hide one another's latencies behind short rings. Tiles that do not fill the GPU once have an SM each,
   // which hides them behind a ring of all its shared memory: W comes from HBM, 1 us away, and a stage of 64 columns is

@@ -1,6 +1,7 @@
-"""Projections of 65 rows and more in 64- and 128-column tiles, on both sides of the line between short rings and long ones
-(148 tiles), K in fewer blocks than a ring has stages and in more: a tile's sums do not depend on the ring, so every row
-and column equals that of a call on the other side of the line bit for bit."""
+"""Projections of 65 rows and more in tiles of 64 or 128 rows and 32, 64 or 128 columns, on both sides of the lines between
+the tiles and between short rings and long ones (148 tiles), K in fewer blocks than a ring has stages and in more: a tile's
+sums do not depend on its size or its ring, so every row and column equals that of a call on the other side of a line bit
+for bit."""
 
 import pytest
 import torch
@@ -12,9 +13,11 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("epilogue", ["none", "residual", "swiglu"])
-# tiles: 2 x 74 and 2 x 75 of 64 columns; 1 x 148 and 1 x 149 of 64; 5 x 28 and 5 x 30 of 128; ragged rows and columns
+# tiles: 2 x 74 and 2 x 75 of 64 columns; 1 x 148 and 1 x 149 of 64; 5 x 28 and 5 x 30 of 128; ragged rows and columns;
+# 64-row tiles: 3 x 49 of 32 columns and 3 x 50; 2 x 74 of 64 columns and 2 x 75
 @pytest.mark.parametrize("m,k,n,fewer", [(130, 896, 4800, 4736), (77, 64, 9500, 9470), (128, 456, 9536, 9472),
-                                         (515, 1032, 3840, 3584), (600, 8, 3840, 3520)])
+                                         (515, 1032, 3840, 3584), (600, 8, 3840, 3520),
+                                         (130, 1096, 1600, 1568), (65, 328, 4800, 4736), (129, 4864, 912, 896)])
 def test_sums_do_not_depend_on_the_ring(m, k, n, fewer, epilogue, dtype):
     g = torch.Generator(device="cuda").manual_seed(m + k + n)
     x, w = ((torch.randn(*s, generator=g, device="cuda") * k ** -0.25).to(dtype) for s in ((m, k), (n, k)))
