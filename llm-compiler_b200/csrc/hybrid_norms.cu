@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(Q == 1 ? 1024 : 512) residual_norm_quads_kerne
   float* x = p.x + row * p.width;
   const T* post = static_cast<const T*>(p.w_post);
   const T* next = static_cast<const T*>(p.w_next);
-  // The weights come from HBM in a model larger than L2, and are wanted one after the other, each behind a sum.
+  // The weights come from HBM in a model larger than L2, and are wanted one after the other, each behind a sum (32 rows x
+  // 2048 in a chain of launches, with more of the partial sums in flight: 6.1 -> 5.2 us).
   const int line = threadIdx.x * (128 / static_cast<int>(sizeof(T)));
   if (line < p.width) {
     if (post != nullptr) prefetch_l2(post + line);

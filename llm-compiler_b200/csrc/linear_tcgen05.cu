@@ -1,7 +1,7 @@
 // serve.linear on the 5th-generation tensor cores: tcgen05.mma with the accumulator in tensor
 // memory (TMEM), operands staged in shared memory by TMA.
 //
-// y[M,N] = x[M,K] W[N,K]^T, both operands K-major and both bf16 or both fp16. One CTA computes a 128 x bn tile over
+// y[M,N] = x[M,K] W[N,K]^T, both operands K-major and both bf16 or both fp16. One CTA computes an A_ROWS x bn tile over
 // one K slice (bn: a runtime multiple of 16 up to the template's BN accumulator columns of
 // TMEM, fp32). Roles inside the CTA of 4 warps:
 //   warp 0, one elected lane  TMA producer: per k-block one A_ROWS x 64 box of x and one bn x 64
@@ -19,12 +19,12 @@
 //   all 4 warps               epilogue: tcgen05.ld of the warp's 32 TMEM lanes (= 32 output
 //                             rows) x 32 columns at a time; bias / residual / SwiGLU with the
 //                             reference's bf16 rounding points, or fp32 split-K partials.
-// Decode-size M (A_ROWS 64): the x box has 64 rows and the MMA, which always spans 128, reads on
-// into the W tile behind it; accumulator lanes 64..127 then hold junk that nobody reads.
+// Tiles of 64 rows (A_ROWS 64: decode sizes, short prompts): the x box has 64 rows and the MMA, which always spans 128,
+// reads on into the W tile behind it; accumulator lanes 64..127 then hold junk that nobody reads.
 // Every mbarrier wait is bounded; a wait that gives up sets B200_STATUS_WAIT_TIMEOUT, the CTA
-// still frees its TMEM columns and returns. No cluster launch, no load shared between CTAs:
-// each CTA fetches its own tiles; with BN 128 at prefill sizes a second CTA resident on the SM
-// overlaps its main loop with this one's epilogue (2 x 96 KB of stages, 2 x 128 TMEM columns).
+// still frees its TMEM columns and returns. No load is shared between CTAs: each fetches its own tiles; with BN 128 and
+// more tiles than SMs a second CTA resident on the SM overlaps its main loop with this one's epilogue (2 x 96 KB of
+// stages, 2 x 128 TMEM columns).
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -838,9 +838,8 @@ struct PartialPlan {
   int bn, splits;
 };
 
-// Decode-size GEMMs with rings just deep enough for their K slice: the CTAs of the next kernel
-// of the chain then fit on the SM beside them and run their set-up (and first weight fetches)
-// early. B200_GEMM_RINGS=deep keeps the deep rings.
+// Short rings for the shortest K slices (up to 4 blocks), and in the plans: how many clusters are resident together, and so
+// the number of K slices, is decided for them, whatever ring is launched. B200_GEMM_RINGS=deep: deep rings everywhere.
 bool small_rings() {
   static const bool value = [] {
     const char* text = getenv("B200_GEMM_RINGS");
