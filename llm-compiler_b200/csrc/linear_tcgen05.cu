@@ -1256,8 +1256,9 @@ int linear_partial_tcgen05(const void* input, const void* weight, float* partial
   p.drop_loads = drop_loads();
   if (a_rows == 64) {
     // A K slice of many k-blocks is a long weight stream: it wants about 2 us x 44 GB/s of
-    // loads in flight per SM, twice what the 96 KB rings of the short slices hold.
-    const bool long_slice = ceil_div(ceil_div(k, kBK), splits) >= 24;
+    // loads in flight per SM, twice what the 96 KB rings of the short slices hold. (From 8 blocks on: 32 rows, 9 slices of
+    // 15 blocks of 2048 x 8192 in a Bazirax step, 4616 -> 4536 us for 8 steps; a Lozanex step, 4 or 8 blocks a slice, the same.)
+    const bool long_slice = ceil_div(ceil_div(k, kBK), splits) >= 8;
     if (plan.bn == 32)
       return small_rings() && ceil_div(ceil_div(k, kBK), splits) <= 4 ? launch<32, 4, 64, kFormPartial>(p, a_map, b_map, stream)
                                                                       : launch<32, 8, 64, kFormPartial>(p, a_map, b_map, stream);
