@@ -33,3 +33,19 @@ def test_sums_do_not_depend_on_the_ring(m, k, n, fewer, epilogue, dtype):
         bound = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * exact.abs() + \
             (k / 16 + 8) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + 1e-6
         assert ((full.double() - exact).abs() <= bound).all()
+
+
+# K blocks a slice (64 rows: 6 or 4 stages up to 7 blocks, 12 or 8 from 8 on): 7, 8 (one of them ragged), 12, 15, 15 in one slice
+@pytest.mark.parametrize("k,n", [(448, 18944), (4096, 1024), (4040, 1016), (3584, 3584), (8200, 2048), (904, 18944)])
+@pytest.mark.parametrize("m", [9, 64])
+def test_partial_sums_do_not_depend_on_the_ring(m, k, n):
+    g = torch.Generator(device="cuda").manual_seed(m + k + n)
+    x = (torch.randn(65, k, generator=g, device="cuda") * k ** -0.25).bfloat16()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.25).bfloat16()
+    taller = kernels.b200_linear_partial(x, w)  # 128-row tiles, short rings
+    few = kernels.b200_linear_partial(x[:m], w)
+    assert few.shape[0] == taller.shape[0] and torch.equal(few, taller[:, :m])
+    # fp32 sums in one chain of products a slice, the slices added in 64 bits
+    exact = x[:m].double() @ w.double().T
+    bound = (k / 16 + 8) * 2.0 ** -23 * (x[:m].double().abs() @ w.double().abs().T) + 1e-6
+    assert ((few.double().sum(0) - exact).abs() <= bound).all()
