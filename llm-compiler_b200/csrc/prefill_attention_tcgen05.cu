@@ -482,8 +482,9 @@ prefill_attention_tcgen05_kernel(const PrefillTcParams p, const __grid_constant_
         const bool raise = __any_sync(0xffffffffu, m_tile > m_ref + kRescaleThreshold);
         // P and O are in use until the group's previous product has completed
         ok = __all_sync(0xffffffffu, mbarrier_wait_ready_first(smem_u32(&o_done[g]), (j - 1) & 1, p.wait_limit));
+        // ... and what this thread does to tensor memory next, the stores of P as well as the moves of O, comes behind it
+        if (ok) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ok && raise) {  // warp-uniform: move the reference maximum of the warp's rows
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const float m_new = fmaxf(m_ref, m_tile);
           // (a row that has seen only -inf so far holds O = 0 and sum 0: any factor keeps them)
           const float factor = m_ref == -INFINITY ? 0.0f : exp2_fast(m_ref - m_new);

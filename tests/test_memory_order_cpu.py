@@ -1,0 +1,19 @@
+"""Orderings between threads, grids and the tensor core that no run can be relied on to show: read off the kernels' source."""
+
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "llm-compiler_b200" / "csrc"
+
+
+def test_probabilities_in_tensor_memory_are_stored_behind_the_product_before():
+    """Prompt attention keeps one buffer of P a group. The product that read it is behind the wait on o_done, but only a
+    fence orders a thread's next access to tensor memory behind a wait: it belongs between the wait and the stores on every
+    path, not only where O is moved as well."""
+
+    source = (CSRC / "prefill_attention_tcgen05.cu").read_text()
+    wait = re.search(r"mbarrier_wait_ready_first\(smem_u32\(&o_done\[g\]\), \(j - 1\) & 1", source)
+    move = source.index("if (ok && raise)", wait.end())
+    store = source.index("tmem_store_32x16(p_taddr", move)
+    assert wait.end() < move < store
+    assert re.search(r'if \(ok\) asm volatile\("tcgen05\.fence::after_thread_sync;"', source[wait.end():move])

@@ -1,0 +1,32 @@
+"""Kernels whose operands are written while they are already resident, or reused while the tensor core may still read."""
+
+import pytest
+import torch
+
+import llm_compiler_b200 as b200
+from llm_compiler_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("size", [64, 128])
+def test_prompt_attention_whose_reference_maximum_stays(size):
+    """Scores within 8 of the first tile's maximum (log2 domain): no tile moves O, so that the stores of P follow the wait for
+    the product before directly, 17 times a group. Many heads, so that SMs run different query blocks side by side."""
+
+    g = torch.Generator(device="cuda").manual_seed(size)
+    tokens, heads, kv_heads = 2100, 14, 2
+    q, k, v = (torch.randn(1, h, tokens, size, generator=g, device="cuda").bfloat16() for h in (heads, kv_heads, kv_heads))
+    first = b200.b200_prefill_attention(q, k, v, None, scale=size ** -0.5, causal=True)
+    for _ in range(20):
+        assert torch.equal(b200.b200_prefill_attention(q, k, v, None, scale=size ** -0.5, causal=True), first)
+    kernels.runtime().check_status()
+    seen = torch.ones(tokens, tokens, dtype=torch.bool, device="cuda").tril()
+    for head in (0, 6, 13):
+        scores = (q[0, head].double() @ k[0, head // 7].double().T * size ** -0.5).masked_fill(~seen, -torch.inf)
+        weights, values = torch.softmax(scores, -1), v[0, head // 7].double()
+        exact = weights @ values
+        # probabilities and results are rounded to bf16 once each: 8 significant bits, so by 2^-8 of the value at most
+        # (2^-9 just below a power of two); fp32 sums and exponentials err far less
+        bound = 1.01 * 2.0 ** -8 * (weights @ values.abs() + exact.abs()) + 1e-6
+        assert ((first[0, head].double() - exact).abs() <= bound).all()
