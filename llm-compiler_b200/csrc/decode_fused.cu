@@ -10,6 +10,8 @@
 //
 // Rounding points are those of the separate reference ops (linear -> add -> rms_norm, and
 // linear -> rope -> kv.store), so the fusion changes launch counts, not numerics.
+// (No __restrict__: the kernel before may still be writing when these are resident, and nothing but constant weights may be
+// read ahead of the wait.)
 #include "common.cuh"
 
 namespace b200 {
@@ -19,10 +21,10 @@ constexpr int kNormThreads = 1024;  // one element per thread at hidden <= 1024
 constexpr int kMaxPerThread = 4;    // hidden <= 4096 kept in registers
 
 __global__ void __launch_bounds__(kNormThreads)
-reduce_residual_rms_norm_kernel(const float* __restrict__ partials, int splits,
-                                const __nv_bfloat16* __restrict__ residual,
-                                const __nv_bfloat16* __restrict__ weight,
-                                __nv_bfloat16* __restrict__ x_out, __nv_bfloat16* __restrict__ h_out,
+reduce_residual_rms_norm_kernel(const float* partials, int splits,
+                                const __nv_bfloat16* residual,
+                                const __nv_bfloat16* weight,
+                                __nv_bfloat16* x_out, __nv_bfloat16* h_out,
                                 int rows, int hidden, float epsilon, int compat,
                                 int early_weight) {
   TraceScope trace(2);
@@ -66,9 +68,13 @@ reduce_residual_rms_norm_kernel(const float* __restrict__ partials, int splits,
       float v = round_bf16(sum_slices(prow + c, slice, splits));
       if (residual != nullptr) v = round_bf16(__fadd_rn(v, r[i]));
       x[i] = v;
-      x_out[static_cast<int64_t>(row) * hidden + c] = __float2bfloat16_rn(v);
       sum = fmaf(v, v, sum);
     }
+  }
+#pragma unroll
+  for (int i = 0; i < kMaxPerThread; ++i) {  // (stored behind every load: nothing says that they do not overlap)
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c < hidden) x_out[static_cast<int64_t>(row) * hidden + c] = __float2bfloat16_rn(x[i]);
   }
   if (h_out == nullptr) {
     trace.mark(1);
@@ -99,14 +105,14 @@ reduce_residual_rms_norm_kernel(const float* __restrict__ partials, int splits,
 }
 
 // One thread handles one (sequence, head, rotation pair d / d + D/2).
-__global__ void reduce_rope_kv_store_kernel(const float* __restrict__ partials, int splits,
-                                            const __nv_bfloat16* __restrict__ bias,
-                                            const __nv_bfloat16* __restrict__ cosine,
-                                            const __nv_bfloat16* __restrict__ sine,
-                                            __nv_bfloat16* __restrict__ q_out,
-                                            __nv_bfloat16* __restrict__ kbuf,
-                                            __nv_bfloat16* __restrict__ vbuf,
-                                            const int64_t* __restrict__ positions, int batch,
+__global__ void reduce_rope_kv_store_kernel(const float* partials, int splits,
+                                            const __nv_bfloat16* bias,
+                                            const __nv_bfloat16* cosine,
+                                            const __nv_bfloat16* sine,
+                                            __nv_bfloat16* q_out,
+                                            __nv_bfloat16* kbuf,
+                                            __nv_bfloat16* vbuf,
+                                            const int64_t* positions, int batch,
                                             int q_heads, int kv_heads, int dim, int capacity,
                                             int32_t* status) {
   TraceScope trace(3);

@@ -543,11 +543,11 @@ constexpr int64_t kArgmaxClusterRows = 96;
 // CTAs of a cluster, 1024 threads together, each with four loads in flight. 151936 bf16, one CTA per row -> a cluster:
 // 1 row 10.2 -> 5.5 us, 64 rows 10.5 -> 8.8; 32 rows of 32768 4.3 -> 3.2. Rows that fill the GPU by themselves keep a CTA
 // each (593 rows: 47 us, 66 with four loads a thread).
-// (Which thread looks at which element, and the order of the comparisons, are the same in both forms.)
+// (Which thread looks at which element, and the order of the comparisons, are the same in both forms. No __restrict__: a
+// cluster may be resident while the logits are still being written, and nothing may be read ahead of the wait.)
 template <typename T, int parts>
 __global__ void __launch_bounds__(kArgmaxThreads / parts)
-argmax_kernel(const T* __restrict__ logits, int64_t* __restrict__ ids, int64_t vocab, int64_t row_stride,
-              bool vector_ok) {
+argmax_kernel(const T* logits, int64_t* ids, int64_t vocab, int64_t row_stride, bool vector_ok) {
   constexpr int per = Elem<T>::kPerVec, kAhead = parts > 1 ? 4 : 1;
   __shared__ float s_val[32];
   __shared__ int64_t s_idx[32];

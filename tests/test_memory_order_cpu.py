@@ -17,3 +17,14 @@ def test_probabilities_in_tensor_memory_are_stored_behind_the_product_before():
     store = source.index("tmem_store_32x16(p_taddr", move)
     assert wait.end() < move < store
     assert re.search(r'if \(ok\) asm volatile\("tcgen05\.fence::after_thread_sync;"', source[wait.end():move])
+
+
+def test_kernels_that_wait_on_the_device_promise_nothing_about_their_operands():
+    """A kernel of a programmatic launch is resident while the kernel before it still writes. __restrict__ on a read-only
+    operand would promise that it does not change for as long as the kernel runs, and let loads move ahead of the wait."""
+
+    for path in [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]:
+        for kernel in re.split(r"__global__", path.read_text())[1:]:
+            parameters, _, body = kernel.partition("{")
+            if "grid_dependency_wait" in body:
+                assert "__restrict__" not in parameters, f"{path.name}: {parameters.strip()}"

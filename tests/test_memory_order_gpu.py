@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import llm_compiler_b200 as b200
-from llm_compiler_b200 import kernels
+from llm_compiler_b200 import _lib, kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +30,34 @@ def test_prompt_attention_whose_reference_maximum_stays(size):
         # (2^-9 just below a power of two); fp32 sums and exponentials err far less
         bound = 1.01 * 2.0 ** -8 * (weights @ values.abs() + exact.abs()) + 1e-6
         assert ((first[0, head].double() - exact).abs() <= bound).all()
+
+
+def projection(x, w, out):
+    """b200_linear into a buffer of the caller's."""
+
+    code = _lib.load().b200_linear(x.data_ptr(), w.data_ptr(), None, None, out.data_ptr(), x.shape[0], x.shape[1],
+                                   w.shape[0], x.shape[1], _lib.BF16, _lib.EPILOGUE_NONE, None, 0,
+                                   kernels.runtime().status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert code == 0
+
+
+@pytest.mark.parametrize("rows", [1, 16, 64])
+def test_tokens_chosen_behind_a_projection_in_flight(rows):
+    """The cluster form is resident while the projection writes the logits: what the buffer held before is never chosen."""
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 896, generator=g, device="cuda").bfloat16()
+    w = torch.randn(151936, 896, generator=g, device="cuda").bfloat16()
+    logits = torch.empty(rows, 151936, dtype=torch.bfloat16, device="cuda")
+    projection(x, w, logits)
+    want = kernels.b200_argmax(logits)
+    chosen = torch.empty_like(want)
+    for turn in range(20):
+        logits.fill_(0)
+        logits[:, turn * 7901 % 151936] = 3e4
+        torch.cuda.synchronize()
+        with kernels.launch_mode(programmatic=True, constant_weights=True):
+            projection(x, w, logits)
+            kernels.b200_argmax(logits, chosen)
+        assert torch.equal(chosen, want)
+    kernels.runtime().check_status()
