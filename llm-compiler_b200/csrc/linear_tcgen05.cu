@@ -1256,9 +1256,13 @@ int linear_partial_tcgen05(const void* input, const void* weight, float* partial
   p.drop_loads = drop_loads();
   if (a_rows == 64) {
     // A K slice of many k-blocks is a long weight stream: it wants about 2 us x 44 GB/s of
-    // loads in flight per SM, twice what the 96 KB rings of the short slices hold. (From 8 blocks on: 32 rows, 9 slices of
-    // 15 blocks of 2048 x 8192 in a Bazirax step, 4616 -> 4536 us for 8 steps; a Lozanex step, 4 or 8 blocks a slice, the same.)
-    const bool long_slice = ceil_div(ceil_div(k, kBK), splits) >= 8;
+    // loads in flight per SM, twice what the 96 KB rings of the short slices hold. (From 24 blocks on whatever the grid;
+    // from 8 on where every CTA has an SM to itself: 32 rows, 9 slices of 15 blocks of 2048 x 8192 in a Bazirax step,
+    // 4616 -> 4536 us for 8 steps; a Lozanex step, 4 or 8 blocks a slice, the same. The plan rounds to up to 1.5 times as
+    // many CTAs as SMs, and of long rings an SM holds one, so that the rest would be a second wave: 48 rows, long -> short,
+    // 152 CTAs of 8 blocks 7.6 -> 4.7 us, 160 of 13 13.0 -> 9.9, 158 of 23 19.0 -> 16.2.)
+    const int64_t slice_blocks = ceil_div(ceil_div(k, kBK), splits);
+    const bool long_slice = slice_blocks >= 24 || (slice_blocks >= 8 && ceil_div(n, plan.bn) * splits <= kNumSMs);
     if (plan.bn == 32)
       return small_rings() && ceil_div(ceil_div(k, kBK), splits) <= 4 ? launch<32, 4, 64, kFormPartial>(p, a_map, b_map, stream)
                                                                       : launch<32, 8, 64, kFormPartial>(p, a_map, b_map, stream);

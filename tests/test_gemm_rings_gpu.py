@@ -49,3 +49,36 @@ def test_partial_sums_do_not_depend_on_the_ring(m, k, n):
     exact = x[:m].double() @ w.double().T
     bound = (k / 16 + 8) * 2.0 ** -23 * (x[:m].double().abs() @ w.double().abs().T) + 1e-6
     assert ((few.double().sum(0) - exact).abs() <= bound).all()
+
+
+# CTAs: 152 against 148 of 8 blocks; 160 against 145 of 13; 158 against 148 of 23
+@pytest.mark.parametrize("k,n,fewer", [(960, 4864, 4736), (4096, 4096, 3712), (2880, 10032, 9472)])
+def test_partial_sums_of_more_ctas_than_sms_are_no_second_wave(k, n, fewer):
+    """A few more columns take a few more CTAs, which short rings hold beside the others: the time grows by the columns (8 % at
+    most here) and what two CTAs on an SM take from one another, where long rings, one CTA an SM, would add a wave."""
+
+    def microseconds(columns):
+        weights = [(torch.randn(columns, k, device="cuda") * k ** -0.5).bfloat16() for _ in range(2 + 300_000_000 // (2 * k * n))]
+        x = torch.randn(48, k, device="cuda").bfloat16()
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream), kernels.launch_mode(programmatic=True, constant_weights=True):
+            kernels.b200_linear_partial(x, weights[0])
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph, stream=stream):
+                for w in weights:
+                    kernels.b200_linear_partial(x, w)
+        graph.replay()
+        best = float("inf")
+        for _ in range(10):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            graph.replay()
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(end))
+        return best * 1e3 / len(weights)
+
+    few, more = microseconds(fewer), microseconds(n)
+    print(f"{fewer}: {few:.2f} us, {n}: {more:.2f} us")
+    assert more <= 1.3 * few
