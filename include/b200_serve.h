@@ -457,6 +457,8 @@ int b200_linear_rms_input(const void* input, const void* folded_weight, const vo
 int b200_rms_norm_linear(const void* input, const void* norm_weight, const void* weight, const void* bias,
                          void* output, int64_t m, int64_t k, int64_t n, int64_t input_row_stride,
                          double epsilon, int dtype, int epilogue, void* stream);
+/* 1 where that one launch is the faster form, 0 where b200_rms_norm and b200_linear are (or it does not apply). */
+int b200_rms_norm_linear_pays(int64_t m, int64_t k, int64_t n);
 int64_t b200_linear_splitk_slices(int64_t m, int64_t k, int64_t n);
 int b200_linear_splitk_residual(const void* input, const void* weight, const void* residual,
                                 void* output, void* row_squares_out, int64_t m, int64_t k,

@@ -183,6 +183,7 @@ SIGNATURES = {
     "b200_linear_rms_input": (c_int, [c_void_p] * 5 + [c_int64] * 5 + [c_double, c_int, c_void_p,
                                                                        c_void_p]),
     "b200_rms_norm_linear": (c_int, [c_void_p] * 5 + [c_int64] * 4 + [c_double, c_int, c_int, c_void_p]),
+    "b200_rms_norm_linear_pays": (c_int, [c_int64] * 3),
     "b200_linear_splitk_slices": (c_int64, [c_int64] * 3),
     "b200_linear_splitk_residual": (c_int, [c_void_p] * 5 + [c_int64] * 4 + [c_void_p, c_void_p]),
     "b200_embedding": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int,

@@ -270,8 +270,7 @@ __device__ __forceinline__ float sum_transposed(float (&v)[32], int lane) {
 //
 // NORM: the RMS norm in front of the projection as well. A row's factor rsqrt(mean(x^2) + eps) does not depend on k, so
 // the products take x times the norm's weight, every CTA adds the squares of the x that it reads anyway, and the factor
-// scales the sums: no launch for the norm, and none of its round trips. A decode step of Qwen2-0.5B in fp32, 4 sequences x
-// 600 tokens: 1028 -> 983 us (with the faster choice of tokens; the norms alone were 49 launches of some 2 us each).
+// scales the sums: no launch for the norm, and none of its round trips (where that pays: norm_pays_inside).
 //
 // ROWS: rows of x a CTA takes (4 or 8)
 template <int ROWS, bool NORM>
@@ -627,23 +626,53 @@ static bool streams_rows(int64_t m, int64_t k, int64_t n) {
                              k >= 192 * (tall - 1));
 }
 
-template <int ROWS, bool NORM>
-static int launch_rows_of(const LinearParamsGeneric<float>& p, cudaStream_t s) {
+// How a streamed projection is cut: groups of columns x row tiles x CTAs of a cluster along K, and the stages of a ring.
+struct RowsGrid {
+  int64_t groups, tall, splits;
+  int slots;
+};
+static RowsGrid rows_grid(int rows, int64_t m, int64_t k, int64_t n) {
   // with few columns as many CTAs of a cluster along K as it takes to hold W in one ring each, up to some eight an SM
-  const int64_t groups = ceil_div(p.n, kRowsColumns), tall = ceil_div(p.m, ROWS), chunks = ceil_div(p.k, kRowsChunk);
+  const int64_t groups = ceil_div(n, kRowsColumns), tall = ceil_div(m, static_cast<int64_t>(rows)), chunks = ceil_div(k, kRowsChunk);
   int64_t splits = ceil_div(chunks, kRowsWarps * kRowsRing);
   if (splits > 8 * kNumSMs / (groups * tall)) splits = 8 * kNumSMs / (groups * tall);
   if (splits > 8) splits = 8;
   if (splits < 1) splits = 1;
   const int64_t most = ceil_div(chunks, kRowsWarps * splits);
-  const int slots = static_cast<int>(most < kRowsRing ? most : kRowsRing), smem = kRowsWarps * slots * kRowsChunkBytes;
+  return RowsGrid{groups, tall, splits, static_cast<int>(most < kRowsRing ? most : kRowsRing)};
+}
+
+// Whether the norm belongs inside: that saves a launch, but every CTA squares and scales x beside its products (a quarter
+// more arithmetic) and holds more registers, so that an SM may hold fewer. It pays while both forms take one wave of CTAs
+// (240 random sizes in chains of launches: 0.61 to 0.91 of the two launches), and mostly with two waves each (0.75 to 1.06;
+// 4 rows with full rings excepted: 0.99 to 1.09). Beyond, or where the norm adds a wave, it loses: 32 rows, 2560 x 454
+// 8.6 -> 11.8 us, 9 rows, 512 x 23918 31 -> 38, 1 row, 4096 x 14648 44 -> 58. Decode steps, two launches -> one everywhere
+// -> by this rule: 24 layers of Qwen2-0.5B, 4 sequences 980 -> 944 -> 943 us, 32 sequences 2938 -> 3159 -> 2944; 4 layers
+// of Qwen2-7B, 1 sequence 853 -> 1005 -> 847.
+static bool norm_pays_inside(int64_t m, int64_t k, int64_t n) {
+  const int rows = m <= 4 ? 4 : 8;
+  const RowsGrid g = rows_grid(rows, m, k, n);
+  auto waves = [&](int64_t registers) {
+    const int64_t by_registers = 64 * 1024 / (registers * kRowsThreads);
+    const int64_t by_memory = 227 * 1024 / (kRowsWarps * g.slots * kRowsChunkBytes + 3 * 1024);
+    return ceil_div(g.groups * g.tall * g.splits, kNumSMs * (by_registers < by_memory ? by_registers : by_memory));
+  };
+  // registers of a thread as the compiler reports them: linear_rows_kernel<4> 80, with the norm 96; <8> 128 and 160
+  const int64_t with = waves(rows == 4 ? 96 : 160), without = waves(rows == 4 ? 80 : 128);
+  return with == without && (with == 1 || (with == 2 && (rows == 8 || g.slots < kRowsRing)));
+}
+
+template <int ROWS, bool NORM>
+static int launch_rows_of(const LinearParamsGeneric<float>& p, cudaStream_t s) {
+  const RowsGrid g = rows_grid(ROWS, p.m, p.k, p.n);
+  const int smem = kRowsWarps * g.slots * kRowsChunkBytes;
   if (cudaFuncSetAttribute((linear_rows_kernel<ROWS, NORM>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kRowsWarps * kRowsRing * kRowsChunkBytes) != cudaSuccess)
     return B200_ERR_LAUNCH;
-  const dim3 grid(static_cast<unsigned>(groups), static_cast<unsigned>(tall), static_cast<unsigned>(splits));
+  const dim3 grid(static_cast<unsigned>(g.groups), static_cast<unsigned>(g.tall), static_cast<unsigned>(g.splits));
   const int early = (launch_mode() & B200_LAUNCH_CONSTANT_WEIGHTS) != 0 ? 1 : 0;
   return launch_chained_cluster_xz(linear_rows_kernel<ROWS, NORM>, grid, dim3(kRowsThreads), static_cast<size_t>(smem), s, 1u,
-                                   static_cast<unsigned>(splits), p, slots, early) == cudaSuccess
+                                   static_cast<unsigned>(g.splits), p, g.slots, early) == cudaSuccess
              ? launch_status() : B200_ERR_LAUNCH;
 }
 template <bool NORM>
@@ -760,6 +789,10 @@ extern "C" int b200_linear(const void* input, const void* weight, const void* bi
   if (!aligned16(input) || !aligned16(weight)) return B200_ERR_ALIGNMENT;
   return linear_tensor_core<__nv_bfloat16>(input, weight, bias, residual, output, m, k, n, input_row_stride, dtype,
                                            epilogue, workspace, workspace_bytes, status, s);
+}
+
+extern "C" int b200_rms_norm_linear_pays(int64_t m, int64_t k, int64_t n) {
+  return m > 0 && k > 0 && n > 0 && streams_rows(m, k, n) && norm_pays_inside(m, k, n) ? 1 : 0;
 }
 
 extern "C" int b200_rms_norm_linear(const void* input, const void* norm_weight, const void* weight, const void* bias,

@@ -488,10 +488,11 @@ class Qwen2Engine(ServingEngine):
         q_size, kv_size = cfg.q_size, cfg.kv_size
 
         def normed_linear(x, norm_weight, weight, bias=None, epilogue="none"):
-            """The norm and the projection behind it: one launch for a few fp32 rows, else two."""
+            """The norm and the projection behind it: one launch for a few fp32 rows where that pays, else two."""
 
             y = None
-            if self.dtype == torch.float32 and self.mode == "fast":
+            if self.dtype == torch.float32 and self.mode == "fast" and \
+                    kernels.rms_norm_linear_pays(batch, weight.shape[1], weight.shape[0]):
                 y = kernels.b200_rms_norm_linear(x, norm_weight, weight, bias, epsilon=cfg.rms_norm_eps,
                                                  epilogue=epilogue)
             if y is None:

@@ -1297,6 +1297,12 @@ def b200_linear_rms_input(tensor: torch.Tensor, folded_weight: torch.Tensor,
     return output
 
 
+def rms_norm_linear_pays(m: int, k: int, n: int) -> bool:
+    """Whether b200_rms_norm_linear is faster than the two operators one after the other."""
+
+    return bool(_lib.load().b200_rms_norm_linear_pays(m, k, n))
+
+
 def b200_rms_norm_linear(tensor: torch.Tensor, norm_weight: torch.Tensor, weight: torch.Tensor,
                          bias: Optional[torch.Tensor] = None, *, epsilon: float,
                          epilogue: str = "none") -> Optional[torch.Tensor]:
