@@ -537,12 +537,14 @@ __global__ void classify_causal_mask_kernel(const T* __restrict__ mask, int64_t 
 }
 
 constexpr int kArgmaxThreads = 1024, kArgmaxParts = 8;
-constexpr int64_t kArgmaxClusterRows = 96;
 
-// A few rows (the last launch of a decode step but one) are bound by the latency of their loads: a row is shared by the
-// CTAs of a cluster, 1024 threads together, each with four loads in flight. 151936 bf16, one CTA per row -> a cluster:
-// 1 row 10.2 -> 5.5 us, 64 rows 10.5 -> 8.8; 32 rows of 32768 4.3 -> 3.2. Rows that fill the GPU by themselves keep a CTA
-// each (593 rows: 47 us, 66 with four loads a thread).
+// Few rows (the last launch of a decode step but one) are bound by the latency of their loads: a row is shared by the
+// CTAs of a cluster, 1024 threads together, each with four loads in flight. bf16, one CTA per row -> a cluster: 1 row of
+// 151936 10.1 -> 5.2 us, 64 rows 13.1 -> 11.0, 32 rows of 32768 4.2 -> 2.9.
+// Rows that one round of a CTA's loads covers (16 KB) have nothing to share: 64 rows of 4096 2.46 us and 2.60 in a cluster,
+// 1 row 2.4 and 2.3. From some 80 rows on (96 of 32-bit elements) they fill the GPU by themselves: 96 rows of 8192 to 151936
+// 0.96 to 1.03 of the time in a cluster, of 151936 in fp32 0.83; 120 rows with a CTA each take 0.88 to 0.97 of what they
+// did before the rows were read through one loop.
 // (Which thread looks at which element, and the order of the comparisons, are the same in both forms. No __restrict__: a
 // cluster may be resident while the logits are still being written, and nothing may be read ahead of the wait.)
 template <typename T, int parts>
@@ -935,12 +937,11 @@ int b200_argmax(const void* logits, int64_t* ids, int64_t rows, int64_t vocab,
   const bool known = with_element_type(dtype, [&](auto tag) {
     using T = typename decltype(tag)::type;
     const T* from = static_cast<const T*>(logits);
-    if (rows > kArgmaxClusterRows)
-      argmax_kernel<T, 1><<<static_cast<unsigned>(rows), kArgmaxThreads, 0, s>>>(from, ids, vocab, row_stride, vec);
-    else
-      launched = launch_chained_cluster(argmax_kernel<T, kArgmaxParts>, dim3(static_cast<unsigned>(rows * kArgmaxParts)),
-                                        dim3(kArgmaxThreads / kArgmaxParts), 0, s, kArgmaxParts, from, ids, vocab,
-                                        row_stride, vec) == cudaSuccess;
+    const bool share = rows <= (sizeof(T) == 4 ? 96 : 80) && vocab * static_cast<int64_t>(sizeof(T)) >= 16 * kArgmaxThreads;
+    const int parts = share ? kArgmaxParts : 1;
+    launched = launch_chained_cluster(share ? argmax_kernel<T, kArgmaxParts> : argmax_kernel<T, 1>,
+                                      dim3(static_cast<unsigned>(rows * parts)), dim3(kArgmaxThreads / parts), 0, s, parts,
+                                      from, ids, vocab, row_stride, vec) == cudaSuccess;
   });
   if (!launched) return B200_ERR_LAUNCH;
   return known ? launch_status() : B200_ERR_UNSUPPORTED;
