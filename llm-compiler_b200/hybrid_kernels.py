@@ -327,6 +327,13 @@ def conv_tail(inputs: "_lib.DeltaInputs", sequences: int, dtype: torch.dtype, de
     _count(rt)
 
 
+def _require_prepared(*operands: Optional[torch.Tensor]) -> None:
+    """The kernels read prepared operands as contiguous fp32, whatever the tensors say."""
+
+    if any(t is not None and (t.dtype != torch.float32 or not t.is_contiguous()) for t in operands):
+        raise ValueError("the recurrence's operands are contiguous fp32 tensors")
+
+
 def recurrence_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Optional[torch.Tensor],
                     decay: torch.Tensor, state: torch.Tensor, batch: SequenceBatch) -> torch.Tensor:
     """Token by token recurrence over prepared fp32 operands; state [slots, heads, dim, row] is updated
@@ -334,12 +341,13 @@ def recurrence_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: Opt
     [rows, heads, dim or 1]. Returns the read-out [rows, heads, vdim]."""
 
     device = _require_cuda(q, k, v, beta, decay, state)
+    _require_prepared(q, k, v, beta, decay)
     rows, kv_heads, dim = q.shape
     heads, vdim = v.shape[1], v.shape[2]
     if state.dtype != torch.float32 or state.ndim != 4 or not state.is_contiguous() or \
             state.shape[1] != heads or state.shape[2] != dim or state.shape[3] < vdim:
         raise ValueError("the state must be contiguous fp32 [slots, heads, dim, >= vdim]")
-    output = v.new_empty((rows, heads, vdim))
+    output = v.new_empty((rows, heads, vdim), dtype=torch.float32)
     rt = runtime(device)
     code = _lib.load().b200_recurrence_scan(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(beta), decay.data_ptr(), state.data_ptr(), output.data_ptr(),
@@ -355,6 +363,7 @@ def recurrence_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: 
     """recurrence_scan in chunks of 64 tokens on the tensor cores; None where the sizes do not fit."""
 
     device = _require_cuda(q, k, v, beta, decay, state)
+    _require_prepared(q, k, v, beta, decay)
     rows, kv_heads, dim = q.shape
     heads, vdim = v.shape[1], v.shape[2]
     if state.dtype != torch.float32 or state.ndim != 4 or not state.is_contiguous() or \
@@ -365,7 +374,7 @@ def recurrence_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: 
     need = int(library.b200_recurrence_chunked_workspace_bytes(chunks, heads, dim, vdim, int(beta is not None)))
     if need == 0:
         return None
-    output = v.new_empty((rows, heads, vdim))
+    output = v.new_empty((rows, heads, vdim), dtype=torch.float32)
     rt = runtime(device)
     workspace = rt.workspace("recurrence_chunked", need)
     code = library.b200_recurrence_chunked(

@@ -165,6 +165,23 @@ def test_a_decay_per_head_equals_equal_decays_per_channel():
         assert float((a - b).abs().max()) < 2e-4 and float((one - per_channel).abs().max()) < 2e-4
 
 
+@pytest.mark.parametrize("form", [hk.recurrence_scan, hk.recurrence_chunked])
+def test_a_recurrence_takes_contiguous_fp32_operands_only(form):
+    """The kernels write an fp32 read-out and read fp32 operands: a 16-bit tensor would be read, and its like written,
+    beyond its end."""
+    heads, dim, vdim = 3, 64, 48
+    batch = batch_of([(0, 0, 70)])
+    rand = lambda *shape: torch.randn(*shape, device="cuda")
+    whole = dict(q=rand(70, heads, dim), k=rand(70, heads, dim), v=rand(70, heads, vdim), beta=rand(70, heads),
+                 decay=-rand(70, heads, 1).abs())
+    state = torch.zeros(1, heads, dim, vdim, device="cuda")
+    for name, tensor in whole.items():
+        for other in (tensor.bfloat16(), tensor.half(), tensor[:1].expand_as(tensor)):
+            with pytest.raises(ValueError):
+                form(*{**whole, name: other}.values(), state, batch)
+    assert form(*whole.values(), state, batch).dtype == torch.float32
+
+
 # -------------------------------------------------------------------------- attention ----
 ATTENTION = [
     dict(heads=6, kv_heads=2, dim=24, vdim=40, scale=0.3, rot=dict(base=1e4, dims=16), mask=dict(size=48)),
