@@ -312,7 +312,10 @@ __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearP
   const float* x = p.x + m0 * p.x_row_stride;
   for (int c = 0; c < count; ++c) {
     const int k = (first + c) * kRowsChunk + lane * 4;
-    float4 xv[ROWS];
+    float4 xv[ROWS], scale = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (NORM && k < p.k)
+      asm volatile("ld.global.ca.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(scale.x), "=f"(scale.y), "=f"(scale.z), "=f"(scale.w)
+                   : "l"(p.norm_weight + k) : "memory");
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
       xv[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -321,7 +324,6 @@ __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(const LinearP
                      : "l"(x + i * p.x_row_stride + k) : "memory");
     }
     if (NORM) {
-      const float4 scale = k < p.k ? __ldg(reinterpret_cast<const float4*>(p.norm_weight + k)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
       for (int i = 0; i < ROWS; ++i) {
         squares[i] = fmaf(xv[i].w, xv[i].w, fmaf(xv[i].z, xv[i].z, fmaf(xv[i].y, xv[i].y, fmaf(xv[i].x, xv[i].x, squares[i]))));
@@ -657,8 +659,8 @@ static bool norm_pays_inside(int64_t m, int64_t k, int64_t n) {
     const int64_t by_memory = 227 * 1024 / (kRowsWarps * g.slots * kRowsChunkBytes + 3 * 1024);
     return ceil_div(g.groups * g.tall * g.splits, kNumSMs * (by_registers < by_memory ? by_registers : by_memory));
   };
-  // registers of a thread as the compiler reports them: linear_rows_kernel<4> 80, with the norm 96; <8> 128 and 160
-  const int64_t with = waves(rows == 4 ? 96 : 160), without = waves(rows == 4 ? 80 : 128);
+  // registers of a thread as the compiler reports them: linear_rows_kernel<4> 80, with the norm 96; <8> 128 and 168
+  const int64_t with = waves(rows == 4 ? 96 : 168), without = waves(rows == 4 ? 80 : 128);
   return with == without && (with == 1 || (with == 2 && (rows == 8 || g.slots < kRowsRing)));
 }
 

@@ -97,7 +97,7 @@ __device__ __forceinline__ void add_bias(const Tcgen05ParamsOf<T>& p, int col0, 
     if (whole && (reinterpret_cast<uintptr_t>(p.bias + col0) & 15u) == 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(p.bias + col0) + i);
+        const uint4 b = reinterpret_cast<const uint4*>(p.bias + col0)[i];
         v[8 * i] += Elem<T>::lo(b.x); v[8 * i + 1] += Elem<T>::hi(b.x);
         v[8 * i + 2] += Elem<T>::lo(b.y); v[8 * i + 3] += Elem<T>::hi(b.y);
         v[8 * i + 4] += Elem<T>::lo(b.z); v[8 * i + 5] += Elem<T>::hi(b.z);

@@ -28,3 +28,14 @@ def test_kernels_that_wait_on_the_device_promise_nothing_about_their_operands():
             parameters, _, body = kernel.partition("{")
             if "grid_dependency_wait" in body:
                 assert "__restrict__" not in parameters, f"{path.name}: {parameters.strip()}"
+
+
+def test_operands_that_a_kernel_in_flight_may_write_are_read_as_such():
+    """__ldg reads through a path that takes its data as constant while the kernel runs. In the projections that wait on the
+    device that holds for no operand (the tiled fp32 product, which does not, keeps it)."""
+
+    for name, kernel in (("linear_tcgen05.cu", "add_bias"), ("linear.cu", "linear_rows_kernel("), ("linear_rows.cu", "")):
+        source = (CSRC / name).read_text()
+        body = source[source.index(kernel):]
+        end = re.search(r"\n}\n", body).end() if kernel else len(body)
+        assert "__ldg" not in body[:end], name
