@@ -63,8 +63,10 @@ extern "C" {
 #define B200_LAUNCH_PREFILL_WARP_LEVEL 16  /* b200_prefill_attention: warp-level kernel         */
 
 /* Launch mode of the CALLING THREAD for the kernels that can wait on the device (linear on tcgen05 incl. the
- * partial-sum, folded-norm and cluster split-K forms, projections of a few rows, the two reduce_* consumers, decode
- * attention, RMS norms, RoPE with the KV store, the hybrid layers' steps; every other kernel, advance_lengths /
+ * partial-sum, folded-norm and cluster split-K forms, projections of a few rows, fp32 projections that stream their
+ * weight, with or without the norm, grouped projections and the routing of experts, the two reduce_* consumers, decode,
+ * prompt and latent attention, per-head products, RMS norms, RoPE with the KV store, the choice of tokens, the hybrid
+ * layers' steps; every other kernel, advance_lengths /
  * embedding / rope table among them, is always
  * launched fully serialised, which is what makes lengths[] stable before the attention's wait).
  * Thread-local: two engines driven from two threads do not see each other's promises; launches
@@ -73,9 +75,10 @@ extern "C" {
  * fully serialised (ReferenceExecutor.run, execution.py:530-575, runs one operation after another).
  * B200_LAUNCH_PROGRAMMATIC: each of those kernels may become resident before its predecessor
  * in the stream has finished and waits on the device (griddepcontrol.wait) before touching
- * any tensor; results are unchanged. B200_LAUNCH_CONSTANT_WEIGHTS additionally lets a linear
- * kernel fetch its `weight` tiles before that wait: only valid while no kernel that writes a
- * weight tensor is in flight on the device. B200_LAUNCH_STABLE_KV_PREFIX lets decode attention
+ * any tensor; results are unchanged. B200_LAUNCH_CONSTANT_WEIGHTS additionally lets the
+ * linear kernels, the per-head products (b200_head_linear), the experts' router and b200_reduce_residual_rms_norm fetch
+ * their weight operands before that wait: only valid while no kernel that writes a weight tensor is in flight on the
+ * device. B200_LAUNCH_STABLE_KV_PREFIX lets decode attention
  * read lengths[] and request the KV rows below lengths[b] - 1 before the wait: valid when the
  * only KV row written since the previous synchronisation point is the newest one (row
  * lengths[b] - 1, stored by the kernel just before attention), as in a decode step whose

@@ -551,16 +551,8 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tensor_map
       "l"(reinterpret_cast<uint64_t>(tensor_map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tensor_map, uint32_t bar,
-                                            int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4}], [%2];\n" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(tensor_map)), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
 
-// The box a tma_load_2d at these coordinates would copy, requested into L2 only: no shared
+// The box that a 2-D load at these coordinates would copy, requested into L2 only: no shared
 // memory, no barrier, nothing to wait for.
 __device__ __forceinline__ void tma_prefetch_l2_2d(const void* tensor_map, int c0, int c1) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];\n" ::"l"(
