@@ -305,6 +305,33 @@ def test_latent_attention_over_ragged_batches_and_growing_scores():
         close(out[i], torch.softmax(scores, -1)[:, :-1] @ rows, torch.bfloat16)
 
 
+# 16 rows of a sequence and fewer (columns of the 16-column form), one tile of latents in the ring and every latent twice;
+# three tokens of five heads: rows that see one key more than the one before
+@pytest.mark.parametrize("heads,tokens", [(16, 1), (3, 1), (5, 3)])
+@pytest.mark.parametrize("rank", [192, 512])
+def test_narrow_latent_attention_over_ragged_batches_and_growing_scores(heads, tokens, rank):
+    """The same in 16 columns: O^T moved again and again, an idle row, fewer rows than columns."""
+    g = torch.Generator().manual_seed(heads + rank)
+    capacity, lengths = 1100, [3, 4, 127, 128, 129, 700, 1099, 5]
+    direction = torch.randn(rank, generator=g)
+    direction /= direction.norm()
+    cache = 0.3 * torch.randn(9, capacity, rank, generator=g) + torch.linspace(0, 60, capacity)[:, None] * direction
+    cache = cache.to(torch.bfloat16)
+    q = (torch.randn(8 * tokens, heads, rank, generator=g) + 4 * direction).to(torch.bfloat16)
+    batch = batch_of([(slot, n - tokens, tokens) for slot, n in enumerate(lengths)])
+    batch.slots[7] = -1
+    sink = torch.randn(heads, generator=g).to(torch.bfloat16)
+    out = hk.latent_attention(q.cuda(), cache.cuda(), sink.cuda(), batch, scale=0.7).view(8, tokens, heads, rank)
+    kernels.runtime().check_status()
+    assert torch.all(out[7] == 0)
+    for i, n in enumerate(lengths[:7]):
+        for t in range(tokens):
+            rows = cache[i, :n - tokens + 1 + t].double()
+            scores = torch.einsum("hr,kr->hk", q[i * tokens + t].double(), rows) * 0.7
+            weights = torch.softmax(torch.cat([scores, sink.double()[:, None]], -1), -1)[:, :-1]
+            close(out[i, t], weights @ rows, torch.bfloat16)
+
+
 @pytest.mark.parametrize("size", [64, 128])
 @pytest.mark.parametrize("context", [0, 1, 63, 64, 127, 128, 129, 300])
 def test_portion_attention_on_the_prefill_kernel(size, context):

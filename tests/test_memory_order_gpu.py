@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import llm_compiler_b200 as b200
+from llm_compiler_b200 import hybrid_kernels as hk
 from llm_compiler_b200 import _lib, kernels
 
 pytestmark = pytest.mark.gpu
@@ -60,4 +61,26 @@ def test_tokens_chosen_behind_a_projection_in_flight(rows):
             projection(x, w, logits)
             kernels.b200_argmax(logits, chosen)
         assert torch.equal(chosen, want)
+    kernels.runtime().check_status()
+
+
+# 16-row and 64-row tiles, CTAs with an SM each (long rings) and without
+@pytest.mark.parametrize("rows,heads,k,n", [(1, 16, 512, 128), (16, 14, 256, 192), (32, 16, 512, 128), (64, 40, 128, 512)])
+def test_per_head_products_behind_a_projection_in_flight(rows, heads, k, n):
+    """W comes ahead of the dependency wait, x does not: what the buffer of x held before is never multiplied."""
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    rows_in = torch.randn(rows, 896, generator=g, device="cuda").bfloat16()
+    w_in = torch.randn(heads * k, 896, generator=g, device="cuda").bfloat16()
+    w = torch.randn(heads, n, k, generator=g, device="cuda").bfloat16()
+    x = torch.empty(rows, heads, k, dtype=torch.bfloat16, device="cuda")
+    projection(rows_in, w_in, x)
+    want = hk.head_linear(x, w)
+    for _ in range(20):
+        x.fill_(float("nan"))
+        torch.cuda.synchronize()
+        with kernels.launch_mode(programmatic=True, constant_weights=True):
+            projection(rows_in, w_in, x)
+            y = hk.head_linear(x, w)
+        assert torch.equal(y, want)
     kernels.runtime().check_status()
