@@ -23,8 +23,8 @@
 // products are issued group by group (S and O of one, then of the other), so that the second group
 // falls half a tile behind the first. Both S first, then both O, kept the groups in step, all warps
 // in their loads and then all in their exponentials. 4 sequences x 14 heads x 4096 tokens, D 64:
-// 240 -> 224 us with P in tensor memory, 205 in this order; 28 heads x 4096, D 128: 135 -> 128 us in
-// this order. Neither unit binds alone: the exponentials take 110 us, the products 55. (exp2 by a
+// 228 us with a lone issuing thread and P in shared memory, 240 issued by a warp, 224 with P in tensor
+// memory as well, 205 in this order; 28 heads x 4096, D 128: 135 -> 128 us in this order. Neither unit binds alone: the exponentials take 110 us, the products 55. (exp2 by a
 // polynomial on every fourth key, or a second buffer of P in shared memory, made it slower.)
 // Roles: warps 0-7 and 8-15 softmax groups, warp 16 (one lane) TMA producer (two K buffers, two
 // V buffers at D = 64, one at D = 128; K one tile ahead of V), warp 17 (an elected lane) MMA issuer and

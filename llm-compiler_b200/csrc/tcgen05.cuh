@@ -48,8 +48,8 @@ __host__ __device__ constexpr uint32_t instruction_descriptor(int m, int n, bool
 
 // One product of 16 along K (M and N from the instruction descriptor). The issuing warp walks its loops as a whole, so
 // that descriptors stay in uniform registers, and the one lane that passes a leader other than 0 issues (elect_one;
-// always the same lane: a commit covers its own thread's products). A product of M 128 x N takes N / 2 cycles, 48 at
-// least at N 64, 39 at N 16, dependent on the one before or not. A lone thread in a branch of its own could not issue
+// always the same lane: a commit covers its own thread's products). A product of M 128 x N takes N / 2 cycles where
+// N is wide and never less than some 40 (48 at N 64, 39 at N 16), dependent on the one before or not. A lone thread in a branch of its own could not issue
 // that fast: 46 cycles a product, 57 with a commit behind every fourth, and its polls waited behind them. Projections on
 // 128 rows x 64 columns a CTA, K 4864, 515 rows: 27.8 -> 24.4 us, 16 rows x 3584 x 3584 22.1 -> 17.3; 16384 rows, 128 x
 // 256 columns a CTA, 234 -> 216 (9728 x 896).
